@@ -111,7 +111,7 @@ def draw(rng):
         if c["recipe"] == "moist":
             c["ipptls"] = rng.choice((2, 2, 3, 4, 5))
         c["tke"] = rng.random() < 0.25
-        c["lehmann"] = rng.random() < 0.5
+        c["lehmann"] = rng.random() < 0.5 or c["recipe"] == "dry"  # a tracer's weights are Lehmann's
         c["rotated"] = c["recipe"] == "dry" and rng.random() < 0.25
         if rng.random() < 0.25:
             c.update(nadv=2, nsound=rng.choice((2, 3)), steps=min(8, c["steps"]))
