@@ -11,9 +11,7 @@
 // sums in the file-scope device array below instead of allocating them.
 //
 // Limits and sharing rules:
-// * the scratch holds kBudgetBlocks partial records; one block reduces up to
-//   kBudgetRowsPerBlock rows (i, k), so a domain may have at most
-//   kBudgetBlocks * kBudgetRowsPerBlock = 32768 rows ((iy-1) * kz); larger
+// * a domain may have at most kBudgetRows = 32768 rows ((iy-1) * kz); larger
 //   domains are rejected with MLC_ERR_TOO_LARGE;
 // * every GPU that loads the library holds the 256 KiB array until exit;
 // * all calls share the one array: calls whose kernels overlap on the GPU
@@ -32,10 +30,14 @@
 namespace {
 
 constexpr int kBudgetBlocks = 4096;
-constexpr int kBudgetRowsPerBlock = 8;
+constexpr long long kBudgetRows = 32768;
 constexpr int kBudgetRecord = 8;  // dry, dryadv, qmass, qadv, ps max, ps min, bad, pad
 constexpr int kBudgetThreads = 256;
 constexpr int kMaxDevices = 64;
+// Blocks an SM the rows are dealt to: with 3 every warp of the 512x512x41
+// domain takes 6 rows and the blocks are resident at once (178 us; 1: 371,
+// 2: 212, 4: 208, 8: 196, the reduction's tail growing with the blocks).
+constexpr int kBudgetBlocksSM = 3;
 
 static __device__ __align__(256) double g_budget_scratch[kBudgetBlocks * kBudgetRecord];
 
@@ -97,124 +99,129 @@ int scratch_for_current_device(double **out) {
   return MLC_OK;
 }
 
-__device__ double tree_sum(double x, double *sh) {
-  const int t = threadIdx.x;
-  sh[t] = x;
-  __syncthreads();
-  for (int s = kBudgetThreads / 2; s > 0; s >>= 1) {
-    if (t < s) sh[t] = sh[t] + sh[t + s];
-    __syncthreads();
-  }
-  const double r = sh[0];
-  __syncthreads();
-  return r;
+// The block's sums and extrema, in warp order (a fixed order), by thread 0.
+struct Budget {
+  double dry, dadv, qm, qadv, pmax, pmin;
+  int bad;
+};
+__device__ __forceinline__ Budget budget_zero() { return {0, 0, 0, 0, -INFINITY, INFINITY, 0}; }
+__device__ __forceinline__ void budget_add(Budget &a, const Budget &b) {
+  a.dry += b.dry; a.dadv += b.dadv; a.qm += b.qm; a.qadv += b.qadv;
+  a.pmax = fmax(a.pmax, b.pmax); a.pmin = fmin(a.pmin, b.pmin);
+  a.bad |= b.bad;
 }
-
-__device__ double tree_ext(double x, double *sh, bool take_max) {
-  const int t = threadIdx.x;
-  sh[t] = x;
-  __syncthreads();
-  for (int s = kBudgetThreads / 2; s > 0; s >>= 1) {
-    if (t < s) sh[t] = take_max ? fmax(sh[t], sh[t + s]) : fmin(sh[t], sh[t + s]);
-    __syncthreads();
+__device__ Budget block_budget(Budget a) {
+  __shared__ Budget sh[kBudgetThreads / 32];
+  const unsigned full = 0xffffffffu;
+  for (int off = 16; off > 0; off >>= 1) {
+    const Budget b{__shfl_down_sync(full, a.dry, off),  __shfl_down_sync(full, a.dadv, off),
+                   __shfl_down_sync(full, a.qm, off),   __shfl_down_sync(full, a.qadv, off),
+                   __shfl_down_sync(full, a.pmax, off), __shfl_down_sync(full, a.pmin, off),
+                   __shfl_down_sync(full, a.bad, off)};
+    budget_add(a, b);
   }
-  const double r = sh[0];
+  if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = a;
   __syncthreads();
-  return r;
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kBudgetThreads / 32; ++w) budget_add(a, sh[w]);
+  return a;
 }
 
 // Arrays are in the packed reference layout: cross (jx-1, iy-1, kz),
 // u (jx, iy-1, kz), v (jx-1, iy, kz), qx (jx-1, iy-1, kz, nqx), ps (jx-1, iy-1).
+//
+// Interior rows (i, k) go to warps, rows_per_warp in turn each, lanes along j
+// (rows start on 8 bytes only, so wider loads are not possible).  dx^2 is applied to the sums and the
+// species of a point are added before they are weighted by dz*rho: 2 + nqx
+// FP64 instructions a point.  On GB300, whose FP64 pipe runs two a clock and
+// SM, that pipe bounds the kernel (142 us at 512x512x41 with 5 species; the
+// 0.6 GB of loads need 89 us); the form with each species weighted by itself
+// needed 23 a point.  The lateral fluxes and the ps extrema are grid-stride
+// loops over their own items.  Measured, both kernels, 512x512x41, 5 species:
+// 1.71 ms before, 0.18 ms now.
+// NQ: species (0: nqx at run time).
+template <int NQ>
 __global__ void __launch_bounds__(kBudgetThreads) k_budget_partial(
-    int jx, int iy, int kz, int nqx, double dx, double dt, const double *__restrict__ rho,
+    int jx, int iy, int kz, int nqx, double dx, double dt, int rows_per_warp, const double *__restrict__ rho,
     const double *__restrict__ dz, const double *__restrict__ qx, const double *__restrict__ u,
     const double *__restrict__ v, const double *__restrict__ ps, double *scratch) {
-  __shared__ double sh[kBudgetThreads];
-  const int nc = jx - 1;
+  const int nc = jx - 1, nq = NQ > 0 ? NQ : nqx;
   const size_t c2 = (size_t)nc * (iy - 1);
   const size_t c3 = c2 * kz;
-  auto cx = [&](int j, int i, int k) { return (size_t)(j - 1) + (size_t)nc * (i - 1) + c2 * (k - 1); };
-  auto ux = [&](int j, int i, int k) {
-    return (size_t)(j - 1) + (size_t)jx * (i - 1) + (size_t)jx * (iy - 1) * (k - 1);
-  };
-  auto vx = [&](int j, int i, int k) {
-    return (size_t)(j - 1) + (size_t)nc * (i - 1) + (size_t)nc * iy * (k - 1);
-  };
-  const double dxsq = dx * dx;
-  double dry = 0, dadv = 0, qm = 0, qadv = 0, pmax = -INFINITY, pmin = INFINITY, bad = 0;
-  const int nrows = (iy - 1) * kz;
-  const int r0 = blockIdx.x * kBudgetRowsPerBlock;
-  for (int r = r0; r < min(r0 + kBudgetRowsPerBlock, nrows); ++r) {
-    const int i = r % (iy - 1) + 1, k = r / (iy - 1) + 1;
-    if (i >= 2 && i <= iy - 2) {
-      for (int j = 2 + threadIdx.x; j <= jx - 2; j += kBudgetThreads) {
-        const size_t o = cx(j, i, k);
-        const double dzr = dz[o], rh = rho[o];
-        dry += dxsq * dzr * rh;
-        for (int n = 0; n < nqx; ++n) qm += qx[o + n * c3] * dxsq * dzr * rh;
-      }
-    }
-    if (threadIdx.x == 0) {
-      const size_t ow = cx(1, i, k), oe = cx(jx - 1, i, k);
-      const double uw = u[ux(1, i, k)], ue = u[ux(jx, i, k)];
-      dadv += uw * dt * dx * dz[ow] * rho[ow];
-      dadv -= ue * dt * dx * dz[oe] * rho[oe];
-      for (int n = 0; n < nqx; ++n) {
-        qadv += qx[ow + n * c3] * uw * dt * dx * dz[ow] * rho[ow];
-        qadv -= qx[oe + n * c3] * ue * dt * dx * dz[oe] * rho[oe];
-      }
-    }
-    if (i == 1 || i == iy - 1) {
-      const int iv = (i == 1) ? 1 : iy;
-      const bool south = (i == 1);
-      for (int j = 2 + threadIdx.x; j <= jx - 2; j += kBudgetThreads) {
-        const size_t o = cx(j, i, k);
-        const double vv = v[vx(j, iv, k)];
-        const double fl = vv * dt * dx * dz[o] * rho[o];
-        dadv = south ? dadv + fl : dadv - fl;
-        for (int n = 0; n < nqx; ++n) {
-          const double q = qx[o + n * c3] * vv * dt * dx * dz[o] * rho[o];
-          qadv = south ? qadv + q : qadv - q;
-        }
-      }
-    }
-    if (k == 1 && i >= 2 && i <= iy - 2) {
-      for (int j = 2 + threadIdx.x; j <= jx - 2; j += kBudgetThreads) {
-        const double x = ps[(size_t)(j - 1) + (size_t)nc * (i - 1)];
-        if (!isfinite(x)) bad = 1;
-        else { pmax = fmax(pmax, x); pmin = fmin(pmin, x); }
-      }
+  Budget a = budget_zero();
+  const int lane = (int)(threadIdx.x & 31u);
+  const int warp = (int)(blockIdx.x * (kBudgetThreads / 32) + (threadIdx.x >> 5));
+  const int ni = iy - 3, rows = ni * kz;
+  const int r1 = min(rows, (warp + 1) * rows_per_warp);
+  for (int r = warp * rows_per_warp; r < r1; ++r) {
+    const int k = r / ni, i = r - k * ni + 1;  // 0-based level and row
+    const size_t o0 = c2 * k + (size_t)nc * i;
+#pragma unroll 1  // unrolled by 4 (the compiler's choice) 211 us instead of 178
+    for (int j = 1 + lane; j <= nc - 2; j += 32) {
+      const size_t o = o0 + j;
+      const double m = dz[o] * rho[o];
+      double q = qx[o];
+#pragma unroll
+      for (int n = 1; n < nq; ++n) q += qx[o + n * c3];
+      a.dry += m;
+      a.qm += q * m;
     }
   }
-  dry = tree_sum(dry, sh);
-  dadv = tree_sum(dadv, sh);
-  qm = tree_sum(qm, sh);
-  qadv = tree_sum(qadv, sh);
-  bad = tree_sum(bad, sh);
-  pmax = tree_ext(pmax, sh, true);
-  pmin = tree_ext(pmin, sh, false);
+  a.dry *= dx * dx;
+  a.qm *= dx * dx;
+  const int gt = (int)(blockIdx.x * kBudgetThreads + threadIdx.x), gs = (int)(gridDim.x * kBudgetThreads);
+  // flux through one face of the cross point at o: sign * wind * dt*dx*dz*rho
+  auto face = [&](size_t o, double wind) {
+    const double f = wind * dt * dx * dz[o] * rho[o];
+    double q = qx[o];
+    for (int n = 1; n < nq; ++n) q += qx[o + n * c3];
+    a.dadv += f;
+    a.qadv += q * f;
+  };
+  // west (u at 1, in) and east (u at jx, out) columns of every row
+  for (int e = gt; e < (iy - 1) * kz; e += gs) {
+    face((size_t)nc * e, u[(size_t)jx * e]);
+    face((size_t)nc * e + nc - 1, -u[(size_t)jx * e + jx - 1]);
+  }
+  // the south and north rows and ps by warps, 32 columns of a row at a time
+  const int chunks = (jx - 3 + 31) / 32, nwarp = (int)(gridDim.x * (kBudgetThreads / 32));
+  // south (v at 1, in) and north (v at iy, out) rows, j in jci
+  for (int e = warp; e < chunks * kz; e += nwarp) {
+    const int k = e / chunks, j = (e - k * chunks) * 32 + lane + 1;
+    if (j > nc - 2) continue;
+    const size_t ov = (size_t)nc * iy * k + j;
+    face(c2 * k + j, v[ov]);
+    face(c2 * k + (size_t)nc * (iy - 2) + j, -v[ov + (size_t)nc * (iy - 1)]);
+  }
+  for (int e = warp; e < chunks * ni; e += nwarp) {
+    const int i = e / chunks, j = (e - i * chunks) * 32 + lane + 1;
+    if (j > nc - 2) continue;
+    const double x = ps[(size_t)nc * (i + 1) + j];
+    if (!isfinite(x)) a.bad = 1;
+    else { a.pmax = fmax(a.pmax, x); a.pmin = fmin(a.pmin, x); }
+  }
+  a = block_budget(a);
   if (threadIdx.x == 0) {
     double *rec = scratch + (size_t)blockIdx.x * kBudgetRecord;
-    rec[0] = dry; rec[1] = dadv; rec[2] = qm; rec[3] = qadv;
-    rec[4] = pmax; rec[5] = pmin; rec[6] = bad; rec[7] = 0.0;
+    rec[0] = a.dry; rec[1] = a.dadv; rec[2] = a.qm; rec[3] = a.qadv;
+    rec[4] = a.pmax; rec[5] = a.pmin; rec[6] = a.bad; rec[7] = 0.0;
   }
 }
 
-__global__ void k_budget_final(const double *scratch, int nblocks, double *out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double a[4] = {0, 0, 0, 0}, pmax = -INFINITY, pmin = INFINITY;
-  bool bad = false;
-  for (int b = 0; b < nblocks; ++b) {
+// One block adds the records, a few a thread in record order, then as the
+// blocks do (one thread adding them all took 1.4 ms of a 1.7 ms call).
+__global__ void __launch_bounds__(kBudgetThreads) k_budget_final(const double *scratch, int nblocks, double *out) {
+  Budget a = budget_zero();
+  for (int b = (int)threadIdx.x; b < nblocks; b += kBudgetThreads) {
     const double *rec = scratch + (size_t)b * kBudgetRecord;
-    for (int q = 0; q < 4; ++q) a[q] += rec[q];
-    pmax = fmax(pmax, rec[4]);
-    pmin = fmin(pmin, rec[5]);
-    if (rec[6] != 0.0) bad = true;
+    budget_add(a, Budget{rec[0], rec[1], rec[2], rec[3], rec[4], rec[5], rec[6] != 0.0});
   }
-  out[0] = a[0]; out[1] = a[1]; out[2] = a[2]; out[3] = a[3];
-  out[4] = bad ? NAN : pmax;
-  out[5] = bad ? NAN : pmin;
-  out[6] = bad ? 1.0 : 0.0;
+  a = block_budget(a);
+  if (threadIdx.x != 0) return;
+  out[0] = a.dry; out[1] = a.dadv; out[2] = a.qm; out[3] = a.qadv;
+  out[4] = a.bad ? NAN : a.pmax;
+  out[5] = a.bad ? NAN : a.pmin;
+  out[6] = a.bad ? 1.0 : 0.0;
 }
 
 }  // namespace
@@ -226,14 +233,18 @@ extern "C" int mlc_mass_budget_noalloc(const mlc_dims *d, double dx, double dt,
   if (!d || !rho || !dz || !qx || !u || !v || !ps || !out) return MLC_ERR_INVALID;
   if (d->jx < 5 || d->iy < 5 || d->kz < 1 || d->nqx < 1) return MLC_ERR_INVALID;
   const long long nrows = (long long)(d->iy - 1) * d->kz;
-  if (nrows > (long long)kBudgetBlocks * kBudgetRowsPerBlock) return MLC_ERR_TOO_LARGE;
+  if (nrows > kBudgetRows) return MLC_ERR_TOO_LARGE;
   double *scratch = nullptr;
   const int st = scratch_for_current_device(&scratch);
   if (st != MLC_OK) return st;
-  const int nblocks = (int)((nrows + kBudgetRowsPerBlock - 1) / kBudgetRowsPerBlock);
+  // whole rows a warp, as few as fill kBudgetBlocksSM blocks on each of 152 SMs
+  constexpr int kWarps = kBudgetThreads / 32, kFull = 152 * kBudgetBlocksSM * kWarps;
+  const int rows = (d->iy - 3) * d->kz, per = (rows + kFull - 1) / kFull;
+  const int nblocks = (rows + per * kWarps - 1) / (per * kWarps);
+  static_assert(kFull / kWarps <= kBudgetBlocks, "the scratch holds every block's record");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  k_budget_partial<<<nblocks, kBudgetThreads, 0, s>>>(d->jx, d->iy, d->kz, d->nqx, dx, dt, rho,
-                                                      dz, qx, u, v, ps, scratch);
-  k_budget_final<<<1, 32, 0, s>>>(scratch, nblocks, out);
+  auto part = d->nqx == 5 ? k_budget_partial<5> : d->nqx == 2 ? k_budget_partial<2> : k_budget_partial<0>;
+  part<<<nblocks, kBudgetThreads, 0, s>>>(d->jx, d->iy, d->kz, d->nqx, dx, dt, per, rho, dz, qx, u, v, ps, scratch);
+  k_budget_final<<<1, kBudgetThreads, 0, s>>>(scratch, nblocks, out);
   return cudaGetLastError() == cudaSuccess ? MLC_OK : MLC_ERR_CUDA;
 }
