@@ -34,7 +34,6 @@ using namespace mlc;
 namespace {
 
 constexpr size_t kAlign = 256;
-constexpr int kMaxLevels = 128;
 constexpr int kMaxSlots = 4096;
 constexpr int kMaxExtent = 32768;
 
@@ -351,7 +350,7 @@ struct mlc_ctx {
   WorkItem *wl_buf = nullptr;
   size_t wl_cap = 0;           // entries
   bool wl_dirty = true;        // members changed since the lists were built
-  int wl_key[6] = {-1, -1, -1, -1, -1, -1};
+  int wl_key[7] = {-1, -1, -1, -1, -1, -1, -1};
   const WorkItem *wl_ptr[7] = {};  // the lists in wl_buf (null: none) ...
   int wl_n[7] = {};                // ... and their lengths
 };
@@ -501,6 +500,27 @@ int remove_member(mlc_ctx *x, int slot) {
   return MLC_OK;
 }
 
+// The form of the column solves for these members, by their 32-column row
+// segments n an SM (152).  Several warps a column while the segments are few;
+// a thread a column, streamed, once they fill the GPU.  Measured, us a launch
+// (six coefficient warps | three | streamed), moist, 41 levels:
+//   n     FP64               mixed
+//   0.8   30.0  38.5  92.8   17.5  25.2  62.8
+//   3.3   69.5  61.4  93.4   23.0  30.1  64.1
+//   5.2    101   110   104   37.2  34.1  72.6
+//   7.1*   118   101   107   36.4  32.9  62.0   (* 35 levels)
+//   9.1    165   166   134   58.4  64.9  72.9
+//   13.4   229   224   179   79.5  72.8  78.6
+//   20.9   356   332   312    120   107   104
+template <class R>
+int solve_kind(const std::vector<Dom<R>> &t) {
+  long n = 0;
+  for (const Dom<R> &D : t) n += (long)((D.g.jx - 1 + 31) / 32) * (D.g.iy - 3);
+  const bool f64 = sizeof(R) == sizeof(double);
+  if (n <= (f64 ? 2 : 4) * 152) return kSolveCols6;
+  return n <= (f64 ? 8 : 16) * 152 ? kSolveCols3 : kSolveStream;
+}
+
 // Upload the descriptor table of the active members and derive the launch
 // geometry (maxima over the members; the launch shapes are kept).
 template <class R>
@@ -539,6 +559,7 @@ int refresh(mlc_ctx *x) {
     if (m.c.tke) k.any_tke = 1;
   }
   L.nmem = (int)t.size();
+  L.solve = solve_kind<R>(t);
   if (!t.empty()) {
     MLC_TRY(cudaMemcpyAsync(x->table, t.data(), t.size() * sizeof(Dom<R>), cudaMemcpyHostToDevice,
                             x->stream));
@@ -565,7 +586,7 @@ int ensure_lists(mlc_ctx *x) {
   bool uneven = false;
   for (const Member *m : act)
     uneven = uneven || m->g.jx != L.jx || m->g.iy != L.iy || m->g.kz != L.kz;
-  const int key[6] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, L.htile};
+  const int key[7] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, L.htile, L.solve};
   // the launch geometry always takes the lists from the context (a copy of
   // an older geometry may carry stale ones)
   auto apply = [&]() {
@@ -612,12 +633,12 @@ int ensure_lists(mlc_ctx *x) {
         for (int bi = 0; bi < cdiv(g.iy, 4); ++bi)
           for (int bj = 0; bj < cdiv(g.jx, 128); ++bj) push(m, bj, bi, kc);
     }
-  // column solves: 128-column segments of the rows i = 2 .. iy-2
+  // column solves: solve_segment-column segments of the rows i = 2 .. iy-2
   off[2] = all.size();
   for (int m = 0; m < (int)act.size(); ++m) {
     const Geom &g = act[m]->g;
     for (int r = 0; r < g.iy - 3; ++r)
-      for (int bj = 0; bj < cdiv(g.jx - 1, f64 ? kSolveColsD : kSolveColsF); ++bj) push(m, bj, r, 0);
+      for (int bj = 0; bj < cdiv(g.jx - 1, solve_segment(L.solve, (int)sizeof(R))); ++bj) push(m, bj, r, 0);
   }
   // vertical WAF: column tiles, the member's own fields of the R table
   off[3] = all.size();
@@ -1180,10 +1201,10 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
     MLC_CHK(put3<double>(x, g, cu.data(), W(a.mo_cu), jx, iy - 1, 1, 0));
     MLC_CHK(put3<double>(x, g, cvv.data(), W(a.mo_cv), jx - 1, iy, 1, 0));
     MLC_TRY(cudaStreamSynchronize(x->stream));
-    // the solve's factors, in the kernel's operand order: (bw*dtrdz)*fmz,
-    // zcs2*fmz and dtrdz*fmz (dtrdz = dtsound*rdzita, zcs2 = dtrdz^2*R/cv)
+    // the solve's factors: (bw*dtrdz)*fmz, (dtrdz*R/cv)*fmz and dtrdz*fmz
+    // (dtrdz = dtsound*rdzita)
     const double sdtrdz = c.dtsound * c.rdzita;
-    const double zcs2 = (sdtrdz * sdtrdz) * kRdrcv;
+    const double zcs = sdtrdz * kRdrcv;
     const int nsp = p.nspgx;
     std::vector<double> fa(nc * kz), fb(nc * kz);
     for (int k = 0; k < kz; ++k)
@@ -1194,7 +1215,7 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
           const int ib = s->ibnd_cr[e2];
           const double bw = ib > 0 ? 1.0 - s->hefc[(size_t)(ib - 1) + (size_t)k * nsp] : 1.0;
           fa[e3] = (bw * sdtrdz) * s->fmz[e3];
-          fb[e3] = zcs2 * s->fmz[e3];
+          fb[e3] = zcs * s->fmz[e3];
         }
     MLC_CHK(put3<double>(x, g, fa.data(), W(a.sv_a), jx - 1, iy - 1, kz, 0));
     MLC_CHK(put3<double>(x, g, fb.data(), W(a.sv_b), jx - 1, iy - 1, kz, 0));

@@ -79,8 +79,8 @@ struct Stat {
   //              g*dts*hy*gzitakh(k) (3-D), coru*dts and corv*dts (2-D)
   const double *dv_cu, *dv_cv, *dv_cf, *mo_du, *mo_dv, *mo_gu, *mo_gv, *mo_cu, *mo_cv;
   //   sound_solve (3-D, cross points): (bw*dtrdz)*fmz with bw the relaxation
-  //              weight 1 - hefc of the point's zone (1 outside), zcs2*fmz
-  //              and dtrdz*fmz
+  //              weight 1 - hefc of the point's zone (1 outside),
+  //              (dtrdz*R/cv)*fmz and dtrdz*fmz
   const double *sv_a, *sv_b, *sv_c;
   // spectral nudging: sine bases bvx (km2 rows of jx) and bvy (lm2 rows of
   // iy), the level weights cnudge (kz)
@@ -257,7 +257,7 @@ __device__ __forceinline__ F2 fast_two_sum(float a, float b) {  // needs |a| >= 
   return {s, b - (s - a)};
 }
 __device__ __forceinline__ F2 two_prod(float a, float b) {
-  const float p = a * b;
+  const float p = __fmul_rn(a, b);  // never fused into a following sum
   return {p, fmaf(a, b, -p)};
 }
 __device__ __forceinline__ F2 df_add(F2 a, F2 b) {
@@ -270,7 +270,7 @@ __device__ __forceinline__ F2 df_add_f(F2 a, float b) {
 }
 __device__ __forceinline__ F2 df_mul(F2 a, F2 b) {
   const F2 p = two_prod(a.hi, b.hi);
-  return fast_two_sum(p.hi, p.lo + (a.hi * b.lo + a.lo * b.hi));
+  return fast_two_sum(p.hi, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, p.lo)));
 }
 __device__ __forceinline__ F2 df_mul_f(F2 a, float b) {
   const F2 p = two_prod(a.hi, b);
@@ -300,8 +300,8 @@ __device__ __forceinline__ F2 df_div(F2 a, F2 b) {
 __device__ __forceinline__ F2 df_recip(F2 b) {
   const float rc = __fdividef(1.f, b.hi);
   const F2 p = two_prod(rc, b.hi);
-  const float e = ((1.f - p.hi) - p.lo) - rc * b.lo;
-  return fast_two_sum(rc, rc * e);
+  const float e = fmaf(-rc, b.lo, (1.f - p.hi) - p.lo);
+  return fast_two_sum(rc, __fmul_rn(rc, e));
 }
 // a - b rounded to FP32 (the hi difference is exact for values within 2x)
 __device__ __forceinline__ float df_diff(F2 a, F2 b) { return (a.hi - b.hi) + (a.lo - b.lo); }
@@ -326,7 +326,7 @@ struct DF {
 // per entry instead, and each entry names the member and the block's tile in
 // the kernel's own coordinates, so only the members' own tiles are launched:
 //   point kernels   a = tile along j, b = tile along i, c = level chunk
-//   column solves   a = 128-column segment, b = row index (i - 2)
+//   column solves   a = segment of solve_segment columns, b = row index (i - 2)
 //   vertical WAF    a = column tile along j, b = tile along i, c = field
 //   horizontal WAF  a = tile along j, b = tile along i, c = level - 1
 // The lists are built on the host whenever the members or the launch shapes

@@ -14,19 +14,21 @@
 
 namespace mlc {
 
-// Columns of a column-solve block (one row segment, one thread a column):
-// FP64 members and mixed members.
-#ifndef MLC_DV_W
-#define MLC_DV_W 128
-#endif
-constexpr int kSolveColsD = MLC_DV_W;
-constexpr int kSolveColsF = 128;
+// Forms of the column solves (mlc_sound.cu) and the columns of a block's row
+// segment in each.
+constexpr int kSolveStream = 0, kSolveCols3 = 3, kSolveCols6 = 6;
+constexpr int solve_segment(int kind, int elem_bytes) {
+  return kind == kSolveStream && elem_bytes == 4 ? 128 : 32;
+}
+// Levels of a domain, at most.
+constexpr int kMaxLevels = 128;
 
 // Extents of a launch (maxima over the members) and the launch shapes.
 struct LaunchGeom {
   int jx, iy, kz, nmem;
   int col_x, col_y;      // column kernels
-  int solve_x, solve_y;  // kept in the tune report; the solves use fixed 128-column blocks
+  int solve_x, solve_y;  // kept in the tune report; not used by the solves
+  int solve;             // form of the column solves (kSolveStream ...)
   int vert_x, vert_y;    // adv_vertical
   int htile;             // adv_horizontal tile shape (hshape)
   int nadv_r;            // advected fields of type R per member
@@ -37,7 +39,7 @@ struct LaunchGeom {
   // largest member) and their lengths, one per tiling
   const WorkItem *wl_pt;     // col_x x col_y tiles, level chunks
   const WorkItem *wl_v4;     // 128 x 4 tiles, level chunks
-  const WorkItem *wl_solve;  // 128-column row segments
+  const WorkItem *wl_solve;  // row segments of solve_segment columns
   const WorkItem *wl_vert;   // vert_x x vert_y column tiles, R fields
   const WorkItem *wl_vinc;   // the same, the two double-float fields
   const WorkItem *wl_h;      // horizontal WAF tiles (shape htile), levels

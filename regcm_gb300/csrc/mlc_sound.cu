@@ -9,17 +9,20 @@
 //   sound_solve     per interior column, one thread per column: the 5-point
 //                   divergence filter, the vertical divergence term, the
 //                   implicit w-Exner tridiagonal system (Eq. 19, Thomas
-//                   algorithm with the column held in shared memory), the
+//                   algorithm, the column streamed through shared memory), the
 //                   Exner update and, after the last substep, the completed s.
 //   sound_momentum  u and v (Eq. 17/18): divergence damping, Coriolis with
 //                   the substep's initial winds, pressure gradient with the new
 //                   Exner function, terrain term, relaxation-zone weight.  It
 //                   writes the other half of a ping-pong pair, which is how the
 //                   reference's ud/vd copies are kept without a copy.
-// Every expression keeps the reference's operands and association order; the
-// only departures are FMA contraction by the compiler and the relaxation
-// weight bdywt recomputed from ibnd and hefc instead of read from an array
-// (the same value, Main/mod_bdycod.F90:4033-4047).
+// theta_v does not change during the substeps, so what it enters is formed
+// once a round by sound_prep: the solve's hydrostatic factor Z =
+// cp*theta_v(half)*fmzf*dtrdz with its decrement per unit w, and the
+// momentum's pressure-gradient coefficients.  Departures from the reference's
+// operand order: those factors, FMA contraction, and the relaxation weight
+// bdywt recomputed from ibnd and hefc instead of read from an array (the same
+// value, Main/mod_bdycod.F90:4033-4047).
 #include "mlc_kernels.cuh"
 #include "mlc_tma.cuh"
 
@@ -27,6 +30,24 @@ namespace mlc {
 
 namespace {
 
+// The scratch planes of the acoustic loop (the WAF's wz planes, free then).
+// FP64: the filtered divergence and the multipliers between the solve's two
+// passes, then G, Cu, Cv.  Mixed: those two are double-float planes (wz_d),
+// and there is no Cu, Cv.
+template <class R>
+struct SoundScratch {
+  R *zf, *mul, *g, *cu, *cv;
+  R *w_lo, *mul_lo;  // mixed: low parts of the eliminated w and the multipliers
+};
+template <class R>
+__device__ __forceinline__ SoundScratch<R> sound_scratch(const Dom<R> &D) {
+  if constexpr (sizeof(R) == sizeof(double)) {
+    return {D.wz[0], D.wz[1], D.wz[2], D.wz[3], D.wz[4], nullptr, nullptr};
+  } else {
+    float *zf = reinterpret_cast<float *>(D.wz_d[0]), *mul = reinterpret_cast<float *>(D.wz_d[1]);
+    return {zf, mul, D.wz[2], nullptr, nullptr, zf + D.g.field3(), mul + D.g.field3()};
+  }
+}
 
 __device__ __forceinline__ double relax_weight(const int32_t *ibnd, const double *hefc, int nsp,
                                                size_t ij, int k) {
@@ -34,6 +55,20 @@ __device__ __forceinline__ double relax_weight(const int32_t *ibnd, const double
   return ib > 0 ? 1.0 - hefc[(size_t)(ib - 1) + (size_t)(k - 1) * nsp] : 1.0;
 }
 
+// What the substeps of one advection round read of theta_v (constant over
+// them), at cross point (j, i), level k:
+//   Z(k)  = theta_v(half) * cp*fmzf*dtrdz, k = 2..kz (:564-566 with the
+//           factor of :641), which the solves lower by w*G every substep
+//   G(k)  = (fmzf*dtrdz)*(theta_v(k-1) - theta_v(k)) * cp*fmzf*dtrdz
+//   Cu, Cv = zcx*cp/2*(theta_v sum) of the momentum's pressure gradients
+//           (an FP64 member's)
+// in tetavf and the scratch planes the solves leave free.  Per substep this
+// takes six FP64 instructions a point out of the momentum and nine out of the
+// solve for thirteen here once a round; in the mixed solve a double-float
+// product and 12 bytes a point.  A mixed member's momentum, bound by memory,
+// reads theta_v itself: two coefficient planes would be as many bytes and cost
+// their writing here (measured 353 + 92 against 366 + 73 us a step of four
+// substeps at 512x512x41).
 template <class R>
 __global__ void k_sound_prep(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
@@ -44,22 +79,35 @@ __global__ void k_sound_prep(const Dom<R> *__restrict__ doms, int advoff, int ti
   const Pt q = point_at(wi, 1, 1);
   if (q.j > g.jx - 1 || q.i > g.iy - 1 || q.k > g.kz) return;
   const int adv = (D.clk->adv_role + advoff) & 1;
+  const Scal &c = D.c;
+  const Stat<R> &sa = D.sa;
   const double *__restrict__ tetav = D.tetav[adv];
-  double *__restrict__ tetavf = D.tetavf;
-  // Main/mod_moloch.F90:564-566, levels 2..kz
+  const SoundScratch<R> ss = sound_scratch(D);
+  const size_t ij = g.at2(q.j, q.i), S = (size_t)g.P;
+  double cx = 0.0, cy = 0.0;
+  if constexpr (sizeof(R) == sizeof(double)) {
+    cx = c.dtrdxs * sa.msfu[ij] * (0.5 * kCpd);
+    cy = (c.lrotllr ? c.dtrdxs : c.dtrdxs * sa.msfv[ij]) * (0.5 * kCpd);
+  }
 #pragma unroll
-  for (int k = q.k < 2 ? 2 : q.k; k < q.k + kPtLevels && k <= g.kz; ++k) {
+  for (int k = q.k; k < q.k + kPtLevels && k <= g.kz; ++k) {
     const size_t o = g.at(q.j, q.i, k), om = o - g.PS;
     if constexpr (sizeof(R) == sizeof(float)) {
-      // double-float theta_v; also theta_v(k-1) - theta_v(k) for the substeps'
-      // solves (the scratch wz[2] is free until the advection of this round)
-      const DF th(tetav, g.field3()), tf(tetavf, g.PS * (size_t)(g.kz + 1));
-      const F2 lo = th.ld(om), hi = th.ld(o);
-      const F2 sm = df_add(lo, hi);
-      tf.st(o, F2{0.5f * sm.hi, 0.5f * sm.lo});
-      D.wz[2][o] = df_diff(lo, hi);
+      const DF th(tetav, g.field3()), zz(D.tetavf, g.PS * (size_t)(g.kz + 1));
+      if (k < 2) continue;
+      const F2 tm = th.ld(om), t0 = th.ld(o);
+      const F2 sm = df_add(tm, t0);
+      const F2 cf = DF(sa.cfz, g.PS * (size_t)(g.kz + 1)).ld(o);
+      zz.st(o, df_mul(F2{0.5f * sm.hi, 0.5f * sm.lo}, cf));
+      ss.g[o] = sa.fmzf[o] * (c.dtsoundf * c.rdzitaf) * df_diff(tm, t0) * df_f(cf);
     } else {
-      tetavf[o] = 0.5 * (tetav[om] + tetav[o]);
+      const double t0 = tetav[o];
+      if (q.j >= 2) ss.cu[o] = cx * (tetav[o - 1] + t0);
+      if (q.i >= 2) ss.cv[o] = cy * (tetav[o - S] + t0);
+      if (k < 2) continue;
+      const double tm = tetav[om], fd = sa.fmzf[o] * (c.dtsound * c.rdzita), cf = kCpd * fd;
+      D.tetavf[o] = (0.5 * (tm + t0)) * cf;
+      ss.g[o] = (fd * (tm - t0)) * cf;
     }
   }
 }
@@ -133,45 +181,487 @@ __global__ void k_sound_div(const Dom<R> *__restrict__ doms, int uvoff, int tile
   }
 }
 
-// The implicit w-Exner solve of an FP64 member (Main/mod_moloch.F90:627-671,
-// s :728-734): per interior column the filtered divergence plus its vertical
-// part, the Thomas elimination k = kz..2, back substitution, the Exner
-// update and (after the last substep) s.  Same structure as the mixed solve
-// below: a block is one 128-column row segment, one thread per column, the
-// downward pass forms each level's coefficients and eliminates at once, the
-// upward pass substitutes back and updates Exner a level behind; every
-// level's planes arrive in shared memory as 1 KB row segments by bulk copies
-// kDvStages levels ahead (the raw divergence with a 2-column halo).  Between
-// the passes the eliminated w stays in w, the multipliers and the filtered
-// divergence in the scratch planes wz[1] and wz[0] (free during the acoustic
-// loop).  The per-level expressions are the reference's, in its order.
-// (Measured on the 512x512x41 step: 3.99 ms of solves a step against 5.68
-// for a column-in-shared-memory form, whose 66 KB a block left 6 warps an SM.)
-// Levels read between two block barriers of the streamed column solves (a
-// barrier frees the stages read since the last one for their refill).
-#ifndef MLC_SOLVE_SYNC
-#define MLC_SOLVE_SYNC 1
-#endif
-constexpr int kSolveSync = MLC_SOLVE_SYNC;
-#ifndef MLC_DV_STAGES
-#define MLC_DV_STAGES 3
-#endif
-constexpr int kDvStages = MLC_DV_STAGES;  // FP64 solve: levels in flight
-constexpr int kDvW = kSolveColsD;
-constexpr int kDvZW = kDvW + 4;                   // raw divergence row, 2-column halo each side
-// The FP64 solve reads its metric products from bind time - (bw*dtrdz)*fmz,
-// zcs2*fmz, dtrdz*fmz, the same roundings as forming them per level - (1),
-// or forms them from fmz and the zone weight every level (0).
-#ifndef MLC_SOLVE_PRE
-#define MLC_SOLVE_PRE 1
-#endif
-constexpr bool kSolvePre = MLC_SOLVE_PRE != 0;
-constexpr int kDvStage = 3 * kDvZW + (kSolvePre ? 8 : 7) * kDvW;   // doubles of one stage
-template <class R>
-__global__ void __launch_bounds__(kDvW, 4) k_sound_solve(const Dom<R> *__restrict__ doms, int advoff, int last,
-    const WorkItem *__restrict__ wl) {
+// ---- the implicit w-Exner solves ---------------------------------------------
+// 1/x of a positive x: the FP32 reciprocal of x's leading bits, moved between
+// the formats by integer instructions, and one third-order step
+// r0 + r0*(e + e^2), e = 1 - x*r0 (Householder's method of order two for the
+// reciprocal): with e below 2^-21 the remaining error, e^3, is below 2^-63, so
+// the result is the rounding of the last fused multiply-add (half an ulp).
+// Three FP64 instructions where the division takes six.  Outside FP32's range,
+// and for NaN, infinite, zero and negative x, the division itself.
+__device__ __forceinline__ double recip_d(double x) {
+  const unsigned h = (unsigned)__double2hiint(x);
+  if (h - 0x38200000u >= 0x47d00000u - 0x38200000u) return 1.0 / x;
+  const float xf = __uint_as_float(((h - 0x38000000u) << 3) | ((unsigned)__double2loint(x) >> 29));
+  const unsigned r = __float_as_uint(__fdividef(1.f, xf));
+  const double r0 = __hiloint2double((int)((r >> 3) + 0x38000000u), (int)(r << 29));
+  const double e = __fma_rn(-x, r0, 1.0);
+  return __fma_rn(r0, __fma_rn(e, e, e), r0);
+}
+
+// Two forms of each solve, picked by the number of column segments
+// (solve_kind).  Their level arithmetic is the functions below, every rounding
+// explicit, so the forms agree bit for bit: a member's result does not depend
+// on what else a launch holds.
+//
+// FP64 (Main/mod_moloch.F90:627-671).  The FP64 instructions bound the large
+// grids, so the arithmetic is arranged for few of them: with Z =
+// cp*theta_v(half)*fmzf*dtrdz (sound_prep) lowered by w*G,
+//   w_expl = w - Z*(dpai - R/cv*d(pai*zf)) - g*dts,   d = (m) - (k) = above - below
+//   zu, zd = Z*(b*pai) + ffilt,                       b = dtrdz*R/cv*fmz
+// with pai*zf and b*pai of a level formed once and carried to the next: 31 a
+// column and level, against 47 for the reference's own association.
+struct LevelD {
+  double s, pai, zf, pz, bp;  // pz: pai*zf, bp: b*pai
+};
+// z: the raw divergence here, w/e/s/n its neighbours (:531-543); fza:
+// (bw*dtrdz)*fmz; ds: s here minus s below (:627-630)
+__device__ __forceinline__ void level_d(LevelD &v, bool filt, double xk, double z, double zw, double ze, double zs,
+                                        double zn, double fza, double ds, double fzb) {
+  if (filt) z = __fma_rn(xk, __fma_rn(-4.0, z, zw + ze + zs + zn), z);
+  v.zf = __fma_rn(fza, ds, z);
+  v.pz = __dmul_rn(v.pai, v.zf);
+  v.bp = __dmul_rn(fzb, v.pai);
+}
+struct CoefD {
+  double zw, zd, zu, den;  // w_expl; den: 1 + zd + zu
+};
+__device__ __forceinline__ CoefD coef_d(const LevelD &vm, const LevelD &vk, double Z, double wold, double ff,
+                                        double gdts) {
+  // the hydrostatic balance -Z*dpai - g*dts in one fused multiply-add
+  const double e = __fma_rn(-kRdrcv, __dsub_rn(vm.pz, vk.pz), vm.pai - vk.pai);
+  CoefD c;
+  c.zw = __dadd_rn(wold, __fma_rn(-Z, e, -gdts));
+  c.zu = __fma_rn(vm.bp, Z, ff);
+  c.zd = __fma_rn(vk.bp, Z, ff);
+  c.den = __dadd_rn(__dadd_rn(1.0, c.zd), c.zu);
+  return c;
+}
+// one level of the elimination: the eliminated w and the multiplier
+__device__ __forceinline__ void eliminate_d(double &w, double &mul, const CoefD &c) {
+  const double r = recip_d(__fma_rn(-c.zd, mul, c.den));
+  w = __dmul_rn(r, __fma_rn(c.zd, w, c.zw));
+  mul = __dmul_rn(r, c.zu);
+}
+__device__ __forceinline__ double exner_d(double pai, double zf, double fzc, double w, double wbelow) {
+  return __dmul_rn(pai, __fma_rn(-kRdrcv, __fma_rn(fzc, __dsub_rn(w, wbelow), zf), 1.0));
+}
+
+// Mixed members, in FP32 only.  Where rounding is amplified the values are
+// double-floats: Z, the hydrostatic balance -Z*(pai(k-1) - pai(k)) - g*dts of
+// the w equation (two terms of ~g*dts whose difference drives w), the Exner
+// update pai - pai*increment and, with DFR, the recurrence.  The divergence
+// filter and the elimination coefficients (O(1)-conditioned) run in plain FP32.
+struct LevelF {
+  float s, zf, fp, pz;  // fp: dtrdz*fmz*pai, pz: pai*zf
+  F2 pai;
+};
+__device__ __forceinline__ void level_f(LevelF &v, bool filt, float xk, float z, float zw, float ze, float zs,
+                                        float zn, float bw, float fz, float ds) {
+  if (filt) z = fmaf(xk, fmaf(-4.f, z, zw + ze + zs + zn), z);
+  v.zf = fmaf(__fmul_rn(bw, fz), ds, z);
+  const float p = df_f(v.pai);
+  v.fp = __fmul_rn(fz, p);
+  v.pz = __fmul_rn(p, v.zf);
+}
+struct CoefF {
+  F2 zw;
+  float zd, zu;
+};
+__device__ __forceinline__ CoefF coef_f(const LevelF &vm, const LevelF &vk, F2 Z, float wold, float ff, F2 ngdts) {
+  const F2 dp = two_sum(vm.pai.hi - vk.pai.hi, vm.pai.lo - vk.pai.lo);
+  const F2 bal = df_add(ngdts, df_mul(F2{-Z.hi, -Z.lo}, dp));
+  const float zr = __fmul_rn(float(kRdrcv), df_f(Z));
+  CoefF c;
+  c.zw = df_add_f(df_add_f(bal, wold), __fmul_rn(zr, __fsub_rn(vm.pz, vk.pz)));
+  c.zu = fmaf(zr, vm.fp, ff);
+  c.zd = fmaf(zr, vk.fp, ff);
+  return c;
+}
+// (den >= 1: the pivot of a diagonally dominant system)
+template <bool DFR>
+__device__ __forceinline__ void eliminate_f(F2 &w, F2 &mul, const CoefF &c) {
+  if constexpr (DFR) {
+    const F2 den = df_add(two_sum(__fadd_rn(1.f, c.zd), c.zu), df_mul_f(F2{-mul.hi, -mul.lo}, c.zd));
+    const F2 r = df_recip(den);
+    w = df_mul(r, df_add(c.zw, df_mul_f(w, c.zd)));
+    mul = df_mul_f(r, c.zu);
+  } else {
+    const float r = 1.f / fmaf(-c.zd, mul.hi, __fadd_rn(__fadd_rn(1.f, c.zd), c.zu));
+    w.hi = __fmul_rn(r, fmaf(c.zd, w.hi, df_f(c.zw)));
+    mul.hi = __fmul_rn(r, c.zu);
+  }
+}
+template <bool DFR>
+__device__ __forceinline__ F2 back_f(F2 wel, F2 mul, F2 wabove) {
+  if constexpr (DFR) return df_add(wel, df_mul(mul, wabove));
+  else return F2{fmaf(mul.hi, wabove.hi, wel.hi), 0.f};
+}
+// dzf: dtrdz*fmz
+__device__ __forceinline__ F2 exner_f(F2 pai, float zf, float dzf, F2 w, F2 wbelow) {
+  const float inc = __fmul_rn(float(kRdrcv), fmaf(dzf, df_diff(w, wbelow), zf));
+  const F2 d = df_mul_f(pai, inc);
+  return df_add(pai, F2{-d.hi, -d.lo});
+}
+
+// ---- the solves, a column by several warps ------------------------------------
+// A block is 32 columns of a row (lanes are columns).  AW warps form the
+// coefficients, kSolveLevels interfaces in turn each, and leave them in shared
+// memory; one warp runs the elimination behind them, an mbarrier a round
+// telling it that the round's coefficients are there.  The column stays on
+// chip: the back substitution overwrites the eliminated values, and all warps
+// update Exner (and s after the last substep) level by level.  The elimination
+// warp's place rotates with the block, so that the SM's four schedulers get it
+// equally often.
+//
+// Why: on GB300 an FP64 instruction of a warp takes 64 clocks of its scheduler's FP64
+// unit, however many lanes are active, and a column's elimination is a serial
+// chain; with one warp a segment three of an SM's four units idle unless many
+// segments share the SM, and the mixed solve is a chain of double-float
+// operations the same way.
+constexpr int kSolveCols = 32;
+// interfaces a coefficient warp forms a round (a round's first level costs the
+// filtered divergence once more; 1 and 4 measured slower)
+constexpr int kSolveLevels = 2;
+constexpr int kSolveArrays = 5;  // shared values a column and level
+// threads of a block: with six coefficient warps two share each scheduler but
+// the elimination's, whose second warp only joins the Exner update
+constexpr int solve_threads(int aw) { return 32 * (aw > 3 ? 8 : 4); }
+
+// This thread's part of a block: its role (0 eliminates, 1..3 coefficients)
+// and its column; lanes outside the interior work on the nearest interior
+// column and store nothing.
+struct SolveLane {
+  int role, lane, col;  // col: j - 1
+  bool act;
+};
+template <int AW>
+__device__ __forceinline__ SolveLane solve_lane(const Geom &g, int x0) {
+  SolveLane l;
+  l.lane = (int)threadIdx.x & 31;
+  const int wp = (int)threadIdx.x >> 5;
+  // warps p and p+4 share a scheduler: the eliminating warp's is left to it
+  const int q = (wp + (int)(blockIdx.x + blockIdx.y)) & 3;
+  l.role = q == 0 ? (wp < 4 ? 0 : AW + 1) : wp < 4 ? q : q + 3;
+  const int j = x0 + l.lane + 1;
+  l.act = j >= 2 && j <= g.jx - 2;
+  l.col = min(max(j, 2), g.jx - 2) - 1;
+  return l;
+}
+
+// FP64 members (s :728-734).
+template <class R, int AW>
+__global__ void __launch_bounds__(solve_threads(AW), 512 / solve_threads(AW)) k_solve_cols_d(const Dom<R> *__restrict__ doms, int advoff,
+                                                                  int last, const WorkItem *__restrict__ wl) {
   static_assert(sizeof(R) == sizeof(double), "FP64 member");
-  constexpr int NS = kDvStages;
+  constexpr int NL = kSolveLevels, NR = AW * NL;  // interfaces a warp, a round
+  extern __shared__ __align__(16) double dv_smem[];
+  __shared__ __align__(8) uint64_t mbar[kMaxLevels / NR + 1];  // a round's coefficients are there
+  const WorkItem wi = wl ? wl[blockIdx.x]
+                          : WorkItem{(int16_t)blockIdx.z, (int16_t)blockIdx.x, (int16_t)blockIdx.y, 0};
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const Geom g = D.g;
+  const int x0 = (int)wi.a * kSolveCols, i = (int)wi.b + 2;
+  if (x0 + 1 > g.jx - 2 || i > g.iy - 2) return;  // uniform over the block
+  const SolveLane l = solve_lane<AW>(g, x0);
+  const int kz = g.kz, PS = (int)g.PS, P = g.P;
+  if ((int)threadIdx.x <= kMaxLevels / NR) {
+    mbar_init(&mbar[threadIdx.x], AW);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const Scal &c = D.c;
+  const Stat<R> &sa = D.sa;
+  const int adv = (D.clk->adv_role + advoff) & 1;
+  const size_t r0 = g.at2(1, i) + (size_t)l.col;
+  const double *__restrict__ zraw = D.zdiv2 + r0;
+  const double *__restrict__ fza = sa.sv_a + r0;
+  const double *__restrict__ fzb = sa.sv_b + r0;
+  const double *__restrict__ gg = sound_scratch(D).g + r0;
+  double *__restrict__ s = D.s + r0;
+  double *__restrict__ w = D.w + r0;
+  double *__restrict__ pai = D.pai[adv] + r0;
+  double *__restrict__ zp = D.tetavf + r0;
+  const bool filt = c.divfilter != 0;
+  // rows k = 0 .. kz+1 of 32 columns: 1 + zd + zu; zd; zu, then the
+  // multiplier; w_expl, then the eliminated w, then w; filtered divergence
+  const int rows = (kz + 2) * 32;
+  double *sa_ = dv_smem + l.lane, *sd = sa_ + rows, *su = sd + rows, *sw = su + rows, *sf = sw + rows;
+  auto level = [&](int m, double s_below, bool keep) {
+    const int o = (m - 1) * PS;
+    LevelD v;
+    v.s = s[o];
+    v.pai = pai[o];
+    const double z = zraw[o];
+    if (filt)
+      level_d(v, true, sa.xknu[m - 1], z, zraw[o - 1], zraw[o + 1], zraw[o - P], zraw[o + P], fza[o], v.s - s_below,
+              fzb[o]);
+    else
+      level_d(v, false, 0.0, z, 0.0, 0.0, 0.0, 0.0, fza[o], v.s - s_below, fzb[o]);
+    if (keep) sf[m * 32] = v.zf;
+    return v;
+  };
+  const double gdts = kGrav * c.dtsound;
+  double wnext = 0.0, wkp1 = 0.0;
+  if (l.role == 0) {
+    wnext = w[kz * PS];  // w(kz+1) = -s(kz+1)
+    sw[(kz + 1) * 32] = wnext;
+    sw[32] = w[0];       // w(1) = 0
+  }
+  const int nr = (kz - 1 + NR - 1) / NR;
+  bool ok = true;
+  if (l.role >= 1 && l.role <= AW) {
+    for (int r = 0; r < nr; ++r) {
+      const int kt = kz - r * NR - (l.role - 1) * NL;  // this warp's first interface
+      if (kt >= 2) {
+        LevelD vk = level(kt, s[kt * PS], kt == kz);
+#pragma unroll
+        for (int n = 0; n < NL; ++n) {
+          const int k = kt - n;
+          if (k < 2) break;
+          const int o = (k - 1) * PS;
+          const double wold = w[o];
+          const LevelD vm = level(k - 1, vk.s, true);
+          const double Z = __fma_rn(-wold, gg[o], zp[o]);
+          if (l.act) zp[o] = Z;
+          const CoefD cf = coef_d(vm, vk, Z, wold, sa.ffilt[k - 1], gdts);
+          sw[k * 32] = cf.zw;
+          sd[k * 32] = cf.zd;
+          su[k * 32] = cf.zu;
+          sa_[k * 32] = cf.den;
+          vk = vm;
+        }
+      }
+      __syncwarp();
+      if (l.lane == 0) mbar_arrive(&mbar[r]);
+    }
+  } else if (l.role == 0) {
+    for (int r = 0; r < nr && ok; ++r) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&mbar[r], 0u));
+      const int k0 = kz - r * NR, k1 = max(2, k0 - NR + 1);
+      for (int k = k0; k >= k1; --k) {
+        eliminate_d(wnext, wkp1, CoefD{sw[k * 32], sd[k * 32], su[k * 32], sa_[k * 32]});
+        sw[k * 32] = wnext;
+        su[k * 32] = wkp1;
+      }
+    }
+    double wp = sw[32];
+    for (int k = 2; k <= kz; ++k) {
+      wp = __fma_rn(su[k * 32], wp, sw[k * 32]);
+      sw[k * 32] = wp;
+      if (l.act) w[(k - 1) * PS] = wp;
+    }
+  }
+  if (__syncthreads_or(!ok)) {
+    if (threadIdx.x == 0) atomicOr(&D.clk->fault, 1);
+    return;
+  }
+  if (!l.act) return;
+  // Exner (:668-671) and s (:728-734), a level a warp
+  const double *__restrict__ fzc = sa.sv_c + r0;
+  const double *__restrict__ fzf = sa.fmzf_d + r0;
+#pragma unroll 3
+  for (int m = 1 + l.role; m <= kz; m += solve_threads(AW) / 32) {
+    const int o = (m - 1) * PS;
+    const double wm = sw[m * 32];
+    pai[o] = exner_d(pai[o], sf[m * 32], fzc[o], wm, sw[(m + 1) * 32]);
+    if (last) s[o] = m >= 2 ? (wm + s[o]) * fzf[o] : 0.0;
+  }
+  if (last && l.role == 0) s[kz * PS] = 0.0;
+}
+
+// Mixed members.
+template <class R, int AW, bool DFR>
+__global__ void __launch_bounds__(solve_threads(AW), 1024 / solve_threads(AW)) k_solve_cols_f(const Dom<R> *__restrict__ doms, int advoff,
+                                                                  int last, const WorkItem *__restrict__ wl) {
+  static_assert(sizeof(R) == sizeof(float), "FP32 fields");
+  constexpr int NL = kSolveLevels, NR = AW * NL;
+  extern __shared__ __align__(16) float sv_smem[];
+  __shared__ __align__(8) uint64_t mbar[kMaxLevels / NR + 1];
+  const WorkItem wi = wl ? wl[blockIdx.x]
+                          : WorkItem{(int16_t)blockIdx.z, (int16_t)blockIdx.x, (int16_t)blockIdx.y, 0};
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const Geom g = D.g;
+  const int x0 = (int)wi.a * kSolveCols, i = (int)wi.b + 2;
+  if (x0 + 1 > g.jx - 2 || i > g.iy - 2) return;  // uniform over the block
+  const SolveLane l = solve_lane<AW>(g, x0);
+  const int kz = g.kz, PS = (int)g.PS, P = g.P;
+  if ((int)threadIdx.x <= kMaxLevels / NR) {
+    mbar_init(&mbar[threadIdx.x], AW);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const Scal &c = D.c;
+  const Stat<R> &sa = D.sa;
+  const int adv = (D.clk->adv_role + advoff) & 1;
+  const unsigned F = (unsigned)g.field3(), F1 = F + (unsigned)PS;
+  const size_t r0 = g.at2(1, i) + (size_t)l.col;
+  const float *__restrict__ zraw = D.zdiv2 + r0;
+  const float *__restrict__ fmz = sa.fmz + r0;
+  const float *__restrict__ gg = sound_scratch(D).g + r0;
+  float *__restrict__ s = D.s + r0;
+  float *__restrict__ w = D.w + r0;
+  float *__restrict__ pai = reinterpret_cast<float *>(D.pai[adv]) + r0;
+  float *__restrict__ zp = reinterpret_cast<float *>(D.tetavf) + r0;
+  const float dtrdz = c.dtsoundf * c.rdzitaf;
+  const bool filt = c.divfilter != 0;
+  const int32_t ib = sa.ibnd_cr[r0];
+  // rows k = 0 .. kz+1 of 32 columns: zd, then the multiplier's low part; zu,
+  // then the multiplier; w_expl, then the eliminated w, then w (low part; high
+  // part); filtered divergence
+  const int rows = (kz + 2) * 32;
+  float *sd = sv_smem + l.lane, *su = sd + rows, *swl = su + rows, *sw = swl + rows, *sf = sw + rows;
+  auto level = [&](int m, float s_below, bool keep) {
+    const int o = (m - 1) * PS;
+    LevelF v;
+    v.s = s[o];
+    v.pai = F2{pai[o], pai[o + F]};
+    const float z = zraw[o], fz = __fmul_rn(dtrdz, fmz[o]);
+    const float bw = ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(m - 1) * c.nspgx] : 1.f;
+    if (filt)
+      level_f(v, true, sa.xknu_r[m - 1], z, zraw[o - 1], zraw[o + 1], zraw[o - P], zraw[o + P], bw, fz, v.s - s_below);
+    else
+      level_f(v, false, 0.f, z, 0.f, 0.f, 0.f, 0.f, bw, fz, v.s - s_below);
+    if (keep) sf[m * 32] = v.zf;
+    return v;
+  };
+  const F2 ngdts{-c.gdts_hi, -c.gdts_lo};
+  F2 wnext{0.f, 0.f}, wkp1{0.f, 0.f};
+  if (l.role == 0) {
+    wnext.hi = w[kz * PS];
+    sw[(kz + 1) * 32] = wnext.hi;
+    swl[(kz + 1) * 32] = 0.f;
+    sw[32] = w[0];
+    swl[32] = 0.f;
+  }
+  const int nr = (kz - 1 + NR - 1) / NR;
+  bool ok = true;
+  if (l.role >= 1 && l.role <= AW) {
+    for (int r = 0; r < nr; ++r) {
+      const int kt = kz - r * NR - (l.role - 1) * NL;
+      if (kt >= 2) {
+        LevelF vk = level(kt, s[kt * PS], kt == kz);
+#pragma unroll
+        for (int n = 0; n < NL; ++n) {
+          const int k = kt - n;
+          if (k < 2) break;
+          const int o = (k - 1) * PS;
+          const float wold = w[o];
+          const LevelF vm = level(k - 1, vk.s, true);
+          const F2 Z = df_add_f(F2{zp[o], zp[o + F1]}, -__fmul_rn(wold, gg[o]));
+          if (l.act) {
+            zp[o] = Z.hi;
+            zp[o + F1] = Z.lo;
+          }
+          const CoefF cf = coef_f(vm, vk, Z, wold, sa.ffilt_r[k - 1], ngdts);
+          sd[k * 32] = cf.zd;
+          su[k * 32] = cf.zu;
+          sw[k * 32] = cf.zw.hi;
+          swl[k * 32] = cf.zw.lo;
+          vk = vm;
+        }
+      }
+      __syncwarp();
+      if (l.lane == 0) mbar_arrive(&mbar[r]);
+    }
+  } else if (l.role == 0) {
+    for (int r = 0; r < nr && ok; ++r) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&mbar[r], 0u));
+      const int k0 = kz - r * NR, k1 = max(2, k0 - NR + 1);
+      for (int k = k0; k >= k1; --k) {
+        eliminate_f<DFR>(wnext, wkp1, CoefF{F2{sw[k * 32], swl[k * 32]}, sd[k * 32], su[k * 32]});
+        sw[k * 32] = wnext.hi;
+        swl[k * 32] = wnext.lo;
+        su[k * 32] = wkp1.hi;
+        sd[k * 32] = wkp1.lo;
+      }
+    }
+    F2 wp{sw[32], 0.f};
+    for (int k = 2; k <= kz; ++k) {
+      wp = back_f<DFR>(F2{sw[k * 32], swl[k * 32]}, F2{su[k * 32], sd[k * 32]}, wp);
+      sw[k * 32] = wp.hi;
+      swl[k * 32] = wp.lo;
+      if (l.act) w[(k - 1) * PS] = df_f(wp);
+    }
+  }
+  if (__syncthreads_or(!ok)) {
+    if (threadIdx.x == 0) atomicOr(&D.clk->fault, 1);
+    return;
+  }
+  if (!l.act) return;
+#pragma unroll 3
+  for (int m = 1 + l.role; m <= kz; m += solve_threads(AW) / 32) {
+    const int o = (m - 1) * PS;
+    const F2 pp{pai[o], pai[o + F]}, wm{sw[m * 32], swl[m * 32]};
+    const F2 pn = exner_f(pp, sf[m * 32], __fmul_rn(dtrdz, fmz[o]), wm, F2{sw[(m + 1) * 32], swl[(m + 1) * 32]});
+    pai[o] = pn.hi;
+    pai[o + F] = pn.lo;
+    if (last) s[o] = m >= 2 ? (df_f(wm) + s[o]) * sa.fmzf[r0 + o] : 0.f;
+  }
+  if (last && l.role == 0) s[kz * PS] = 0.f;
+}
+
+// ---- the solves, streamed: one thread a column --------------------------------
+// Where the grid fills the GPU (solve_kind).
+// A block is a row segment of CW columns (one thread a column).  The downward
+// pass forms each level's coefficients and eliminates at once, the upward pass
+// substitutes back and updates Exner (and s after the last substep) a level
+// behind.  Every level's planes arrive in shared memory as row segments by
+// untiled bulk copies kStages levels ahead of the level being solved (the raw
+// divergence with a halo); the lanes of warp 0 issue them, one plane a lane,
+// each lane keeping its plane's address.  Between the passes the eliminated w
+// stays in w, the multipliers and the filtered divergence in scratch planes.
+//
+// Shared layout of a stage, in elements: three rows of the raw divergence
+// (i, i-1, i+1; kHalo columns either side, which keeps 16-byte alignment),
+// then kPlanes rows of CW.  The upward pass uses the divergence rows for its
+// last two planes.
+template <class R, int CW>
+struct SolveShape {
+  static constexpr bool kF64 = sizeof(R) == sizeof(double);
+  static constexpr int kHalo = 16 / (int)sizeof(R) > 2 ? 16 / (int)sizeof(R) : 2;
+  static constexpr int kZW = CW + 2 * kHalo;
+  static constexpr int kPlanes = kF64 ? 7 : 8;
+  static constexpr int kStage = 3 * kZW + kPlanes * CW;
+  static constexpr int kStages = kF64 ? (CW == 32 ? 4 : 3) : (CW == 32 ? 6 : 4);
+};
+
+// One plane's copies: where the segment lies in the plane at level 1, where
+// it goes in a stage, and its bytes (0: this lane copies nothing).
+template <class R>
+struct PlaneCopy {
+  const R *src;
+  int dst;
+  unsigned bytes;
+};
+
+// whether x holds for some thread of the block, a block barrier
+template <int CW>
+__device__ __forceinline__ bool block_any(bool x) {
+  if constexpr (CW == 32) {
+    x = __any_sync(0xffffffffu, x);
+    __syncwarp();
+    return x;
+  } else {
+    return __syncthreads_or(x);
+  }
+}
+template <int CW>
+__device__ __forceinline__ void block_sync() {
+  if constexpr (CW == 32) __syncwarp();
+  else __syncthreads();
+}
+
+// The FP64 form: the arithmetic of k_solve_cols_d, 31 FP64 instructions a
+// column and level.
+template <class R, int CW>
+__global__ void __launch_bounds__(CW, CW == 32 ? 24 : 768 / CW) k_solve_stream_d(const Dom<R> *__restrict__ doms,
+    int advoff, int last, const WorkItem *__restrict__ wl) {
+  static_assert(sizeof(R) == sizeof(double), "FP64 member");
+  using Sh = SolveShape<R, CW>;
+  constexpr int NS = Sh::kStages, ZW = Sh::kZW;
   extern __shared__ __align__(16) double dv_smem[];
   __shared__ __align__(8) uint64_t mbar[NS];
   const WorkItem wi = wl ? wl[blockIdx.x]
@@ -180,7 +670,7 @@ __global__ void __launch_bounds__(kDvW, 4) k_sound_solve(const Dom<R> *__restric
   if (!D.active) return;
   const Geom g = D.g;
   const int t = (int)threadIdx.x;
-  const int x0 = (int)wi.a * kDvW;
+  const int x0 = (int)wi.a * CW;
   const int i = (int)wi.b + 2;
   if (x0 + 1 > g.jx - 2 || i > g.iy - 2) return;  // uniform over the block
   const int j = x0 + t + 1;
@@ -191,70 +681,60 @@ __global__ void __launch_bounds__(kDvW, 4) k_sound_solve(const Dom<R> *__restric
   const int adv = (D.clk->adv_role + advoff) & 1;
   const int PS = (int)g.PS, P = g.P;
   const size_t r0 = g.at2(1, i);
+  const SoundScratch<R> ss = sound_scratch(D);
   const double *__restrict__ zraw = D.zdiv2 + r0;
   double *__restrict__ s = D.s + r0;
   double *__restrict__ w = D.w + r0;
   double *__restrict__ pai = D.pai[adv] + r0;
-  const double *__restrict__ tetav = D.tetav[adv] + r0;
-  double *__restrict__ tetavf = D.tetavf + r0;
-  // with the products from bind time, fmz's place (down pass, up pass) holds
-  // (bw*dtrdz)*fmz and dtrdz*fmz, and zcs2*fmz comes as an eighth plane
-  const double *__restrict__ fmz = (kSolvePre ? sa.sv_a : sa.fmz_d) + r0;
-  const double *__restrict__ fmz_up = (kSolvePre ? sa.sv_c : sa.fmz_d) + r0;
-  const double *__restrict__ fmzb = (kSolvePre ? sa.sv_b : sa.fmz_d) + r0;
-  const double *__restrict__ fmzf = sa.fmzf_d + r0;
-  double *__restrict__ zfs = D.wz[0] + r0;   // free during the acoustic loop
-  double *__restrict__ mul = D.wz[1] + r0;
-  const double dts = c.dtsound;
-  const double dtrdz = dts * c.rdzita;
-  const double zcs2 = (dtrdz * dtrdz) * kRdrcv;
+  double *__restrict__ zp = D.tetavf + r0;
+  double *__restrict__ zfs = ss.zf + r0;
+  double *__restrict__ mul = ss.mul + r0;
+  const double gdts = kGrav * c.dtsound;
   const int ij_off = j - 1;
-  const size_t ij = r0 + (size_t)ij_off;
   const bool filt = c.divfilter != 0;
-  const int xe = min(x0 + kDvW, P);
-  const int zs = x0 >= 2 ? x0 - 2 : 0, ze = min(x0 + kDvW + 2, P);
+  const int xe = min(x0 + CW, P);
+  const int zs = x0 >= Sh::kHalo ? x0 - Sh::kHalo : 0, ze = min(x0 + CW + Sh::kHalo, P);
   const unsigned wb = (unsigned)(xe - x0) * 8u, zb = (unsigned)(ze - zs) * 8u;
   const int zc = x0 + t - zs;
-  auto stage = [&](int b) { return dv_smem + (size_t)b * kDvStage; };
-  auto fld = [&](double *st, int f) { return st + 3 * kDvZW + f * kDvW; };
-  const int nd = kz - 1;
-  // down unit u (m = kz-1-u): zraw rows, s, fmz, pai, tetav at m; w, fmzf, tetavf at m+1
-  auto issue_down = [&](int u, int b) {
-    const int m = kz - 1 - u;
-    double *st = stage(b);
-    uint64_t *bar = &mbar[b];
-    fence_proxy_async();
-    mbar_expect_tx(bar, (filt ? 3u : 1u) * zb + (kSolvePre ? 8u : 7u) * wb);
-    const int o = (m - 1) * PS, ob = m * PS;
-    bulk_load(st, zraw + o + zs, zb, bar);
-    if (filt) {
-      bulk_load(st + kDvZW, zraw + o - P + zs, zb, bar);
-      bulk_load(st + 2 * kDvZW, zraw + o + P + zs, zb, bar);
+  auto stage = [&](int b) { return dv_smem + (size_t)b * Sh::kStage; };
+  constexpr int F0 = 3 * ZW;  // the first plane's offset
+  const int nd = kz - 1, nu = kz;
+  // this lane's plane of the downward pass (level m: divergence, s, the
+  // vertical divergence factor, pai, b; interface m+1: w, Z, G)
+  PlaneCopy<R> pc{nullptr, 0, 0u};
+  unsigned dn_bytes = (filt ? 3u : 1u) * zb + 7u * wb;
+  if (t < 32) {
+    switch (t) {
+      case 0: pc = {zraw + zs, 0, zb}; break;
+      case 1: pc = {zraw - P + zs, ZW, filt ? zb : 0u}; break;
+      case 2: pc = {zraw + P + zs, 2 * ZW, filt ? zb : 0u}; break;
+      case 3: pc = {s + x0, F0, wb}; break;
+      case 4: pc = {sa.sv_a + r0 + x0, F0 + CW, wb}; break;
+      case 5: pc = {pai + x0, F0 + 2 * CW, wb}; break;
+      case 6: pc = {sa.sv_b + r0 + x0, F0 + 3 * CW, wb}; break;
+      case 7: pc = {w + PS + x0, F0 + 4 * CW, wb}; break;
+      case 8: pc = {zp + PS + x0, F0 + 5 * CW, wb}; break;
+      case 9: pc = {ss.g + r0 + PS + x0, F0 + 6 * CW, wb}; break;
+      default: break;
     }
-    bulk_load(fld(st, 0), s + o + x0, wb, bar);
-    bulk_load(fld(st, 1), fmz + o + x0, wb, bar);
-    bulk_load(fld(st, 2), pai + o + x0, wb, bar);
-    bulk_load(fld(st, 3), tetav + o + x0, wb, bar);
-    bulk_load(fld(st, 4), w + ob + x0, wb, bar);
-    bulk_load(fld(st, 5), fmzf + ob + x0, wb, bar);
-    bulk_load(fld(st, 6), tetavf + ob + x0, wb, bar);
-    if constexpr (kSolvePre) bulk_load(fld(st, 7), fmzb + o + x0, wb, bar);
-  };
-  // up unit v (m = v + 2): w(m), mul(m) (m <= kz); pai, zfs, fmz, s, fmzf at m-1
-  auto issue_up = [&](int v, int b) {
-    const int m = v + 2;
-    double *st = stage(b);
-    uint64_t *bar = &mbar[b];
+  }
+  // warp 0: the copies of down unit u (m = kz-1-u) or up unit v (m = v+2)
+  auto issue_down = [&](int u, int b) {
     fence_proxy_async();
-    mbar_expect_tx(bar, (m <= kz ? 7u : 6u) * wb);
-    const int o = (m - 1) * PS, op = (m - 2) * PS;
-    bulk_load(fld(st, 0), w + o + x0, wb, bar);
-    if (m <= kz) bulk_load(fld(st, 1), mul + o + x0, wb, bar);
-    bulk_load(fld(st, 2), pai + op + x0, wb, bar);
-    bulk_load(fld(st, 3), zfs + op + x0, wb, bar);
-    bulk_load(fld(st, 4), fmz_up + op + x0, wb, bar);
-    bulk_load(fld(st, 5), s + op + x0, wb, bar);
-    bulk_load(fld(st, 6), fmzf + op + x0, wb, bar);
+    if (t == 0) {
+      mbar_expect_tx(&mbar[b], dn_bytes);
+    }
+    __syncwarp();
+    if (pc.bytes) bulk_load(stage(b) + pc.dst, pc.src + (kz - 2 - u) * PS, pc.bytes, &mbar[b]);
+  };
+  auto issue_up = [&](int v, int b) {
+    const bool top = v == kz - 1;
+    fence_proxy_async();
+    if (t == 0) {
+      mbar_expect_tx(&mbar[b], ((last ? 7u : 5u) - (top ? 1u : 0u)) * wb);
+    }
+    __syncwarp();
+    if (pc.bytes && !(top && t == 1)) bulk_load(stage(b) + pc.dst, pc.src + v * PS, pc.bytes, &mbar[b]);
   };
   auto bail = [&](int gnext, int gend) {
     if (t == 0) {
@@ -266,32 +746,24 @@ __global__ void __launch_bounds__(kDvW, 4) k_sound_solve(const Dom<R> *__restric
     for (int q = 0; q < NS; ++q) mbar_init(&mbar[q], 1);
     fence_mbar_init();
   }
-  __syncthreads();
-  if (t == 0)
+  block_sync<CW>();
+  if (t < 32)
     for (int u = 0; u < NS && u < nd; ++u) issue_down(u, u);
-  // filtered divergence plus the vertical part of level m (:531-543, :627-630)
-  // fz: fmz, or (bw*dtrdz)*fmz from bind time
-  auto zf_of = [&](int m, double z, double lap, double fz, double sm, double sm1) {
-    if (filt) z = z + sa.xknu[m - 1] * lap;
-    if constexpr (kSolvePre) return z + fz * (sm - sm1);
-    const double bw = relax_weight(sa.ibnd_cr, sa.hefc, c.nspgx, ij, m);
-    return z + bw * dtrdz * fz * (sm - sm1);
-  };
-  // fmz_k: fmz of level k, or zcs2*fmz from bind time
-  double wnext = 0.0, wkp1 = 0.0, zfk = 0.0, pai_k = 0.0, tet_k = 0.0, fmz_k = 0.0, s_k = 0.0;
+  // carried from the level below
+  LevelD vk{};
+  double wnext = 0.0, wkp1 = 0.0;
   if (act) {
     const int o = (kz - 1) * PS + ij_off;
-    const double z = zraw[o];
-    const double lap = filt ? (zraw[o - 1] + zraw[o + 1] + zraw[o - P] + zraw[o + P] - 4.0 * z) : 0.0;
-    s_k = s[o];
-    fmz_k = fmzb[o];
-    zfk = zf_of(kz, z, lap, fmz[o], s_k, s[kz * PS + ij_off]);
-    pai_k = pai[o];
-    tet_k = tetav[o];
+    vk.s = s[o];
+    vk.pai = pai[o];
+    const double ds = vk.s - s[kz * PS + ij_off];
+    if (filt)
+      level_d(vk, true, sa.xknu[kz - 1], zraw[o], zraw[o - 1], zraw[o + 1], zraw[o - P], zraw[o + P],
+              sa.sv_a[r0 + o], ds, sa.sv_b[r0 + o]);
+    else
+      level_d(vk, false, 0.0, zraw[o], 0.0, 0.0, 0.0, 0.0, sa.sv_a[r0 + o], ds, sa.sv_b[r0 + o]);
     wnext = w[kz * PS + ij_off];  // w(kz+1) = -s(kz+1)
   }
-  bool ok = true;
-  int synced = 0;  // first unit read since the last block barrier
   for (int u = 0; u < nd; ++u) {
     const int k = kz - u, m = k - 1;
     const int b = u % NS;
@@ -299,140 +771,90 @@ __global__ void __launch_bounds__(kDvW, 4) k_sound_solve(const Dom<R> *__restric
     const double *st = stage(b);
     if (act) {
       const int o = (k - 1) * PS + ij_off;
-      const double z = st[zc];
-      const double lap = filt ? (st[zc - 1] + st[zc + 1] + st[kDvZW + zc] + st[2 * kDvZW + zc] - 4.0 * z) : 0.0;
-      const double *f0 = st + 3 * kDvZW + t;
-      const double s_m = f0[0], fza_m = f0[kDvW], pai_m = f0[2 * kDvW], tet_m = f0[3 * kDvW];
-      const double wold = f0[4 * kDvW], fmzf_k = f0[5 * kDvW], tvf0 = f0[6 * kDvW];
-      const double fmz_m = kSolvePre ? f0[7 * kDvW] : fza_m;
-      const double zf_m = zf_of(m, z, lap, fza_m, s_m, s_k);
-      zfs[o] = zfk;
-      const double tvf = tvf0 - wold * fmzf_k * dtrdz * (tet_m - tet_k);
-      tetavf[o] = tvf;
-      const double zrom1w = kCpd * tvf * fmzf_k;
-      double zwexpl = wold - zrom1w * dtrdz * (pai_m - pai_k) - kGrav * dts;
-      zwexpl = zwexpl + kRdrcv * zrom1w * dtrdz * (pai_m * zf_m - pai_k * zfk);
-      const double ff = sa.ffilt[k - 1];
-      double zu, zd;
-      if constexpr (kSolvePre) {
-        zu = fmz_m * zrom1w * pai_m + ff;  // fmz_m = zcs2*fmz
-        zd = fmz_k * zrom1w * pai_k + ff;
-      } else {
-        zu = zcs2 * fmz_m * zrom1w * pai_m + ff;
-        zd = zcs2 * fmz_k * zrom1w * pai_k + ff;
-      }
-      const double zrapp = 1.0 / (1.0 + zd + zu - zd * wkp1);
-      wnext = zrapp * (zwexpl + zd * wnext);
-      wkp1 = zrapp * zu;
+      const double *f0 = st + F0 + t;
+      LevelD vm;
+      vm.s = f0[0];
+      vm.pai = f0[2 * CW];
+      const double wold = f0[4 * CW];
+      if (filt)
+        level_d(vm, true, sa.xknu[m - 1], st[zc], st[zc - 1], st[zc + 1], st[ZW + zc], st[2 * ZW + zc], f0[CW],
+                vm.s - vk.s, f0[3 * CW]);
+      else
+        level_d(vm, false, 0.0, st[zc], 0.0, 0.0, 0.0, 0.0, f0[CW], vm.s - vk.s, f0[3 * CW]);
+      const double Z = __fma_rn(-wold, f0[6 * CW], f0[5 * CW]);
+      zfs[o] = vk.zf;
+      zp[o] = Z;
+      eliminate_d(wnext, wkp1, coef_d(vm, vk, Z, wold, sa.ffilt[k - 1], gdts));
       w[o] = wnext;
       mul[o] = wkp1;
-      zfk = zf_m;
-      pai_k = pai_m; tet_k = tet_m; fmz_k = fmz_m; s_k = s_m;
+      vk = vm;
     }
-    ok = ok && landed;
-    if ((u + 1) % kSolveSync == 0 || u + 1 == nd) {
-      if (__syncthreads_or(!ok)) {
-        bail(u + 1, min(nd, synced + NS));  // the units issued and not read
-        return;
-      }
-      // the stages read since the last barrier are free: refill them
-      if (t == 0)
-        for (int r = synced; r <= u; ++r)
-          if (r + NS < nd) issue_down(r + NS, r % NS);
-      synced = u + 1;
+    if (block_any<CW>(!landed)) {
+      bail(u + 1, min(nd, u + NS));  // the units issued and not read
+      return;
+    }
+    // stage b is read: refill it
+    if (t < 32 && u + NS < nd) issue_down(u + NS, b);
+  }
+  if (act) zfs[ij_off] = vk.zf;  // level 1
+  if (t < 32) {
+    pc = {nullptr, 0, 0u};
+    // this lane's plane of the upward pass (level m-1: pai, divergence, dtrdz*fmz and,
+    // after the last substep, s and fmzf; interface m: w, multiplier)
+    switch (t) {
+      case 0: pc = {w + PS + x0, F0, wb}; break;
+      case 1: pc = {mul + PS + x0, F0 + CW, wb}; break;  // not at m = kz+1
+      case 2: pc = {pai + x0, F0 + 2 * CW, wb}; break;
+      case 3: pc = {zfs + x0, F0 + 3 * CW, wb}; break;
+      case 4: pc = {sa.sv_c + r0 + x0, F0 + 4 * CW, wb}; break;
+      case 5: pc = {s + x0, F0 + 5 * CW, last ? wb : 0u}; break;
+      case 6: pc = {sa.fmzf_d + r0 + x0, F0 + 6 * CW, last ? wb : 0u}; break;
+      default: break;
     }
   }
-  if (act) zfs[ij_off] = zfk;  // level 1
   fence_proxy_async_global();
-  __syncthreads();
-  const int nu = kz;
-  if (t == 0)
+  block_sync<CW>();
+  if (t < 32)
     for (int v = 0; v < NS && v < nu; ++v) issue_up(v, (nd + v) % NS);
-  // Exner (:668-671) of level m once w(m+1) is known, and s (:728-734)
-  // fz: fmz, or dtrdz*fmz from bind time
-  auto exner = [&](int m, double wm, double wmp, double pk, double zf, double fz, double sm, double fzf) {
-    const int o = (m - 1) * PS + ij_off;
-    if constexpr (kSolvePre) pai[o] = pk * (1.0 - kRdrcv * (zf + (fz * (wm - wmp))));
-    else pai[o] = pk * (1.0 - kRdrcv * (zf + (dtrdz * fz * (wm - wmp))));
-    if (last && m >= 2) s[o] = (wm + sm) * fzf;
-  };
+  // Exner (:668-671) of level k-1 once w(k) is known, and s (:728-734)
   double wprev = act ? w[ij_off] : 0.0;  // w(1) = 0
-  ok = true;
-  synced = 0;
   for (int v = 0; v < nu; ++v) {
     const int k = v + 2, gu = nd + v;
     const int b = gu % NS;
     const bool landed = mbar_wait_bounded(&mbar[b], (unsigned)((gu / NS) & 1));
     if (act) {
-      const double *f0 = stage(b) + 3 * kDvZW + t;
-      const double wel = f0[0];
-      const double cp = f0[2 * kDvW], czf = f0[3 * kDvW], cfz_ = f0[4 * kDvW], cs = f0[5 * kDvW],
-                   cfzf = f0[6 * kDvW];
+      const double *f0 = stage(b) + F0 + t;
+      const int o = v * PS + ij_off;
+      double wk = f0[0];
       if (k <= kz) {
-        const double wk = wel + f0[kDvW] * wprev;
-        w[(k - 1) * PS + ij_off] = wk;
-        exner(k - 1, wprev, wk, cp, czf, cfz_, cs, cfzf);
-        wprev = wk;
-      } else {
-        exner(kz, wprev, wel, cp, czf, cfz_, cs, cfzf);
+        wk = __fma_rn(f0[CW], wprev, wk);
+        w[o + PS] = wk;
       }
+      pai[o] = exner_d(f0[2 * CW], f0[3 * CW], f0[4 * CW], wprev, wk);
+      if (last && k >= 3) s[o] = (wprev + f0[5 * CW]) * f0[6 * CW];
+      wprev = wk;
     }
-    ok = ok && landed;
-    if ((v + 1) % kSolveSync == 0 || v + 1 == nu) {
-      if (__syncthreads_or(!ok)) {
-        bail(gu + 1, nd + min(nu, synced + NS));
-        return;
-      }
-      if (t == 0)
-        for (int r = synced; r <= v; ++r)
-          if (r + NS < nu) issue_up(r + NS, (nd + r) % NS);
-      synced = v + 1;
+    if (block_any<CW>(!landed)) {
+      bail(gu + 1, nd + min(nu, v + NS));
+      return;
     }
+    if (t < 32 && v + NS < nu) issue_up(v + NS, b);
   }
   if (last && act) {
     s[ij_off] = 0.0;
     s[kz * PS + ij_off] = 0.0;
   }
 }
-#ifndef MLC_SV_STAGES
-#define MLC_SV_STAGES 4
-#endif
-constexpr int kSvStages = MLC_SV_STAGES;  // levels in flight ahead of the one being solved
-constexpr int kSvW = kSolveColsF;          // columns of a block (one row segment)
-constexpr int kSvZW = kSvW + 8;      // raw divergence rows with a 4-column halo each side
-constexpr int kSvStage = 3 * kSvZW + 11 * kSvW;  // floats of one stage
 
-// The solve of a mixed member (same equations as k_sound_solve), in FP32
-// only, one thread per column.  Where rounding is amplified the values are
-// double-floats: theta_v at half levels, the hydrostatic balance
-// -cp*theta_v*fmzf*dtrdz*(pai(k-1) - pai(k)) - g*dts of the w equation (two
-// terms of ~g*dts whose difference drives w), and the Exner update
-// pai - pai*increment.  The divergence filter, the elimination coefficients
-// (O(1)-conditioned), the recurrence and the back substitution run in plain
-// FP32.  The downward pass forms each level's coefficients and eliminates at
-// once; the upward pass substitutes back and updates Exner (and, after the
-// last substep, s) a level behind.  Between the passes the column's
-// eliminated w stays in w, its multipliers and filtered divergence in the
-// FP32 planes of wz_d[1] and wz_d[0] (free during the acoustic loop).
-// wz[2] holds theta_v(k-1) - theta_v(k) from sound_prep.
-//
-// The inputs stream through shared memory: a block is 128 consecutive
-// columns of one row, and the copy engine brings each level's planes as
-// 512-byte row segments (untiled bulk copies, 16-byte aligned: the segment
-// starts at a multiple of 128 columns, the raw divergence's halo of 4
-// columns keeps that alignment) kSvStages levels ahead of the level being
-// solved, so the per-level chain of dependent arithmetic never waits on
-// memory.  The copies of one level (11 planes and 1 or 3 divergence rows)
-// complete on one mbarrier; a stage is refilled after every thread has read
-// it (one block barrier a level).  The upward pass reads back w, the
-// multipliers and the filtered divergence the threads stored in the
-// downward pass, after a proxy fence.  (Measured on the 512x512x41 step:
-// 0.73 ms of solves a step against 0.95 for the same thread-per-column
-// kernel with register prefetch of one level.)
-template <class R, bool DFR>
-__global__ void __launch_bounds__(128, 4) k_solve_mixed(const Dom<R> *__restrict__ doms, int advoff, int last,
-    const WorkItem *__restrict__ wl) {
-  constexpr int NS = kSvStages;
+// The mixed form: the arithmetic of k_solve_cols_f.
+// Seven blocks an SM (64 registers): 793 us of four solves at 512x512x41; six
+// 804, eight (56 registers) 817, five 893.
+template <class R, int CW, bool DFR>
+__global__ void __launch_bounds__(CW, 7) k_solve_stream_f(const Dom<R> *__restrict__ doms,
+    int advoff, int last, const WorkItem *__restrict__ wl) {
+  static_assert(sizeof(R) == sizeof(float), "FP32 fields");
+  using Sh = SolveShape<R, CW>;
+  constexpr int NS = Sh::kStages, ZW = Sh::kZW;
   extern __shared__ __align__(16) float sv_smem[];
   __shared__ __align__(8) uint64_t mbar[NS];
   const WorkItem wi = wl ? wl[blockIdx.x]
@@ -441,7 +863,7 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const Dom<R> *__restrict
   if (!D.active) return;
   const Geom g = D.g;
   const int t = (int)threadIdx.x;
-  const int x0 = (int)wi.a * kSvW;          // first column (0-based j-1) of the block
+  const int x0 = (int)wi.a * CW;            // first column (0-based j-1) of the block
   const int i = (int)wi.b + 2;
   if (x0 + 1 > g.jx - 2 || i > g.iy - 2) return;  // uniform over the block
   const int j = x0 + t + 1;
@@ -453,89 +875,69 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const Dom<R> *__restrict
   const size_t F = g.field3(), F1 = g.PS * (size_t)(kz + 1);
   const int PS = (int)g.PS, P = g.P;
   const size_t r0 = g.at2(1, i);                  // row i, column 1
+  const SoundScratch<R> ss = sound_scratch(D);
   // row bases (column 1 of row i, level 1)
   float *__restrict__ pai_h = reinterpret_cast<float *>(D.pai[adv]) + r0;
   float *__restrict__ pai_l = pai_h + F;
-  float *__restrict__ tvf_h = reinterpret_cast<float *>(D.tetavf) + r0;
-  float *__restrict__ tvf_l = tvf_h + F1;
-  const float *__restrict__ cfz_h = reinterpret_cast<const float *>(sa.cfz) + r0;
-  const float *__restrict__ cfz_l = cfz_h + F1;
-  float *__restrict__ zfs = reinterpret_cast<float *>(D.wz_d[0]) + r0;
-  float *__restrict__ mul = reinterpret_cast<float *>(D.wz_d[1]) + r0;
-  // DFR: the low parts of the eliminated w and of the multipliers, in the
-  // free lo planes of the same scratch allocations
-  float *__restrict__ w_lo = zfs + F;
-  float *__restrict__ mul_lo = mul + F;
+  float *__restrict__ z_h = reinterpret_cast<float *>(D.tetavf) + r0;
+  float *__restrict__ z_l = z_h + F1;
+  float *__restrict__ zfs = ss.zf + r0;
+  float *__restrict__ mul = ss.mul + r0;
+  float *__restrict__ w_lo = ss.w_lo + r0;
+  float *__restrict__ mul_lo = ss.mul_lo + r0;
   const float *__restrict__ zraw = D.zdiv2 + r0;
-  const float *__restrict__ dtet = D.wz[2] + r0;
   const float *__restrict__ fmz = sa.fmz + r0;
-  const float *__restrict__ fmzf = sa.fmzf + r0;
   float *__restrict__ s = D.s + r0;
   float *__restrict__ w = D.w + r0;
   const float dtrdz = c.dtsoundf * c.rdzitaf;
-  const float rdrcv = float(kRdrcv);
-  const float rdt = rdrcv * dtrdz;
   const F2 ngdts{-c.gdts_hi, -c.gdts_lo};
   const int ij_off = j - 1;                       // this thread's column offset in a row
   const int32_t ib = act ? sa.ibnd_cr[r0 + ij_off] : 0;
   const int nsp = c.nspgx;
   const bool filt = c.divfilter != 0;
   // copy extents: the block's columns, and the raw divergence with its halo
-  const int xe = min(x0 + kSvW, P);
-  const int zs = x0 >= 4 ? x0 - 4 : 0, ze = min(x0 + kSvW + 4, P);
+  const int xe = min(x0 + CW, P);
+  const int zs = x0 >= Sh::kHalo ? x0 - Sh::kHalo : 0, ze = min(x0 + CW + Sh::kHalo, P);
   const unsigned wb = (unsigned)(xe - x0) * 4u, zb = (unsigned)(ze - zs) * 4u;
   const int zc = x0 + t - zs;                     // this column in a halo row
-  auto stage = [&](int b) { return sv_smem + (size_t)b * kSvStage; };
-  // stage layout: zraw rows i, i-1, i+1 (kSvZW each), then 11 fields of kSvW
-  auto fld = [&](float *st, int f) { return st + 3 * kSvZW + f * kSvW; };
-  const int nd = kz - 1;                          // down units: m = kz-1 .. 1
-  // down unit u: A(m) = zraw, s, fmz, pai at level m; B(m+1) = w, fmzf,
-  // dtet, tvf, cfz at interface m+1 (m = kz-1-u)
+  auto stage = [&](int b) { return sv_smem + (size_t)b * Sh::kStage; };
+  constexpr int F0 = 3 * ZW;
+  const int nd = kz - 1, nu = kz;                 // down units: m = kz-1 .. 1, up units: m = 2 .. kz+1
+  PlaneCopy<R> pc{nullptr, 0, 0u};
+  const unsigned dn_bytes = (filt ? 3u : 1u) * zb + 8u * wb;
+  if (t < 32) {
+    switch (t) {
+      case 0: pc = {zraw + zs, 0, zb}; break;
+      case 1: pc = {zraw - P + zs, ZW, filt ? zb : 0u}; break;
+      case 2: pc = {zraw + P + zs, 2 * ZW, filt ? zb : 0u}; break;
+      case 3: pc = {s + x0, F0, wb}; break;
+      case 4: pc = {fmz + x0, F0 + CW, wb}; break;
+      case 5: pc = {pai_h + x0, F0 + 2 * CW, wb}; break;
+      case 6: pc = {pai_l + x0, F0 + 3 * CW, wb}; break;
+      case 7: pc = {w + PS + x0, F0 + 4 * CW, wb}; break;
+      case 8: pc = {ss.g + r0 + PS + x0, F0 + 5 * CW, wb}; break;
+      case 9: pc = {z_h + PS + x0, F0 + 6 * CW, wb}; break;
+      case 10: pc = {z_l + PS + x0, F0 + 7 * CW, wb}; break;
+      default: break;
+    }
+  }
   auto issue_down = [&](int u, int b) {
-    const int m = kz - 1 - u;
-    float *st = stage(b);
-    uint64_t *bar = &mbar[b];
     fence_proxy_async();
-    mbar_expect_tx(bar, (filt ? 3u : 1u) * zb + 11u * wb);
-    const int o = (m - 1) * PS, ob = m * PS;
-    bulk_load(st, zraw + o + zs, zb, bar);
-    if (filt) {
-      bulk_load(st + kSvZW, zraw + o - P + zs, zb, bar);
-      bulk_load(st + 2 * kSvZW, zraw + o + P + zs, zb, bar);
+    if (t == 0) {
+      mbar_expect_tx(&mbar[b], dn_bytes);
     }
-    bulk_load(fld(st, 0), s + o + x0, wb, bar);
-    bulk_load(fld(st, 1), fmz + o + x0, wb, bar);
-    bulk_load(fld(st, 2), pai_h + o + x0, wb, bar);
-    bulk_load(fld(st, 3), pai_l + o + x0, wb, bar);
-    bulk_load(fld(st, 4), w + ob + x0, wb, bar);
-    bulk_load(fld(st, 5), fmzf + ob + x0, wb, bar);
-    bulk_load(fld(st, 6), dtet + ob + x0, wb, bar);
-    bulk_load(fld(st, 7), tvf_h + ob + x0, wb, bar);
-    bulk_load(fld(st, 8), tvf_l + ob + x0, wb, bar);
-    bulk_load(fld(st, 9), cfz_h + ob + x0, wb, bar);
-    bulk_load(fld(st, 10), cfz_l + ob + x0, wb, bar);
+    __syncwarp();
+    if (pc.bytes) bulk_load(stage(b) + pc.dst, pc.src + (kz - 2 - u) * PS, pc.bytes, &mbar[b]);
   };
-  // up unit v (m = v + 2): w(m), mul(m) (m <= kz), and pai, zfs, fmz, s,
-  // fmzf at level m-1
   auto issue_up = [&](int v, int b) {
-    const int m = v + 2;
-    float *st = stage(b);
-    uint64_t *bar = &mbar[b];
+    const bool top = v == kz - 1;
     fence_proxy_async();
-    mbar_expect_tx(bar, (m <= kz ? (DFR ? 10u : 8u) : 7u) * wb);
-    const int o = (m - 1) * PS, op = (m - 2) * PS;
-    bulk_load(fld(st, 0), w + o + x0, wb, bar);
-    if (m <= kz) bulk_load(fld(st, 1), mul + o + x0, wb, bar);
-    if (DFR && m <= kz) {
-      bulk_load(fld(st, 8), w_lo + o + x0, wb, bar);
-      bulk_load(fld(st, 9), mul_lo + o + x0, wb, bar);
+    if (t == 0) {
+      mbar_expect_tx(&mbar[b], (5u + (last ? 2u : 0u) + (top ? 0u : DFR ? 3u : 1u)) * wb);
     }
-    bulk_load(fld(st, 2), pai_h + op + x0, wb, bar);
-    bulk_load(fld(st, 3), pai_l + op + x0, wb, bar);
-    bulk_load(fld(st, 4), zfs + op + x0, wb, bar);
-    bulk_load(fld(st, 5), fmz + op + x0, wb, bar);
-    bulk_load(fld(st, 6), s + op + x0, wb, bar);
-    bulk_load(fld(st, 7), fmzf + op + x0, wb, bar);
+    __syncwarp();
+    if (pc.bytes && !(top && t >= 1 && t <= 3))
+      bulk_load(stage(b) + pc.dst, pc.src + v * PS, pc.bytes, &mbar[b]);
   };
   // a failed wait (a copy that never landed): record it, let the copies in
   // flight land (bounded) and leave
@@ -549,37 +951,28 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const Dom<R> *__restrict
     for (int q = 0; q < NS; ++q) mbar_init(&mbar[q], 1);
     fence_mbar_init();
   }
-  __syncthreads();
-  if (t == 0)
+  block_sync<CW>();
+  if (t < 32)
     for (int u = 0; u < NS && u < nd; ++u) issue_down(u, u);
 
-  struct LvA {
-    float z, lap, s, fmz;
-    F2 pai;
-  };
-  auto zf_of = [&](int m, const LvA &a, float s_above) {
-    float z = a.z;
-    if (filt) z = z + sa.xknu_r[m - 1] * a.lap;
-    const float bw = ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(m - 1) * nsp] : 1.f;
-    return z + bw * dtrdz * a.fmz * (a.s - s_above);
+  auto bweight = [&](int m) {
+    return ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(m - 1) * nsp] : 1.f;
   };
   // level kz and the interface below it straight from memory (once)
-  LvA ak{};
-  float wnext = 0.f, zfk = 0.f;
+  LevelF vk{};
+  F2 wnext{0.f, 0.f}, wkp1{0.f, 0.f};
   if (act) {
     const int o = (kz - 1) * PS + ij_off;
-    ak.z = zraw[o];
-    ak.lap = filt ? (zraw[o - 1] + zraw[o + 1] + zraw[o - P] + zraw[o + P] - 4.f * ak.z) : 0.f;
-    ak.s = s[o];
-    ak.fmz = fmz[o];
-    ak.pai = F2{pai_h[o], pai_l[o]};
-    wnext = w[kz * PS + ij_off];
-    zfk = zf_of(kz, ak, s[kz * PS + ij_off]);
+    vk.s = s[o];
+    vk.pai = F2{pai_h[o], pai_l[o]};
+    const float fz = __fmul_rn(dtrdz, fmz[o]), ds = vk.s - s[kz * PS + ij_off];
+    if (filt)
+      level_f(vk, true, sa.xknu_r[kz - 1], zraw[o], zraw[o - 1], zraw[o + 1], zraw[o - P], zraw[o + P], bweight(kz),
+              fz, ds);
+    else
+      level_f(vk, false, 0.f, zraw[o], 0.f, 0.f, 0.f, 0.f, bweight(kz), fz, ds);
+    wnext.hi = w[kz * PS + ij_off];
   }
-  float wkp1 = 0.f;
-  F2 wnextd{wnext, 0.f}, wkp1d{0.f, 0.f};
-  bool ok = true;
-  int synced = 0;  // first unit read since the last block barrier
   for (int u = 0; u < nd; ++u) {
     const int k = kz - u, m = k - 1;
     const int b = u % NS;
@@ -587,141 +980,100 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const Dom<R> *__restrict
     const float *st = stage(b);
     if (act) {
       const int o = (k - 1) * PS + ij_off;
-      LvA am;
-      am.z = st[zc];
-      am.lap = filt ? (st[zc - 1] + st[zc + 1] + st[kSvZW + zc] + st[2 * kSvZW + zc] - 4.f * am.z) : 0.f;
-      const float *f0 = st + 3 * kSvZW + t;
-      am.s = f0[0];
-      am.fmz = f0[kSvW];
-      am.pai = F2{f0[2 * kSvW], f0[3 * kSvW]};
-      const float wold = f0[4 * kSvW], bfmzf = f0[5 * kSvW], bdtet = f0[6 * kSvW];
-      const F2 btvf{f0[7 * kSvW], f0[8 * kSvW]}, bcfz{f0[9 * kSvW], f0[10 * kSvW]};
-      const float zf_m = zf_of(m, am, ak.s);
-      zfs[o] = zfk;
-      const F2 pai_m = am.pai, pai_k = ak.pai;
-      const float corr = wold * bfmzf * dtrdz * bdtet;
-      const F2 tvf = df_add_f(btvf, -corr);
-      tvf_h[o] = tvf.hi;
-      tvf_l[o] = tvf.lo;
-      const F2 zrd = df_mul(tvf, bcfz);
-      const F2 dp = two_sum(pai_m.hi - pai_k.hi, pai_m.lo - pai_k.lo);
-      const F2 bal = df_add(ngdts, df_mul(F2{-zrd.hi, -zrd.lo}, dp));
-      const float zr = df_f(zrd), pm = df_f(pai_m), pk = df_f(pai_k);
-      const float ff = sa.ffilt_r[k - 1];
-      const float zu = rdt * am.fmz * zr * pm + ff;
-      const float zd = rdt * ak.fmz * zr * pk + ff;
+      const float *f0 = st + F0 + t;
+      LevelF vm;
+      vm.s = f0[0];
+      vm.pai = F2{f0[2 * CW], f0[3 * CW]};
+      const float fz = __fmul_rn(dtrdz, f0[CW]), wold = f0[4 * CW];
+      if (filt)
+        level_f(vm, true, sa.xknu_r[m - 1], st[zc], st[zc - 1], st[zc + 1], st[ZW + zc], st[2 * ZW + zc], bweight(m),
+                fz, vm.s - vk.s);
+      else
+        level_f(vm, false, 0.f, st[zc], 0.f, 0.f, 0.f, 0.f, bweight(m), fz, vm.s - vk.s);
+      zfs[o] = vk.zf;
+      const F2 Z = df_add_f(F2{f0[6 * CW], f0[7 * CW]}, -__fmul_rn(wold, f0[5 * CW]));
+      z_h[o] = Z.hi;
+      z_l[o] = Z.lo;
+      eliminate_f<DFR>(wnext, wkp1, coef_f(vm, vk, Z, wold, sa.ffilt_r[k - 1], ngdts));
+      w[o] = wnext.hi;
+      mul[o] = wkp1.hi;
       if constexpr (DFR) {
-        // the recurrence in double-float: the explicit w keeps the hydrostatic
-        // balance's low part, the pivots and multipliers carry theirs
-        F2 zw = df_add_f(bal, wold);
-        zw = df_add_f(zw, rdrcv * zr * (pm * zf_m - pk * zfk));
-        const F2 den = df_add(two_sum(1.f + zd, zu), df_mul_f(F2{-wkp1d.hi, -wkp1d.lo}, zd));
-        const F2 zrapp = df_recip(den);  // den >= 1: the pivot of a diagonally dominant system
-        wnextd = df_mul(zrapp, df_add(zw, df_mul_f(wnextd, zd)));
-        wkp1d = df_mul_f(zrapp, zu);
-        w[o] = wnextd.hi;
-        w_lo[o] = wnextd.lo;
-        mul[o] = wkp1d.hi;
-        mul_lo[o] = wkp1d.lo;
-      } else {
-        float zw = wold + df_f(bal);
-        zw = zw + rdrcv * zr * (pm * zf_m - pk * zfk);
-        const float zrapp = 1.f / (1.f + zd + zu - zd * wkp1);
-        wnext = zrapp * (zw + zd * wnext);
-        wkp1 = zrapp * zu;
-        w[o] = wnext;
-        mul[o] = wkp1;
+        w_lo[o] = wnext.lo;
+        mul_lo[o] = wkp1.lo;
       }
-      zfk = zf_m;
-      ak = am;
+      vk = vm;
     }
-    ok = ok && landed;
-    if ((u + 1) % kSolveSync == 0 || u + 1 == nd) {
-      if (__syncthreads_or(!ok)) {
-        bail(u + 1, min(nd, synced + NS));  // the units issued and not read
-        return;
-      }
-      // the stages read since the last barrier are free: refill them
-      if (t == 0)
-        for (int r = synced; r <= u; ++r)
-          if (r + NS < nd) issue_down(r + NS, r % NS);
-      synced = u + 1;
+    if (block_any<CW>(!landed)) {
+      bail(u + 1, min(nd, u + NS));  // the units issued and not read
+      return;
+    }
+    // stage b is read: refill it
+    if (t < 32 && u + NS < nd) issue_down(u + NS, b);
+  }
+  if (act) zfs[ij_off] = vk.zf;  // level 1
+  // this thread's stores of w, mul and zfs are read back by the copy engine
+  if (t < 32) {
+    pc = {nullptr, 0, 0u};
+    // s and fmzf (after the last substep) go where the divergence rows lay
+    switch (t) {
+      case 0: pc = {w + PS + x0, F0, wb}; break;
+      case 1: pc = {mul + PS + x0, F0 + CW, wb}; break;             // these three
+      case 2: pc = {w_lo + PS + x0, F0 + 2 * CW, DFR ? wb : 0u}; break;    // not at
+      case 3: pc = {mul_lo + PS + x0, F0 + 3 * CW, DFR ? wb : 0u}; break;  // m = kz+1
+      case 4: pc = {pai_h + x0, F0 + 4 * CW, wb}; break;
+      case 5: pc = {pai_l + x0, F0 + 5 * CW, wb}; break;
+      case 6: pc = {zfs + x0, F0 + 6 * CW, wb}; break;
+      case 7: pc = {fmz + x0, F0 + 7 * CW, wb}; break;
+      case 8: pc = {s + x0, 0, last ? wb : 0u}; break;
+      case 9: pc = {sa.fmzf + r0 + x0, ZW, last ? wb : 0u}; break;
+      default: break;
     }
   }
-  if (act) zfs[ij_off] = zfk;  // level 1
-  // this thread's stores of w, mul and zfs are read back by the copy engine
   fence_proxy_async_global();
-  __syncthreads();
-  const int nu = kz;  // up units: m = 2 .. kz+1
-  if (t == 0)
+  block_sync<CW>();
+  if (t < 32)
     for (int v = 0; v < NS && v < nu; ++v) issue_up(v, (nd + v) % NS);
-  auto exner = [&](int m, float wm, float dw, F2 pk, float zf, float fz, float sm, float fzf) {
-    const int o = (m - 1) * PS + ij_off;
-    const float inc = rdrcv * (zf + (dtrdz * fz * dw));
-    const F2 d = df_mul_f(pk, inc);
-    const F2 pn = df_add(pk, F2{-d.hi, -d.lo});
-    pai_h[o] = pn.hi;
-    pai_l[o] = pn.lo;
-    if (last && m >= 2) s[o] = (wm + sm) * fzf;
-  };
-  float wprev = act ? w[ij_off] : 0.f;  // w(1) = 0
-  F2 wprevd{wprev, 0.f};
-  ok = true;
-  synced = 0;
+  F2 wprev{act ? w[ij_off] : 0.f, 0.f};  // w(1) = 0
   for (int v = 0; v < nu; ++v) {
     const int k = v + 2, gu = nd + v;
     const int b = gu % NS;
     const bool landed = mbar_wait_bounded(&mbar[b], (unsigned)((gu / NS) & 1));
     if (act) {
-      const float *f0 = stage(b) + 3 * kSvZW + t;
-      const float wel = f0[0];
-      const F2 cp{f0[2 * kSvW], f0[3 * kSvW]};
-      const float czf = f0[4 * kSvW], cfz_ = f0[5 * kSvW], cs = f0[6 * kSvW], cfzf = f0[7 * kSvW];
-      if constexpr (DFR) {
-        if (k <= kz) {
-          const F2 wk = df_add(F2{wel, f0[8 * kSvW]},
-                               df_mul(F2{f0[kSvW], f0[9 * kSvW]}, wprevd));
-          const float wkf = df_f(wk);
-          w[(k - 1) * PS + ij_off] = wkf;
-          exner(k - 1, df_f(wprevd), df_diff(wprevd, wk), cp, czf, cfz_, cs, cfzf);
-          wprevd = wk;
-        } else {
-          exner(kz, df_f(wprevd), df_f(df_add_f(wprevd, -wel)), cp, czf, cfz_, cs, cfzf);
-        }
-      } else {
-        if (k <= kz) {
-          const float wk = wel + f0[kSvW] * wprev;
-          w[(k - 1) * PS + ij_off] = wk;
-          exner(k - 1, wprev, wprev - wk, cp, czf, cfz_, cs, cfzf);
-          wprev = wk;
-        } else {
-          exner(kz, wprev, wprev - wel, cp, czf, cfz_, cs, cfzf);
-        }
+      const float *st = stage(b);
+      const float *f0 = st + F0 + t;
+      const int o = v * PS + ij_off;
+      F2 wk{f0[0], 0.f};
+      if (k <= kz) {
+        if constexpr (DFR) wk = back_f<DFR>(F2{wk.hi, f0[2 * CW]}, F2{f0[CW], f0[3 * CW]}, wprev);
+        else wk = back_f<DFR>(wk, F2{f0[CW], 0.f}, wprev);
+        w[o + PS] = df_f(wk);
       }
+      // Exner of level k-1 (and s after the last substep)
+      const F2 pn = exner_f(F2{f0[4 * CW], f0[5 * CW]}, f0[6 * CW], __fmul_rn(dtrdz, f0[7 * CW]), wprev, wk);
+      pai_h[o] = pn.hi;
+      pai_l[o] = pn.lo;
+      if (last && k >= 3) s[o] = (df_f(wprev) + st[t]) * st[ZW + t];
+      wprev = wk;
     }
-    ok = ok && landed;
-    if ((v + 1) % kSolveSync == 0 || v + 1 == nu) {
-      if (__syncthreads_or(!ok)) {
-        bail(gu + 1, nd + min(nu, synced + NS));
-        return;
-      }
-      if (t == 0)
-        for (int r = synced; r <= v; ++r)
-          if (r + NS < nu) issue_up(r + NS, (nd + r) % NS);
-      synced = v + 1;
+    if (block_any<CW>(!landed)) {
+      bail(gu + 1, nd + min(nu, v + NS));
+      return;
     }
+    if (t < 32 && v + NS < nu) issue_up(v + NS, b);
   }
   if (last && act) {
     s[ij_off] = 0.f;
     s[kz * PS + ij_off] = 0.f;
   }
 }
-// Main/mod_moloch.F90:677-721 with divergence_damping :738-765 folded in
+
+// Main/mod_moloch.F90:677-721 with divergence_damping :738-765 folded in, FP64
 template <class R>
 __global__ void k_sound_momentum(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
                                  int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
+  static_assert(sizeof(R) == sizeof(double), "FP64 member");
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
   const Geom g = D.g;
@@ -735,107 +1087,39 @@ __global__ void k_sound_momentum(const Dom<R> *__restrict__ doms, int uvoff, int
   R *__restrict__ v_out = D.v[uv ^ 1];
   const R *__restrict__ zraw = D.zdiv2;
   const double *__restrict__ pai = D.pai[adv];
-  const double *__restrict__ tetav = D.tetav[adv];
+  const SoundScratch<R> ss = sound_scratch(D);
   const Pt q = point_at(wi, 1, 1);
   const int j = q.j, i = q.i;
   if (j > g.jx || i > g.iy || q.k > g.kz) return;
-  constexpr bool mixed = sizeof(R) == sizeof(float);
-  const R dts = pick<R>(c.dtsound, c.dtsoundf);
-  const R dtrdx = pick<R>(c.dtrdxs, c.dtrdxsf), dtrdy = dtrdx;
-  const R dxrdt = pick<R>(c.dxrdt, c.dxrdtf);
-  const size_t F = g.field3();
-  // mixed member: theta_v and Exner are double-floats (hi, lo planes)
-  const float *__restrict__ th_f = reinterpret_cast<const float *>(tetav);
-  const float *__restrict__ pa_f = reinterpret_cast<const float *>(pai);
-  // relaxation weight 1 - hefc(ib, k) (Main/mod_bdycod.F90:4033-4047)
-  auto bweight = [&](const int32_t *ibnd, size_t ij0, int k) -> R {
-    if constexpr (mixed) {
-      const int ib = ibnd[ij0];
-      return ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(k - 1) * c.nspgx] : 1.f;
-    } else {
-      return R(relax_weight(ibnd, sa.hefc, c.nspgx, ij0, k));
-    }
-  };
-  // theta_v(a) + theta_v(b) and pai(a) - pai(b) in the field type
-  auto tsum = [&](size_t a, size_t b) -> R {
-    if constexpr (mixed) return (th_f[a] + th_f[b]) + (th_f[a + F] + th_f[b + F]);
-    else return R(tetav[a] + tetav[b]);
-  };
-  auto pdif = [&](size_t a, size_t b) -> R {
-    if constexpr (mixed) return (pa_f[a] - pa_f[b]) + (pa_f[a + F] - pa_f[b + F]);
-    else return R(pai[a] - pai[b]);
-  };
-  const R zfz = R(kGrav) * dts;
-  const R halfcp = R(0.5) * R(kCpd);
   const size_t ij = g.at2(j, i);
   const size_t PS = g.PS;
   const bool has_u = i <= g.iy - 1;
   const bool has_v = j <= g.jx - 1;
   const bool upd_u = has_u && j >= 2 && j <= g.jx - 1 && i >= 2 && i <= g.iy - 2;
   const bool upd_v = has_v && j >= 2 && j <= g.jx - 2 && i >= 2 && i <= g.iy - 1;
-  R mu = 0, zcx = 0, hxk = 0, cor_u = 0, zcy = 0, hyk = 0, cor_v = 0, mv = 0;
-  if (upd_u) {
-    mu = sa.msfu[ij];
-    zcx = dtrdx * mu;
-    hxk = sa.hx[ij];
-    cor_u = sa.coru[ij];
-  }
-  if (upd_v) {
-    mv = sa.msfv[ij];
-    zcy = c.lrotllr ? dtrdy : dtrdy * mv;
-    hyk = sa.hy[ij];
-    cor_v = sa.corv[ij];
-  }
+  const double cor_u = upd_u ? sa.mo_cu[ij] : 0.0, cor_v = upd_v ? sa.mo_cv[ij] : 0.0;
   const size_t W = 1, S = (size_t)g.P;
+  // Six FP64 instructions a wind point (the pipe that bounds this kernel):
+  // the constant products dxrdt*xkdamp*msfu, g*dts*hx*gzitakh and coru*dts
+  // come from bind time, zcx*cp/2*(theta_v sum) from sound_prep.
 #pragma unroll
   for (int k = q.k; k < q.k + kPtLevels && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * PS;
-    const R gk = sa.gzitakh_r[k - 1];
     if (has_u) {
-      R un = u_in[o];
+      double un = u_in[o];
       if (upd_u) {
-        // FP64: the constant products dxrdt*xkdamp*msfu, g*dts*hx*gzitakh and
-        // coru*dts come from bind time (same operands, same order)
-        if (c.divdamp) {
-          R xdam;
-          if constexpr (mixed) xdam = dxrdt * sa.xkdamp_r[k - 1] * mu;
-          else xdam = sa.mo_du[o];
-          un = un + xdam * (zraw[o] - zraw[o - W]);
-        }
-        const R zrom1u = halfcp * tsum(o - W, o);
-        R zcor1u, zg;
-        if constexpr (mixed) {
-          zcor1u = cor_u * dts * v_in[o];
-          zg = zfz * hxk * gk;
-        } else {
-          zcor1u = sa.mo_cu[ij] * v_in[o];
-          zg = sa.mo_gu[o];
-        }
-        const R bw = bweight(sa.ibnd_ud, ij, k);
-        un = un + bw * (zcor1u - zg - zcx * zrom1u * pdif(o, o - W));
+        if (c.divdamp) un = __fma_rn(sa.mo_du[o], zraw[o] - zraw[o - W], un);
+        const double r = __fma_rn(-ss.cu[o], pai[o] - pai[o - W], __fma_rn(cor_u, v_in[o], -sa.mo_gu[o]));
+        un = __fma_rn(relax_weight(sa.ibnd_ud, sa.hefc, c.nspgx, ij, k), r, un);
       }
       u_out[o] = un;
     }
     if (has_v) {
-      R vn = v_in[o];
+      double vn = v_in[o];
       if (upd_v) {
-        if (c.divdamp) {
-          R xdam;
-          if constexpr (mixed) xdam = c.lrotllr ? dxrdt * sa.xkdamp_r[k - 1] : dxrdt * sa.xkdamp_r[k - 1] * mv;
-          else xdam = sa.mo_dv[o];
-          vn = vn + xdam * (zraw[o] - zraw[o - S]);
-        }
-        const R zrom1v = halfcp * tsum(o - S, o);
-        R zcor1v, zg;
-        if constexpr (mixed) {
-          zcor1v = cor_v * dts * u_in[o];
-          zg = zfz * hyk * gk;
-        } else {
-          zcor1v = sa.mo_cv[ij] * u_in[o];
-          zg = sa.mo_gv[o];
-        }
-        const R bw = bweight(sa.ibnd_vd, ij, k);
-        vn = vn + bw * (-zcor1v - zg - zcy * zrom1v * pdif(o, o - S));
+        if (c.divdamp) vn = __fma_rn(sa.mo_dv[o], zraw[o] - zraw[o - S], vn);
+        const double r = __fma_rn(-ss.cv[o], pai[o] - pai[o - S], __fma_rn(-cor_v, u_in[o], -sa.mo_gv[o]));
+        vn = __fma_rn(relax_weight(sa.ibnd_vd, sa.hefc, c.nspgx, ij, k), r, vn);
       }
       v_out[o] = vn;
     }
@@ -1103,8 +1387,8 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const
         const float zcor1u = cu4[q] * dts * vo[q];
         const int ib = ibu[q];
         const float bw = ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(k - 1) * nsp] : 1.f;
-        const float zcx = dtrdx * mu[q];
         const float pd = (ph.x[q] - ph.at(q - 1)) + (pl.x[q] - pl.at(q - 1));
+        const float zcx = dtrdx * mu[q];
         a = a + bw * (zcor1u - zfz * hx4[q] * gk - zcx * zrom1u * pd);
       }
       un[q] = a;
@@ -1118,8 +1402,8 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const
         const float zcor1v = cv4[q] * dts * uo[q];
         const int ib = ibv[q];
         const float bw = ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(k - 1) * nsp] : 1.f;
-        const float zcy = c.lrotllr ? dtrdy : dtrdy * mv[q];
         const float pd = (ph.x[q] - ps[q]) + (pl.x[q] - psl[q]);
+        const float zcy = c.lrotllr ? dtrdy : dtrdy * mv[q];
         b = b + bw * (-zcor1v - zfz * hy4[q] * gk - zcy * zrom1v * pd);
       }
       vn[q] = b;
@@ -1152,6 +1436,10 @@ inline dim3 pt_grid(const LaunchGeom &L, int nj, int ni, int &tiles_j) {
 }
 }  // namespace
 
+// shared memory of a solve block of columns of kz levels
+template <class R>
+constexpr size_t solve_smem(int kz) { return (size_t)kSolveArrays * (kz + 2) * 32 * sizeof(R); }
+
 template <class R>
 void Launch<R>::sound_prep(const LaunchGeom &L, const Dom<R> *d, int advoff, cudaStream_t s) {
   int tj;
@@ -1174,27 +1462,39 @@ void Launch<R>::sound_div(const LaunchGeom &L, const Dom<R> *d, int uvoff, cudaS
   }
 }
 
+template <class R, int AW>
+void launch_cols(const LaunchGeom &L, const Dom<R> *d, dim3 grid, int advoff, int last, cudaStream_t s) {
+  const size_t smem = solve_smem<R>(L.kz);
+  if constexpr (sizeof(R) == sizeof(float)) {
+    if (L.solve_df) k_solve_cols_f<R, AW, true><<<grid, solve_threads(AW), smem, s>>>(d, advoff, last, L.wl_solve);
+    else k_solve_cols_f<R, AW, false><<<grid, solve_threads(AW), smem, s>>>(d, advoff, last, L.wl_solve);
+  } else {
+    k_solve_cols_d<R, AW><<<grid, solve_threads(AW), smem, s>>>(d, advoff, last, L.wl_solve);
+  }
+}
+
 template <class R>
 void Launch<R>::sound_solve(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool last,
                             cudaStream_t s) {
   (void)uvoff;
-  // one block per 128-column row segment in both precisions (the solve
-  // launch shape of LaunchGeom is not used)
-  if constexpr (sizeof(R) == sizeof(float)) {
-    const int tj = (L.jx - 1 + kSvW - 1) / kSvW;
-    const dim3 grid = L.wl_solve ? dim3((unsigned)L.n_solve, 1, 1)
-                                 : dim3((unsigned)tj, (unsigned)(L.iy - 3), (unsigned)L.nmem);
-    const size_t smem = (size_t)kSvStages * kSvStage * sizeof(float);
-    if (L.solve_df)
-      k_solve_mixed<R, true><<<grid, kSvW, smem, s>>>(d, advoff, last ? 1 : 0, L.wl_solve);
-    else
-      k_solve_mixed<R, false><<<grid, kSvW, smem, s>>>(d, advoff, last ? 1 : 0, L.wl_solve);
+  // (LaunchGeom's solve_x and solve_y are not used)
+  constexpr int CW = solve_segment(kSolveStream, (int)sizeof(R));
+  const int w = solve_segment(L.solve, (int)sizeof(R)), lst = last ? 1 : 0;
+  const dim3 grid = L.wl_solve ? dim3((unsigned)L.n_solve, 1, 1)
+                               : dim3((unsigned)((L.jx - 1 + w - 1) / w), (unsigned)(L.iy - 3), (unsigned)L.nmem);
+  if (L.solve == kSolveCols6) {
+    launch_cols<R, 6>(L, d, grid, advoff, lst, s);
+  } else if (L.solve == kSolveCols3) {
+    launch_cols<R, 3>(L, d, grid, advoff, lst, s);
   } else {
-    const int tj = (L.jx - 1 + kDvW - 1) / kDvW;
-    const dim3 grid = L.wl_solve ? dim3((unsigned)L.n_solve, 1, 1)
-                                 : dim3((unsigned)tj, (unsigned)(L.iy - 3), (unsigned)L.nmem);
-    k_sound_solve<R><<<grid, kDvW, (size_t)kDvStages * kDvStage * sizeof(double), s>>>(
-        d, advoff, last ? 1 : 0, L.wl_solve);
+    using Sh = SolveShape<R, CW>;
+    constexpr size_t smem = (size_t)Sh::kStages * Sh::kStage * sizeof(R);
+    if constexpr (sizeof(R) == sizeof(float)) {
+      if (L.solve_df) k_solve_stream_f<R, CW, true><<<grid, CW, smem, s>>>(d, advoff, lst, L.wl_solve);
+      else k_solve_stream_f<R, CW, false><<<grid, CW, smem, s>>>(d, advoff, lst, L.wl_solve);
+    } else {
+      k_solve_stream_d<R, CW><<<grid, CW, smem, s>>>(d, advoff, lst, L.wl_solve);
+    }
   }
 }
 
@@ -1217,11 +1517,22 @@ void Launch<R>::sound_momentum(const LaunchGeom &L, const Dom<R> *d, int uvoff, 
 
 template <class R>
 cudaError_t Launch<R>::configure_sound() {
-  if constexpr (sizeof(R) == sizeof(float))
-    return cudaSuccess;  // the mixed solve uses no dynamic shared memory
-  else
-    return cudaFuncSetAttribute(k_sound_solve<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                200 * 1024);
+  // k_solve_cols holds a column of up to kMaxLevels levels in shared memory
+  const int most = (int)solve_smem<R>(kMaxLevels);
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](auto k) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  };
+  if constexpr (sizeof(R) == sizeof(float)) {
+    allow(k_solve_cols_f<R, 3, true>);
+    allow(k_solve_cols_f<R, 3, false>);
+    allow(k_solve_cols_f<R, 6, true>);
+    allow(k_solve_cols_f<R, 6, false>);
+  } else {
+    allow(k_solve_cols_d<R, 3>);
+    allow(k_solve_cols_d<R, 6>);
+  }
+  return e;
 }
 
 template struct Launch<double>;

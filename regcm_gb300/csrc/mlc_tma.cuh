@@ -27,6 +27,11 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
                "r"(bytes)
                : "memory");
 }
+// one arrival (release: this thread's earlier shared stores, and those it has
+// synchronised with, are visible to whoever sees the phase complete)
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // one tiled copy of the box at (x, y, z) of the tensor map into shared memory
 __device__ __forceinline__ void tma_load_3d(void *dst, const void *tmap, int x, int y, int z,
                                             uint64_t *bar) {
