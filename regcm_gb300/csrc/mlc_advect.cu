@@ -314,7 +314,7 @@ __device__ __forceinline__ void field_t(const Dom<R> &D, int set, int f, int adv
   }
 }
 
-template <class R>
+template <class R, int LV>
 __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -328,7 +328,7 @@ __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advof
   R *__restrict__ ux = D.ux[adv];
   R *__restrict__ vx = D.vx[adv];
   R *__restrict__ wx = D.wx[adv];
-  const Pt q_ = point_at(wi, 1, 1);
+  const Pt q_ = point_at<LV>(wi, 1, 1);
   const int j = q_.j, k0 = q_.k;
   if (k0 > g.kz) return;
   const int i = q_.i;
@@ -336,29 +336,29 @@ __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advof
   if (j > jx - 1 || i > iy - 1) return;
   const size_t ij = g.at2(j, i), PS = g.PS, S = (size_t)g.P;
 #pragma unroll
-  for (int k = k0; k < k0 + kPtLevels && k <= g.kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * PS;
     // uvstagtouvx :1535-1549
     R a;
     if (j == 1) a = R(0.5) * (u[o] + u[o + 1]);
     else if (j == jx - 1) a = R(0.5) * (u[o + 1] + u[o]);
-    else a = R(0.5625) * (u[o + 1] + u[o]) - R(0.0625) * (u[o + 2] + u[o - 1]);
+    else a = interp4<R>(u[o + 1], u[o], u[o + 2], u[o - 1]);
     ux[o] = a;
     // :1553-1566
     if (i == 1) a = R(0.5) * (v[o] + v[o + S]);
     else if (i == iy - 1) a = R(0.5) * (v[o + S] + v[o]);
-    else a = R(0.5625) * (v[o + S] + v[o]) - R(0.0625) * (v[o + 2 * S] + v[o - S]);
+    else a = interp4<R>(v[o + S], v[o], v[o + 2 * S], v[o - S]);
     vx[o] = a;
     // zstagtoh :1445-1459
     if (k == 1) a = R(0.5) * (w[o + PS] + w[o]);
     else if (k == kz) a = R(0.5) * (w[o + PS] + w[o]);
-    else a = R(0.5625) * (w[o + PS] + w[o]) - R(0.0625) * (w[o + 2 * PS] + w[o - PS]);
+    else a = interp4<R>(w[o + PS], w[o], w[o + 2 * PS], w[o - PS]);
     wx[o] = a;
     if (D.c.tke) {
       // zstagtoh(tke, tkex) (Main/mod_moloch.F90:782-784)
       const R *__restrict__ tk = D.tke;
       if (k == 1 || k == kz) a = R(0.5) * (tk[o + PS] + tk[o]);
-      else a = R(0.5625) * (tk[o + PS] + tk[o]) - R(0.0625) * (tk[o + 2 * PS] + tk[o - PS]);
+      else a = interp4<R>(tk[o + PS], tk[o], tk[o + 2 * PS], tk[o - PS]);
       D.tkex[adv][o] = a;
     }
     if constexpr (sizeof(R) == sizeof(double)) {
@@ -1052,26 +1052,26 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
 
 // Species that are not advected (ipptls = 0: qx(iqfrst:nqx)) keep their
 // values when the advected fields move to the other half of their pairs.
-template <class R>
+template <class R, int LV>
 __global__ void k_species_copy(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
   const Geom g = D.g;
-  const Pt q = point_at(wi, 1, 1);
+  const Pt q = point_at<LV>(wi, 1, 1);
   if (D.c.ipptls > 0 || q.j > g.jx - 1 || q.i > g.iy - 1 || q.k > g.kz) return;
   const int adv = (D.clk->adv_role + advoff) & 1;
   const size_t F = g.field3();
 #pragma unroll
-  for (int k = q.k; k < q.k + kPtLevels && k <= g.kz; ++k) {
+  for (int k = q.k; k < q.k + LV && k <= g.kz; ++k) {
     const size_t o = g.at(q.j, q.i, k);
     for (int n = 1; n < g.nqx; ++n) D.qx[adv ^ 1][o + (size_t)n * F] = D.qx[adv][o + (size_t)n * F];
   }
 }
 
 // :809-825
-template <class R>
+template <class R, int LV>
 __global__ void k_adv_curvature(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -1083,7 +1083,7 @@ __global__ void k_adv_curvature(const Dom<R> *__restrict__ doms, int advoff, int
   const int adv = (D.clk->adv_role + advoff) & 1;
   R *__restrict__ ux = D.ux[adv];
   R *__restrict__ vx = D.vx[adv];
-  const Pt q_ = point_at(wi, 2, 2);
+  const Pt q_ = point_at<LV>(wi, 2, 2);
   const int j = q_.j, k0 = q_.k;
   if (k0 > g.kz) return;
   const int i = q_.i;
@@ -1092,26 +1092,25 @@ __global__ void k_adv_curvature(const Dom<R> *__restrict__ doms, int advoff, int
   const R dta = pick<R>(c.dtstepa, c.dtstepaf);
   R tanx, tany;
   if (c.lrotllr) {
-    const double dlat = kDegrad * 0.5 * (sa.rlat[i - 1] + sa.rlat[i]);
-    tanx = R(sin(dlat)) * sa.msfx[ij] * R(kRearthRad);
+    tanx = R(sa.slat[i - 1]) * sa.msfx[ij] * R(kRearthRad);
     tany = tanx;
   } else {
     tanx = (sa.msfu[ij - 1] - sa.msfu[ij]) * pick<R>(c.rdx, c.rdxf);
     tany = (sa.msfv[ij - (size_t)g.P] - sa.msfv[ij]) * pick<R>(c.rdx, c.rdxf);
   }
 #pragma unroll
-  for (int k = k0; k < k0 + kPtLevels && k <= g.kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * g.PS;
     R a = ux[o];
     const R b = vx[o];
-    a = a + a * b * tanx * dta;
+    a = fma_r(mul_r(mul_r(a, b), tanx), dta, a);
     ux[o] = a;
-    vx[o] = b - a * a * tany * dta;
+    vx[o] = fma_r(-mul_r(mul_r(a, a), tany), dta, b);
   }
 }
 
 // uvxtouvstag :1477-1522 and htozstag :1461-1475
-template <class R>
+template <class R, int LV>
 __global__ void k_adv_back(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -1125,7 +1124,7 @@ __global__ void k_adv_back(const Dom<R> *__restrict__ doms, int uvoff, int advof
   R *__restrict__ u = D.u[uv];
   R *__restrict__ v = D.v[uv];
   R *__restrict__ w = D.w;
-  const Pt q_ = point_at(wi, 1, 1);
+  const Pt q_ = point_at<LV>(wi, 1, 1);
   const int j = q_.j, k0 = q_.k;
   if (k0 > g.kz) return;
   const int i = q_.i;
@@ -1136,33 +1135,33 @@ __global__ void k_adv_back(const Dom<R> *__restrict__ doms, int uvoff, int advof
   const bool do_v = (j >= 2 && j <= jx - 2 && i >= 2 && i <= iy - 1);
   const bool do_w = (j <= jx - 1 && i <= iy - 1);
 #pragma unroll
-  for (int k = k0; k < k0 + kPtLevels && k <= g.kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * PS;
     if (do_u) {
       R a;
       if (j == jx - 1) a = R(0.5) * (ux[o - 1] + ux[o]);
       else if (j == 2) a = R(0.5) * (ux[o] + ux[o - 1]);
-      else a = R(0.5625) * (ux[o] + ux[o - 1]) - R(0.0625) * (ux[o + 1] + ux[o - 2]);
+      else a = interp4<R>(ux[o], ux[o - 1], ux[o + 1], ux[o - 2]);
       u[o] = a;
     }
     if (do_v) {
       R a;
       if (i == iy - 1) a = R(0.5) * (vx[o - S] + vx[o]);
       else if (i == 2) a = R(0.5) * (vx[o] + vx[o - S]);
-      else a = R(0.5625) * (vx[o] + vx[o - S]) - R(0.0625) * (vx[o + S] + vx[o - 2 * S]);
+      else a = interp4<R>(vx[o], vx[o - S], vx[o + S], vx[o - 2 * S]);
       v[o] = a;
     }
     if (do_w && k >= 2) {
       R a;
       if (k == 2) a = R(0.5) * (wx[o] + wx[o - PS]);
       else if (k == kz) a = R(0.5) * (wx[o] + wx[o - PS]);
-      else a = R(0.5625) * (wx[o] + wx[o - PS]) - R(0.0625) * (wx[o + PS] + wx[o - 2 * PS]);
+      else a = interp4<R>(wx[o], wx[o - PS], wx[o + PS], wx[o - 2 * PS]);
       w[o] = a;
       if (D.c.tke) {
         // htozstag(tkex, tke) (Main/mod_moloch.F90:831-834)
         const R *__restrict__ tx = D.tkex[adv];
         if (k == 2 || k == kz) a = R(0.5) * (tx[o] + tx[o - PS]);
-        else a = R(0.5625) * (tx[o] + tx[o - PS]) - R(0.0625) * (tx[o + PS] + tx[o - 2 * PS]);
+        else a = interp4<R>(tx[o], tx[o - PS], tx[o + PS], tx[o - 2 * PS]);
         D.tke[o] = a;
       }
     }
@@ -1660,8 +1659,7 @@ inline dim3 pt_grid(const LaunchGeom &L, int nj, int ni, int &tiles_j) {
   tiles_j = (nj + L.col_x - 1) / L.col_x;
   if (L.wl_pt) return dim3((unsigned)L.n_pt, 1, 1);  // one block per work item
   const int ti = (ni + L.col_y - 1) / L.col_y;
-  return dim3((unsigned)(tiles_j * ti), (unsigned)((L.kz + kPtLevels - 1) / kPtLevels),
-              (unsigned)L.nmem);
+  return dim3((unsigned)(tiles_j * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
 }
 
 }  // namespace
@@ -1671,7 +1669,8 @@ void Launch<R>::adv_prep(const LaunchGeom &L, const Dom<R> *d, int uvoff, int ad
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  k_adv_prep<R><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_adv_prep<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_adv_prep<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R, class T>
@@ -1761,7 +1760,8 @@ void Launch<R>::adv_species_copy(const LaunchGeom &L, const Dom<R> *d, int advof
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  k_species_copy<R><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_species_copy<R, 1><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
+  else k_species_copy<R, 4><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1769,7 +1769,8 @@ void Launch<R>::adv_curvature(const LaunchGeom &L, const Dom<R> *d, int advoff, 
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 3, L.iy - 3, tj);
-  k_adv_curvature<R><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_adv_curvature<R, 1><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
+  else k_adv_curvature<R, 4><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1777,7 +1778,8 @@ void Launch<R>::adv_back(const LaunchGeom &L, const Dom<R> *d, int uvoff, int ad
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-  k_adv_back<R><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_adv_back<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_adv_back<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>

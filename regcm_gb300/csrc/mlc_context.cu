@@ -174,7 +174,7 @@ void carve_dom(Carver &cv, Dom<R> &D, const Geom &g, const mlc_dims &d, const ml
   s.hefc = cv.take<double>((size_t)p.nspgx * d.kz); s.fcx = cv.take<double>(p.nspgx);
   s.tnudge = cv.take<double>(d.kz); s.ffilt = cv.take<double>(d.kz); s.gzitakh = cv.take<double>(d.kz);
   s.xkdamp = cv.take<double>(d.kz); s.xknu = cv.take<double>(d.kz); s.gzitak = cv.take<double>(d.kz + 1);
-  s.rlat = cv.take<double>(d.iy);
+  s.slat = cv.take<double>(d.iy);
   if (f64) {
     s.dv_cu = cv.take<double>(F); s.dv_cv = cv.take<double>(F); s.dv_cf = cv.take<double>(F);
     s.mo_du = cv.take<double>(F); s.mo_dv = cv.take<double>(F);
@@ -350,9 +350,9 @@ struct mlc_ctx {
   WorkItem *wl_buf = nullptr;
   size_t wl_cap = 0;           // entries
   bool wl_dirty = true;        // members changed since the lists were built
-  int wl_key[7] = {-1, -1, -1, -1, -1, -1, -1};
-  const WorkItem *wl_ptr[7] = {};  // the lists in wl_buf (null: none) ...
-  int wl_n[7] = {};                // ... and their lengths
+  int wl_key[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
+  const WorkItem *wl_ptr[9] = {};  // the lists in wl_buf (null: none) ...
+  int wl_n[9] = {};                // ... and their lengths
 };
 
 namespace {
@@ -500,6 +500,13 @@ int remove_member(mlc_ctx *x, int slot) {
   return MLC_OK;
 }
 
+// Levels a thread of the point kernels runs: one while the points are few,
+// because a thread's levels wait on memory one after the other.  Step times
+// with one and four levels: mixed 64x64x30 0.166 and 0.213 ms, FP64 64x64x30
+// 0.331 and 0.369, 201x157x35 (1.1 M points) 2.72 and 2.77, 256x256x41 (2.7 M)
+// 4.36 both, 512x512x41 15.6 and 15.5; mixed 6.8 M points 3.09 and 3.01.
+int point_levels(size_t points) { return points <= (size_t)152 * 16384 ? 1 : 4; }
+
 // The form of the column solves for these members, by their 32-column row
 // segments n an SM (152).  Several warps a column while the segments are few;
 // a thread a column, streamed, once they fill the GPU.  Measured, us a launch
@@ -560,6 +567,15 @@ int refresh(mlc_ctx *x) {
   }
   L.nmem = (int)t.size();
   L.solve = solve_kind<R>(t);
+  size_t pts = 0;
+  L.frame_points = 0;
+  for (const Dom<R> &D : t) {
+    const int nx = D.g.jx - 1, ny = D.g.iy - 1, f = 2 * D.c.frame;
+    pts += (size_t)D.g.jx * D.g.iy * D.g.kz;
+    L.frame_points = std::max(L.frame_points, nx * ny - std::max(0, nx - f) * std::max(0, ny - f));
+  }
+  L.lv = point_levels(pts);
+  L.wind_rows = !x->mixed ? 0 : pts <= (size_t)256 << 10 ? 2 : 4;  // (eight and more measured slower)
   if (!t.empty()) {
     MLC_TRY(cudaMemcpyAsync(x->table, t.data(), t.size() * sizeof(Dom<R>), cudaMemcpyHostToDevice,
                             x->stream));
@@ -586,19 +602,19 @@ int ensure_lists(mlc_ctx *x) {
   bool uneven = false;
   for (const Member *m : act)
     uneven = uneven || m->g.jx != L.jx || m->g.iy != L.iy || m->g.kz != L.kz;
-  const int key[7] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, L.htile, L.solve};
+  const int key[9] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, L.htile, L.solve, L.lv, L.wind_rows};
   // the launch geometry always takes the lists from the context (a copy of
   // an older geometry may carry stale ones)
   auto apply = [&]() {
     L.wl_pt = x->wl_ptr[0]; L.wl_v4 = x->wl_ptr[1]; L.wl_solve = x->wl_ptr[2];
     L.wl_vert = x->wl_ptr[3]; L.wl_vinc = x->wl_ptr[4]; L.wl_h = x->wl_ptr[5];
-    L.wl_hinc = x->wl_ptr[6];
+    L.wl_hinc = x->wl_ptr[6]; L.wl_vec = x->wl_ptr[7]; L.wl_wind = x->wl_ptr[8];
     L.n_pt = x->wl_n[0]; L.n_v4 = x->wl_n[1]; L.n_solve = x->wl_n[2]; L.n_vert = x->wl_n[3];
-    L.n_vinc = x->wl_n[4]; L.n_h = x->wl_n[5]; L.n_hinc = x->wl_n[6];
+    L.n_vinc = x->wl_n[4]; L.n_h = x->wl_n[5]; L.n_hinc = x->wl_n[6]; L.n_vec = x->wl_n[7]; L.n_wind = x->wl_n[8];
     return MLC_OK;
   };
   if (!x->wl_dirty && std::memcmp(key, x->wl_key, sizeof(key)) == 0) return apply();
-  for (int q = 0; q < 7; ++q) {
+  for (int q = 0; q < 9; ++q) {
     x->wl_ptr[q] = nullptr;
     x->wl_n[q] = 0;
   }
@@ -615,12 +631,12 @@ int ensure_lists(mlc_ctx *x) {
   auto push = [&](int m, int a, int b, int c) {
     all.push_back(WorkItem{(int16_t)m, (int16_t)a, (int16_t)b, (int16_t)c});
   };
-  size_t off[7];
+  size_t off[9];
   // point kernels: col_x x col_y tiles over jx x iy, level chunks
   off[0] = all.size();
   for (int m = 0; m < (int)act.size(); ++m) {
     const Geom &g = act[m]->g;
-    for (int kc = 0; kc < cdiv(g.kz, kPtLevels); ++kc)
+    for (int kc = 0; kc < cdiv(g.kz, L.lv); ++kc)
       for (int bi = 0; bi < cdiv(g.iy, L.col_y); ++bi)
         for (int bj = 0; bj < cdiv(g.jx, L.col_x); ++bj) push(m, bj, bi, kc);
   }
@@ -629,7 +645,7 @@ int ensure_lists(mlc_ctx *x) {
   if (!f64)
     for (int m = 0; m < (int)act.size(); ++m) {
       const Geom &g = act[m]->g;
-      for (int kc = 0; kc < cdiv(g.kz, kPtLevels); ++kc)
+      for (int kc = 0; kc < cdiv(g.kz, L.lv); ++kc)
         for (int bi = 0; bi < cdiv(g.iy, 4); ++bi)
           for (int bj = 0; bj < cdiv(g.jx, 128); ++bj) push(m, bj, bi, kc);
     }
@@ -673,6 +689,21 @@ int ensure_lists(mlc_ctx *x) {
   htiles(hshape((int)sizeof(R), L.htile));
   off[6] = all.size();
   if (!f64) htiles(hshape_inc(L.htile));
+  // the step end: 16-byte lanes, and the winds' tiles
+  off[7] = all.size();
+  for (int m = 0; m < (int)act.size(); ++m) {
+    const Geom &g = act[m]->g;
+    for (int kc = 0; kc < cdiv(g.kz, L.lv); ++kc)
+      for (int bi = 0; bi < cdiv(g.iy - 1, 4); ++bi)
+        for (int bj = 0; bj < cdiv(g.jx - 1, f64 ? 64 : 128); ++bj) push(m, bj, bi, kc);
+  }
+  off[8] = all.size();
+  for (int m = 0; m < (int)act.size() && L.wind_rows; ++m) {
+    const Geom &g = act[m]->g;
+    for (int k = 0; k < g.kz; ++k)
+      for (int bi = 0; bi < wind_tiles_i(g.iy, L.wind_rows); ++bi)
+        for (int bj = 0; bj < wind_tiles_j(g.jx); ++bj) push(m, bj, bi, k);
+  }
   const size_t total = all.size();
   if (total > x->wl_cap) {
     if (x->wl_buf) MLC_TRY(cudaFree(x->wl_buf));
@@ -689,8 +720,8 @@ int ensure_lists(mlc_ctx *x) {
   MLC_TRY(cudaMemcpyAsync(x->wl_buf, all.data(), total * sizeof(WorkItem), cudaMemcpyHostToDevice,
                           x->stream));
   MLC_TRY(cudaStreamSynchronize(x->stream));
-  for (int q = 0; q < 7; ++q) {
-    const size_t end = q == 6 ? total : off[q + 1];
+  for (int q = 0; q < 9; ++q) {
+    const size_t end = q == 8 ? total : off[q + 1];
     x->wl_n[q] = (int)(end - off[q]);
     x->wl_ptr[q] = x->wl_n[q] ? x->wl_buf + off[q] : nullptr;
   }
@@ -781,6 +812,22 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
   if (phase != kStepFinish) {
     // the ring first: the point pass after it does tvirt, t and the relaxation
     if (x->prm.do_apply_bdy) { REC("bdy_ring", K::bdy_ring(L, d, uvo, ao, s)); ++nl; }
+    if (phase == kStepAll && !(x->prm.do_apply_bdy && x->prm.mo_spectral_nudge)) {
+      REC("end_frame", K::end_frame(L, d, uvo, ao, s)); ++nl;
+      REC("end_point", K::end_point(L, d, uvo, ao, s)); ++nl;
+      int flip = 0;
+      if (L.wind_rows) {
+        // (the winds end in the other half of their pairs)
+        REC("end_winds", K::end_winds(L, d, uvo, ao, s)); ++nl;
+        flip = 1;
+      } else {
+        REC("end_uvx", K::end_uvx(L, d, uvo, ao, s)); ++nl;
+        REC("end_uvstag", K::end_uvstag(L, d, uvo, ao, s)); ++nl;
+      }
+      if (x->key.any_tke) { REC("end_tke", K::end_tke(L, d, true, s)); ++nl; }
+      REC("end_reduce", K::end_reduce(L, d, uvo + flip, ao, true, s)); ++nl;
+      return nl;
+    }
     REC("end_relax", K::end_relax(L, d, uvo, ao, s)); ++nl;
     if (x->prm.do_apply_bdy && x->prm.mo_spectral_nudge) {
       REC("bdy_spectral", K::bdy_spectral(L, d, uvo, ao, s));
@@ -788,7 +835,7 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
     }
   }
   if (phase == kStepAll) {
-    REC("end_cross", K::end_cross(L, d, uvo, ao, s)); ++nl;
+    REC("end_cross", K::end_cross(L, d, uvo, ao, s)); nl += 2;
   } else if (phase == kStepDynamics) {
     REC("end_mkslice", K::end_cross_split(L, d, uvo, ao, false, s)); nl += 2;
     return nl;
@@ -797,7 +844,7 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
   }
   if (x->key.any_tke) { REC("end_tke", K::end_tke(L, d, phase == kStepAll, s)); ++nl; }
   REC("end_uvstag", K::end_uvstag(L, d, uvo, ao, s)); ++nl;
-  REC("end_reduce", K::end_reduce(L, d, uvo, ao, s)); ++nl;
+  REC("end_reduce", K::end_reduce(L, d, uvo, ao, false, s)); ++nl;
   return nl;
 }
 
@@ -1086,6 +1133,14 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
     return 0;
   };
   c.hb_cr = any_pos(s->ibnd_cr); c.hb_ud = any_pos(s->ibnd_ud); c.hb_vd = any_pos(s->ibnd_vd);
+  // how deep the zones lie inside the domain, in cross points
+  c.frame = 1;
+  for (int i = 1; i <= iy; ++i)
+    for (int j = 1; j <= jx; ++j) {
+      const size_t e = (size_t)(j - 1) + (size_t)(i - 1) * jx;
+      if (s->ibnd_cr[e] > 0 || s->ibnd_ud[e] > 0 || s->ibnd_vd[e] > 0)
+        c.frame = std::max(c.frame, 1 + std::max(0, std::min(std::min(j - 1, jx - 1 - j), std::min(i - 1, iy - 1 - i))));
+    }
   // the curvature terms vanish identically with uniform map factors
   {
     bool curv = p.lrotllr != 0;
@@ -1098,7 +1153,7 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
   }
   // 1-D vertical arrays, Main/mod_moloch.F90:262-300
   std::vector<double> v1(kz + 1);
-  for (int k = 1; k <= kz + 1; ++k) v1[k - 1] = gzita(s->zita[k - 1], p.mo_ztop, p.mo_a0);
+  for (int k = 1; k <= kz + 1; ++k) v1[k - 1] = -0.25 * gzita(s->zita[k - 1], p.mo_ztop, p.mo_a0);
   MLC_CHK(put1(x, v1.data(), a.gzitak, kz + 1));
   MLC_CHK(put1r<R>(x, v1.data(), a.gzitak_r, kz + 1));
   for (int k = 1; k <= kz; ++k) v1[k - 1] = gzita(s->zitah[k - 1], p.mo_ztop, p.mo_a0);
@@ -1135,7 +1190,12 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
     MLC_CHK(put1(x, s->fcx, a.fcx, p.nspgx));
     MLC_CHK(put1r<R>(x, s->fcx, a.fcx_r, p.nspgx));
   }
-  if (s->rlat) MLC_CHK(put1(x, s->rlat, a.rlat, iy));
+  if (s->rlat) {
+    // sin of the cross rows' latitude (row i between i and i+1)
+    std::vector<double> sl(iy, 0.0);
+    for (int i = 0; i + 1 < iy; ++i) sl[i] = std::sin(kDegrad * 0.5 * (s->rlat[i] + s->rlat[i + 1]));
+    MLC_CHK(put1(x, sl.data(), a.slat, iy));
+  }
   if (sizeof(R) == sizeof(double)) {
     // the acoustic substep's constant factors, in the kernels' operand order
     // (the same products the kernels formed every substep)

@@ -44,6 +44,9 @@ struct Scal {
   int spectral;             // spectral nudging on
   int km2, lm2;             // sine modes in x and y (2*km, 2*lm)
   int tke;                  // ibltyp = 2: TKE advected, bounded and updated
+  int frame;                // depth of the points the boundary treats one by one: every cross, u and v
+                            // point of a relaxation zone lies in the outermost `frame` rows or columns
+                            // of cross points (at least the ring)
   double dtrad;             // spectral nudging interval
 };
 // sine modes of spectral nudging per direction, at most
@@ -63,8 +66,8 @@ struct Stat {
   const double *hefc;      // (nspgx, kz)
   const double *fcx;       // (nspgx)
   const double *tnudge, *ffilt, *gzitakh, *xkdamp, *xknu;      // (kz), 1-based via [k-1]
-  const double *gzitak;    // (kz+1)
-  const double *rlat;      // (iy)
+  const double *gzitak;    // (kz+1): -G(zita)/4, the factor of s (Eq. 10)
+  const double *slat;      // (iy) sine of the cross rows' latitude (rotated pole)
   // the 1-D arrays, hefc, fcx and dz in the field type (aliases for FP64)
   const R *gzitak_r, *gzitakh_r, *xkdamp_r, *xknu_r, *ffilt_r, *tnudge_r, *hefc_r, *fcx_r, *dz_r;
   // a mixed member's dz - dz_r (dz as the double-float {dz_r, dz_lo}, for the
@@ -234,6 +237,62 @@ __device__ __forceinline__ R pick(double d, float f) {
   else return f;
 }
 
+// ---- FP64 arithmetic of few instructions --------------------------------------
+// GB300's FP64 units run half a lane a clock and scheduler: the FP64 kernels
+// are bound by their FP64 instruction counts.  Explicit roundings also keep
+// two kernels that evaluate one expression bit for bit alike.
+// 1/x of a positive x: the FP32 reciprocal of x's leading bits, moved between
+// the formats by integer instructions, and one third-order step
+// r0 + r0*(e + e^2), e = 1 - x*r0 (Householder's method of order two for the
+// reciprocal): with e below 2^-21 the remaining error, e^3, is below 2^-63, so
+// the result is the rounding of the last fused multiply-add (half an ulp).
+// Three FP64 instructions where the division takes six.  Outside FP32's range,
+// and for NaN, infinite, zero and negative x, the division itself.
+__device__ __forceinline__ double recip_d(double x) {
+  const unsigned h = (unsigned)__double2hiint(x);
+  if (h - 0x38200000u >= 0x47d00000u - 0x38200000u) return 1.0 / x;
+  const float xf = __uint_as_float(((h - 0x38000000u) << 3) | ((unsigned)__double2loint(x) >> 29));
+  const unsigned r = __float_as_uint(__fdividef(1.f, xf));
+  const double r0 = __hiloint2double((int)((r >> 3) + 0x38000000u), (int)(r << 29));
+  const double e = __fma_rn(-x, r0, 1.0);
+  return __fma_rn(r0, __fma_rn(e, e, e), r0);
+}
+
+// a/b: the quotient by the reciprocal, corrected once with the exact remainder
+// (Markstein, IBM J. Res. Dev. 34(1), 1990); six FP64 instructions.
+__device__ __forceinline__ double div_d(double a, double b) {
+  const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu, hb = (unsigned)__double2hiint(b);
+  if (ha - 0x10000000u >= 0x60000000u || hb - 0x38200000u >= 0x47d00000u - 0x38200000u) return a / b;
+  const double r = recip_d(b), q = __dmul_rn(a, r);
+  return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+template <class R>
+__device__ __forceinline__ R divide(R a, R b) {
+  if constexpr (sizeof(R) == sizeof(double)) return div_d(a, b);
+  else return a / b;
+}
+// a*b + c in one rounding, and a*b that no sum fuses, either type
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
+// -x/16 exactly; an FP64 normal's exponent by an integer subtraction
+__device__ __forceinline__ float neg_16th(float x) { return __fmul_rn(-0.0625f, x); }
+__device__ __forceinline__ double neg_16th(double x) {
+  const unsigned h = (unsigned)__double2hiint(x);
+  if ((h & 0x7fffffffu) - 0x00500000u >= 0x7ff00000u - 0x00500000u) return __dmul_rn(-0.0625, x);
+  return __hiloint2double((int)((h ^ 0x80000000u) - 0x00400000u), __double2loint(x));
+}
+// The interpolations between staggered and cross points: fourth order from
+// the two points either side (near a, b; far c, d), and second order at the
+// domain's edges.
+template <class R>
+__device__ __forceinline__ R interp4(R a, R b, R c, R d) {
+  return fma_r(R(0.5625), a + b, neg_16th(c + d));
+}
+template <class R>
+__device__ __forceinline__ R interp2(R a, R b) { return R(0.5) * (a + b); }
+
 // ---- double-float values of a mixed member ----------------------------------
 // theta_v, Exner, theta_v at half levels, the vertical increments of the
 // increment-form advection, cp*fmzf*dtrdz and the boundary Exner values of a
@@ -351,19 +410,14 @@ __device__ __forceinline__ WorkItem work_item(const WorkItem *wl, int tiles_j) {
 struct Pt {
   int j, i, k;
 };
-// Levels one thread of a point kernel runs (its per-thread setup - the
-// member's descriptor, roles and 2-D metric - is shared by them); grid y
-// counts chunks of this many levels and Pt::k is the chunk's first level.
-constexpr int kPtLevels = 4;
-__device__ __forceinline__ Pt point_of(int tiles_j, int j0, int i0) {
-  const int bj = (int)(blockIdx.x % (unsigned)tiles_j), bi = (int)(blockIdx.x / (unsigned)tiles_j);
-  return {bj * (int)blockDim.x + (int)threadIdx.x + j0, bi * (int)blockDim.y + (int)threadIdx.y + i0,
-          (int)blockIdx.y * kPtLevels + 1};
-}
-// the same for the tile of a work item
+// LV: levels one thread of a point kernel runs (its per-thread setup - the
+// member's descriptor, roles and 2-D metric - is shared by them): four, or one
+// where the points are too few to fill the GPU otherwise (point_levels).  Grid
+// y counts chunks of LV levels and Pt::k is the chunk's first level.
+template <int LV>
 __device__ __forceinline__ Pt point_at(const WorkItem &w, int j0, int i0) {
   return {(int)w.a * (int)blockDim.x + (int)threadIdx.x + j0,
-          (int)w.b * (int)blockDim.y + (int)threadIdx.y + i0, (int)w.c * kPtLevels + 1};
+          (int)w.b * (int)blockDim.y + (int)threadIdx.y + i0, (int)w.c * LV + 1};
 }
 
 // The state with the roles the launch works on.

@@ -18,28 +18,43 @@ namespace mlc {
 
 namespace {
 
+// 1 + ep1*qv - condensate (Main/mod_moloch.F90:1608-1648), of the species in q
+template <class R>
+__device__ __forceinline__ R qfactor_of(const R (&q)[5], int ipptls) {
+  const R f = fma_r(R(kEp1), q[0], R(1));
+  if (ipptls > 1) return f - q[1] - q[2] - q[3] - q[4];
+  if (ipptls == 1) return f - q[1];
+  return f;
+}
+// species in the factor
+__device__ __forceinline__ int qfactor_species(int ipptls) { return ipptls > 1 ? 5 : ipptls == 1 ? 2 : 1; }
 template <class R>
 __device__ __forceinline__ R qfactor(const R *qx, size_t o, size_t F, int ipptls) {
-  if (ipptls > 1) return R(1) + R(kEp1) * qx[o] - qx[o + F] - qx[o + 2 * F] - qx[o + 3 * F] - qx[o + 4 * F];
-  if (ipptls == 1) return R(1) + R(kEp1) * qx[o] - qx[o + F];
-  return R(1) + R(kEp1) * qx[o];
+  R q[5] = {};
+  const int nq = qfactor_species(ipptls);
+  for (int n = 0; n < 5; ++n)
+    if (n < nq) q[n] = qx[o + (size_t)n * F];
+  return qfactor_of<R>(q, ipptls);
 }
 // The same factor for a mixed member as the exact double-float 1 + d, with
 // only d = ep1*qv - condensate in FP32.  The step end divides t by qf and
 // multiplies by it again after the relaxation changed qv: an FP32 qf's
 // rounding (6e-8) cancels only where qv did not change, and would otherwise
 // reach theta_v in the relaxation zone every step.
-__device__ __forceinline__ F2 qfactor_df(const float *qx, size_t o, size_t F, int ipptls) {
-  float d;
-  if (ipptls > 1) d = float(kEp1) * qx[o] - qx[o + F] - qx[o + 2 * F] - qx[o + 3 * F] - qx[o + 4 * F];
-  else if (ipptls == 1) d = float(kEp1) * qx[o] - qx[o + F];
-  else d = float(kEp1) * qx[o];
+__device__ __forceinline__ F2 qfactor_df_of(const float (&q)[5], int ipptls) {
+  float d = mul_r(float(kEp1), q[0]);
+  if (ipptls > 1) d = d - q[1] - q[2] - q[3] - q[4];
+  else if (ipptls == 1) d = d - q[1];
   return fast_two_sum(1.f, d);
 }
+__device__ __forceinline__ F2 qfactor_df(const float *qx, size_t o, size_t F, int ipptls) {
+  float q[5] = {};
+  const int nq = qfactor_species(ipptls);
+  for (int n = 0; n < 5; ++n)
+    if (n < nq) q[n] = qx[o + (size_t)n * F];
+  return qfactor_df_of(q, ipptls);
+}
 
-// bdyval, MOLOCH branch (Main/mod_bdycod.F90:1631-1860).  Phase 0 does the
-// west/east columns (corners excluded), phase 1 the south/north rows
-// (corners included), which read the corner values phase 0 left.
 // Boundary blends and relaxations.  An FP64 member evaluates the reference's
 // expressions x0*b0 + x1*b1 and (1 - x)*f + x*fext.  In FP32 both carry a
 // rounding that repeats every step - 1 - x and x0 are rounded once and for
@@ -49,151 +64,128 @@ __device__ __forceinline__ F2 qfactor_df(const float *qx, size_t o, size_t F, in
 // f + x*(fext - f) round only the small correction.
 template <class R>
 __device__ __forceinline__ R bdy_blend(R x0, R x1, R b0, R b1) {
-  if constexpr (sizeof(R) == sizeof(float)) return b0 + x1 * (b1 - b0);
-  else return x0 * b0 + x1 * b1;
+  if constexpr (sizeof(R) == sizeof(float)) return fmaf(x1, b1 - b0, b0);
+  else return __fma_rn(x0, b0, __dmul_rn(x1, b1));
 }
 template <class R>
 __device__ __forceinline__ R bdy_relax_to(R f, R x, R fext) {
-  if constexpr (sizeof(R) == sizeof(float)) return f + x * (fext - f);
-  else return (R(1) - x) * f + x * fext;
+  if constexpr (sizeof(R) == sizeof(float)) return fmaf(x, fext - f, f);
+  else return __fma_rn(R(1) - x, f, __dmul_rn(x, fext));
 }
 
-// One block per level and member runs both phases, a block barrier between
-// them: everything phase 1 reads that phase 0 writes (qx, w at the level,
-// TKE one interface up, written by the same level's phase 0) lies in the
-// block's own level.
-constexpr int kRingThreads = 1024;
+// bdyval, MOLOCH branch (Main/mod_bdycod.F90:1631-1860): the west and east
+// columns (corners excluded), then the south and north rows (corners
+// included).  Species without boundary data, w and TKE take their floor on
+// inflow and the value of the point inside on outflow; for a row's first and
+// last point that is the column's new value, which the thread forms itself, so
+// every ring point is independent: one thread a point and level.  (A block a
+// level with a barrier between columns and rows took 204 us a step for 32
+// members of 128x128x30, whose 960 blocks waited on memory one after the
+// other.)
+constexpr int kRingThreads = 128;
 template <class R>
 __global__ void __launch_bounds__(kRingThreads) k_bdy_ring(const Dom<R> *__restrict__ doms, int uvoff,
                                                            int advoff) {
-  const Dom<R> &D = doms[blockIdx.y];
+  const Dom<R> &D = doms[blockIdx.z];
   if (!D.active) return;
   const Geom g = D.g;
+  const int jx = g.jx, iy = g.iy;
+  const int k = (int)blockIdx.y + 1;
+  if (k > g.kz) return;
+  const int n0 = iy - 2, n1 = jx;  // points a side: columns i = 2..iy-1, rows j = 1..jx
+  int e = (int)(blockIdx.x * kRingThreads + threadIdx.x);
+  if (e >= 2 * (n0 + n1)) return;
+  const bool column = e < 2 * n0;
+  if (!column) e -= 2 * n0;
+  const bool far = e >= (column ? n0 : n1);  // east, north
+  if (far) e -= column ? n0 : n1;
   const Scal &c = D.c;
   const Bdy<R> &bd = D.bd;
   const Clock *clk = D.clk;
   const State<R> st = state_of(D, (clk->uv_role + uvoff) & 1, (clk->adv_role + advoff) & 1);
-  const int jx = g.jx, iy = g.iy;
-  const int k = blockIdx.x + 1;
-  if (k > g.kz) return;                                  // a member with fewer levels (whole block)
   const double xb = clk->xbctime;
   const double x1 = (xb + c.dt) * c.rtb;
   const double x0 = 1.0 - x1;
-  const double cx1 = (xb + c.dt) / c.dtbdys;  // chem_bdyval_uncoupled
-  const double cx0 = 1.0 - cx1;
   const R rx0 = R(x0), rx1 = R(x1);
   const size_t PS = g.PS, F = g.field3(), ko = (size_t)(k - 1) * PS;
-  // Exner at a ring point: x0*b0 + x1*b1 (a mixed member: b0 + x1*(b1 - b0)
-  // in double-float)
-  auto set_pai_ring = [&](size_t ob) {
-    if constexpr (sizeof(R) == sizeof(float)) {
-      const DF b0(bd.xpaib[0], F), b1(bd.xpaib[1], F);
-      const F2 a = b0.ld(ob);
-      DF(st.pai, F).st(ob, df_add_f(a, float(x1) * df_diff(b1.ld(ob), a)));
-    } else {
-      st.pai[ob] = x0 * bd.xpaib[0][ob] + x1 * bd.xpaib[1][ob];
-    }
-  };
   auto blend = [&](const R *const *b, size_t o) { return bdy_blend<R>(rx0, rx1, b[0][o], b[1][o]); };
-  // t at a ring point: the blend (a mixed member: double-float, lo in wz[1])
-  auto set_t_ring = [&](size_t ob) {
-    if constexpr (sizeof(R) == sizeof(float)) {
-      const DF b0(bd.xtb[0], F), b1(bd.xtb[1], F);
-      const F2 a = b0.ld(ob);
-      const F2 t = df_add_f(a, float(x1) * df_diff(b1.ld(ob), a));
-      st.t[ob] = t.hi;
-      D.wz[1][ob] = t.lo;
-    } else {
-      st.t[ob] = x0 * bd.xtb[0][ob] + x1 * bd.xtb[1][ob];
-    }
-  };
-  const int nqx = g.nqx;
-  // side 0 = west/south, 1 = east/north; idx the position along the side
-  auto point = [&](int phase, int side, int idx) {
-  if (phase == 0) {
-    const int i = idx + 2;  // i in idi = 2..iy-1 (v), ici = 2..iy-2 (others)
-    if (i > iy - 1) return;
-    const int jb = side == 0 ? 1 : jx - 1;   // jce1 / jce2
-    const int jd = side == 0 ? 1 : jx;       // jde1 / jde2
-    const int jin = side == 0 ? 2 : jx - 2;  // jci1 / jci2
-    const size_t ob = g.at2(jb, i) + ko, od = g.at2(jd, i) + ko, oi = g.at2(jin, i) + ko;
-    st.v[ob] = blend(bd.dvb, ob);
-    if (i > iy - 2) return;
-    if (k == 1) st.ps[g.at2(jb, i)] = x0 * bd.xpsb[0][g.at2(jb, i)] + x1 * bd.xpsb[1][g.at2(jb, i)];
-    const R un = blend(bd.dub, od);
-    st.u[od] = un;
-    set_t_ring(ob);
-    set_pai_ring(ob);
-    st.qx[ob] = blend(bd.xqb, ob);
-    if (c.present_qc) st.qx[ob + F] = blend(bd.xlb, ob);
-    if (c.present_qi && c.ipptls > 1) st.qx[ob + 2 * F] = blend(bd.xib, ob);
-    const bool inflow = side == 0 ? (un > R(0)) : (un < R(0));
-    for (int n = 1; n < nqx; ++n) {
-      if ((c.present_qc && n == 1) || (c.present_qi && n == 2)) continue;
-      const size_t on = (size_t)n * F;
-      st.qx[ob + on] = inflow ? R(qx_zero(n)) : st.qx[oi + on];
-    }
-    st.w[ob] = inflow ? R(0) : st.w[oi];
-    if (c.tke) {
-      // Main/mod_bdycod.F90:1684-1695 (west), 1742-1753 (east): the floor at
-      // the top interface, below it inflow by u(k) + u(k-1) of the new ring
-      if (k == 1) {
-        st.tke[ob] = R(kTkeMin);
-      } else {
-        const R us = un + blend(bd.dub, od - PS);
-        const bool in2 = side == 0 ? (us > R(0)) : (us < R(0));
-        st.tke[ob + PS] = in2 ? R(kTkeMin) : st.tke[oi + PS];
-      }
-    }
-    for (int n = 0; n < g.ntr; ++n) {
-      const size_t on = (size_t)n * F;
-      st.trac[ob + on] = bdy_blend<R>(R(cx0), R(cx1), bd.chib[0][ob + on], bd.chib[1][ob + on]);
-    }
+  // j and i of the ring point (cross points), of the point inside it, and of
+  // the wind normal to the side (u at jn in a column, v at row in)
+  int j, i, jin, iin, jn, in;
+  if (column) {
+    i = in = iin = e + 2;
+    j = far ? jx - 1 : 1; jin = far ? jx - 2 : 2; jn = far ? jx : 1;
   } else {
-    const int j = idx + 1;  // j in jde = 1..jx (u), jce = 1..jx-1 (others)
-    if (j > jx) return;
-    const int ib = side == 0 ? 1 : iy - 1;   // ice1 / ice2
-    const int id = side == 0 ? 1 : iy;       // ide1 / ide2
-    const int iin = side == 0 ? 2 : iy - 2;  // ici1 / ici2
-    const size_t ou = g.at2(j, ib) + ko;
-    st.u[ou] = blend(bd.dub, ou);
+    j = jn = jin = e + 1;
+    i = far ? iy - 1 : 1; iin = far ? iy - 2 : 2; in = far ? iy : 1;
+  }
+  const size_t on = g.at2(jn, in) + ko;
+  // the winds along the side reach one point further than the cross points
+  if (column) {
+    st.v[g.at2(j, i) + ko] = blend(bd.dvb, g.at2(j, i) + ko);
+    if (i > iy - 2) return;
+  } else {
+    st.u[g.at2(j, i) + ko] = blend(bd.dub, g.at2(j, i) + ko);
     if (j > jx - 1) return;
-    const size_t ob = g.at2(j, ib) + ko, od = g.at2(j, id) + ko, oi = g.at2(j, iin) + ko;
-    if (k == 1) st.ps[g.at2(j, ib)] = x0 * bd.xpsb[0][g.at2(j, ib)] + x1 * bd.xpsb[1][g.at2(j, ib)];
-    const R vn = blend(bd.dvb, od);
-    st.v[od] = vn;
-    set_t_ring(ob);
-    set_pai_ring(ob);
-    st.qx[ob] = blend(bd.xqb, ob);
-    if (c.present_qc) st.qx[ob + F] = blend(bd.xlb, ob);
-    if (c.present_qi && c.ipptls > 1) st.qx[ob + 2 * F] = blend(bd.xib, ob);
-    const bool inflow = side == 0 ? (vn > R(0)) : (vn < R(0));
-    for (int n = 1; n < nqx; ++n) {
-      if ((c.present_qc && n == 1) || (c.present_qi && n == 2)) continue;
-      const size_t on = (size_t)n * F;
-      st.qx[ob + on] = inflow ? R(qx_zero(n)) : st.qx[oi + on];
-    }
-    st.w[ob] = inflow ? R(0) : st.w[oi];
-    if (c.tke) {
-      // Main/mod_bdycod.F90:1800-1811 (south), 1858-1869 (north)
-      if (k == 1) {
-        st.tke[ob] = R(kTkeMin);
-      } else {
-        const R vs = vn + blend(bd.dvb, od - PS);
-        const bool in2 = side == 0 ? (vs > R(0)) : (vs < R(0));
-        st.tke[ob + PS] = in2 ? R(kTkeMin) : st.tke[oi + PS];
-      }
-    }
-    for (int n = 0; n < g.ntr; ++n) {
-      const size_t on = (size_t)n * F;
-      st.trac[ob + on] = bdy_blend<R>(R(cx0), R(cx1), bd.chib[0][ob + on], bd.chib[1][ob + on]);
+  }
+  const R *const *nb = column ? bd.dub : bd.dvb;
+  const R wind = blend(nb, on);
+  (column ? st.u : st.v)[on] = wind;
+  const size_t ob = g.at2(j, i) + ko;
+  if (k == 1) {
+    const size_t o2 = g.at2(j, i);
+    st.ps[o2] = bdy_blend<double>(x0, x1, bd.xpsb[0][o2], bd.xpsb[1][o2]);
+  }
+  // t and Exner: x0*b0 + x1*b1 (a mixed member: b0 + x1*(b1 - b0) in
+  // double-float, the low part of t in wz[1])
+  if constexpr (sizeof(R) == sizeof(float)) {
+    const DF t0(bd.xtb[0], F), t1(bd.xtb[1], F), p0(bd.xpaib[0], F), p1(bd.xpaib[1], F);
+    const F2 a = t0.ld(ob), b = p0.ld(ob);
+    const F2 t = df_add_f(a, mul_r(float(x1), df_diff(t1.ld(ob), a)));
+    st.t[ob] = t.hi;
+    D.wz[1][ob] = t.lo;
+    DF(st.pai, F).st(ob, df_add_f(b, mul_r(float(x1), df_diff(p1.ld(ob), b))));
+  } else {
+    st.t[ob] = bdy_blend<double>(x0, x1, bd.xtb[0][ob], bd.xtb[1][ob]);
+    st.pai[ob] = bdy_blend<double>(x0, x1, bd.xpaib[0][ob], bd.xpaib[1][ob]);
+  }
+  st.qx[ob] = blend(bd.xqb, ob);
+  if (c.present_qc) st.qx[ob + F] = blend(bd.xlb, ob);
+  if (c.present_qi && c.ipptls > 1) st.qx[ob + 2 * F] = blend(bd.xib, ob);
+  // the point inside; at a row's ends a column point, whose own value is its
+  // floor or that of the point inside it
+  const bool west = !column && j == 1, east = !column && j == jx - 1;
+  const size_t oi = g.at2(west ? 2 : east ? jx - 2 : jin, iin) + ko;
+  const size_t oc = g.at2(west ? 1 : jx, iin) + ko;  // u of that column point
+  auto inflow_of = [&](R x, bool hi) { return hi ? x < R(0) : x > R(0); };
+  const bool floor1 = inflow_of(wind, far);
+  const bool floor2 = (west || east) && inflow_of(blend(bd.dub, oc), east);
+  const bool floor = floor1 || floor2;
+  for (int n = 1; n < g.nqx; ++n) {
+    if ((c.present_qc && n == 1) || (c.present_qi && n == 2)) continue;
+    const size_t of = (size_t)n * F;
+    st.qx[ob + of] = floor ? R(qx_zero(n)) : st.qx[oi + of];
+  }
+  st.w[ob] = floor ? R(0) : st.w[oi];
+  if (c.tke) {
+    // Main/mod_bdycod.F90:1684-1695, 1742-1753, 1800-1811, 1858-1869: the floor
+    // at the top interface, below it inflow by the winds of levels k and k-1
+    if (k == 1) {
+      st.tke[ob] = R(kTkeMin);
+    } else {
+      const bool f1 = inflow_of(wind + blend(nb, on - PS), far);
+      const bool f2 = (west || east) && inflow_of(blend(bd.dub, oc) + blend(bd.dub, oc - PS), east);
+      st.tke[ob + PS] = f1 || f2 ? R(kTkeMin) : st.tke[oi + PS];
     }
   }
-  };
-  const int n0 = iy - 2, n1 = jx;  // positions a side: phase 0 i = 2..iy-1, phase 1 j = 1..jx
-  for (int e = (int)threadIdx.x; e < 2 * n0; e += kRingThreads) point(0, e >= n0 ? 1 : 0, e >= n0 ? e - n0 : e);
-  __syncthreads();
-  for (int e = (int)threadIdx.x; e < 2 * n1; e += kRingThreads) point(1, e >= n1 ? 1 : 0, e >= n1 ? e - n1 : e);
+  if (g.ntr) {
+    const double cx1 = (xb + c.dt) / c.dtbdys;  // chem_bdyval_uncoupled
+    const double cx0 = 1.0 - cx1;
+    for (int n = 0; n < g.ntr; ++n) {
+      const size_t of = (size_t)n * F;
+      st.trac[ob + of] = bdy_blend<R>(R(cx0), R(cx1), bd.chib[0][ob + of], bd.chib[1][ob + of]);
+    }
+  }
 }
 
 // The step end's point pass, after the boundary ring: virtual temperature
@@ -207,7 +199,7 @@ __global__ void __launch_bounds__(kRingThreads) k_bdy_ring(const Dom<R> *__restr
 // temperature pass does not write, and it writes only ring points, where
 // this pass leaves t alone; tvirt at the ring points is recomputed by the
 // status update.  The relaxation's clock has already moved by dtsec.
-template <class R>
+template <class R, int LV>
 __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -219,7 +211,7 @@ __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advo
   const Bdy<R> &bd = D.bd;
   const Clock *clk = D.clk;
   const State<R> st = state_of(D, (clk->uv_role + uvoff) & 1, (clk->adv_role + advoff) & 1);
-  const Pt q_ = point_at(wi, 1, 1);
+  const Pt q_ = point_at<LV>(wi, 1, 1);
   const int j = q_.j, k0 = q_.k;
   if (k0 > g.kz) return;
   const int i = q_.i;
@@ -272,18 +264,12 @@ __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advo
 #pragma unroll
     for (int n = 0; n < 5; ++n) x.q[n] = n < nq ? st.qx[o + (size_t)n * F] : R(0);
   };
-  // qfactor of the loaded species, in its association
-  auto qf_of = [&](const TvIn &x) -> R {
-    if (ipp > 1) return R(1) + R(kEp1) * x.q[0] - x.q[1] - x.q[2] - x.q[3] - x.q[4];
-    if (ipp == 1) return R(1) + R(kEp1) * x.q[0] - x.q[1];
-    return R(1) + R(kEp1) * x.q[0];
-  };
   TvIn cur, nxt;
   load_in(ij + (size_t)(k0 - 1) * PS, cur);
 #pragma unroll
-  for (int k = k0; k < k0 + kPtLevels && k <= g.kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * PS;
-    if (k + 1 < k0 + kPtLevels && k + 1 <= g.kz) load_in(o + PS, nxt);
+    if (k + 1 < k0 + LV && k + 1 <= g.kz) load_in(o + PS, nxt);
     // ---- tvirt and t (every cross point; t only inside the ring) ----
     F2 tdf{0.f, 0.f};  // a mixed member's double-float t
     R tr = R(0);       // an FP64 member's t
@@ -294,18 +280,14 @@ __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advo
       const F2 tv = df_mul(F2{cur.th, cur.thl}, F2{cur.pa, cur.pal});
       st.tvirt[o] = df_f(tv);
       if (inner) {
-        float d;  // qfactor_df of the loaded species
-        if (ipp > 1) d = float(kEp1) * cur.q[0] - cur.q[1] - cur.q[2] - cur.q[3] - cur.q[4];
-        else if (ipp == 1) d = float(kEp1) * cur.q[0] - cur.q[1];
-        else d = float(kEp1) * cur.q[0];
-        tdf = df_div(tv, fast_two_sum(1.f, d));
+        tdf = df_div(tv, qfactor_df_of(cur.q, ipp));
       } else if (!c.apply_bdy) {
         D.wz[1][o] = 0.f;  // (with the boundary on, the ring wrote it)
       }
     } else {
-      const R tv = R(cur.th * cur.pa);
+      const R tv = mul_r(cur.th, cur.pa);
       st.tvirt[o] = tv;
-      if (inner) tr = tv / qf_of(cur);
+      if (inner) tr = divide<R>(tv, qfactor_of<R>(cur.q, ipp));
     }
     cur = nxt;
     // ---- motopnudge and morelax ----
@@ -338,15 +320,15 @@ __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advo
         // (1-x)*t + x*b as t + x*(b - t) on the double-float t
         const DF b0(bd.xtb[0], F), b1(bd.xtb[1], F);
         const F2 a = b0.ld(o);
-        const F2 bt = df_add_f(a, float(x1) * df_diff(b1.ld(o), a));
-        if (nud) tdf = df_add_f(tdf, xfn * df_diff(bt, tdf));
+        const F2 bt = df_add_f(a, mul_r(float(x1), df_diff(b1.ld(o), a)));
+        if (nud) tdf = df_add_f(tdf, mul_r(xfn, df_diff(bt, tdf)));
         if (ibc > 0) {
           const float xf = sa.hefc_r[(size_t)(ibc - 1) + (size_t)(k - 1) * nsp];
-          tdf = df_add_f(tdf, xf * df_diff(bt, tdf));
+          tdf = df_add_f(tdf, mul_r(xf, df_diff(bt, tdf)));
         }
       } else {
-        const double bt = x0 * bd.xtb[0][o] + x1 * bd.xtb[1][o];
-        if (nud) tr = (R(1) - xfn) * tr + xfn * R(bt);
+        const double bt = bdy_blend<double>(x0, x1, bd.xtb[0][o], bd.xtb[1][o]);
+        if (nud) tr = bdy_relax_to<R>(tr, xfn, R(bt));
         if (ibc > 0) tr = relax(tr, R(bt), ibc, k);
       }
     }
@@ -364,11 +346,10 @@ __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advo
       const float xf = sa.hefc_r[(size_t)(ibc - 1) + (size_t)(k - 1) * nsp];
       const DF pa(st.pai, F), b0(bd.xpaib[0], F), b1(bd.xpaib[1], F);
       const F2 pp = pa.ld(o), a = b0.ld(o);
-      pa.st(o, df_add_f(pp, xf * (df_diff(a, pp) + float(x1) * df_diff(b1.ld(o), a))));
+      pa.st(o, df_add_f(pp, mul_r(xf, fmaf(float(x1), df_diff(b1.ld(o), a), df_diff(a, pp)))));
     } else {
       const double xf = sa.hefc[(size_t)(ibc - 1) + (size_t)(k - 1) * nsp];
-      const double fext = x0 * bd.xpaib[0][o] + x1 * bd.xpaib[1][o];
-      st.pai[o] = (1.0 - xf) * st.pai[o] + xf * fext;
+      st.pai[o] = bdy_relax_to<double>(st.pai[o], xf, bdy_blend<double>(x0, x1, bd.xpaib[0][o], bd.xpaib[1][o]));
     }
     st.qx[o] = relax(st.qx[o], blend(bd.xqb, o), ibc, k);
     {
@@ -430,7 +411,7 @@ __device__ __forceinline__ R spec_departure(const Dom<R> &D, const State<R> &st,
       const F2 bt = df_add_f(a, float(x1) * df_diff(b1.ld(o), a));
       return df_diff(bt, F2{st.t[o], D.wz[1][o]});
     } else {
-      return (x0 * bd.xtb[0][o] + x1 * bd.xtb[1][o]) - st.t[o];
+      return bdy_blend<double>(x0, x1, bd.xtb[0][o], bd.xtb[1][o]) - st.t[o];
     }
   }
   const R *const *b = f == 1 ? bd.dub : bd.dvb;
@@ -514,8 +495,8 @@ __global__ void __launch_bounds__(256) k_spec_modes(const Dom<R> *__restrict__ d
 }
 
 // f(j,i,k) += cnudge(k) sum_m bvx(j,m) G(i,m) for t, u and v at one point
-// (j, i from 2), kPtLevels levels per thread.
-template <class R>
+// (j, i from 2), LV levels per thread.
+template <class R, int LV>
 __global__ void k_spec_apply(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -525,7 +506,7 @@ __global__ void k_spec_apply(const Dom<R> *__restrict__ doms, int uvoff, int adv
   const Clock *clk = D.clk;
   if (!spectral_due(c, clk)) return;
   const Geom g = D.g;
-  const Pt q_ = point_at(wi, 2, 2);
+  const Pt q_ = point_at<LV>(wi, 2, 2);
   const int j = q_.j, i = q_.i, k0 = q_.k;
   if (k0 > g.kz || j > g.jx - 1 || i > g.iy - 1) return;
   const State<R> st = state_of(D, (clk->uv_role + uvoff) & 1, (clk->adv_role + advoff) & 1);
@@ -540,7 +521,7 @@ __global__ void k_spec_apply(const Dom<R> *__restrict__ doms, int uvoff, int adv
   };
   const bool tp = j == 2 && i <= g.iy - 2, up = i <= g.iy - 2, vp = j <= g.jx - 2;
 #pragma unroll
-  for (int k = k0; k < k0 + kPtLevels && k <= g.kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * g.PS;
     const R cn = D.sa.cnudge[k - 1];
     if (tp) {
@@ -557,14 +538,21 @@ __global__ void k_spec_apply(const Dom<R> *__restrict__ doms, int uvoff, int adv
   }
 }
 
-// extrapolate_surface_pressure (:1592-1606) of the interior column at ij,
-// from t and q at the two lowest levels before status_update clamps q, and p
-// at the lowest level (the same expression k_end_cross stores).
+// extrapolate_surface_pressure (:1592-1606) from the virtual temperatures and
+// heights of the levels kz-1 and kz and the pressure of the lowest.
+__device__ __forceinline__ double surface_pressure(double tv1, double tv2, double z1, double z2, double p2) {
+  double lrt = div_d(tv1 - tv2, z1 - z2);
+  if (lrt < -kGovcp) lrt = -kGovcp;
+  else if (lrt > -0.005) lrt = __fma_rn(0.65, lrt, -0.35 * kLrate);
+  const double tv = __fma_rn(__dmul_rn(-lrt, 0.5), z2, tv2);
+  return __dmul_rn(p2, exp(div_d(__dmul_rn(kGovr, z2), tv)));
+}
+// The same of the interior column at ij, from t and q before status_update
+// clamps q, and p at the lowest level (the expression k_end_cross stores).
 template <class R>
 __device__ __forceinline__ void ps_column(const Dom<R> &D, const State<R> &st, size_t ij) {
   const Geom &g = D.g;
   const Scal &c = D.c;
-  const Stat<R> &sa = D.sa;
   const size_t PS = g.PS, F = g.field3();
   const int ipp = c.ipptls, kz = g.kz;
   // tvirt at kz-1, kz before the clamps: from the boundary's temp_to_tvirt,
@@ -572,8 +560,8 @@ __device__ __forceinline__ void ps_column(const Dom<R> &D, const State<R> &st, s
   const size_t o1 = ij + (size_t)(kz - 2) * PS, o2 = ij + (size_t)(kz - 1) * PS;
   double tv1, tv2;
   if (c.apply_bdy) {
-    tv1 = (double)(st.t[o1] * qfactor(st.qx, o1, F, ipp));
-    tv2 = (double)(st.t[o2] * qfactor(st.qx, o2, F, ipp));
+    tv1 = (double)mul_r(st.t[o1], qfactor(st.qx, o1, F, ipp));
+    tv2 = (double)mul_r(st.t[o2], qfactor(st.qx, o2, F, ipp));
   } else {
     tv1 = (double)st.tvirt[o1];
     tv2 = (double)st.tvirt[o2];
@@ -581,16 +569,11 @@ __device__ __forceinline__ void ps_column(const Dom<R> &D, const State<R> &st, s
   R p2;
   if constexpr (sizeof(R) == sizeof(float)) p2 = exner_to_pressure_f(df_f(DF(st.pai, F).ld(o2)));
   else p2 = (R)exner_to_pressure(st.pai[o2]);
-  const double z1 = sa.zeta[o1], z2 = sa.zeta[o2];
-  double lrt = (tv1 - tv2) / (z1 - z2);
-  if (lrt < -kGovcp) lrt = -kGovcp;
-  else if (lrt > -0.005) lrt = 0.65 * lrt - 0.35 * kLrate;
-  const double tv = tv2 - lrt * 0.5 * z2;
-  st.ps[ij] = (double)p2 * exp(kGovr * z2 / tv);
+  st.ps[ij] = surface_pressure(tv1, tv2, D.sa.zeta[o1], D.sa.zeta[o2], (double)p2);
 }
 
-// ps of every interior column, for the split step (the whole step's
-// k_end_cross forms it in the thread that owns the column's lowest levels)
+// ps of every interior column, for the split step and steps with spectral
+// nudging (the reduction forms it in the others)
 template <class R>
 __global__ void k_end_ps(const Dom<R> *__restrict__ doms, int uvoff, int advoff) {
   const Dom<R> &D = doms[blockIdx.z];
@@ -624,13 +607,52 @@ __device__ __forceinline__ bool below_pos(R q, double c) {
   }
 }
 
+// pfwsat (Share/pfwsat.inc) of FP64 fields with few FP64 instructions: the
+// range tests on the bit patterns, explicit fused multiply-adds, div_d.
+__device__ __forceinline__ double pfwsat_d(double t, double p) {
+  double td = t - kTzero;
+  const long long b = bits_of_d(td), mag = b & 0x7fffffffffffffffLL;
+  const bool num = mag <= 0x7ff0000000000000LL;
+  if (num && b < 0 && mag > __double_as_longlong(75.0)) td = -75.0;
+  if (num && b > __double_as_longlong(100.0)) td = 100.0;
+  double es;
+  if (num && b >= 0) {
+    es = __fma_rn(td, 0.209339997e-13, -0.373208410e-10);
+    es = __fma_rn(td, es, 0.892344772e-08);
+    es = __fma_rn(td, es, 0.196237241e-05);
+    es = __fma_rn(td, es, 0.305903558e-03);
+    es = __fma_rn(td, es, 0.264461437e-01);
+    es = __fma_rn(td, es, 0.143064234e+01);
+    es = __fma_rn(td, es, 0.444007856e+02);
+    es = __fma_rn(td, es, 0.611213476e+03);
+  } else {
+    es = __fma_rn(td, 0.262655803e-12, 0.149436277e-09);
+    es = __fma_rn(td, es, 0.387940929e-07);
+    es = __fma_rn(td, es, 0.602780717e-05);
+    es = __fma_rn(td, es, 0.614396778e-03);
+    es = __fma_rn(td, es, 0.420547422e-01);
+    es = __fma_rn(td, es, 0.188369801e+01);
+    es = __fma_rn(td, es, 0.503109514e+02);
+    es = __fma_rn(td, es, 0.611123516e+03);
+  }
+  // (pressures and saturation pressures are positive, so they order like
+  // their patterns; a NaN stays)
+  const double cap = __dmul_rn(0.15, p);
+  const long long be = bits_of_d(es);
+  if (be <= 0x7ff0000000000000LL && bits_of_d(cap) < be) es = cap;
+  return __dmul_rn(kEp2, div_d(es, p - es));
+}
+
+// x differs from c in its bits (-0 from 0 too), on the integer pipe
+__device__ __forceinline__ bool bits_differ(double x, double c) { return bits_of_d(x) != __double_as_longlong(c); }
+__device__ __forceinline__ bool bits_differ(float x, float c) { return __float_as_uint(x) != __float_as_uint(c); }
+
 // Cross-point work after the boundary, per point: uvstagtouvx and
 // temp_to_tvirt of boundary (:520-523), p (:348-352), the edits mkslice
 // makes to the state (Main/mod_slice.F90:136-147: qx and tracer floors),
 // then status_update (:1403-1443): tendencies, q clamps, tvirt, tetav, rho,
-// qsat.  The surface pressure is extrapolated before the clamps: in the
-// whole step by the thread holding the column's two lowest levels (chunks
-// of levels are counted from the top), in the split step by k_end_ps.
+// qsat.  The surface pressure is extrapolated before, by k_end_ps.  Whole
+// steps take k_end_point and k_end_winds instead unless they nudge spectrally.
 //   kEndAll   the whole sequence with zero tendencies (mlc_step).  rho and
 //             qsat of :348-352, and tvirt and tetav of the boundary, are
 //             recomputed from the same inputs by status_update, so they are
@@ -639,7 +661,7 @@ __device__ __forceinline__ bool below_pos(R q, double c) {
 //   kEndPost  status_update with the member's tendencies (Dom::tend).
 constexpr int kEndAll = 0, kEndPre = 1, kEndPost = 2;
 constexpr double kTracFloor = 1.0e-50;  // mkslice's tracer floor (Main/mod_slice.F90:141-147)
-template <class R, int PH>
+template <class R, int PH, int LV>
 __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -649,18 +671,14 @@ __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advo
   const Scal &c = D.c;
   const Stat<R> &sa = D.sa;
   const State<R> st = state_of(D, (D.clk->uv_role + uvoff) & 1, (D.clk->adv_role + advoff) & 1);
-  const Pt q_ = point_at(wi, 1, 1);
+  const Pt q_ = point_at<LV>(wi, 1, 1);
   const int j = q_.j, i = q_.i;
   const int jx = g.jx, iy = g.iy, kz = g.kz;
-  // level chunks counted from the top, so the chunk holding kz also holds
-  // kz-1 (the levels ps is extrapolated from)
-  const int khi = kz - (int)wi.c * kPtLevels, klo = max(1, khi - kPtLevels + 1);
-  if (j > jx - 1 || i > iy - 1 || khi < 1) return;
+  const int klo = q_.k, khi = min(kz, klo + LV - 1);
+  if (j > jx - 1 || i > iy - 1 || klo > kz) return;
   const size_t ij = g.at2(j, i), PS = g.PS, F = g.field3(), S = (size_t)g.P;
   const bool inner = j >= 2 && j <= jx - 2 && i >= 2 && i <= iy - 2;
   const int ipp = c.ipptls;
-  // the whole step: ps before this thread clamps q at kz-1, kz
-  if (PH == kEndAll && khi == kz && inner) ps_column<R>(D, st, ij);
 #pragma unroll
   for (int k = klo; k <= khi; ++k) {
   const size_t o = ij + (size_t)(k - 1) * PS;
@@ -670,11 +688,11 @@ __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advo
       R a;
       if (j == 1) a = R(0.5) * (u[o] + u[o + 1]);
       else if (j == jx - 1) a = R(0.5) * (u[o + 1] + u[o]);
-      else a = R(0.5625) * (u[o + 1] + u[o]) - R(0.0625) * (u[o + 2] + u[o - 1]);
+      else a = interp4<R>(u[o + 1], u[o], u[o + 2], u[o - 1]);
       st.ux[o] = a;
       if (i == 1) a = R(0.5) * (v[o] + v[o + S]);
       else if (i == iy - 1) a = R(0.5) * (v[o + S] + v[o]);
-      else a = R(0.5625) * (v[o + S] + v[o]) - R(0.0625) * (v[o + 2 * S] + v[o - S]);
+      else a = interp4<R>(v[o + S], v[o], v[o + 2 * S], v[o - S]);
       st.vx[o] = a;
     }
   }
@@ -688,17 +706,17 @@ __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advo
     // floors), rho and qsat of :348-352, then mkslice's floors
     const R tk = st.t[o], pk = st.p[o];
     if (c.apply_bdy) {
-      st.tvirt[o] = tk * qfactor(st.qx, o, F, ipp);
+      st.tvirt[o] = mul_r(tk, qfactor(st.qx, o, F, ipp));
       if constexpr (sizeof(R) == sizeof(float)) {
         const F2 t2{tk, D.wz[1][o]};
         DF(st.tetav, F).st(o, df_div(df_mul(t2, qfactor_df(st.qx, o, F, ipp)), DF(st.pai, F).ld(o)));
       } else {
-        st.tetav[o] = (double)st.tvirt[o] / st.pai[o];
+        st.tetav[o] = div_d((double)st.tvirt[o], st.pai[o]);
       }
     }
-    st.rho[o] = pk / (R(kRgas) * tk);
+    st.rho[o] = divide<R>(pk, mul_r(R(kRgas), tk));
     if constexpr (sizeof(R) == sizeof(float)) st.qsat[o] = pfwsat_f(tk, pk);
-    else st.qsat[o] = (R)pfwsat((double)tk, (double)pk);
+    else st.qsat[o] = (R)pfwsat_d((double)tk, (double)pk);
     if (inner) {
       for (int n = 0; n < g.nqx; ++n) {
         const size_t on = o + (size_t)n * F;
@@ -755,10 +773,10 @@ __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advo
     }
     const R tk = st.t[o];
     const R qf = qfactor(st.qx, o, F, ipp);
-    const R tv = tk * qf;
+    const R tv = mul_r(tk, qf);
     st.tvirt[o] = tv;
     const R pk = st.p[o];
-    st.rho[o] = pk / (R(kRgas) * tk);
+    st.rho[o] = divide<R>(pk, mul_r(R(kRgas), tk));
     if constexpr (sizeof(R) == sizeof(float)) {
       // theta_v = tvirt/pai from the double-float t (Main/mod_moloch.F90:1403-1443):
       // where nothing relaxed t, t*qf/pai gives back theta_v to ~1e-14
@@ -766,186 +784,576 @@ __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advo
       DF(st.tetav, F).st(o, df_div(df_mul(t2, qfactor_df(st.qx, o, F, ipp)), DF(st.pai, F).ld(o)));
       st.qsat[o] = pfwsat_f(tk, pk);
     } else {
-      st.tetav[o] = (double)tv / st.pai[o];
-      st.qsat[o] = (R)pfwsat((double)tk, (double)pk);
+      st.tetav[o] = div_d((double)tv, st.pai[o]);
+      st.qsat[o] = (R)pfwsat_d((double)tk, (double)pk);
     }
   }
   }
 }
 
-// 16 bytes at p (16-byte aligned) as 4 floats; a float4 store
-__device__ __forceinline__ void ld4f(float (&x)[4], const float *p) {
-  const float4 v = *reinterpret_cast<const float4 *>(p);
-  x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+// V elements at p in one access (4 to 16 bytes, aligned), and back where ok
+template <class R, int V>
+__device__ __forceinline__ void ldv(R (&x)[V], const R *p) {
+  if constexpr (V == 1) {
+    x[0] = *p;
+  } else {
+    static_assert(V * sizeof(R) == 16, "16-byte lanes");
+    const uint4 w = *reinterpret_cast<const uint4 *>(p);
+    memcpy(x, &w, 16);
+  }
 }
-__device__ __forceinline__ void st4f(float *p, const float (&x)[4]) {
-  *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
+template <class R, int V>
+__device__ __forceinline__ void stv(R *p, const R (&x)[V], const bool (&ok)[V], bool all) {
+  if (V > 1 && all) {
+    uint4 w;
+    memcpy(&w, x, 16);
+    *reinterpret_cast<uint4 *>(p) = w;
+  } else {
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+      if (ok[q]) p[q] = x[q];
+  }
 }
 
-// k_end_cross of a mixed member with lanes of four consecutive columns
-// (16-byte loads and stores; the same expressions): ux, vx, p, the
-// status_update clamps, tvirt, rho, theta_v (double-float) and qsat.  A block
-// is 32 lanes x 4 rows; grid x = 128-column tiles times row tiles, y = level
-// chunks, z = member.
+// A whole step's pointwise end in one pass (steps that nudge spectrally take
+// k_end_relax and k_end_cross): virtual temperature and temperature of
+// dynamical_core :1121-1123, motopnudge (Main/mod_bdycod.F90:4049-4083) and
+// morelax on every field (boundary, Main/mod_moloch.F90:478-497), p
+// (:348-352), mkslice's floors and status_update with zero tendencies
+// (:1403-1443), rho and qsat; the virtual temperatures that ps is extrapolated
+// from go to the scratch plane wz[0].
+//
+// Two launches share the points.  FRAME: the ring and the relaxation zone
+// (Scal::frame points deep), a point a thread.  Else the points inside it,
+// lanes of 16 bytes of a row (two FP64 or four FP32 columns), where a level is
+// nudged as a whole or not at all and no lane leaves the common path; with the
+// zone's code in the same warps every row of a 128-column domain ran it four
+// columns at a time (1000 us a step for 32 members of 128x128x30; 483 now, the
+// passes before it 819).  Seven and ten blocks an SM: measured best of three to
+// twelve, by up to a quarter.
+// Bound by the FP64 pipe or, mixed, by memory: 56 bytes a point at five
+// species, where the passes it replaces moved 140 (t and its low part,
+// theta_v, Exner and the species went through memory between them).
+// Mixed: where nothing changed t or the species of its factor, theta_v is what
+// it was and is left alone.  FP64 forms t*qf/pai everywhere, as the split step
+// does (the two are bit for bit equal).
+// us a step, this pass and k_end_winds against k_end_relax, k_end_cross and
+// k_end_uvstag: mixed 512x512x41 258 against 546, 12 uneven domains 325 against
+// 619; FP64 512x512x41 1765 (with k_end_uvx and k_end_uvstag) against 2180.
+template <class R, int LV, bool FRAME>
+__global__ void __launch_bounds__(128, FRAME ? 10 : 7) k_end_point(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
+                                                   int tiles_j, const WorkItem *__restrict__ wl) {
+  constexpr int V = FRAME ? 1 : 16 / (int)sizeof(R);
+  constexpr bool mixed = sizeof(R) == sizeof(float);
+  const WorkItem wi = FRAME ? WorkItem{(int16_t)blockIdx.z, 0, 0, (int16_t)blockIdx.y} : work_item(wl, tiles_j);
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const Geom g = D.g;
+  const Scal &c = D.c;
+  const int jx = g.jx, iy = g.iy, kz = g.kz, fr = c.frame;
+  const int k0 = (int)wi.c * LV + 1;
+  if (k0 > kz) return;
+  int e0, i;  // 0-based first column, row
+  if constexpr (FRAME) {
+    // the south and north rows of the frame, then its columns between them
+    const int nx = jx - 1, ny = iy - 1;
+    const int s = min(fr, ny), n = min(fr, ny - s), w = min(fr, nx), we = w + min(fr, nx - w);
+    int e = (int)(blockIdx.x * 128u + threadIdx.x);
+    if (e < (s + n) * nx) {
+      const int r = e / nx;
+      e0 = e - r * nx;
+      i = r < s ? r + 1 : ny - (r - s);
+    } else {
+      e -= (s + n) * nx;
+      const int r = e / we, q = e - r * we;
+      if (r >= ny - s - n) return;
+      i = s + 1 + r;
+      e0 = q < w ? q : nx - we + q;
+    }
+  } else {
+    e0 = ((int)wi.a * 32 + (int)(threadIdx.x & 31u)) * V;
+    i = (int)wi.b * 4 + (int)(threadIdx.x >> 5) + 1;
+    if (e0 + V - 1 < fr || e0 > jx - 2 - fr || i <= fr || i > iy - 1 - fr) return;
+  }
+  const Stat<R> &sa = D.sa;
+  const Bdy<R> &bd = D.bd;
+  const Clock *clk = D.clk;
+  const State<R> st = state_of(D, (clk->uv_role + uvoff) & 1, (clk->adv_role + advoff) & 1);
+  const size_t F = g.field3();
+  const unsigned PS = (unsigned)g.PS, ij = (unsigned)e0 + (unsigned)(i - 1) * (unsigned)g.P;
+  const R *__restrict__ th_p = reinterpret_cast<const R *>(st.tetav);
+  const R *__restrict__ pa_p = reinterpret_cast<const R *>(st.pai);
+  R *__restrict__ qx = st.qx;
+  const bool bdy = c.apply_bdy != 0;
+  // the lane's own columns, and in the frame whether its point is inside the
+  // ring and its zone as a cross, u and v point (0: not in the zone, -2: no
+  // point that the boundary changes)
+  bool has[V], all = true;
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    has[e] = FRAME || (e0 + e >= fr && e0 + e <= jx - 2 - fr);
+    all = all && has[e];
+  }
+  bool inner = true;
+  int ibc = 0, ibu = 0, ibv = 0;
+  if constexpr (FRAME) {
+    const int j = e0 + 1;
+    inner = j >= 2 && j <= jx - 2 && i >= 2 && i <= iy - 2;
+    ibc = bdy && inner ? sa.ibnd_cr[ij] : -2;
+    ibu = bdy && j >= 2 && i >= 2 && i <= iy - 2 ? sa.ibnd_ud[ij] : -2;
+    ibv = bdy && j >= 2 && i >= 2 && j <= jx - 2 ? sa.ibnd_vd[ij] : -2;
+  }
+  const bool zone = ibc > 0 || ibu > 0 || ibv > 0;
+  const int ipp = c.ipptls, nq = qfactor_species(ipp), nztop = bdy && c.top_nudge ? c.nztop : 0;
+  // the boundary clock has moved by dtsec (Main/mod_bdycod.F90:2653)
+  double x0 = 0.0, x1 = 0.0, cx0 = 0.0, cx1 = 0.0;
+  if (zone || k0 <= nztop) {
+    const double xb = clk->xbctime + c.dtsec;
+    x1 = (xb + c.dt) * c.rtb;
+    x0 = 1.0 - x1;
+    if (FRAME && g.ntr) {
+      cx1 = (xb + c.dt) / c.dtbdys;
+      cx0 = 1.0 - cx1;
+    }
+  }
+  const R rx0 = R(x0), rx1 = R(x1);
+  constexpr double trtau = 1.0 / (2.0 * 3600.0), wrtau = 1.0 / (3600.0 / 4.0);
+#pragma unroll 1
+  for (int k = k0; k < k0 + LV && k <= kz; ++k) {
+    const unsigned o = ij + (unsigned)(k - 1) * PS;
+    R th[V], pa[V], thl[V], pal[V], q[5][V];
+    ldv<R, V>(th, th_p + o);
+    ldv<R, V>(pa, pa_p + o);
+    if constexpr (mixed) {
+      ldv<R, V>(thl, th_p + F + o);
+      ldv<R, V>(pal, pa_p + F + o);
+    }
+#pragma unroll
+    for (int n = 0; n < 5; ++n)
+      if (n < nq) ldv<R, V>(q[n], qx + o + (size_t)n * F);
+      else
+#pragma unroll
+        for (int e = 0; e < V; ++e) q[n][e] = R(0);
+    auto species = [&](int e, R (&x)[5]) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) x[n] = q[n][e];
+    };
+    // ---- tvirt and t (t of the ring is the boundary's) ----
+    R t[V], tl[V], tv[V], qf[V];  // FP64: t, theta_v*pai, the factor; mixed: t and its low part, theta_v*pai
+    bool chg[V];                  // theta_v is formed anew
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      R x[5];
+      species(e, x);
+      chg[e] = !inner;
+      if constexpr (mixed) {
+        const F2 v2 = df_mul(F2{th[e], thl[e]}, F2{pa[e], pal[e]});
+        const F2 t2 = inner ? df_div(v2, qfactor_df_of(x, ipp)) : F2{st.t[o], bdy ? D.wz[1][o] : 0.f};
+        t[e] = t2.hi;
+        tl[e] = t2.lo;
+        tv[e] = df_f(v2);
+      } else {
+        tv[e] = mul_r(th[e], pa[e]);
+        qf[e] = qfactor_of<R>(x, ipp);
+        t[e] = inner ? divide<R>(tv[e], qf[e]) : st.t[o];
+      }
+    }
+    // ---- motopnudge and morelax ----
+    const bool nud = k <= nztop;
+    R xfn = R(0);
+    if (nud) {
+      if constexpr (mixed) xfn = mul_r(sa.tnudge_r[k - 1], float(trtau * c.dtsec));
+      else xfn = sa.tnudge[k - 1] * trtau * c.dtsec;
+    }
+    if (k == 2 && bdy && c.top_nudge && inner) {  // w sponge, before the level's relaxation
+      const R xf = R(wrtau * c.dtsec);
+      R w2[V];
+      ldv<R, V>(w2, st.w + o);
+#pragma unroll
+      for (int e = 0; e < V; ++e) w2[e] = bdy_relax_to<R>(w2[e], xf, R(0) * w2[e]);
+      stv<R, V>(st.w + o, w2, has, all);
+    }
+    if (nud || zone) {
+      const R *hefc = sa.hefc_r + (size_t)(k - 1) * c.nspgx - 1;  // hefc[zone]
+      // nudged, then relaxed in the zone
+      auto wind = [&](R *f, const R *const *b, int ib) {
+        if (ib == -2 || !(nud || ib > 0)) return;
+        R x[V], b0[V], b1[V];
+        ldv<R, V>(x, f + o);
+        ldv<R, V>(b0, b[0] + o);
+        ldv<R, V>(b1, b[1] + o);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const R ext = bdy_blend<R>(rx0, rx1, b0[e], b1[e]);
+          if (nud) x[e] = bdy_relax_to<R>(x[e], xfn, ext);
+          if (FRAME && ib > 0) x[e] = bdy_relax_to<R>(x[e], hefc[ib], ext);
+        }
+        stv<R, V>(f + o, x, has, all);
+      };
+      wind(st.u, bd.dub, ibu);
+      wind(st.v, bd.dvb, ibv);
+      if (ibc != -2 && (nud || ibc > 0)) {
+        const R *b0p = reinterpret_cast<const R *>(bd.xtb[0]), *b1p = reinterpret_cast<const R *>(bd.xtb[1]);
+        R b0[V], b1[V], b0l[V], b1l[V];
+        ldv<R, V>(b0, b0p + o);
+        ldv<R, V>(b1, b1p + o);
+        if constexpr (mixed) {
+          ldv<R, V>(b0l, b0p + F + o);
+          ldv<R, V>(b1l, b1p + F + o);
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          chg[e] = true;
+          if constexpr (mixed) {
+            // (1-x)*t + x*b as t + x*(b - t) on the double-float t
+            const F2 a{b0[e], b0l[e]};
+            const F2 bt = df_add_f(a, mul_r(float(x1), df_diff(F2{b1[e], b1l[e]}, a)));
+            F2 t2{t[e], tl[e]};
+            if (nud) t2 = df_add_f(t2, mul_r(xfn, df_diff(bt, t2)));
+            if (FRAME && ibc > 0) t2 = df_add_f(t2, mul_r(hefc[ibc], df_diff(bt, t2)));
+            t[e] = t2.hi;
+            tl[e] = t2.lo;
+          } else {
+            const double bt = bdy_blend<double>(x0, x1, b0[e], b1[e]);
+            if (nud) t[e] = bdy_relax_to<R>(t[e], xfn, bt);
+            if (FRAME && ibc > 0) t[e] = bdy_relax_to<R>(t[e], hefc[ibc], bt);
+          }
+        }
+      }
+      if constexpr (FRAME) {
+        if (ibc > 0) {
+          const R xf = hefc[ibc];
+          auto blend = [&](const R *const *b, size_t at) { return bdy_blend<R>(rx0, rx1, b[0][at], b[1][at]); };
+          if constexpr (mixed) {
+            const DF b0(bd.xpaib[0], F), b1(bd.xpaib[1], F);
+            const F2 pp{pa[0], pal[0]}, a = b0.ld(o);
+            const F2 pn = df_add_f(pp, mul_r(xf, fmaf(float(x1), df_diff(b1.ld(o), a), df_diff(a, pp))));
+            DF(st.pai, F).st(o, pn);
+            pa[0] = pn.hi;
+            pal[0] = pn.lo;
+          } else {
+            pa[0] = bdy_relax_to<double>(pa[0], xf, bdy_blend<double>(x0, x1, bd.xpaib[0][o], bd.xpaib[1][o]));
+            st.pai[o] = pa[0];
+          }
+          q[0][0] = bdy_relax_to<R>(q[0][0], xf, blend(bd.xqb, o));
+          qx[o] = q[0][0];
+          {
+            // morelax_fraction with frac = 0 (:3962-3993)
+            const R f = st.w[o];
+            st.w[o] = bdy_relax_to<R>(f, xf, f * R(0));
+          }
+          if (ipp > 0 && c.present_qc) {
+            q[1][0] = bdy_relax_to<R>(q[1][0], xf, blend(bd.xlb, o));
+            qx[o + F] = q[1][0];
+          }
+          if (ipp > 1 && c.present_qi) {
+            q[2][0] = bdy_relax_to<R>(q[2][0], xf, blend(bd.xib, o));
+            qx[o + 2 * F] = q[2][0];
+          }
+          for (int n = 0; n < g.ntr; ++n) {
+            const size_t on = o + (size_t)n * F;
+            st.trac[on] = bdy_relax_to<R>(st.trac[on], sa.fcx_r[ibc - 1],
+                                          bdy_blend<R>(R(cx0), R(cx1), bd.chib[0][on], bd.chib[1][on]));
+          }
+          if constexpr (!mixed) {
+            R x[5];
+            species(0, x);
+            qf[0] = qfactor_of<R>(x, ipp);
+          }
+        }
+      }
+    }
+    // ---- the virtual temperatures of ps, before the clamps ----
+    if (k >= kz - 1) {
+      R x2[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        x2[e] = tv[e];
+        if constexpr (mixed) {
+          if (bdy && chg[e]) {
+            R x[5];
+            species(e, x);
+            x2[e] = mul_r(t[e], qfactor_of<R>(x, ipp));
+          }
+        } else {
+          if (bdy) x2[e] = mul_r(t[e], qf[e]);
+        }
+      }
+      stv<R, V>(D.wz[0] + o, x2, has, all);
+    }
+    // ---- mkslice's floors, then status_update's clamps with zero tendencies,
+    // one clamp (see k_end_cross); the ring keeps its values ----
+    if (inner) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        if (n >= nq) break;
+        bool ch = false;
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          // (a value that is its floor already changes nothing)
+          if (has[e] && below_pos<R>(q[n][e], qx_check(n)) && bits_differ(q[n][e], R(qx_zero(n)))) {
+            q[n][e] = R(qx_zero(n));
+            chg[e] = ch = true;
+          }
+        if (ch) stv<R, V>(qx + o + (size_t)n * F, q[n], has, all);
+      }
+      for (int n = nq; n < g.nqx; ++n) {
+        R x[V];
+        bool ch = false;
+        ldv<R, V>(x, qx + o + (size_t)n * F);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (has[e] && below_pos<R>(x[e], qx_check(n)) && bits_differ(x[e], R(qx_zero(n)))) {
+            x[e] = R(qx_zero(n));
+            ch = true;
+          }
+        if (ch) stv<R, V>(qx + o + (size_t)n * F, x, has, all);
+      }
+      for (int n = 0; n < g.ntr; ++n) {
+        R x[V];
+        bool ch = false;
+        ldv<R, V>(x, st.trac + o + (size_t)n * F);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          // FP32 holds nothing between zero and the floor
+          const bool low = mixed ? x[e] <= R(0) : below_pos<double>((double)x[e], kTracFloor);
+          if (has[e] && low && bits_differ(x[e], R(0))) {
+            x[e] = R(0);
+            ch = true;
+          }
+        }
+        if (ch) stv<R, V>(st.trac + o + (size_t)n * F, x, has, all);
+      }
+    }
+    // ---- diagnostics and theta_v ----
+    R pp[V], rh[V], qs[V], thn[V], thn_l[V];
+    bool any = false;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      R x[5];
+      species(e, x);
+      any = any || chg[e];
+      if constexpr (mixed) {
+        pp[e] = exner_to_pressure_f(pa[e] + pal[e]);
+        thn[e] = th[e];
+        thn_l[e] = thl[e];
+        if (chg[e]) {
+          const F2 v2 = df_mul(F2{t[e], tl[e]}, qfactor_df_of(x, ipp));
+          const F2 t2 = df_div(v2, F2{pa[e], pal[e]});
+          tv[e] = mul_r(t[e], qfactor_of<R>(x, ipp));
+          thn[e] = t2.hi;
+          thn_l[e] = t2.lo;
+        }
+        qs[e] = pfwsat_f(t[e], pp[e]);
+      } else {
+        pp[e] = exner_to_pressure(pa[e]);
+        if (chg[e]) qf[e] = qfactor_of<R>(x, ipp);
+        tv[e] = mul_r(t[e], qf[e]);
+        thn[e] = div_d(tv[e], pa[e]);
+        qs[e] = pfwsat_d(t[e], pp[e]);
+      }
+      rh[e] = divide<R>(pp[e], mul_r(R(kRgas), t[e]));
+    }
+    if (inner) stv<R, V>(st.t + o, t, has, all);
+    stv<R, V>(st.tvirt + o, tv, has, all);
+    stv<R, V>(st.p + o, pp, has, all);
+    stv<R, V>(st.rho + o, rh, has, all);
+    stv<R, V>(st.qsat + o, qs, has, all);
+    if (!mixed || any) {
+      R *th_o = reinterpret_cast<R *>(st.tetav);
+      stv<R, V>(th_o + o, thn, has, all);
+      if constexpr (mixed) stv<R, V>(th_o + F + o, thn_l, has, all);
+    }
+  }
+}
+
+// A whole step's winds at its end: ux, vx from the relaxed u, v (boundary
+// :520-523, uvstagtouvx :1535-1566; the advected ux, vx with the boundary off)
+// and u, v from them (uvxtouvstag, status_update :1440).  The new winds go to
+// the other half of their pairs, because the stencils of other tiles still
+// read the old ones.  A warp marches `rows` rows along i, holding four rows of
+// v and of vx in registers; a lane holds four columns, whose neighbours along
+// j come by shuffles, so a warp's 128 columns write the middle 120.  Each
+// field is read and written once, a row ahead of its use.  Bound by memory: 67
+// us at 512x512x41 (24 bytes a point: 38), 120 as two point passes.  FP64
+// members keep the two passes (k_end_uvx, k_end_uvstag): their arithmetic is
+// the bound there, and this form does a fifth more of it for its halo (503
+// against 383 us).
 template <class R>
-__global__ void __launch_bounds__(128) k_end_cross_v4(const Dom<R> *__restrict__ doms, int uvoff,
-                                                      int advoff, int tiles_j,
-    const WorkItem *__restrict__ wl) {
+__global__ void __launch_bounds__(32 * kWindWarps) k_end_winds(const Dom<R> *__restrict__ doms, int uvoff,
+                                                               int advoff, int rows, int tiles_j,
+                                                               const WorkItem *__restrict__ wl) {
+  constexpr int V = 4;
   static_assert(sizeof(R) == sizeof(float), "FP32 fields");
+  static_assert(kWindCols == 32 * V - 8, "a lane either side is halo");
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
   const Geom g = D.g;
-  const int jx = g.jx, iy = g.iy, kz = g.kz;
-  const int bj = wi.a, bi = wi.b;
-  const int e0 = (bj * 32 + (int)threadIdx.x) * 4;
-  const int i = bi * (int)blockDim.y + (int)threadIdx.y + 1;
-  // level chunks counted from the top (the chunk holding kz holds kz-1)
-  const int khi = kz - (int)wi.c * kPtLevels, klo = max(1, khi - kPtLevels + 1);
-  if (e0 + 1 > jx - 1 || i > iy - 1 || khi < 1) return;
-  const Scal &c = D.c;
-  const State<R> st = state_of(D, (D.clk->uv_role + uvoff) & 1, (D.clk->adv_role + advoff) & 1);
-  const float *__restrict__ u = st.u;
-  const float *__restrict__ v = st.v;
-  float *__restrict__ ux = st.ux;
-  float *__restrict__ vx = st.vx;
-  float *__restrict__ pp = st.p;
-  float *__restrict__ tt = st.t;
-  float *__restrict__ tvir = st.tvirt;
-  float *__restrict__ rho = st.rho;
-  float *__restrict__ qsat = st.qsat;
-  float *__restrict__ qx = st.qx;
-  float *__restrict__ trac = st.trac;
-  const float *__restrict__ tlo = D.wz[1];
-  const size_t F = g.field3();
-  float *__restrict__ pa_h = reinterpret_cast<float *>(st.pai);
-  float *__restrict__ th_h = reinterpret_cast<float *>(st.tetav);
-  const unsigned P = (unsigned)g.P, PS = (unsigned)g.PS;
-  const unsigned ij = (unsigned)e0 + (unsigned)(i - 1) * P;
-  const int ipp = c.ipptls;
-  bool has[4], inner[4];
-  bool all = true;
-  int nvalid = 0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int j = e0 + q + 1;
-    has[q] = j <= jx - 1;
-    inner[q] = j >= 2 && j <= jx - 2 && i >= 2 && i <= iy - 2;
-    all = all && has[q];
-    nvalid += has[q] ? 1 : 0;
-  }
-  const bool any_inner = inner[0] || inner[1] || inner[2] || inner[3];
-  auto store = [&](float *dst, const float (&x)[4]) {
-    if (all) {
-      st4f(dst, x);
+  const int jx = g.jx, iy = g.iy, k = (int)wi.c + 1;
+  if (k > g.kz) return;
+  const int lane = (int)threadIdx.x & 31;
+  const int i0 = ((int)wi.b * kWindWarps + ((int)threadIdx.x >> 5)) * rows + 1;
+  if (i0 > iy) return;  // (a warp)
+  const int i1 = min(i0 + rows - 1, iy);
+  const int e0 = (int)wi.a * kWindCols - V + V * lane;
+  const bool inrow = e0 >= 0 && e0 + V <= g.P, wr = inrow && lane >= 1 && lane <= 30 && e0 < jx;
+  const bool ends = e0 <= 1 || e0 + V >= jx - 1;  // the lane holds columns near the domain's first or last
+  const bool bdy = D.c.apply_bdy != 0;
+  const int uv = (D.clk->uv_role + uvoff) & 1, adv = (D.clk->adv_role + advoff) & 1;
+  const unsigned ko = (unsigned)(k - 1) * (unsigned)g.PS, P = (unsigned)g.P;
+  const R *__restrict__ u_in = D.u[uv] + ko;
+  const R *__restrict__ v_in = D.v[uv] + ko;
+  R *__restrict__ u_out = D.u[uv ^ 1] + ko;
+  R *__restrict__ v_out = D.v[uv ^ 1] + ko;
+  R *ux = D.ux[adv] + ko;
+  R *vx = D.vx[adv] + ko;
+  auto load = [&](R (&x)[V], const R *p, int r, int rmax) {
+    if (inrow && r >= 1 && r <= rmax) {
+      ldv<R, V>(x, p + (unsigned)e0 + (unsigned)(r - 1) * P);
     } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (has[q]) dst[q] = x[q];
+      for (int q = 0; q < V; ++q) x[q] = R(0);
     }
   };
-  // ps of the lane's interior columns before this thread clamps q at kz-1, kz
-  if (khi == kz)
+  // (the columns past a field's last lie in the row's padding)
+  auto store = [&](R *p, int r, const R (&x)[V]) {
+    if (!wr) return;
+    *reinterpret_cast<float4 *>(p + (unsigned)e0 + (unsigned)(r - 1) * P) = make_float4(x[0], x[1], x[2], x[3]);
+  };
+  const unsigned full = 0xffffffffu;
+  auto pick4 = [](const R (&n)[V + 3], int lo, int q) {  // n[lo + q], q in 0 .. 3
+    return q == 0 ? n[lo] : q == 1 ? n[lo + 1] : q == 2 ? n[lo + 2] : n[lo + 3];
+  };
+  // rows r-1 .. r+2 of v, and r-3 .. r-1 of vx
+  R va[V], vb[V], vc[V], vd[V], xa[V], xb[V], xc[V];
+  // the next rows of v and u, loaded a row ahead
+  R vn[V], un[V];
+  load(va, v_in, i0 - 3, iy);
+  load(vb, v_in, i0 - 2, iy);
+  load(vc, v_in, i0 - 1, iy);
+  load(vn, v_in, i0, iy);
+  load(un, u_in, i0, iy - 1);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (inner[q]) ps_column<R>(D, st, (size_t)ij + (size_t)q);
-  for (int k = klo; k <= khi; ++k) {
-    const unsigned o = ij + (unsigned)(k - 1) * PS;
-    if (c.apply_bdy) {
-      // u at j-1 .. j+2 and v at rows i-1 .. i+2 (:1535-1566)
-      float uc[4], ue1 = 0.f, ue2 = 0.f, uw = 0.f;
-      ld4f(uc, u + o);
-      if (e0 >= 1) uw = u[o - 1];
-      if (nvalid == 4) ue1 = u[o + 4];          // j+1 of the last column (<= jx)
-      if (e0 + 4 <= jx - 2) ue2 = u[o + 5];     // j+2 of the last column
-      const float un[6] = {uw, uc[0], uc[1], uc[2], uc[3], ue1};  // u at j-1 .. j+4 of column 0
-      float a[4];
+  for (int q = 0; q < V; ++q) xa[q] = xb[q] = xc[q] = R(0);
+  for (int r = i0 - 2; r <= i1 + 1; ++r) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = e0 + q + 1;
-        const float u0 = un[q + 1], u1 = un[q + 2], um = un[q];
-        const float u2 = q < 3 ? un[q + 3] : ue2;
-        if (j == 1) a[q] = 0.5f * (u0 + u1);
-        else if (j == jx - 1) a[q] = 0.5f * (u1 + u0);
-        else a[q] = 0.5625f * (u1 + u0) - 0.0625f * (u2 + um);
-      }
-      store(ux + o, a);
-      float vc[4], vn[4], vs[4] = {0.f, 0.f, 0.f, 0.f}, vnn[4] = {0.f, 0.f, 0.f, 0.f};
-      ld4f(vc, v + o);
-      ld4f(vn, v + o + P);
-      if (i >= 2 && i <= iy - 2) {
-        ld4f(vs, v + o - P);
-        ld4f(vnn, v + o + 2 * P);
-      }
+    for (int q = 0; q < V; ++q) vd[q] = vn[q];
+    load(vn, v_in, r + 3, r < i1 + 1 ? iy : 0);
+    // vx of row r
+    R x[V];
+    if (!bdy) {
+      load(x, vx, r, iy - 1);
+    } else {
+      if (r == 1 || r == iy - 1) {  // (a warp)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (i == 1) a[q] = 0.5f * (vc[q] + vn[q]);
-        else if (i == iy - 1) a[q] = 0.5f * (vn[q] + vc[q]);
-        else a[q] = 0.5625f * (vn[q] + vc[q]) - 0.0625f * (vnn[q] + vs[q]);
+        for (int q = 0; q < V; ++q) x[q] = interp2<R>(vb[q], vc[q]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q) x[q] = interp4<R>(vc[q], vb[q], vd[q], va[q]);
       }
-      store(vx + o, a);
+      if (r >= i0 && r <= i1 && r <= iy - 1) store(vx, r, x);
     }
-    // pressure (FP32 of the double-float Exner)
-    float ph[4], pl[4], pk[4];
-    ld4f(ph, pa_h + o);
-    ld4f(pl, pa_h + F + o);
+    // v of row r-1, from vx of rows r-3 .. r
+    const int ro = r - 1;
+    if (ro >= i0) {
+      R y[V];
+      if (ro < 2 || ro > iy - 1) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) pk[q] = exner_to_pressure_f(ph[q] + pl[q]);
-    store(pp + o, pk);
-    // mkslice's floors, then status_update's (zero tendencies): at inner
-    // points qx below its check value becomes its zero value, and a tracer
-    // below 1e-50 becomes 0 (in FP32 every value below 1e-50 is <= 0)
-    if (any_inner) {
-      for (int n = 0; n < g.nqx; ++n) {
-        float x[4];
-        ld4f(x, qx + o + (size_t)n * F);
-        bool ch = false;
+        for (int q = 0; q < V; ++q) y[q] = va[q];
+      } else if (ro == 2 || ro == iy - 1) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (inner[q] && x[q] < float(qx_check(n))) {
-            x[q] = float(qx_zero(n));
-            ch = true;
+        for (int q = 0; q < V; ++q) y[q] = interp2<R>(xb[q], xc[q]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q) y[q] = interp4<R>(xc[q], xb[q], x[q], xa[q]);
+      }
+      if (ends) {  // v keeps its values at the first and last column
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+          if (e0 + q + 1 < 2 || e0 + q + 1 > jx - 2) y[q] = va[q];
+      }
+      store(v_out, ro, y);
+    }
+    // ux and u of row r
+    if (r >= i0 && r <= i1 && r <= iy - 1) {
+      R u[V], a[V], y[V];
+#pragma unroll
+      for (int q = 0; q < V; ++q) u[q] = un[q];
+      load(un, u_in, r + 1, r < i1 ? iy - 1 : 0);
+      if (!bdy) {
+        load(a, ux, r, iy - 1);
+      } else {
+        const R uw = __shfl_up_sync(full, u[V - 1], 1);
+        const R ue = __shfl_down_sync(full, u[0], 1), uf = __shfl_down_sync(full, u[1], 1);
+        const R n[V + 3] = {uw, u[0], u[1], u[2], u[3], ue, uf};  // columns -1 .. V+1
+#pragma unroll
+        for (int q = 0; q < V; ++q) a[q] = interp4<R>(n[q + 2], n[q + 1], n[q + 3], n[q]);
+        if (ends) {  // columns 1 and jx-1, one a lane at most
+          const R x = e0 == 0 ? interp2<R>(n[1], n[2]) : interp2<R>(pick4(n, 1, jx - 2 - e0), pick4(n, 2, jx - 2 - e0));
+#pragma unroll
+          for (int q = 0; q < V; ++q)
+            if (e0 + q + 1 == 1 || e0 + q + 1 == jx - 1) a[q] = x;
+        }
+        store(ux, r, a);
+      }
+      const R x1 = __shfl_up_sync(full, a[V - 1], 1), x2 = __shfl_up_sync(full, a[V - 2], 1);
+      const R xe = __shfl_down_sync(full, a[0], 1);
+      const R n[V + 3] = {x2, x1, a[0], a[1], a[2], a[3], xe};  // columns -2 .. V
+      if (r < 2 || r > iy - 2) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) y[q] = u[q];
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q) y[q] = interp4<R>(n[q + 2], n[q + 1], n[q + 3], n[q]);
+        if (ends) {  // columns 2 and jx-1
+          const R x = e0 == 0 ? interp2<R>(n[2], n[3]) : interp2<R>(pick4(n, 1, jx - 2 - e0), pick4(n, 2, jx - 2 - e0));
+#pragma unroll
+          for (int q = 0; q < V; ++q) {
+            const int j = e0 + q + 1;
+            if (j == 2 || j == jx - 1) y[q] = x;
+            else if (j < 2 || j > jx - 1) y[q] = u[q];
           }
-        if (ch) store(qx + o + (size_t)n * F, x);
+        }
       }
-      for (int n = 0; n < g.ntr; ++n) {
-        float x[4];
-        ld4f(x, trac + o + (size_t)n * F);
-        bool ch = false;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (inner[q] && x[q] <= 0.f) {
-            x[q] = 0.f;
-            ch = true;
-          }
-        if (ch) store(trac + o + (size_t)n * F, x);
-      }
+      store(u_out, r, y);
     }
-    float tk[4], tl[4], tv[4], rh[4], th_o[4], tl_o[4], qs[4];
-    ld4f(tk, tt + o);
-    ld4f(tl, tlo + o);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const size_t oq = o + q;
-      const float qf = qfactor(qx, oq, F, ipp);
-      tv[q] = tk[q] * qf;
-      rh[q] = pk[q] / (float(kRgas) * tk[q]);
-      // theta_v = tvirt/pai from the double-float t (Main/mod_moloch.F90:1403-1443)
-      const F2 th2 = df_div(df_mul(F2{tk[q], tl[q]}, qfactor_df(qx, oq, F, ipp)), F2{ph[q], pl[q]});
-      th_o[q] = th2.hi;
-      tl_o[q] = th2.lo;
-      qs[q] = pfwsat_f(tk[q], pk[q]);
+    for (int q = 0; q < V; ++q) {
+      va[q] = vb[q]; vb[q] = vc[q]; vc[q] = vd[q];
+      xa[q] = xb[q]; xb[q] = xc[q]; xc[q] = x[q];
     }
-    store(tvir + o, tv);
-    store(rho + o, rh);
-    store(th_h + o, th_o);
-    store(th_h + F + o, tl_o);
-    store(qsat + o, qs);
+  }
+}
+
+// ux, vx from the relaxed u, v (boundary :520-523, uvstagtouvx :1535-1566)
+template <class R, int LV>
+__global__ void k_end_uvx(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
+    const WorkItem *__restrict__ wl) {
+  const WorkItem wi = work_item(wl, tiles_j);
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active || !D.c.apply_bdy) return;
+  const Geom g = D.g;
+  const int uv = (D.clk->uv_role + uvoff) & 1, adv = (D.clk->adv_role + advoff) & 1;
+  const R *__restrict__ u = D.u[uv];
+  const R *__restrict__ v = D.v[uv];
+  R *__restrict__ ux = D.ux[adv];
+  R *__restrict__ vx = D.vx[adv];
+  const Pt q = point_at<LV>(wi, 1, 1);
+  const int j = q.j, i = q.i, jx = g.jx, iy = g.iy;
+  if (j > jx - 1 || i > iy - 1 || q.k > g.kz) return;
+  const size_t ij = g.at2(j, i), S = (size_t)g.P;
+#pragma unroll
+  for (int k = q.k; k < q.k + LV && k <= g.kz; ++k) {
+    const size_t o = ij + (size_t)(k - 1) * g.PS;
+    ux[o] = j == 1 || j == jx - 1 ? interp2<R>(u[o], u[o + 1]) : interp4<R>(u[o + 1], u[o], u[o + 2], u[o - 1]);
+    vx[o] = i == 1 || i == iy - 1 ? interp2<R>(v[o], v[o + S])
+                                  : interp4<R>(v[o + S], v[o], v[o + 2 * S], v[o - S]);
   }
 }
 
 // uvxtouvstag at the end of status_update (:1440)
-template <class R>
+template <class R, int LV>
 __global__ void k_end_uvstag(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
@@ -957,7 +1365,7 @@ __global__ void k_end_uvstag(const Dom<R> *__restrict__ doms, int uvoff, int adv
   const R *__restrict__ vx = D.vx[adv];
   R *__restrict__ u = D.u[uv];
   R *__restrict__ v = D.v[uv];
-  const Pt q_ = point_at(wi, 1, 1);
+  const Pt q_ = point_at<LV>(wi, 1, 1);
   const int j = q_.j, k0 = q_.k;
   if (k0 > g.kz) return;
   const int i = q_.i;
@@ -968,28 +1376,28 @@ __global__ void k_end_uvstag(const Dom<R> *__restrict__ doms, int uvoff, int adv
   const bool do_v = (j >= 2 && j <= jx - 2 && i >= 2 && i <= iy - 1);
   if (!do_u && !do_v) return;
 #pragma unroll
-  for (int k = k0; k < k0 + kPtLevels && k <= g.kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * PS;
     if (do_u) {
       R a;
       if (j == jx - 1) a = R(0.5) * (ux[o - 1] + ux[o]);
       else if (j == 2) a = R(0.5) * (ux[o] + ux[o - 1]);
-      else a = R(0.5625) * (ux[o] + ux[o - 1]) - R(0.0625) * (ux[o + 1] + ux[o - 2]);
+      else a = interp4<R>(ux[o], ux[o - 1], ux[o + 1], ux[o - 2]);
       u[o] = a;
     }
     if (do_v) {
       R a;
       if (i == iy - 1) a = R(0.5) * (vx[o - S] + vx[o]);
       else if (i == 2) a = R(0.5) * (vx[o] + vx[o - S]);
-      else a = R(0.5625) * (vx[o] + vx[o - S]) - R(0.0625) * (vx[o + S] + vx[o - 2 * S]);
+      else a = interp4<R>(vx[o], vx[o - S], vx[o + S], vx[o - 2 * S]);
       v[o] = a;
     }
   }
 }
 
-// Mass budget (Main/mod_massck.F90:77-170) and ps extrema.  Block b sums the
-// rows (i,k) it owns in a fixed order and writes seven partials; the single-
-// block pass then adds the partials in block order, so the result does not
+// Mass budget (Main/mod_massck.F90:77-170) and ps extrema.  The member's
+// blocks sum their rows in a fixed order and write seven partials each; the
+// last block to finish adds them in a fixed order, so the result does not
 // depend on scheduling and a domain gives the same bits alone or in a batch.
 constexpr int kRedThreads = 256;
 constexpr int kRedWarps = kRedThreads / 32;
@@ -1001,68 +1409,63 @@ __device__ __forceinline__ const R *pick_dz(const Stat<R> &sa) {
   if constexpr (sizeof(R) == sizeof(float)) return sa.dz_r;
   else return sa.dz;
 }
-// 16 bytes at p (16-byte aligned) as V elements
-template <class R, int V>
-__device__ __forceinline__ void ld_vec16(R (&x)[V], const R *p) {
-  const uint4 w = *reinterpret_cast<const uint4 *>(p);
-  memcpy(x, &w, 16);
-}
 
-// Partial sums of the mass budget (Main/mod_massck.F90:57-369) and the ps
-// extrema of one member, per block.  The interior sums run over the member's
-// 3-D arrays as flat vectors of 16 bytes (every row starts on 128 bytes, so a
-// vector never straddles a row); a grid-stride loop over the vectors keeps
-// many loads in flight.  The species of a point are summed before they are
-// weighted by its dry mass dx^2*dz*rho.  FP32 members form the point products
-// in FP32, add each vector's in FP32 and accumulate them as double-floats;
-// dx^2 is applied once per thread.  The lateral fluxes and the ps extrema
-// are grid-stride loops over their own items.  Sums are in a fixed order for
-// a given member, whatever else the launch holds.
-// Per member, by one warp of the reduction's last block: add the partials
-// (lanes stride over the blocks in block order, then a fixed shuffle tree,
-// so the result does not depend on which block finished last), store the
-// diagnostics, then advance the boundary clock and the buffer roles to the
-// next step's and re-arm the block count.
-template <class R>
-__device__ void reduce_finish(const Dom<R> &D, int uvoff, int advoff, int lane) {
-  const double *part = D.partials;
-  const int nblocks = D.red_blocks;
-  double a[4] = {0, 0, 0, 0}, pmax = -INFINITY, pmin = INFINITY, bad = 0;
-  for (int b = lane; b < nblocks; b += 32) {
-    const double *p = part + (size_t)b * kNPart;
-    for (int q = 0; q < 4; ++q) a[q] += __ldcg(p + q);
-    pmax = fmax(pmax, __ldcg(p + 4));
-    pmin = fmin(pmin, __ldcg(p + 5));
-    bad += __ldcg(p + 6);
-  }
+// A block's sums: every warp's by shuffles, then the first warp adds the
+// warps'.  The result is thread 0's.
+struct RedSum {
+  double dry, dadv, qm, qadv;
+  long long pmax, pmin;  // keys of ps
+  int bad;
+};
+// a double's pattern ordered like its value, as a signed integer (its own
+// inverse on the patterns): maxima on the integer pipe
+__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
+__device__ __forceinline__ RedSum red_zero() {
+  return {0, 0, 0, 0, order_key(__double_as_longlong(-INFINITY)), order_key(__double_as_longlong(INFINITY)), 0};
+}
+__device__ __forceinline__ void red_step(RedSum &a, int off, bool flux) {
   const unsigned full = 0xffffffffu;
-  for (int off = 16; off > 0; off >>= 1) {
-    for (int q = 0; q < 4; ++q) a[q] += __shfl_down_sync(full, a[q], off);
-    pmax = fmax(pmax, __shfl_down_sync(full, pmax, off));
-    pmin = fmin(pmin, __shfl_down_sync(full, pmin, off));
-    bad += __shfl_down_sync(full, bad, off);
+  a.dry += __shfl_down_sync(full, a.dry, off);
+  a.qm += __shfl_down_sync(full, a.qm, off);
+  if (flux) {
+    a.dadv += __shfl_down_sync(full, a.dadv, off);
+    a.qadv += __shfl_down_sync(full, a.qadv, off);
   }
-  if (lane != 0) return;
-  DiagDev *diag = D.diag;
-  Clock *clk = D.clk;
-  const bool isbad = bad != 0.0;
-  diag->drymass = a[0]; diag->dryadv = a[1]; diag->qmass = a[2]; diag->qadv = a[3];
-  diag->ps_max = isbad ? NAN : pmax;
-  diag->ps_min = isbad ? NAN : pmin;
-  diag->nonfinite = isbad ? 1 : 0;
-  if (isbad && !clk->nonfinite) { clk->nonfinite = 1; clk->bad_step = clk->step; }
-  if (D.c.apply_bdy) clk->xbctime = clk->xbctime + D.c.dtsec;
-  if (D.c.apply_bdy && D.c.spectral) clk->tspectral = clk->tspectral + D.c.dtsec;
-  clk->step = clk->step + 1;
-  clk->uv_role = (clk->uv_role + uvoff) & 1;
-  clk->adv_role = (clk->adv_role + advoff) & 1;
-  clk->red_done = 0u;
+  a.pmax = max(a.pmax, __shfl_down_sync(full, a.pmax, off));
+  a.pmin = min(a.pmin, __shfl_down_sync(full, a.pmin, off));
+  a.bad |= __shfl_down_sync(full, a.bad, off);
+}
+// flux: whether the warp holds lateral fluxes
+__device__ __forceinline__ RedSum red_block(RedSum a, bool flux, RedSum *sh) {
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+  for (int off = 16; off > 0; off >>= 1) red_step(a, off, flux);
+  if (lane == 0) sh[warp] = a;
+  __syncthreads();
+  if (warp == 0) {
+    a = sh[lane < kRedWarps ? lane : 0];
+    for (int off = kRedWarps / 2; off > 0; off >>= 1) red_step(a, off, true);
+  }
+  return a;
 }
 
+// Partial sums of the mass budget and the ps extrema of one member, per block.
+// Interior rows go to warps, lanes along the row in 16-byte vectors (every row
+// starts on 128 bytes); the species of a point are summed before they are
+// weighted by its dry mass, and dx^2 and dt*dx are applied to the sums.  FP32
+// members: dz is the double-float {dz_r, dz_lo}, dz*rho, the species' sum and
+// its share are double-floats, and so are the running sums (about 1e-14
+// relative against the FP64 sums of the same FP32 state).  The lateral fluxes
+// and ps are grid-stride loops over their own items.  form_ps: ps is
+// extrapolated here, from the virtual temperatures k_end_point left in wz[0].
+// (Row pieces a warp instead of flat vectors with two integer divisions each,
+// the species summed first, a block instead of a warp adding the partials, and
+// ps formed here: 110 us a step at 512x512x41 mixed, 182 FP64, against 113 and
+// 230 without ps; 20 against 25 and 28 at 64x64x30.)
 template <class R>
 __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__restrict__ doms,
-                                                                int uvoff, int advoff) {
-  __shared__ double sh[kRedWarps][kNPart];
+                                                                int uvoff, int advoff, int form_ps) {
+  __shared__ RedSum sh[kRedWarps];
+  __shared__ bool last;
   const Dom<R> &D = doms[blockIdx.y];
   if (!D.active) return;
   const int nb = D.red_blocks;
@@ -1072,150 +1475,172 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__
   const Stat<R> &sa = D.sa;
   const State<R> st = state_of(D, (D.clk->uv_role + uvoff) & 1, (D.clk->adv_role + advoff) & 1);
   const int jx = g.jx, iy = g.iy, kz = g.kz, nqx = g.nqx;
-  const double dx = c.dx, dt = c.dt, dxsq = dx * dx;
   const size_t F = g.field3();
-  const unsigned gt = blockIdx.x * kRedThreads + threadIdx.x;  // this thread's first item
-  const unsigned gs = (unsigned)nb * kRedThreads;              // stride
-  double dry = 0, dadv = 0, qm = 0, qadv = 0, pmax = -INFINITY, pmin = INFINITY, bad = 0;
-  const bool budget = c.debug_level > 0;
-  if (budget) {
+  const int lane = (int)threadIdx.x & 31;
+  const int gt = (int)(blockIdx.x * kRedThreads + threadIdx.x), gs = nb * kRedThreads;
+  RedSum a = red_zero();
+  bool flux = false;
+  if (c.debug_level > 0) {
     constexpr int V = 16 / (int)sizeof(R);
-    const unsigned nvec = (unsigned)(g.PS * (size_t)kz) / V;  // below 2^31 / V
-    const unsigned P = (unsigned)g.P;
     const R *__restrict__ dzp = pick_dz<R>(sa);
+    const R *__restrict__ rho = st.rho;
+    const R *__restrict__ qx = st.qx;
     F2 dry2{0.f, 0.f}, qm2{0.f, 0.f};
-    for (unsigned v = gt; v < nvec; v += gs) {
-      const unsigned base = v * V;
-      const unsigned r = base / P;               // (i-1) + (k-1)*iy
-      const int c0 = (int)(base - r * P);        // j-1 of the vector's first element
-      const int i = (int)(r % (unsigned)iy) + 1;
-      if (i < 2 || i > iy - 2 || c0 + 1 > jx - 2) continue;
-      R dz[V], rh[V], qs[V], q1[V];
-      ld_vec16<R, V>(dz, dzp + base);
-      ld_vec16<R, V>(rh, st.rho + base);
+    // a warp's items: pieces of 32*V columns of the interior rows, in order;
+    // two items' loads in flight
+    const int ni = iy - 3, np = (jx - 2 + 32 * V - 1) / (32 * V), items = ni * kz * np;
+    const int nw = nb * kRedWarps, per = (items + nw - 1) / nw;
+    const int t0 = (gt >> 5) * per, t1 = min(items, t0 + per);
+#pragma unroll 2
+    for (int it = t0; it < t1; ++it) {
+      const int r = it / np, kk = r / ni, ii = r - kk * ni + 1;  // 0-based level and row
+      const int e = (it - r * np) * 32 * V + lane * V;
+      if (e >= jx - 2) continue;
+      const size_t o = (size_t)kk * g.PS + (size_t)ii * g.P + e;
+      R dz[V], rh[V], q[5][V];
+      ldv<R, V>(dz, dzp + o);
+      ldv<R, V>(rh, rho + o);
+#pragma unroll
+      for (int n = 0; n < 5; ++n)
+        if (n < nqx) ldv<R, V>(q[n], qx + o + (size_t)n * F);
       if constexpr (sizeof(R) == sizeof(float)) {
-        // FP32 state, FP64-accurate sums: dz as the double-float {dz_r,
-        // dz_lo}, dz*rho and each species' share as double-float products,
-        // double-float running sums (about 1e-14 relative against the FP64
-        // sums of the same FP32 state)
-        R dzl[V];
-        ld_vec16<R, V>(dzl, sa.dz_lo + base);
-        F2 dr[V];
+        R dl[V];
+        ldv<R, V>(dl, sa.dz_lo + o);
+        F2 qs[V];
 #pragma unroll
-        for (int q = 0; q < V; ++q) {
-          const int j = c0 + q + 1;
-          dr[q] = (j >= 2 && j <= jx - 2) ? df_mul_f(F2{dz[q], dzl[q]}, rh[q]) : F2{0.f, 0.f};
-          dry2 = df_add(dry2, dr[q]);
+        for (int x = 0; x < V; ++x) {
+          qs[x] = F2{q[0][x], 0.f};
+#pragma unroll
+          for (int n = 1; n < 5; ++n)
+            if (n < nqx) qs[x] = df_add_f(qs[x], q[n][x]);
         }
-        for (int n = 0; n < nqx; ++n) {
-          ld_vec16<R, V>(q1, st.qx + base + (size_t)n * F);
+        for (int n = 5; n < nqx; ++n) {
+          ldv<R, V>(q[0], qx + o + (size_t)n * F);
 #pragma unroll
-          for (int q = 0; q < V; ++q) qm2 = df_add(qm2, df_mul_f(dr[q], q1[q]));
-        }
-      } else {
-        ld_vec16<R, V>(qs, st.qx + base);
-        for (int n = 1; n < nqx; ++n) {
-          ld_vec16<R, V>(q1, st.qx + base + (size_t)n * F);
-#pragma unroll
-          for (int q = 0; q < V; ++q) qs[q] += q1[q];
+          for (int x = 0; x < V; ++x) qs[x] = df_add_f(qs[x], q[0][x]);
         }
 #pragma unroll
-        for (int q = 0; q < V; ++q) {
-          const int j = c0 + q + 1;
-          if (j >= 2 && j <= jx - 2) {
-            const double wpt = dxsq * (double)dz[q] * (double)rh[q];
-            dry += wpt;
-            qm += (double)qs[q] * wpt;
+        for (int x = 0; x < V; ++x)
+          if (e + x >= 1 && e + x <= jx - 3) {
+            const F2 m = df_mul_f(F2{dz[x], dl[x]}, rh[x]);
+            dry2 = df_add(dry2, m);
+            qm2 = df_add(qm2, df_mul(m, qs[x]));
           }
+      } else {
+#pragma unroll
+        for (int n = 1; n < 5; ++n)
+          if (n < nqx)
+#pragma unroll
+            for (int x = 0; x < V; ++x) q[0][x] += q[n][x];
+        for (int n = 5; n < nqx; ++n) {
+          ldv<R, V>(q[1], qx + o + (size_t)n * F);
+#pragma unroll
+          for (int x = 0; x < V; ++x) q[0][x] += q[1][x];
         }
+#pragma unroll
+        for (int x = 0; x < V; ++x)
+          if (e + x >= 1 && e + x <= jx - 3) {
+            const double m = __dmul_rn(dz[x], rh[x]);
+            a.dry += m;
+            a.qm = __fma_rn(q[0][x], m, a.qm);
+          }
       }
     }
+    const double dxsq = c.dx * c.dx;
     if constexpr (sizeof(R) == sizeof(float)) {
-      dry = ((double)dry2.hi + (double)dry2.lo) * dxsq;
-      qm = ((double)qm2.hi + (double)qm2.lo) * dxsq;
+      a.dry = ((double)dry2.hi + (double)dry2.lo) * dxsq;
+      a.qm = ((double)qm2.hi + (double)qm2.lo) * dxsq;
+    } else {
+      a.dry *= dxsq;
+      a.qm *= dxsq;
     }
+    // Lateral fluxes, FP64 products of the state's values in both precisions
+    // (a few thousand terms: the budget stays FP64-accurate for a mixed
+    // member).  wind: into the domain
+    auto face = [&](size_t o, double wind) {
+      const double f = wind * (sa.dz[o] * (double)st.rho[o]);
+      double q = (double)st.qx[o];
+      for (int n = 1; n < nqx; ++n) q += (double)st.qx[o + (size_t)n * F];
+      a.dadv += f;
+      a.qadv = __fma_rn(q, f, a.qadv);
+      flux = true;
+    };
     // west and east columns over i in ice = 1 .. iy-1 (:85-100)
-    const unsigned nwe = (unsigned)((iy - 1) * kz);
-    for (unsigned e = gt; e < nwe; e += gs) {
-      const int i = (int)(e % (unsigned)(iy - 1)) + 1, k = (int)(e / (unsigned)(iy - 1)) + 1;
-      const size_t ko = (size_t)(k - 1) * g.PS;
-      const size_t ow = g.at2(1, i) + ko, oe = g.at2(jx - 1, i) + ko;
-      {
-        // FP64 products of the state's values in both precisions (a few
-        // thousand terms: the budget stays FP64-accurate for a mixed member)
-        const double uw = (double)st.u[g.at2(1, i) + ko], ue = (double)st.u[g.at2(jx, i) + ko];
-        const double dzw = (double)sa.dz[ow], rw = (double)st.rho[ow];
-        const double dze = (double)sa.dz[oe], re = (double)st.rho[oe];
-        dadv += uw * dt * dx * dzw * rw;
-        dadv -= ue * dt * dx * dze * re;
-        for (int n = 0; n < nqx; ++n) {
-          qadv += (double)st.qx[ow + (size_t)n * F] * uw * dt * dx * dzw * rw;
-          qadv -= (double)st.qx[oe + (size_t)n * F] * ue * dt * dx * dze * re;
-        }
-      }
+    for (int e = gt; e < 2 * (iy - 1) * kz; e += gs) {
+      const bool east = (e & 1) != 0;
+      const int r = e >> 1, k = r / (iy - 1), i = r - k * (iy - 1) + 1;
+      const size_t ko = (size_t)k * g.PS;
+      const double u = (double)st.u[g.at2(east ? jx : 1, i) + ko];
+      face(g.at2(east ? jx - 1 : 1, i) + ko, east ? -u : u);
     }
     // south (v at ide1) and north (v at ide2) rows, j in jci (:101-116)
-    const unsigned nsn = (unsigned)(2 * kz * (jx - 3));
-    for (unsigned e = gt; e < nsn; e += gs) {
-      const int j = (int)(e % (unsigned)(jx - 3)) + 2;
-      const unsigned rest = e / (unsigned)(jx - 3);
-      const bool south = (rest & 1u) == 0;
-      const int k = (int)(rest >> 1) + 1;
-      const int i = south ? 1 : iy - 1, iv = south ? 1 : iy;
-      const size_t ko = (size_t)(k - 1) * g.PS;
-      const size_t o = g.at2(j, i) + ko;
-      const double vv = (double)st.v[g.at2(j, iv) + ko];
-      const double dzr = (double)sa.dz[o], rh = (double)st.rho[o];
-      const double fl = vv * dt * dx * dzr * rh;
-      dadv = south ? dadv + fl : dadv - fl;
-      for (int n = 0; n < nqx; ++n) {
-        const double q = (double)st.qx[o + (size_t)n * F] * vv * dt * dx * dzr * rh;
-        qadv = south ? qadv + q : qadv - q;
-      }
+    for (int e = gt; e < 2 * kz * (jx - 3); e += gs) {
+      const int rest = e / (jx - 3), j = e - rest * (jx - 3) + 2;
+      const bool north = (rest & 1) != 0;
+      const size_t ko = (size_t)(rest >> 1) * g.PS;
+      const double v = (double)st.v[g.at2(j, north ? iy : 1) + ko];
+      face(g.at2(j, north ? iy - 1 : 1) + ko, north ? -v : v);
+    }
+    flux = __any_sync(0xffffffffu, flux);
+    if (flux) {
+      a.dadv *= c.dt * c.dx;
+      a.qadv *= c.dt * c.dx;
     }
   }
-  // ps extrema over the interior
-  const unsigned nps = (unsigned)((iy - 3) * (jx - 3));
-  for (unsigned e = gt; e < nps; e += gs) {
-    const int j = (int)(e % (unsigned)(jx - 3)) + 2, i = (int)(e / (unsigned)(jx - 3)) + 2;
-    const double x = st.ps[g.at2(j, i)];
-    if (!isfinite(x)) bad = 1;
-    else { pmax = fmax(pmax, x); pmin = fmin(pmin, x); }
+  // ps and its extrema over the interior
+  for (int e = gt; e < (iy - 3) * (jx - 3); e += gs) {
+    const int i = e / (jx - 3) + 2, j = e - (i - 2) * (jx - 3) + 2;
+    const size_t ij = g.at2(j, i);
+    double x;
+    if (form_ps) {
+      const size_t o1 = ij + (size_t)(kz - 2) * g.PS, o2 = ij + (size_t)(kz - 1) * g.PS;
+      x = surface_pressure((double)D.wz[0][o1], (double)D.wz[0][o2], sa.zeta[o1], sa.zeta[o2], (double)st.p[o2]);
+      st.ps[ij] = x;
+    } else {
+      x = st.ps[ij];
+    }
+    const long long b = __double_as_longlong(x);
+    if ((b & 0x7ff0000000000000LL) == 0x7ff0000000000000LL) a.bad = 1;
+    else { a.pmax = max(a.pmax, order_key(b)); a.pmin = min(a.pmin, order_key(b)); }
   }
-  const unsigned full = 0xffffffffu;
-  for (int off = 16; off > 0; off >>= 1) {
-    dry += __shfl_down_sync(full, dry, off);
-    qm += __shfl_down_sync(full, qm, off);
-    dadv += __shfl_down_sync(full, dadv, off);
-    qadv += __shfl_down_sync(full, qadv, off);
-    bad += __shfl_down_sync(full, bad, off);
-    pmax = fmax(pmax, __shfl_down_sync(full, pmax, off));
-    pmin = fmin(pmin, __shfl_down_sync(full, pmin, off));
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    sh[warp][0] = dry; sh[warp][1] = dadv; sh[warp][2] = qm; sh[warp][3] = qadv;
-    sh[warp][4] = pmax; sh[warp][5] = pmin; sh[warp][6] = bad;
-  }
-  __syncthreads();
-  __shared__ bool last;
+  a = red_block(a, flux, sh);
   if (threadIdx.x == 0) {
-    double a[kNPart] = {0, 0, 0, 0, -INFINITY, INFINITY, 0};
-    for (int w = 0; w < kRedWarps; ++w) {
-      a[0] += sh[w][0]; a[1] += sh[w][1]; a[2] += sh[w][2]; a[3] += sh[w][3];
-      a[4] = fmax(a[4], sh[w][4]); a[5] = fmin(a[5], sh[w][5]); a[6] += sh[w][6];
-    }
     double *p = D.partials + (size_t)blockIdx.x * kNPart;
-    for (int q = 0; q < kNPart; ++q) p[q] = a[q];
+    p[0] = a.dry; p[1] = a.dadv; p[2] = a.qm; p[3] = a.qadv; 
+    p[4] = __longlong_as_double(a.pmax); p[5] = __longlong_as_double(a.pmin); p[6] = a.bad;
     // the member's last block to finish adds the partials: its partials are
     // visible before its ticket, and every other block's before theirs
     __threadfence();
     last = atomicAdd(&D.clk->red_done, 1u) == (unsigned)nb - 1u;
   }
   __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
+  if (!last) return;
   __threadfence();
-  reduce_finish<R>(D, uvoff, advoff, (int)threadIdx.x);
+  // store the diagnostics, then advance the boundary clock and the buffer
+  // roles to the next step's and re-arm the block count
+  RedSum t = red_zero();
+  for (int b = (int)threadIdx.x; b < nb; b += kRedThreads) {
+    const double *p = D.partials + (size_t)b * kNPart;
+    t.dry += __ldcg(p); t.dadv += __ldcg(p + 1); t.qm += __ldcg(p + 2); t.qadv += __ldcg(p + 3);
+    t.pmax = max(t.pmax, __double_as_longlong(__ldcg(p + 4)));
+    t.pmin = min(t.pmin, __double_as_longlong(__ldcg(p + 5)));
+    t.bad |= __ldcg(p + 6) != 0.0;
+  }
+  t = red_block(t, true, sh);
+  if (threadIdx.x != 0) return;
+  DiagDev *diag = D.diag;
+  Clock *clk = D.clk;
+  diag->drymass = t.dry; diag->dryadv = t.dadv; diag->qmass = t.qm; diag->qadv = t.qadv;
+  diag->ps_max = t.bad ? NAN : __longlong_as_double(order_key(t.pmax));
+  diag->ps_min = t.bad ? NAN : __longlong_as_double(order_key(t.pmin));
+  diag->nonfinite = t.bad;
+  if (t.bad && !clk->nonfinite) { clk->nonfinite = 1; clk->bad_step = clk->step; }
+  if (c.apply_bdy) clk->xbctime = clk->xbctime + c.dtsec;
+  if (c.apply_bdy && c.spectral) clk->tspectral = clk->tspectral + c.dtsec;
+  clk->step = clk->step + 1;
+  clk->uv_role = (clk->uv_role + uvoff) & 1;
+  clk->adv_role = (clk->adv_role + advoff) & 1;
+  clk->red_done = 0u;
 }
 
 template <class R>
@@ -1281,37 +1706,38 @@ inline dim3 pt_grid(const LaunchGeom &L, int nj, int ni, int &tiles_j) {
   tiles_j = (nj + L.col_x - 1) / L.col_x;
   if (L.wl_pt) return dim3((unsigned)L.n_pt, 1, 1);  // one block per work item
   const int ti = (ni + L.col_y - 1) / L.col_y;
-  return dim3((unsigned)(tiles_j * ti), (unsigned)((L.kz + kPtLevels - 1) / kPtLevels),
-              (unsigned)L.nmem);
+  return dim3((unsigned)(tiles_j * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
 }
 
 }  // namespace
 
-// some 16 elements per thread, at most 4 blocks per SM
+// Eight row pieces a warp, at most 2 blocks per SM - a block more costs its
+// threads' sums, some 50 FP64 instructions a warp - but down to two pieces a
+// warp for the first 64 blocks, whose loads a small domain waits on.  (Of the
+// member's extents alone: its sums are the same in any batch.)
 int reduce_blocks(const Geom &g) {
-  const size_t n = g.PS * (size_t)g.kz;
-  const size_t per_block = (size_t)kRedThreads * 16;
-  const size_t nb = (n + per_block - 1) / per_block;
-  return (int)std::min<size_t>(std::max<size_t>(nb, 1), 152 * 4);
+  const int items = (g.iy - 3) * g.kz * ((g.jx - 2 + 127) / 128);
+  const int eight = (items + 8 * kRedWarps - 1) / (8 * kRedWarps), two = (items + 2 * kRedWarps - 1) / (2 * kRedWarps);
+  return std::max(1, std::min(std::max(eight, std::min(two, 64)), 152 * 2));
 }
 
 // status_update of the turbulent kinetic energy (Main/mod_moloch.F90:
 // 1419-1424): on jci x ici at the kz+1 interfaces, tke + dtsec * tketen (the
 // physics' tendency; none in a whole step), then the floor tkemin.
-template <class R>
+template <class R, int LV>
 __global__ void k_end_tke(const Dom<R> *__restrict__ doms, int whole, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active || !D.c.tke) return;
   const Geom g = D.g;
-  const Pt q = point_at(wi, 1, 1);
+  const Pt q = point_at<LV>(wi, 1, 1);
   if (q.j < 2 || q.j > g.jx - 2 || q.i < 2 || q.i > g.iy - 2 || q.k > g.kz) return;
   const R *ten = whole ? nullptr : D.tend;
   // tketen follows the kz-plane tendencies (t, u, v, the species, tracers)
   const R *tt = ten ? ten + (size_t)(3 + g.nqx + g.ntr) * g.field3() : nullptr;
   const R dts = pick<R>(D.c.dtsec, D.c.dtsecf);
-  const int klast = q.k + kPtLevels - 1 >= g.kz ? g.kz + 1 : q.k + kPtLevels - 1;
+  const int klast = q.k + LV - 1 >= g.kz ? g.kz + 1 : q.k + LV - 1;
   for (int k = q.k; k <= klast; ++k) {
     const size_t o = g.at(q.j, q.i, k);
     R v = D.tke[o];
@@ -1323,7 +1749,8 @@ __global__ void k_end_tke(const Dom<R> *__restrict__ doms, int whole, int tiles_
 
 template <class R>
 void Launch<R>::bdy_ring(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
-  k_bdy_ring<R><<<dim3((unsigned)L.kz, (unsigned)L.nmem), kRingThreads, 0, s>>>(d, uvoff, advoff);
+  const unsigned nb = (unsigned)((2 * (L.iy - 2) + 2 * L.jx + kRingThreads - 1) / kRingThreads);
+  k_bdy_ring<R><<<dim3(nb, (unsigned)L.kz, (unsigned)L.nmem), kRingThreads, 0, s>>>(d, uvoff, advoff);
 }
 
 template <class R>
@@ -1331,7 +1758,8 @@ void Launch<R>::end_relax(const LaunchGeom &L, const Dom<R> *d, int uvoff, int a
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  k_end_relax<R><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_end_relax<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_end_relax<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1343,37 +1771,64 @@ void Launch<R>::bdy_spectral(const LaunchGeom &L, const Dom<R> *d, int uvoff, in
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 2, L.iy - 2, tj);
-  k_spec_apply<R><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_spec_apply<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_spec_apply<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+}
+
+template <class R>
+void Launch<R>::end_point(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  constexpr int W = 32 * (16 / (int)sizeof(R));
+  const int tj = (L.jx - 1 + W - 1) / W, ti = (L.iy - 1 + 3) / 4;
+  const dim3 grd = L.wl_vec ? dim3((unsigned)L.n_vec, 1, 1)
+                            : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
+  if (L.lv == 1) k_end_point<R, 1, false><<<grd, 128, 0, s>>>(d, uvoff, advoff, tj, L.wl_vec);
+  else k_end_point<R, 4, false><<<grd, 128, 0, s>>>(d, uvoff, advoff, tj, L.wl_vec);
+}
+
+template <class R>
+void Launch<R>::end_frame(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  const dim3 grd((unsigned)((L.frame_points + 127) / 128), (unsigned)L.kz, (unsigned)L.nmem);
+  k_end_point<R, 1, true><<<grd, 128, 0, s>>>(d, uvoff, advoff, 1, nullptr);
+}
+
+template <class R>
+void Launch<R>::end_uvx(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
+  int tj;
+  const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
+  if (L.lv == 1) k_end_uvx<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_end_uvx<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+}
+
+template <class R>
+void Launch<R>::end_winds(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  const int tj = wind_tiles_j(L.jx), ti = wind_tiles_i(L.iy, L.wind_rows);
+  const dim3 grd = L.wl_wind ? dim3((unsigned)L.n_wind, 1, 1)
+                             : dim3((unsigned)(tj * ti), (unsigned)L.kz, (unsigned)L.nmem);
+  if constexpr (sizeof(R) == sizeof(float))
+    k_end_winds<R><<<grd, 32 * kWindWarps, 0, s>>>(d, uvoff, advoff, L.wind_rows, tj, L.wl_wind);
+}
+
+template <class R, int PH>
+void launch_cross(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
+  int tj;
+  const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
+  if (PH != kEndPost) k_end_ps<R><<<grid2(L.jx - 3, L.iy - 3, b, L.nmem), b, 0, s>>>(d, uvoff, advoff);
+  if (L.lv == 1) k_end_cross<R, PH, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_end_cross<R, PH, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
 void Launch<R>::end_cross(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
-  const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
-  if constexpr (sizeof(R) == sizeof(float)) {
-    const int tj = (L.jx - 1 + 127) / 128, ti = (L.iy - 1 + 3) / 4;
-    const dim3 grd = L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
-                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + kPtLevels - 1) / kPtLevels),
-                                    (unsigned)L.nmem);
-    k_end_cross_v4<R><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, advoff, tj, L.wl_v4);
-  } else {
-    int tj;
-    const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-    k_end_cross<R, kEndAll><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  }
+  launch_cross<R, kEndAll>(L, d, uvoff, advoff, s);
 }
 
 template <class R>
 void Launch<R>::end_cross_split(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool post,
                                 cudaStream_t s) {
-  const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
-  int tj;
-  const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (post) {
-    k_end_cross<R, kEndPost><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  } else {
-    k_end_ps<R><<<grid2(L.jx - 3, L.iy - 3, b, L.nmem), b, 0, s>>>(d, uvoff, advoff);
-    k_end_cross<R, kEndPre><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  }
+  if (post) launch_cross<R, kEndPost>(L, d, uvoff, advoff, s);
+  else launch_cross<R, kEndPre>(L, d, uvoff, advoff, s);
 }
 
 template <class R>
@@ -1381,7 +1836,8 @@ void Launch<R>::end_uvstag(const LaunchGeom &L, const Dom<R> *d, int uvoff, int 
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-  k_end_uvstag<R><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_end_uvstag<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  else k_end_uvstag<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1389,14 +1845,15 @@ void Launch<R>::end_tke(const LaunchGeom &L, const Dom<R> *d, bool whole_step, c
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-  k_end_tke<R><<<grd, b, 0, s>>>(d, whole_step ? 1 : 0, tj, L.wl_pt);
+  if (L.lv == 1) k_end_tke<R, 1><<<grd, b, 0, s>>>(d, whole_step ? 1 : 0, tj, L.wl_pt);
+  else k_end_tke<R, 4><<<grd, b, 0, s>>>(d, whole_step ? 1 : 0, tj, L.wl_pt);
 }
 
 template <class R>
-void Launch<R>::end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff,
+void Launch<R>::end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps,
                            cudaStream_t s) {
   k_reduce_partial<R><<<dim3((unsigned)L.red_blocks, (unsigned)L.nmem), kRedThreads, 0, s>>>(
-      d, uvoff, advoff);
+      d, uvoff, advoff, form_ps ? 1 : 0);
 }
 
 template <class R>

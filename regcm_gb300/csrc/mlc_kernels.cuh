@@ -20,6 +20,12 @@ constexpr int kSolveStream = 0, kSolveCols3 = 3, kSolveCols6 = 6;
 constexpr int solve_segment(int kind, int elem_bytes) {
   return kind == kSolveStream && elem_bytes == 4 ? 128 : 32;
 }
+// Tiles of end_winds: a block is kWindWarps warps, a warp a row segment of 128
+// columns of which it writes kWindCols, marching over some rows.
+constexpr int kWindWarps = 4, kWindCols = 120;
+constexpr int wind_tiles_j(int jx) { return (jx + kWindCols - 1) / kWindCols; }
+constexpr int wind_tiles_i(int iy, int rows) { return (iy + kWindWarps * rows - 1) / (kWindWarps * rows); }
+
 // Levels of a domain, at most.
 constexpr int kMaxLevels = 128;
 
@@ -29,6 +35,9 @@ struct LaunchGeom {
   int col_x, col_y;      // column kernels
   int solve_x, solve_y;  // kept in the tune report; not used by the solves
   int solve;             // form of the column solves (kSolveStream ...)
+  int wind_rows;         // rows of a warp of end_winds (0: FP64 members, end_uvx and end_uvstag)
+  int frame_points;      // points a level of the largest member's frame (Scal::frame)
+  int lv;                // levels a thread of the point kernels runs (1 or 4)
   int vert_x, vert_y;    // adv_vertical
   int htile;             // adv_horizontal tile shape (hshape)
   int nadv_r;            // advected fields of type R per member
@@ -39,12 +48,14 @@ struct LaunchGeom {
   // largest member) and their lengths, one per tiling
   const WorkItem *wl_pt;     // col_x x col_y tiles, level chunks
   const WorkItem *wl_v4;     // 128 x 4 tiles, level chunks
+  const WorkItem *wl_vec;    // the step end's: 16-byte lanes (64 or 128 columns) x 4 tiles, level chunks
+  const WorkItem *wl_wind;   // wind_cols columns x kWindWarps*wind_rows rows, levels
   const WorkItem *wl_solve;  // row segments of solve_segment columns
   const WorkItem *wl_vert;   // vert_x x vert_y column tiles, R fields
   const WorkItem *wl_vinc;   // the same, the two double-float fields
   const WorkItem *wl_h;      // horizontal WAF tiles (shape htile), levels
   const WorkItem *wl_hinc;   // increment-form WAF tiles, levels
-  int n_pt, n_v4, n_solve, n_vert, n_vinc, n_h, n_hinc;
+  int n_pt, n_v4, n_vec, n_wind, n_solve, n_vert, n_vinc, n_h, n_hinc;
 };
 
 template <class R> struct Launch {
@@ -74,6 +85,13 @@ template <class R> struct Launch {
   static void bdy_ring(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   static void end_relax(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   static void bdy_spectral(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
+  // a whole step's end without spectral nudging: the pointwise work, then the
+  // winds (a mixed member's end in the other half of their pairs)
+  static void end_point(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
+  // ... of the ring and the relaxation zone
+  static void end_frame(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
+  static void end_uvx(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
+  static void end_winds(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   static void end_cross(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   // the step split at the physics: k_end_ps and the cross-point work up to
   // mkslice (post = false), or status_update with the tendencies (post = true)
@@ -82,7 +100,8 @@ template <class R> struct Launch {
   static void end_uvstag(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   // status_update of the TKE (ibltyp = 2): tendency (split step) and floor
   static void end_tke(const LaunchGeom &L, const Dom<R> *d, bool whole_step, cudaStream_t s);
-  static void end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff,
+  // form_ps: ps from the virtual temperatures end_point left
+  static void end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps,
                          cudaStream_t s);
   // ---- layout conversion (one member, from the host) ----
   static void unpack3(const double *src, R *dst, const Geom &g, int nj, int ni, int nk,

@@ -69,14 +69,14 @@ __device__ __forceinline__ double relax_weight(const int32_t *ibnd, const double
 // reads theta_v itself: two coefficient planes would be as many bytes and cost
 // their writing here (measured 353 + 92 against 366 + 73 us a step of four
 // substeps at 512x512x41).
-template <class R>
+template <class R, int LV>
 __global__ void k_sound_prep(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
   const Geom g = D.g;
-  const Pt q = point_at(wi, 1, 1);
+  const Pt q = point_at<LV>(wi, 1, 1);
   if (q.j > g.jx - 1 || q.i > g.iy - 1 || q.k > g.kz) return;
   const int adv = (D.clk->adv_role + advoff) & 1;
   const Scal &c = D.c;
@@ -90,7 +90,7 @@ __global__ void k_sound_prep(const Dom<R> *__restrict__ doms, int advoff, int ti
     cy = (c.lrotllr ? c.dtrdxs : c.dtrdxs * sa.msfv[ij]) * (0.5 * kCpd);
   }
 #pragma unroll
-  for (int k = q.k; k < q.k + kPtLevels && k <= g.kz; ++k) {
+  for (int k = q.k; k < q.k + LV && k <= g.kz; ++k) {
     const size_t o = g.at(q.j, q.i, k), om = o - g.PS;
     if constexpr (sizeof(R) == sizeof(float)) {
       const DF th(tetav, g.field3()), zz(D.tetavf, g.PS * (size_t)(g.kz + 1));
@@ -112,18 +112,32 @@ __global__ void k_sound_prep(const Dom<R> *__restrict__ doms, int advoff, int ti
   }
 }
 
-// Main/mod_moloch.F90:582-618
+// zdiv2 (Main/mod_moloch.F90:602-618) from the face fluxes u*cu and v*cv, and
+// the terrain-following wind of s (:582-597) from the winds summed over two
+// levels; every rounding explicit (the chunk sizes of the point kernels give
+// the same bits).
 template <class R>
+__device__ __forceinline__ R divergence(R cf, R u0, R cu0, R u1, R cu1, R v0, R cv0, R v1, R cv1) {
+  return mul_r(cf, fma_r(-v0, cv0, fma_r(v1, cv1, fma_r(u1, cu1, -mul_r(u0, cu0)))));
+}
+template <class R>
+__device__ __forceinline__ R slope_wind(R u0, R hx0, R u1, R hx1, R v0, R hy0, R v1, R hy1) {
+  return fma_r(v1, hy1, fma_r(v0, hy0, fma_r(u1, hx1, mul_r(u0, hx0))));
+}
+
+// Main/mod_moloch.F90:582-618, FP64.  Bound by the FP64 pipe: 14 instructions
+// a point (17 with the reference's association).
+template <class R, int LV>
 __global__ void k_sound_div(const Dom<R> *__restrict__ doms, int uvoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  static_assert(sizeof(R) == sizeof(double), "FP64 member");
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
   const Geom g = D.g;
-  const Pt q = point_at(wi, 1, 1);
+  const Pt q = point_at<LV>(wi, 1, 1);
   const int j = q.j, i = q.i, kz = g.kz;
   if (j > g.jx - 1 || i > g.iy - 1 || q.k > kz) return;
-  const Scal &c = D.c;
   const Stat<R> &sa = D.sa;
   const int uv = (D.clk->uv_role + uvoff) & 1;
   const R *__restrict__ u = D.u[uv];
@@ -131,72 +145,32 @@ __global__ void k_sound_div(const Dom<R> *__restrict__ doms, int uvoff, int tile
   R *__restrict__ zdiv2 = D.zdiv2;
   R *__restrict__ s = D.s;
   R *__restrict__ w = D.w;
-  const R dtrdx = pick<R>(c.dtrdxs, c.dtrdxsf), dtrdy = dtrdx;
   const size_t ij = g.at2(j, i), ijE = g.at2(j + 1, i), ijN = g.at2(j, i + 1);
   const bool interior = (j >= 2 && j <= g.jx - 2 && i >= 2 && i <= g.iy - 2);
-  const R rmu0 = sa.rmu[ij], rmu1 = sa.rmu[ijE], rmv0 = sa.rmv[ij], rmv1 = sa.rmv[ijN];
-  const R mfac = c.lrotllr ? sa.msfx[ij] : sa.mx2[ij];
   R hx0 = 0, hx1 = 0, hy0 = 0, hy1 = 0;
   if (interior) {
     hx0 = sa.hx[ij]; hx1 = sa.hx[ijE]; hy0 = sa.hy[ij]; hy1 = sa.hy[ijN];
   }
 #pragma unroll
-  for (int k = q.k; k < q.k + kPtLevels && k <= kz; ++k) {
-  const size_t o = (size_t)(k - 1) * g.PS;
-  const R u0 = u[ij + o], u1 = u[ijE + o], v0 = v[ij + o], v1 = v[ijN + o];
-  if constexpr (sizeof(R) == sizeof(double)) {
-    // the constant factors formed at bind time: u*(dtrdx*rfmzu*rmu) for
-    // dtrdx*u*rfmzu*rmu (one FP64 product a flux instead of three)
-    const R zum = u0 * sa.dv_cu[ij + o], zup = u1 * sa.dv_cu[ijE + o];
-    const R zvm = v0 * sa.dv_cv[ij + o], zvp = v1 * sa.dv_cv[ijN + o];
-    zdiv2[ij + o] = sa.dv_cf[ij + o] * ((zup - zum) + (zvp - zvm));
-  } else {
-  R zum, zup;
-  if (c.lrotllr) {
-    zum = dtrdx * u0 * sa.rfmzu[ij + o];
-    zup = dtrdx * u1 * sa.rfmzu[ijE + o];
-  } else {
-    zum = dtrdx * u0 * sa.rfmzu[ij + o] * rmu0;
-    zup = dtrdx * u1 * sa.rfmzu[ijE + o] * rmu1;
+  for (int k = q.k; k < q.k + LV && k <= kz; ++k) {
+    const size_t o = (size_t)(k - 1) * g.PS;
+    const R u0 = u[ij + o], u1 = u[ijE + o], v0 = v[ij + o], v1 = v[ijN + o];
+    // the constant factors formed at bind time
+    zdiv2[ij + o] = divergence<R>(sa.dv_cf[ij + o], u0, sa.dv_cu[ij + o], u1, sa.dv_cu[ijE + o], v0,
+                                  sa.dv_cv[ij + o], v1, sa.dv_cv[ijN + o]);
+    if (!interior) continue;
+    if (k >= 2) {
+      const size_t om = o - g.PS;  // level k-1
+      s[ij + o] = mul_r(slope_wind<R>(u0 + u[ij + om], hx0, u1 + u[ijE + om], hx1, v0 + v[ij + om], hy0,
+                                      v1 + v[ijN + om], hy1),
+                        sa.gzitak[k - 1]);
+    }
+    if (k == kz) {
+      const R skp1 = -0.5 * slope_wind<R>(u0, hx0, u1, hx1, v0, hy0, v1, hy1);
+      s[ij + (size_t)kz * g.PS] = skp1;
+      w[ij + (size_t)kz * g.PS] = -skp1;
+    }
   }
-  const R zvm = dtrdy * v0 * sa.rfmzv[ij + o] * rmv0;
-  const R zvp = dtrdy * v1 * sa.rfmzv[ijN + o] * rmv1;
-  zdiv2[ij + o] = sa.fmz[ij + o] * mfac * ((zup - zum) + (zvp - zvm));
-  }
-  if (!interior) continue;
-  if (k >= 2) {
-    const size_t om = o - g.PS;  // level k-1
-    const R um = u[ij + om], up = u[ijE + om], vm = v[ij + om], vp = v[ijN + om];
-    const R zuh = (u0 + um) * hx0 + (u1 + up) * hx1;
-    const R zvh = (v0 + vm) * hy0 + (v1 + vp) * hy1;
-    s[ij + o] = -(R(0.25) * (zuh + zvh) * sa.gzitak_r[k - 1]);
-  }
-  if (k == kz) {
-    const R zuh = u0 * hx0 + u1 * hx1;
-    const R zvh = v0 * hy0 + v1 * hy1;
-    const R skp1 = -(R(0.5) * (zuh + zvh));
-    s[ij + (size_t)kz * g.PS] = skp1;
-    w[ij + (size_t)kz * g.PS] = -skp1;
-  }
-  }
-}
-
-// ---- the implicit w-Exner solves ---------------------------------------------
-// 1/x of a positive x: the FP32 reciprocal of x's leading bits, moved between
-// the formats by integer instructions, and one third-order step
-// r0 + r0*(e + e^2), e = 1 - x*r0 (Householder's method of order two for the
-// reciprocal): with e below 2^-21 the remaining error, e^3, is below 2^-63, so
-// the result is the rounding of the last fused multiply-add (half an ulp).
-// Three FP64 instructions where the division takes six.  Outside FP32's range,
-// and for NaN, infinite, zero and negative x, the division itself.
-__device__ __forceinline__ double recip_d(double x) {
-  const unsigned h = (unsigned)__double2hiint(x);
-  if (h - 0x38200000u >= 0x47d00000u - 0x38200000u) return 1.0 / x;
-  const float xf = __uint_as_float(((h - 0x38000000u) << 3) | ((unsigned)__double2loint(x) >> 29));
-  const unsigned r = __float_as_uint(__fdividef(1.f, xf));
-  const double r0 = __hiloint2double((int)((r >> 3) + 0x38000000u), (int)(r << 29));
-  const double e = __fma_rn(-x, r0, 1.0);
-  return __fma_rn(r0, __fma_rn(e, e, e), r0);
 }
 
 // Two forms of each solve, picked by the number of column segments
@@ -1068,7 +1042,7 @@ __global__ void __launch_bounds__(CW, 7) k_solve_stream_f(const Dom<R> *__restri
 }
 
 // Main/mod_moloch.F90:677-721 with divergence_damping :738-765 folded in, FP64
-template <class R>
+template <class R, int LV>
 __global__ void k_sound_momentum(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
                                  int tiles_j,
     const WorkItem *__restrict__ wl) {
@@ -1088,7 +1062,7 @@ __global__ void k_sound_momentum(const Dom<R> *__restrict__ doms, int uvoff, int
   const R *__restrict__ zraw = D.zdiv2;
   const double *__restrict__ pai = D.pai[adv];
   const SoundScratch<R> ss = sound_scratch(D);
-  const Pt q = point_at(wi, 1, 1);
+  const Pt q = point_at<LV>(wi, 1, 1);
   const int j = q.j, i = q.i;
   if (j > g.jx || i > g.iy || q.k > g.kz) return;
   const size_t ij = g.at2(j, i);
@@ -1103,7 +1077,7 @@ __global__ void k_sound_momentum(const Dom<R> *__restrict__ doms, int uvoff, int
   // the constant products dxrdt*xkdamp*msfu, g*dts*hx*gzitakh and coru*dts
   // come from bind time, zcx*cp/2*(theta_v sum) from sound_prep.
 #pragma unroll
-  for (int k = q.k; k < q.k + kPtLevels && k <= g.kz; ++k) {
+  for (int k = q.k; k < q.k + LV && k <= g.kz; ++k) {
     const size_t o = ij + (size_t)(k - 1) * PS;
     if (has_u) {
       double un = u_in[o];
@@ -1153,7 +1127,7 @@ struct West4 {
 // k_sound_div) with lanes of four consecutive columns: 16-byte loads at the
 // lane's points and the row north of them, the east neighbour of the last
 // element read singly, the level below carried from the previous level.
-template <class R>
+template <class R, int LV>
 __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<R> *__restrict__ doms, int uvoff,
                                                       int tiles_j,
     const WorkItem *__restrict__ wl) {
@@ -1166,7 +1140,7 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
   const int bj = wi.a, bi = wi.b;
   const int e0 = (bj * 32 + (int)threadIdx.x) * 4;
   const int i = bi * (int)blockDim.y + (int)threadIdx.y + 1;
-  const int k0 = (int)wi.c * kPtLevels + 1;
+  const int k0 = (int)wi.c * LV + 1;
   if (e0 + 1 > jx - 1 || i > iy - 1 || k0 > kz) return;
   const Scal &c = D.c;
   const Stat<R> &sa = D.sa;
@@ -1176,7 +1150,6 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
   float *__restrict__ zdiv2 = D.zdiv2;
   float *__restrict__ sv = D.s;
   float *__restrict__ w = D.w;
-  const float dtrdx = c.dtrdxsf, dtrdy = dtrdx;
   const unsigned P = (unsigned)g.P, PS = (unsigned)g.PS;
   const unsigned ij = (unsigned)e0 + (unsigned)(i - 1) * P;
   const bool east = e0 + 4 <= jx - 1;  // element 3 has an east neighbour to read
@@ -1205,8 +1178,14 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
   ld4(hy0, sa.hy + ij);
   ld4(hy1, sa.hy + ij + P);
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < 4; ++q) {
     if (!inner[q]) hx0[q] = hx1[q] = hy0[q] = hy1[q] = 0.f;
+    // the face fluxes' 2-D factors dts/dx/m (rotated: dts/dx for u)
+    rmu0[q] = c.lrotllr ? c.dtrdxsf : mul_r(c.dtrdxsf, rmu0[q]);
+    rmu1[q] = c.lrotllr ? c.dtrdxsf : mul_r(c.dtrdxsf, rmu1[q]);
+    rmv0[q] = mul_r(c.dtrdxsf, rmv0[q]);
+    rmv1[q] = mul_r(c.dtrdxsf, rmv1[q]);
+  }
   // the winds of the level below (for s)
   float um[4], upm[4], vm[4], vpm[4];
   if (k0 >= 2 && any_inner) {
@@ -1216,7 +1195,7 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
     ld4(vm, v + om);
     ld4(vpm, v + om + P);
   }
-  for (int k = k0; k < k0 + kPtLevels && k <= kz; ++k) {
+  for (int k = k0; k < k0 + LV && k <= kz; ++k) {
     const unsigned o = ij + (unsigned)(k - 1) * PS;
     float u0[4], u1[4], v0[4], v1[4], fu0[4], fu1[4], fv0[4], fv1[4], fz[4], zd[4];
     ld4(u0, u + o);
@@ -1229,19 +1208,9 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
     ld4(fv1, sa.rfmzv + o + P);
     ld4(fz, sa.fmz + o);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float zum, zup;
-      if (c.lrotllr) {
-        zum = dtrdx * u0[q] * fu0[q];
-        zup = dtrdx * u1[q] * fu1[q];
-      } else {
-        zum = dtrdx * u0[q] * fu0[q] * rmu0[q];
-        zup = dtrdx * u1[q] * fu1[q] * rmu1[q];
-      }
-      const float zvm = dtrdy * v0[q] * fv0[q] * rmv0[q];
-      const float zvp = dtrdy * v1[q] * fv1[q] * rmv1[q];
-      zd[q] = fz[q] * mfac[q] * ((zup - zum) + (zvp - zvm));
-    }
+    for (int q = 0; q < 4; ++q)
+      zd[q] = divergence<float>(mul_r(fz[q], mfac[q]), u0[q], mul_r(fu0[q], rmu0[q]), u1[q], mul_r(fu1[q], rmu1[q]),
+                                v0[q], mul_r(fv0[q], rmv0[q]), v1[q], mul_r(fv1[q], rmv1[q]));
     if (all) {
       *reinterpret_cast<float4 *>(zdiv2 + o) = make_float4(zd[0], zd[1], zd[2], zd[3]);
     } else {
@@ -1254,20 +1223,17 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
         const float gk = sa.gzitak_r[k - 1];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-          if (inner[q]) {
-            const float zuh = (u0[q] + um[q]) * hx0[q] + (u1[q] + upm[q]) * hx1[q];
-            const float zvh = (v0[q] + vm[q]) * hy0[q] + (v1[q] + vpm[q]) * hy1[q];
-            sv[o + q] = -(0.25f * (zuh + zvh) * gk);
-          }
+          if (inner[q])
+            sv[o + q] = mul_r(slope_wind<float>(u0[q] + um[q], hx0[q], u1[q] + upm[q], hx1[q], v0[q] + vm[q], hy0[q],
+                                                v1[q] + vpm[q], hy1[q]),
+                              gk);
       }
       if (k == kz) {
         const unsigned ot = ij + (unsigned)kz * PS;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           if (inner[q]) {
-            const float zuh = u0[q] * hx0[q] + u1[q] * hx1[q];
-            const float zvh = v0[q] * hy0[q] + v1[q] * hy1[q];
-            const float skp1 = -(0.5f * (zuh + zvh));
+            const float skp1 = -0.5f * slope_wind<float>(u0[q], hx0[q], u1[q], hx1[q], v0[q], hy0[q], v1[q], hy1[q]);
             sv[ot + q] = skp1;
             w[ot + q] = -skp1;
           }
@@ -1286,7 +1252,7 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
 // neighbours are the lane's own elements but for the first, read singly.  A
 // block is 32 lanes x 4 rows; grid x = 128-column tiles times row tiles, y =
 // level chunks, z = member.
-template <class R>
+template <class R, int LV>
 __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const Dom<R> *__restrict__ doms,
                                                            int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
@@ -1299,7 +1265,7 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const
   const int bj = wi.a, bi = wi.b;
   const int e0 = (bj * 32 + (int)threadIdx.x) * 4;  // j-1 of the lane's first column
   const int i = bi * (int)blockDim.y + (int)threadIdx.y + 1;
-  const int k0 = (int)wi.c * kPtLevels + 1;
+  const int k0 = (int)wi.c * LV + 1;
   if (e0 + 1 > jx || i > iy || k0 > kz) return;
   const Scal &c = D.c;
   const Stat<R> &sa = D.sa;
@@ -1315,7 +1281,7 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const
   const float *__restrict__ th_l = th_h + F;
   const float *__restrict__ pa_h = reinterpret_cast<const float *>(D.pai[adv]);
   const float *__restrict__ pa_l = pa_h + F;
-  const float dts = c.dtsoundf, dtrdx = c.dtrdxsf, dtrdy = dtrdx, dxrdt = c.dxrdtf;
+  const float dts = c.dtsoundf, dtrdx = c.dtrdxsf, dxrdt = c.dxrdtf;
   const float zfz = float(kGrav) * dts;
   const float halfcp = 0.5f * float(kCpd);
   const unsigned P = (unsigned)g.P;
@@ -1345,7 +1311,18 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const
   ld4i(ibu, sa.ibnd_ud + ij);
   ld4i(ibv, sa.ibnd_vd + ij);
   const int nsp = c.nspgx;
-  for (int k = k0; k < k0 + kPtLevels && k <= kz; ++k) {
+  // the columns' factors coru*dts and g*dts*hx, and v's; 1 for msfv of the
+  // rotated pole
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    cu4[q] = mul_r(cu4[q], dts);
+    hx4[q] = mul_r(zfz, hx4[q]);
+    cv4[q] = mul_r(cv4[q], dts);
+    hy4[q] = mul_r(zfz, hy4[q]);
+    if (c.lrotllr) mv[q] = 1.f;
+  }
+  const float kpg = mul_r(dtrdx, halfcp);
+  for (int k = k0; k < k0 + LV && k <= kz; ++k) {
     const unsigned o = ij + (unsigned)(k - 1) * (unsigned)g.PS;
     float un[4], vn[4], uo[4], vo[4];
     ld4(uo, u_in + o);
@@ -1374,37 +1351,27 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const
       ld4(psl, pa_l + o - P);
     }
     const float gk = sa.gzitakh_r[k - 1];
-    const float xk = sa.xkdamp_r[k - 1];
+    const float xd = mul_r(dxrdt, sa.xkdamp_r[k - 1]);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float a = uo[q];
       if (upd_u[q]) {
-        if (c.divdamp) {
-          const float xdam = dxrdt * xk * mu[q];
-          a = a + xdam * (zr.x[q] - zr.at(q - 1));
-        }
-        const float zrom1u = halfcp * ((th.at(q - 1) + th.x[q]) + (tl.at(q - 1) + tl.x[q]));
-        const float zcor1u = cu4[q] * dts * vo[q];
+        if (c.divdamp) a = fma_r(mul_r(xd, mu[q]), zr.x[q] - zr.at(q - 1), a);
+        const float kp = mul_r(mul_r(kpg, mu[q]), (th.at(q - 1) + th.x[q]) + (tl.at(q - 1) + tl.x[q]));
         const int ib = ibu[q];
         const float bw = ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(k - 1) * nsp] : 1.f;
         const float pd = (ph.x[q] - ph.at(q - 1)) + (pl.x[q] - pl.at(q - 1));
-        const float zcx = dtrdx * mu[q];
-        a = a + bw * (zcor1u - zfz * hx4[q] * gk - zcx * zrom1u * pd);
+        a = fma_r(bw, fma_r(-kp, pd, fma_r(cu4[q], vo[q], -mul_r(hx4[q], gk))), a);
       }
       un[q] = a;
       float b = vo[q];
       if (upd_v[q]) {
-        if (c.divdamp) {
-          const float xdam = c.lrotllr ? dxrdt * xk : dxrdt * xk * mv[q];
-          b = b + xdam * (zr.x[q] - zs[q]);
-        }
-        const float zrom1v = halfcp * ((ts[q] + th.x[q]) + (tsl[q] + tl.x[q]));
-        const float zcor1v = cv4[q] * dts * uo[q];
+        if (c.divdamp) b = fma_r(mul_r(xd, mv[q]), zr.x[q] - zs[q], b);
+        const float kp = mul_r(mul_r(kpg, mv[q]), (ts[q] + th.x[q]) + (tsl[q] + tl.x[q]));
         const int ib = ibv[q];
         const float bw = ib > 0 ? 1.f - sa.hefc_r[(size_t)(ib - 1) + (size_t)(k - 1) * nsp] : 1.f;
         const float pd = (ph.x[q] - ps[q]) + (pl.x[q] - psl[q]);
-        const float zcy = c.lrotllr ? dtrdy : dtrdy * mv[q];
-        b = b + bw * (-zcor1v - zfz * hy4[q] * gk - zcy * zrom1v * pd);
+        b = fma_r(bw, fma_r(-kp, pd, fma_r(-cv4[q], uo[q], -mul_r(hy4[q], gk))), b);
       }
       vn[q] = b;
     }
@@ -1431,8 +1398,7 @@ inline dim3 pt_grid(const LaunchGeom &L, int nj, int ni, int &tiles_j) {
   tiles_j = (nj + L.col_x - 1) / L.col_x;
   if (L.wl_pt) return dim3((unsigned)L.n_pt, 1, 1);  // one block per work item
   const int ti = (ni + L.col_y - 1) / L.col_y;
-  return dim3((unsigned)(tiles_j * ti), (unsigned)((L.kz + kPtLevels - 1) / kPtLevels),
-              (unsigned)L.nmem);
+  return dim3((unsigned)(tiles_j * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
 }
 }  // namespace
 
@@ -1444,7 +1410,8 @@ template <class R>
 void Launch<R>::sound_prep(const LaunchGeom &L, const Dom<R> *d, int advoff, cudaStream_t s) {
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  k_sound_prep<R><<<grd, col_block(L), 0, s>>>(d, advoff, tj, L.wl_pt);
+  if (L.lv == 1) k_sound_prep<R, 1><<<grd, col_block(L), 0, s>>>(d, advoff, tj, L.wl_pt);
+  else k_sound_prep<R, 4><<<grd, col_block(L), 0, s>>>(d, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1452,13 +1419,15 @@ void Launch<R>::sound_div(const LaunchGeom &L, const Dom<R> *d, int uvoff, cudaS
   if constexpr (sizeof(R) == sizeof(float)) {
     const int tj = (L.jx - 1 + 127) / 128, ti = (L.iy - 1 + 3) / 4;
     const dim3 grd = L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
-                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + kPtLevels - 1) / kPtLevels),
+                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv),
                                     (unsigned)L.nmem);
-    k_sound_div_v4<R><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, tj, L.wl_v4);
+    if (L.lv == 1) k_sound_div_v4<R, 1><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, tj, L.wl_v4);
+    else k_sound_div_v4<R, 4><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, tj, L.wl_v4);
   } else {
     int tj;
     const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-    k_sound_div<R><<<grd, col_block(L), 0, s>>>(d, uvoff, tj, L.wl_pt);
+    if (L.lv == 1) k_sound_div<R, 1><<<grd, col_block(L), 0, s>>>(d, uvoff, tj, L.wl_pt);
+    else k_sound_div<R, 4><<<grd, col_block(L), 0, s>>>(d, uvoff, tj, L.wl_pt);
   }
 }
 
@@ -1505,13 +1474,15 @@ void Launch<R>::sound_momentum(const LaunchGeom &L, const Dom<R> *d, int uvoff, 
     // lanes of four columns: 128 columns by 4 rows a block
     const int tj = (L.jx + 127) / 128, ti = (L.iy + 3) / 4;
     const dim3 grd = L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
-                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + kPtLevels - 1) / kPtLevels),
+                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv),
                                     (unsigned)L.nmem);
-    k_sound_momentum_v4<R><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, advoff, tj, L.wl_v4);
+    if (L.lv == 1) k_sound_momentum_v4<R, 1><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, advoff, tj, L.wl_v4);
+    else k_sound_momentum_v4<R, 4><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, advoff, tj, L.wl_v4);
   } else {
     int tj;
     const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-    k_sound_momentum<R><<<grd, col_block(L), 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+    if (L.lv == 1) k_sound_momentum<R, 1><<<grd, col_block(L), 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+    else k_sound_momentum<R, 4><<<grd, col_block(L), 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
   }
 }
 
