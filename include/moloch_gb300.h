@@ -295,11 +295,12 @@ size_t mlc_member_footprint(const mlc_dims *dims, const mlc_params *params);
 typedef struct mlc_tune_report {
   int32_t col_x, col_y;      /* column kernels                        */
   int32_t solve_x, solve_y;  /* accepted for compatibility and reported;
-                                the solves run on 128-column row
-                                segments whatever these say            */
+                                the solves take their form by the
+                                members' sizes whatever these say      */
   int32_t vert_x, vert_y;    /* vertical WAF passes                   */
   int32_t htile;             /* horizontal WAF tile, columns x rows:
-                                0 32x8, 1 64x8, 2 64x4, 3 32x4        */
+                                0 32x8, 1 64x8, 2 64x4, 3 32x4 (until
+                                shapes are set, by the members' sizes) */
   double  ms_fixed;          /* tuned kernel groups, fixed shapes [ms/step] */
   double  ms_tuned;          /* the same groups, picked shapes [ms/step]    */
 } mlc_tune_report;

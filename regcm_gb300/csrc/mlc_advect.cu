@@ -46,32 +46,14 @@ __device__ __forceinline__ long long bits_of(double x) {
   return b;
 }
 
-// -x for an FP64 operand of a fused multiply-add, as a flip of the sign bit
-// in the integer pipe (exact, like the negation itself), so that no FP64
-// instruction forms it (on GB300 every FP64 instruction is 1/64-rate work)
-__device__ __forceinline__ double neg_d(double x) {
-  return __longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ULL);
-}
-
-// x0 + m*(a*b - c*d + e*f) of the horizontal updates.  For FP64 the products
-// are fused explicitly (the second and third into fused multiply-adds), so the
-// rounding does not depend on how the compiler contracts the expression in
-// each tile instantiation: the tile shapes give bit-identical FP64 results.
-// FP32 leaves the contraction to the compiler.  rot: m = 1, no product.
-// chain: the rotated-pole form is x0 + a*b - c*d + e*f, left to right (the
-// zonal update), else x0 + (a*b - c*d + e*f) (the meridional one).
+// x + (gs*cs - gn*cn + dv*p): a WAF update from the fluxes per unit wind of a
+// cell's two faces, the faces' winds times the cell's metric factors, the
+// divergence factor and the field before the update.  The terms, which nearly
+// cancel, are summed before x.  Every rounding is explicit, so the tile shapes
+// give the same bits.
 template <class T>
-__device__ __forceinline__ T stencil_update(T x0, T m, bool rot, bool chain, T a, T b, T c, T d, T e,
-                                            T f) {
-  if constexpr (sizeof(T) == sizeof(double)) {
-    if (rot && chain) return __fma_rn(e, f, __fma_rn(neg_d(c), d, __fma_rn(a, b, x0)));
-    const T t = __fma_rn(e, f, __fma_rn(neg_d(c), d, __dmul_rn(a, b)));
-    return __fma_rn(m, t, x0);  // rot: m = 1, x0 + t exactly as the sum
-  } else {
-    const T z = e * f;
-    if (rot && chain) return x0 + a * b - c * d + z;
-    return rot ? x0 + (a * b - c * d + z) : x0 + m * (a * b - c * d + z);
-  }
+__device__ __forceinline__ T waf_update(T x, T gs, T cs, T gn, T cn, T dv, T p) {
+  return x + fma_r(gs, cs, fma_r(-gn, cn, mul_r(dv, p)));
 }
 
 // The upwind tests zamu >= 0 and zamu > 0.  For FP64 they are made on the
@@ -150,34 +132,18 @@ __device__ __forceinline__ T waf_b(T den, T num) {
   }
   return B;
 }
-template <class T>
-__device__ __forceinline__ T waf_flux(T hvel, bool up, T zamu, T a, T c, T num) {
-  const T den = c - a;
-  const T B = waf_b<T>(den, num);
-  if constexpr (sizeof(T) == sizeof(double)) {
-    // is*den as a choice of den's sign (no FP64 multiply); the fused
-    // multiply-add and the final product are explicit, so that the compiler
-    // cannot fuse them into the caller's arithmetic differently in each tile
-    // instantiation (the tile shapes give bit-identical results)
-    const T sden = up ? den : -den;
-    const T zmi = zamu - (up ? T(1) : T(-1));
-    return __dmul_rn(hvel, (a + c) - __fma_rn(zmi, B, sden));
-  } else {
-    const T is = up ? T(1) : T(-1);
-    return hvel * ((a + c) - (is * den + (zamu - is) * B));
-  }
-}
-// The same flux as vel*(x - zmih*B) with vel = 2*hvel (the wind itself),
-// x = a upwind of a positive zamu (is = +1) else c, and zmih = (zamu - is)/2:
-// (a + c) - is*den = 2x exactly, so in exact arithmetic
-//   hvel*((a + c) - (is*den + (zamu - is)*B)) = vel*(x - zmih*B),
-// one fused multiply-add and one product, with the wind and zmih of an
-// interface formed once for every field.
+// The kernels form it per unit wind: vel*g with vel = 2*hvel (the wind itself),
+// g = x - zmih*B, x = a upwind of a positive zamu (is = +1) else c, and
+// zmih = (zamu - is)/2: (a + c) - is*den = 2x exactly, so in exact arithmetic
+//   hvel*((a + c) - (is*den + (zamu - is)*B)) = vel*(x - zmih*B).
+// One fused multiply-add; the wind joins the cells' metric factors, formed
+// once for every field (FP64, moist 512x512x41, a step: horizontal WAF 4.90 ms
+// with the wind in every flux, 3.65 so; vertical 2.35 and 1.82).
 //
 // FP64 keeps the doubling out of the FP64 pipe: in the regions where B is
-// 2*num or 2*den the flux takes zmi = 2*zmih (exact) as the factor of num or
-// den instead, zmih*(2*sel) = zmi*sel exactly, so only the differences, one
-// fused multiply-add and one product are FP64 instructions.
+// 2*num or 2*den the flux takes 2*zmih (an exponent's increment) as the factor
+// of num or den instead, zmih*(2*sel) = (2*zmih)*sel exactly, so only the
+// differences and one fused multiply-add are FP64 instructions.
 __device__ __forceinline__ double waf_sel(double den, double num, bool &dbl) {
   // the regions of waf_b, tested on the bit patterns
   const long long bden = bits_of(den), bnum = bits_of(num);
@@ -208,45 +174,29 @@ __device__ __forceinline__ T self_diff(T a) {
     return a - a;
   }
 }
-// The same with den = c - a and the upwind value x given (a caller that
-// streams the differences of neighbouring interfaces forms each once: an
-// interface's den is the num of the interfaces on either side)
+// 2x (if dbl) by the exponent, on the integer pipe; zeros, subnormals,
+// infinities and NaN as they are
+__device__ __forceinline__ double twice(double x, bool dbl) {
+  const int h = __double2hiint(x), e = h & 0x7ff00000;
+  return __hiloint2double(dbl && e && e != 0x7ff00000 ? h + 0x00100000 : h, __double2loint(x));
+}
+// g with den = c - a and the upwind value x given (an interface's den is the
+// num of the interfaces on either side: a caller that has the neighbouring
+// differences forms each once); nz = -zmih
 template <class T>
-__device__ __forceinline__ T waf_flux_d(T vel, bool up, T zmih, T zmi, T x, T den, T num) {
+__device__ __forceinline__ T waf_g(T nz, T x, T den, T num) {
   if constexpr (sizeof(T) == sizeof(double)) {
     bool dbl;
     const double sel = waf_sel(den, num, dbl);
-    return __dmul_rn(vel, __fma_rn(neg_d(dbl ? zmi : zmih), sel, x));
+    return __fma_rn(twice(nz, dbl), sel, x);
   } else {
-    (void)zmi;
-    const T B = waf_b<T>(den, num);
-    return vel * fmaf(-zmih, B, x);
+    return fmaf(nz, waf_b<T>(den, num), x);
   }
 }
+// -zmih = (is - zamu)/2 of an interface
 template <class T>
-__device__ __forceinline__ T waf_flux_h(T vel, bool up, T zmih, T zmi, T a, T c, T num) {
-  const T den = c - a;
-  const T x = up ? a : c;
-  if constexpr (sizeof(T) == sizeof(double)) {
-    bool dbl;
-    const double sel = waf_sel(den, num, dbl);
-    return __dmul_rn(vel, __fma_rn(neg_d(dbl ? zmi : zmih), sel, x));
-  } else {
-    (void)zmi;
-    const T B = waf_b<T>(den, num);
-    return vel * fmaf(-zmih, B, x);
-  }
-}
-// zmi = zamu - is and zmih = zmi/2 of an interface (the halving is exact)
-template <class T>
-__device__ __forceinline__ T waf_zmi(T zamu, bool up) {
-  if constexpr (sizeof(T) == sizeof(double)) return __dadd_rn(zamu, up ? -1.0 : 1.0);
-  else return zamu - (up ? 1.f : -1.f);
-}
-template <class T>
-__device__ __forceinline__ T waf_zmih(T zamu, bool up) {
-  if constexpr (sizeof(T) == sizeof(double)) return __dmul_rn(waf_zmi<T>(zamu, up), 0.5);
-  else return waf_zmi<T>(zamu, up) * 0.5f;
+__device__ __forceinline__ T waf_nz(T zamu, bool up) {
+  return fma_r(T(-0.5), zamu, up ? T(0.5) : T(-0.5));
 }
 
 // The advected fields of a member, in the reference's order (tetav, pai,
@@ -362,18 +312,17 @@ __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advof
       D.tkex[adv][o] = a;
     }
     if constexpr (sizeof(R) == sizeof(double)) {
-      // the vertical WAF update's factor s(k)*zu(k) - s(k+1)*zd(k), and the
-      // flux factors of interface k+1 - zamu = s*dtrdz, zmi = zamu - is and
-      // zmih = zmi/2 - once for all fields (FP64 arithmetic is the FP64
-      // path's bound)
+      // the vertical WAF's factors, once for all fields (FP64 arithmetic is
+      // the FP64 path's bound): s(k)*zu(k) and s(k+1)*zd(k) of the level's
+      // fluxes, their difference, and -zmih of interface k+1, whose sign bit
+      // of zamu's factor s(k+1) says which side is upwind
       const double skp = D.s[o + PS];
-      D.vdiv[o] = __fma_rn(neg_d(skp), D.sa.zrfmd[o], __dmul_rn(D.s[o], D.sa.zrfmu[o]));
-      const double dtrdz = 0.5 * (D.c.dtstepa * D.c.rdzita);
-      const double zamu = __dmul_rn(skp, dtrdz);
-      const double zmi = waf_zmi<double>(zamu, nonneg(zamu));
-      D.vzamu[o] = zamu;
-      D.vzmi[o] = zmi;
-      D.vzmih[o] = __dmul_rn(zmi, 0.5);
+      const double cu = __dmul_rn(D.s[o], D.sa.zrfmu[o]), cd = __dmul_rn(skp, D.sa.zrfmd[o]);
+      D.vcu[o] = cu;
+      D.vcd[o] = cd;
+      D.vdiv[o] = cu - cd;
+      const double zamu = __dmul_rn(skp, 0.5 * (D.c.dtstepa * D.c.rdzita));
+      D.vnz[o] = waf_nz<double>(zamu, nonneg(zamu));
     }
   }
 }
@@ -386,49 +335,36 @@ __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advof
 // the column never touches shared memory.  R is the type of the winds and
 // metric, T that of the advected field and of the arithmetic.  Fluxes and
 // updates are the reference's expressions, operand for operand.
+// the flux per unit s through interface k+1 between levels k and k+1, its
+// upwind difference col(k1) - col(k1p1) with the reference's clamps
+// k1p1 = min(k+2, kz), k1 = max(k-1, 1); d: the differences c(k) - c(k+1) of
+// the interface itself, of the one above it (k-1, k) and below it (k+1, k+2)
 template <class T>
-__device__ __forceinline__ T vflux(T dtrdz, T skp, T cm1, T ck, T cp1, T cp2, int k, int kz) {
-  // interface k+1 between levels k and k+1; the upwind difference col(k1) -
-  // col(k1p1) with the reference's clamps k1p1 = min(k+2, kz), k1 = max(k-1, 1)
-  const T zamu = skp * dtrdz;
-  const bool up = nonneg(zamu);
-  T num;
-  if (up) num = k + 2 <= kz ? cp1 - cp2 : cp1 - cp1;
-  else num = k >= 2 ? cm1 - ck : ck - ck;
-  const T zmi = waf_zmi<T>(zamu, up);
-  return waf_flux_h<T>(skp, up, zmi * T(0.5), zmi, cp1, ck, num);
+__device__ __forceinline__ T vflux(T nz, bool up, T ck, T cp1, T d_above, T d, T d_below, int k, int kz) {
+  const T num = up ? (k + 2 <= kz ? d_below : self_diff<T>(cp1)) : (k >= 2 ? d_above : self_diff<T>(ck));
+  return waf_g<T>(nz, up ? cp1 : ck, d, num);
 }
-// the same with the interface's factors given (an FP64 member, k_adv_prep)
-struct VIf {
-  double zamu, zmih, zmi;
-};
-__device__ __forceinline__ double vflux_p(double skp, const VIf &t, double cm1, double ck, double cp1,
-                                          double cp2, int k, int kz) {
-  const bool up = nonneg(t.zamu);
-  double num;
-  if (up) num = k + 2 <= kz ? cp1 - cp2 : cp1 - cp1;
-  else num = k >= 2 ? cm1 - ck : ck - ck;
-  return waf_flux_h<double>(skp, up, t.zmih, t.zmi, cp1, ck, num);
-}
+// (levels inside, where no clamp acts)
 template <class T>
-__device__ __forceinline__ T vupdate(T pk, T fb, T fa, T sk, T skp, T zu, T zd) {
-  const T zdv = (sk * zu - skp * zd) * pk;
-  return pk - fb * zu + fa * zd + zdv;
+__device__ __forceinline__ T vflux_in(T nz, bool up, T ck, T cp1, T d_above, T d, T d_below) {
+  return waf_g<T>(nz, up ? cp1 : ck, d, up ? d_below : d_above);
 }
-// the same with the factor sk*zu - skp*zd given (FP64: from adv_prep), the
-// products fused explicitly
+// pk - gb*cu + ga*cd + dv*pk: gb, ga the fluxes per unit s of the interfaces
+// above and below, cu and cd s times their metric ratios, dv = cu - cd
 template <class T>
-__device__ __forceinline__ T vupdate_f(T pk, T fb, T fa, T dv, T zu, T zd) {
-  return __fma_rn(dv, pk, __fma_rn(fa, zd, __fma_rn(neg_d(fb), zu, pk)));
+__device__ __forceinline__ T vupdate(T pk, T gb, T ga, T dv, T cu, T cd) {
+  return fma_r(dv, pk, fma_r(ga, cd, fma_r(-gb, cu, pk)));
 }
 
 // Blocks of 256 threads an SM the vertical WAF is compiled for, FP64 and FP32
-// (0: no bound, the compiler's own register choice).
+// (0: no bound, the compiler's own register choice).  FP32 3/4/5/6 blocks:
+// 309/283/252/313 us a moist 512x512x41 step; FP64 2 (by its registers) and 3:
+// 1820 and 1988 us.
 #ifndef MLC_VERT_MINB_D
 #define MLC_VERT_MINB_D 0
 #endif
 #ifndef MLC_VERT_MINB_F
-#define MLC_VERT_MINB_F 4
+#define MLC_VERT_MINB_F 5
 #endif
 template <class T>
 constexpr int vert_min_blocks() {
@@ -436,9 +372,6 @@ constexpr int vert_min_blocks() {
 }
 // Levels an FP32 column loads ahead of the one it computes (1 or 2; two
 // measured no faster on the moist 512x512x41 step, 0.256 ms a step both).
-#ifndef MLC_VPF_F
-#define MLC_VPF_F 1
-#endif
 // grid: x = column tiles along j times the fields (field fastest, so the
 // blocks reading one column's s and metric run together), y = row tiles,
 // z = member; block (vert_x, vert_y) columns along (j, i)
@@ -446,7 +379,6 @@ template <class R, class T>
 __global__ void __launch_bounds__(256, vert_min_blocks<T>())
     k_adv_vertical(const Dom<R> *__restrict__ doms, int nf, int set, int advoff,
                                const WorkItem *__restrict__ wl) {
-  constexpr int kVpf = sizeof(T) == sizeof(float) ? MLC_VPF_F : 1;  // levels loaded ahead
   const WorkItem wi = wl ? wl[blockIdx.x]
                           : WorkItem{(int16_t)blockIdx.z, (int16_t)(blockIdx.x / (unsigned)nf),
                                      (int16_t)blockIdx.y, (int16_t)(blockIdx.x % (unsigned)nf)};
@@ -473,151 +405,111 @@ __global__ void __launch_bounds__(256, vert_min_blocks<T>())
   const R *__restrict__ zup = D.sa.zrfmu + ij;
   const R *__restrict__ zdp = D.sa.zrfmd + ij;
   const unsigned PS = (unsigned)g.PS;  // a domain's fields stay below 2^31 elements
-  const T dtrdz = T(0.5) * (pick<T>(c.dtstepa, c.dtstepaf) * pick<T>(c.rdzita, c.rdzitaf));
+  // -1/2 of the factor of s in zamu
+  const T hdtrdz = T(-0.25) * (pick<T>(c.dtstepa, c.dtstepaf) * pick<T>(c.rdzita, c.rdzitaf));
 
-  // windows: pass-1 input at k-1..k+2, pass-1 output at k-3..k-1, s at
-  // k-2..k+1, metric at k-2..k-1, the pass-1 flux at interface k and the
-  // pass-2 flux at interface k-2
-  T c0m1 = T(0), c0k = src[0], c0p1 = src[PS];
-  T c1m3 = T(0), c1m2 = T(0), c1m1 = T(0);
-  T sm2 = T(0), sm1 = T(0), sk = T(sp[0]);
-  T zum2 = T(0), zdm2 = T(0), zum1 = T(0), zdm1 = T(0);
-  T f1k = T(0), f2m = T(0);
-  // differences c(k) - c(k+1) of the pass-1 input at interfaces k-1, k (d1p,
-  // d1c) and of the pass-2 input at m-1, m (d2p, d2c): an interface's den is
-  // the num of its neighbours, so each difference is formed once
-  T d1p = T(0), d1c = T(0), d2p = T(0), d2c = T(0);
-  // FP64 member: the update's divergence factor, precomputed per level
+  // windows: pass-1 input at k..k+1, pass-1 output at k-2..k-1, levels k-2 and
+  // k-1 as loaded, the pass-1 flux at interface k and the pass-2 flux at
+  // interface k-2, and the differences c(k) - c(k+1) of the pass-1 input at
+  // interfaces k-1, k and of the pass-2 input at m-1, m (m = k-2)
   constexpr bool kPre = sizeof(R) == sizeof(double) && sizeof(T) == sizeof(double);
+  // A level's factors: FP64 those of k_adv_prep.  FP32 forms them from s(k),
+  // s(k+1) and the metric (a plane less to read), for the second pass again:
+  // what a level carries between the passes is then four registers instead of
+  // five, which fits five blocks an SM (moist 512x512x41: 252 us a step; 268
+  // with the wind in the fluxes, 280 with the factors kept)
+  struct Fac {
+    T cu, cd, dv, nz;
+    bool up;  // of interface k+1: the cell below is upwind
+  };
+  struct Lev {
+    T a, b, c, d;  // FP64: cu, cd, dv, nz.  FP32: zu, zd
+    T s, sp;       // s(k), s(k+1)
+    bool up;
+  };
+  const double *__restrict__ cup = kPre ? D.vcu + ij : nullptr;
+  const double *__restrict__ cdp = kPre ? D.vcd + ij : nullptr;
   const double *__restrict__ dvp = kPre ? D.vdiv + ij : nullptr;
-  T dvm2 = T(0), dvm1 = T(0), n_dv = kPre ? T(dvp[0]) : T(0);
-  // FP64 member: the interface factors (zamu, hvel, zmi) of interfaces k+1,
-  // k and k-1 (pass 1 at k, pass 2 at k-2), the next level's loaded ahead
-  const double *__restrict__ zap = kPre ? D.vzamu + ij : nullptr;
-  const double *__restrict__ zmp = kPre ? D.vzmih + ij : nullptr;
-  const double *__restrict__ z2p = kPre ? D.vzmi + ij : nullptr;
-  VIf tkm1{0, 0, 0}, tkm2{0, 0, 0};
-  VIf n_t = kPre ? VIf{zap[0], zmp[0], z2p[0]} : VIf{0, 0, 0};
-  // the next level's loads, issued one level ahead (kVpf = 2: the level
-  // after it too, in m_*)
-  T n_s = T(sp[PS]), n_c = src[2 * PS], n_zu = T(zup[0]), n_zd = T(zdp[0]);
-  T m_s = T(0), m_c = T(0), m_zu = T(0), m_zd = T(0), m_dv = T(0);
-  VIf m_t{0, 0, 0};
-  if constexpr (kVpf == 2) {
-    if (kz >= 2) {
-      m_s = T(sp[2 * PS]);
-      m_zu = T(zup[PS]);
-      m_zd = T(zdp[PS]);
-      if constexpr (kPre) {
-        m_dv = T(dvp[PS]);
-        m_t = VIf{zap[PS], zmp[PS], z2p[PS]};
-      }
+  const double *__restrict__ nzp = kPre ? D.vnz + ij : nullptr;
+  auto load = [&](unsigned o) {
+    Lev r{};
+    r.sp = T(sp[o + PS]);
+    if constexpr (kPre) {
+      r.a = T(cup[o]); r.b = T(cdp[o]); r.c = T(dvp[o]); r.d = T(nzp[o]);
+    } else {
+      r.a = T(zup[o]); r.b = T(zdp[o]);
     }
-    if (kz >= 4) m_c = src[3 * PS];
-  }
+    return r;
+  };
+  auto factors = [&](const Lev &r) {
+    if constexpr (kPre) {
+      return Fac{r.a, r.b, r.c, r.d, r.up};
+    } else {
+      const T cu = mul_r(r.s, r.a), cd = mul_r(r.sp, r.b);
+      const bool up = nonneg(r.sp);
+      return Fac{cu, cd, cu - cd, fma_r(r.sp, hdtrdz, up ? T(0.5) : T(-0.5)), up};
+    }
+  };
+  T c0k = src[0], c0p1 = src[PS];
+  T c1m2 = T(0), c1m1 = T(0);
+  T sk = kPre ? T(0) : T(sp[0]);
+  T f1k = T(0), f2m = T(0);
+  T d1p = T(0), d1c = c0k - c0p1, d2p = T(0), d2c = T(0);
+  Lev l1{}, l2{};  // levels k-1, k-2
+  // the next level's loads, issued one level ahead
+  Lev n_l = load(0);
+  T n_c = src[2 * PS];
   // level k; every bound check is known to hold inside the column
-  // (4 <= k <= kz-3, kz-4 with two levels ahead), so the interior steps
-  // carry none
+  // (4 <= k <= kz-3), so the interior steps carry none
   auto step = [&](int k, auto interior) {
     constexpr bool I = decltype(interior)::value;
     const unsigned o = (unsigned)(k - 1) * PS;
-    const T skp1 = n_s, c0p2 = (I || k + 2 <= kz) ? n_c : T(0), zuk = n_zu, zdk = n_zd;
-    const T dvk = n_dv;
-    const VIf tk = n_t;
-    if constexpr (kVpf == 2) {
-      // the level after next: s at k+3, the metric at k+2, c at k+4
-      n_s = m_s; n_zu = m_zu; n_zd = m_zd; n_c = m_c;
-      if constexpr (kPre) { n_dv = m_dv; n_t = m_t; }
-      if (I || k + 2 <= kz) {
-        if constexpr (kPre) {
-          m_dv = T(dvp[o + 2 * PS]);
-          m_t = VIf{zap[o + 2 * PS], zmp[o + 2 * PS], z2p[o + 2 * PS]};
-        }
-        m_s = T(sp[o + 3 * PS]);
-        m_zu = T(zup[o + 2 * PS]);
-        m_zd = T(zdp[o + 2 * PS]);
-        if (I || k + 4 <= kz) m_c = src[o + 4 * PS];
-      }
-    } else if (I || k < kz) {
-      if constexpr (kPre) {
-        n_dv = T(dvp[o + PS]);
-        n_t = VIf{zap[o + PS], zmp[o + PS], z2p[o + PS]};
-      }
-      n_s = T(sp[o + 2 * PS]);
-      n_zu = T(zup[o + PS]);
-      n_zd = T(zdp[o + PS]);
+    Lev l = n_l;
+    const T c0p2 = (I || k + 2 <= kz) ? n_c : T(0);
+    if (I || k < kz) {
+      n_l = load(o + PS);
       if (I || k + 3 <= kz) n_c = src[o + 3 * PS];
     }
-    T f1kp;
-    const T d1n = c0p1 - c0p2;  // the next interface's den, this one's upwind num
     if constexpr (kPre) {
-      if (I) {
-        const bool up = nonneg(tk.zamu);
-        f1kp = waf_flux_d<double>(skp1, up, tk.zmih, tk.zmi, up ? c0p1 : c0k, d1c, up ? d1n : d1p);
-      } else {
-        f1kp = k <= kz - 1 ? vflux_p(skp1, tk, c0m1, c0k, c0p1, c0p2, k, kz) : T(0);
-      }
-    } else if (I) {
-      const T zamu = skp1 * dtrdz;
-      const bool up = nonneg(zamu);
-      const T zmi = waf_zmi<T>(zamu, up);
-      f1kp = waf_flux_d<T>(skp1, up, zmi * T(0.5), zmi, up ? c0p1 : c0k, d1c, up ? d1n : d1p);
+      l.up = nonneg(l.sp);  // zamu has s's sign
     } else {
-      f1kp = k <= kz - 1 ? vflux<T>(dtrdz, skp1, c0m1, c0k, c0p1, c0p2, k, kz) : T(0);
+      l.s = sk;
+      sk = l.sp;
     }
-    T c1k;
-    if constexpr (kPre) c1k = vupdate_f<T>(c0k, f1k, f1kp, dvk, zuk, zdk);
-    else c1k = vupdate<T>(c0k, f1k, f1kp, sk, skp1, zuk, zdk);
+    const Fac t = factors(l);
+    const T d1n = c0p1 - c0p2;  // the next interface's difference, this one's upwind one
+    T f1kp;
+    if (I) f1kp = vflux_in<T>(t.nz, t.up, c0k, c0p1, d1p, d1c, d1n);
+    else f1kp = k <= kz - 1 ? vflux<T>(t.nz, t.up, c0k, c0p1, d1p, d1c, d1n, k, kz) : T(0);
+    const T c1k = vupdate<T>(c0k, f1k, f1kp, t.dv, t.cu, t.cd);
     const T d2n = c1m1 - c1k;
     if (I || k >= 3) {  // pass 2 at level m = k-2
+      const Fac t2 = factors(l2);
       T f2n;
-      if constexpr (kPre) {
-        if (I) {
-          const bool up = nonneg(tkm2.zamu);
-          f2n = waf_flux_d<double>(sm1, up, tkm2.zmih, tkm2.zmi, up ? c1m1 : c1m2, d2c, up ? d2n : d2p);
-        } else {
-          f2n = vflux_p(sm1, tkm2, c1m3, c1m2, c1m1, c1k, k - 2, kz);
-        }
-      } else if (I) {
-        const T zamu = sm1 * dtrdz;
-        const bool up = nonneg(zamu);
-        const T zmi = waf_zmi<T>(zamu, up);
-        f2n = waf_flux_d<T>(sm1, up, zmi * T(0.5), zmi, up ? c1m1 : c1m2, d2c, up ? d2n : d2p);
-      } else {
-        f2n = vflux<T>(dtrdz, sm1, c1m3, c1m2, c1m1, c1k, k - 2, kz);
-      }
-      if constexpr (kPre) dst[o - 2 * PS] = vupdate_f<T>(c1m2, f2m, f2n, dvm2, zum2, zdm2);
-      else dst[o - 2 * PS] = vupdate<T>(c1m2, f2m, f2n, sm2, sm1, zum2, zdm2);
+      if (I) f2n = vflux_in<T>(t2.nz, t2.up, c1m2, c1m1, d2p, d2c, d2n);
+      else f2n = vflux<T>(t2.nz, t2.up, c1m2, c1m1, d2p, d2c, d2n, k - 2, kz);
+      dst[o - 2 * PS] = vupdate<T>(c1m2, f2m, f2n, t2.dv, t2.cu, t2.cd);
       f2m = f2n;
     }
-    c0m1 = c0k; c0k = c0p1; c0p1 = c0p2;
-    c1m3 = c1m2; c1m2 = c1m1; c1m1 = c1k;
+    c0k = c0p1; c0p1 = c0p2;
+    c1m2 = c1m1; c1m1 = c1k;
     d1p = d1c; d1c = d1n; d2p = d2c; d2c = d2n;
-    sm2 = sm1; sm1 = sk; sk = skp1;
-    zum2 = zum1; zdm2 = zdm1; zum1 = zuk; zdm1 = zdk;
-    dvm2 = dvm1; dvm1 = dvk;
-    tkm2 = tkm1; tkm1 = tk;
+    l2 = l1; l1 = l;
     f1k = f1kp;
   };
   using edge = std::integral_constant<bool, false>;
   using mid = std::integral_constant<bool, true>;
-  const int k1 = min(3, kz), k2 = max(4, kz - (kVpf == 2 ? 3 : 2));
+  const int k1 = min(3, kz), k2 = max(4, kz - 2);
   for (int k = 1; k <= k1; ++k) step(k, edge{});
 #pragma unroll 4
   for (int k = 4; k < k2; ++k) step(k, mid{});
   for (int k = k2; k <= kz; ++k) step(k, edge{});
   // pass 2 at levels kz-1 (flux through interface kz) and kz (none above)
   const unsigned ot = (unsigned)(kz - 1) * PS;
-  T f2n;
-  if constexpr (kPre) f2n = vflux_p(sm1, tkm2, c1m3, c1m2, c1m1, c1m1, kz - 1, kz);
-  else f2n = vflux<T>(dtrdz, sm1, c1m3, c1m2, c1m1, c1m1, kz - 1, kz);
-  if constexpr (kPre) {
-    dst[ot - PS] = vupdate_f<T>(c1m2, f2m, f2n, dvm2, zum2, zdm2);
-    dst[ot] = vupdate_f<T>(c1m1, f2n, T(0), dvm1, zum1, zdm1);
-  } else {
-    dst[ot - PS] = vupdate<T>(c1m2, f2m, f2n, sm2, sm1, zum2, zdm2);
-    dst[ot] = vupdate<T>(c1m1, f2n, T(0), sm1, sk, zum1, zdm1);
-  }
+  const Fac t1 = factors(l1), t2 = factors(l2);
+  const T f2n = vflux<T>(t2.nz, t2.up, c1m2, c1m1, d2p, d2c, T(0), kz - 1, kz);
+  dst[ot - PS] = vupdate<T>(c1m2, f2m, f2n, t2.dv, t2.cu, t2.cd);
+  dst[ot] = vupdate<T>(c1m1, f2n, T(0), t1.dv, t1.cu, t1.cd);
 }
 
 // ---- lane vectors ---------------------------------------------------------
@@ -685,20 +577,20 @@ __device__ __forceinline__ void next_col(T (&e)[V], const T (&x)[V]) {
 // flux of row I0+nw); the intermediate p0 follows; the zonal fluxes take
 // their neighbours' p0 from the adjacent lanes by shuffles, and the result
 // goes to the field's other buffer (the halo of other tiles still needs the
-// old values).  A warp's range is 32*v columns, of which it writes the
-// middle 32*v - 4 (a column's zonal update needs p0 two columns either
-// side); tiles overlap by four columns.  Per field the expressions are the
-// reference's, operand for operand.
+// old values).  A warp's range is 32*v columns, of which an inner tile writes
+// the middle 32*v - 4 (hshape_writes); tiles overlap by four columns.
 // Resident warps an SM the WAF tile kernels are compiled for; the register
-// budget follows (65536 / (32 * warps) a thread).  Measured on the moist
-// 512x512x41 step: FP32 horizontal WAF at 40 warps (48 registers, 12 bytes
-// spilled) 0.455 ms a step, at 32 (64 registers) 0.464, at 16 warps (90
-// registers) 0.72; the increment form at 32
-// warps (64 registers, 32 bytes spilled) 0.27 against 0.29 at 24 and 0.37 at
-// 20.  FP64 at 16 warps (128 registers): the FP64 pipe is the bound, but 8
-// warps an SM leave it idle (6.98 against 7.83 ms).
+// budget follows (65536 / (32 * warps) a thread).  FP32, moist 512x512x41, a
+// step: 64-column tiles at 40 warps (48 registers) 0.378 ms, at 32 0.434;
+// 128-column tiles at 32 warps 0.351, at 24 0.394, at 40 (spilled) 0.471.
+// The increment form at 32 warps (64 registers) 0.223 and 0.250 at 40 warps;
+// in 128-column tiles at 16 warps (128 registers) 0.267, at 24 0.313.  FP64
+// at 16 warps (108 registers): the FP64 pipe is the bound.
 #ifndef MLC_HWAF_WARPS
 #define MLC_HWAF_WARPS 40
+#endif
+#ifndef MLC_HWAF_WARPS_4
+#define MLC_HWAF_WARPS_4 32
 #endif
 #ifndef MLC_HWAF_WARPS_D
 #define MLC_HWAF_WARPS_D 16
@@ -706,27 +598,27 @@ __device__ __forceinline__ void next_col(T (&e)[V], const T (&x)[V]) {
 #ifndef MLC_HINC_WARPS
 #define MLC_HINC_WARPS 32
 #endif
+#ifndef MLC_HINC_WARPS_4
+#define MLC_HINC_WARPS_4 16
+#endif
 template <class R>
 constexpr int waf_min_blocks(int warps, int nw) {
   return warps / nw > 1 ? warps / nw : 1;
 }
 template <class R, int V, int NW>
 __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof(float)
-                                                                   ? MLC_HWAF_WARPS
+                                                                   ? (V == 4 ? MLC_HWAF_WARPS_4 : MLC_HWAF_WARPS)
                                                                    : MLC_HWAF_WARPS_D, NW))
     k_adv_horizontal(const Dom<R> *__restrict__ doms,
                                                            int tiles_j, int uvoff, int advoff,
     const WorkItem *__restrict__ wl) {
   using T = R;
   constexpr int W = 32 * V;       // columns of a warp's range
-  constexpr int S = W - 4;        // columns it writes: range columns 2 .. W-3
-  constexpr int OB0 = hshape_ob0(V);
-  constexpr int OFF = hshape_off((int)sizeof(T), V);
-  constexpr int BW = W + 2 * OFF;  // halo tile row: range column c sits at c + OFF
-  constexpr unsigned kBox = (unsigned)((NW + 4) * BW * sizeof(T));
+  constexpr int S = W - 4;        // columns from a tile to the next (hshape_writes)
+  constexpr unsigned kBox = (unsigned)((NW + 4) * W * sizeof(T));
   constexpr unsigned kBuf = (kBox + 127u) / 128u * 128u;
   constexpr int kStages = 4;  // halo tiles in flight: the next three fields land while one is used
-  constexpr int shape = V == 1 ? (NW == 8 ? 0 : 3) : (NW == 8 ? 1 : 2);
+  constexpr int shape = V == 1 ? (NW == 8 ? 0 : 3) : V == 2 ? (NW == 8 ? 1 : 2) : 4;
   static_assert(hshape((int)sizeof(T), shape).v == V && hshape((int)sizeof(T), shape).nw == NW,
                 "tile shape table");
   __shared__ __align__(128) unsigned char wzraw[kStages][kBuf];  // TMA destinations
@@ -743,9 +635,9 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
   const int jx = g.jx, iy = g.iy;
   if (k > g.kz) return;
   const int bj = wi.a, bi = wi.b;
-  const int ob = bj * S + OB0;  // column offset (j - 1) of the range's first column
+  const int ob = bj * S;        // column offset (j - 1) of the range's first column
   const int I0 = bi * NW + 1;
-  if (ob + 3 > jx - 1 || I0 > iy - 1) return;
+  if (bj >= hshape_tiles(V, jx) || I0 > iy - 1) return;
   const Scal &c = D.c;
   const Stat<R> &sa = D.sa;
   const int uv = (D.clk->uv_role + uvoff) & 1, adv = (D.clk->adv_role + advoff) & 1;
@@ -759,15 +651,15 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
   const T *__restrict__ uk = D.u[uv] + ko;
   const T *__restrict__ vk = D.v[uv] + ko;
   const T dta = pick<T>(c.dtstepa, c.dtstepaf);
-  const T dtrdx = dta * pick<T>(c.rdx, c.rdxf), dtrdy = dta * pick<T>(c.rdx, c.rdxf);
+  const T dtr = dta * pick<T>(c.rdx, c.rdxf);
   const bool rot = c.lrotllr != 0;
   const int nf = n_table_r(D);
   const char *tmaps = static_cast<const char *>(D.tmap) + (size_t)shape * kTmapSlots * kTmapBytes;
-  auto tile = [&](int b) { return reinterpret_cast<T(*)[BW]>(wzraw[b]); };
+  auto tile = [&](int b) { return reinterpret_cast<T(*)[W]>(wzraw[b]); };
   auto issue = [&](int fld, int b) {  // one thread: the halo tile of field fld into buffer b
     fence_proxy_async();
     mbar_expect_tx(&mbar[b], kBox);
-    tma_load_3d(wzraw[b], tmaps + (size_t)fld * kTmapBytes, ob - OFF, I0 - 3, k - 1, &mbar[b]);
+    tma_load_3d(wzraw[b], tmaps + (size_t)fld * kTmapBytes, ob, I0 - 3, k - 1, &mbar[b]);
   };
   if (tid == 0) {
     for (int q = 0; q < kStages; ++q) mbar_init(&mbar[q], 1);
@@ -804,22 +696,23 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
   // forms more than three flux rows' worth before the block barrier (the
   // last warp alone would form four); with one column a lane the last warp
   // takes them.  ec0 is the range column of the lane's first one there.
-  constexpr int VE = V == 2 && NW >= 2 ? 1 : V;
-  const bool eWarp = VE == 1 && V == 2 ? wp >= NW - 2 : wp == NW - 1;
-  const int ec0 = VE == 1 && V == 2 ? (wp - (NW - 2)) * 32 + lane : V * lane;
+  constexpr int VE = NW >= V ? 1 : V;
+  const bool eWarp = VE == 1 ? wp >= NW - V : wp == NW - 1;
+  const int ec0 = VE == 1 ? (wp - (NW - V)) * 32 + lane : V * lane;
   const int eE0 = ob + ec0;
-  T vv[V], zmy[V], vve[VE], zmye[VE];
-  bool mv[V], me[VE];  // meridional flux defined at the column (row i, row I0+NW)
+  // Courant numbers of the faces south of the lane's points, of row I0+NW and
+  // west of the points, as upwind flags (zamu > 0) and -zmih
+  bool upy[V], upe[VE], upx[V];
+  T nzy[V], nze[VE], nzx[V];
   {
     T a[V], b[V];
     ld_row<T, V>(a, vk, e0, i, P, okM);
     ld_row<T, V>(b, sa.msfv, e0, i, P, okM && !rot);
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const bool ok = okM && jq[q] >= 1 && jq[q] <= jx - 1;
-      mv[q] = ok;
-      vv[q] = ok ? a[q] : T(0);  // the flux's wind v (= 2*hvel)
-      zmy[q] = ok ? (rot ? a[q] * dtrdy : a[q] * b[q] * dtrdy) : T(0);
+      const T z = mul_r(rot ? a[q] : mul_r(a[q], b[q]), dtr);
+      upy[q] = positive(z);
+      nzy[q] = waf_nz<T>(z, upy[q]);
     }
     const int ie = I0 + NW;
     const bool okE = eWarp && eE0 >= 0 && eE0 + VE <= g.P && ie >= 2 && ie <= iy - 1;
@@ -828,17 +721,18 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
     ld_row<T, VE>(be, sa.msfv, eE0, ie, P, okE && !rot);
 #pragma unroll
     for (int q = 0; q < VE; ++q) {
-      const int je = eE0 + q + 1;
-      const bool ok = okE && je >= 1 && je <= jx - 1;
-      me[q] = ok;
-      vve[q] = ok ? ae[q] : T(0);
-      zmye[q] = ok ? (rot ? ae[q] * dtrdy : ae[q] * be[q] * dtrdy) : T(0);
+      const T z = mul_r(rot ? ae[q] : mul_r(ae[q], be[q]), dtr);
+      upe[q] = positive(z);
+      nze[q] = waf_nz<T>(z, upe[q]);
     }
   }
-  T zs[V], zn[V], dvy[V], m2[V], uu[V], zmx[V], zw[V], ze[V], dvx[V];
-  bool pv[V], xv[V], rv[V];  // p0, zonal flux, interior update defined at the column
+  // the faces' winds times dt/dx and the metric factors of the cell between
+  // them (cs, cn; cw, ce) and the divergence factors (dvy, dvx), with
+  // a = dt/dx*fmz*m^2 (rotated pole: *m).  rfmzu on the south and north faces
+  // as in the reference (Main/mod_moloch.F90:1000-1001).
+  T cs[V], cn[V], dvy[V], cw[V], ce[V], dvx[V];
   {
-    T fz[V], vi[V], vn[V], ri[V], rn[V], fi[V], fn[V], mf[V], ui[V], rmui[V], msu[V];
+    T fz[V], vi[V], vn[V], ri[V], rn[V], fi[V], fn[V], mf[V], ui[V], rw[V], msu[V];
     ld_row<T, V>(fz, sa.fmz + ko, e0, i, P, okP);
     ld_row<T, V>(vi, vk, e0, i, P, okP);
     ld_row<T, V>(vn, vk, e0, i + 1, P, okP);
@@ -848,69 +742,26 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
     ld_row<T, V>(fn, (rot ? sa.rfmzv : sa.rfmzu) + ko, e0, i + 1, P, okP);
     ld_row<T, V>(mf, rot ? sa.msfx : sa.mx2, e0, i, P, okP);
     ld_row<T, V>(ui, uk, e0, i, P, okP);
-    ld_row<T, V>(rmui, sa.rmu, e0, i, P, okP && !rot);
+    ld_row<T, V>(rw, sa.rmu, e0, i, P, okP && !rot);
     ld_row<T, V>(msu, sa.msfu, e0, i, P, okP);
-#pragma unroll
-    for (int q = 0; q < V; ++q) {
-      const int j = jq[q];
-      pv[q] = okP && j >= 1 && j <= jx - 1;
-      xv[q] = okP && j >= 2 && j <= jx - 1;
-      rv[q] = okP && j >= 2 && j <= jx - 2;
-      if (rot) {
-        const T zhxvtn = dtrdy * rn[q] * mf[q];
-        const T zhxvts = dtrdy * ri[q] * mf[q];
-        zn[q] = zhxvtn * fz[q] * fn[q];
-        zs[q] = zhxvts * fz[q] * fi[q];
-        dvy[q] = vn[q] * zn[q] - vi[q] * zs[q];
-        m2[q] = T(1);
-      } else {
-        // rfmzu as in the reference (Main/mod_moloch.F90:1000-1001)
-        zn[q] = dtrdy * fz[q] * fn[q];
-        zs[q] = dtrdy * fz[q] * fi[q];
-        dvy[q] = vn[q] * rn[q] * zn[q] - vi[q] * ri[q] * zs[q];
-        m2[q] = mf[q];
-      }
-      uu[q] = xv[q] ? ui[q] : T(0);  // the zonal flux's wind u (= 2*hvel)
-      zmx[q] = xv[q] ? ui[q] * msu[q] * dtrdx : T(0);
-    }
-    // the zonal update also needs u, rfmzu and rmu one column east
-    T fzu[V], fze[V], ue[V], rme[V];
-    ld_row<T, V>(fzu, sa.rfmzu + ko, e0, i, P, okP);
-    next_col<T, V>(fze, fzu);
+    T fw[V], fe[V], ue[V], re[V];
+    ld_row<T, V>(fw, sa.rfmzu + ko, e0, i, P, okP);
+    next_col<T, V>(fe, fw);
     next_col<T, V>(ue, ui);
-    next_col<T, V>(rme, rmui);
+    next_col<T, V>(re, rw);
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      if (rot) {
-        const T zcostx = dtrdx * mf[q];
-        zw[q] = zcostx * fz[q] * fzu[q];
-        ze[q] = zcostx * fz[q] * fze[q];
-        dvx[q] = ue[q] * ze[q] - ui[q] * zw[q];
-      } else {
-        zw[q] = dtrdx * fz[q] * fzu[q];
-        ze[q] = dtrdx * fz[q] * fze[q];
-        dvx[q] = ue[q] * rme[q] * ze[q] - ui[q] * rmui[q] * zw[q];
-      }
+      const T a = mul_r(dtr, mul_r(fz[q], mf[q]));
+      cs[q] = mul_r(mul_r(vi[q], rot ? mul_r(fi[q], ri[q]) : fi[q]), a);
+      cn[q] = mul_r(mul_r(vn[q], rot ? mul_r(fn[q], rn[q]) : fn[q]), a);
+      cw[q] = mul_r(mul_r(ui[q], fw[q]), a);
+      ce[q] = mul_r(mul_r(ue[q], fe[q]), a);
+      dvy[q] = rot ? cn[q] - cs[q] : fma_r(cn[q], rn[q], -mul_r(cs[q], ri[q]));
+      dvx[q] = rot ? ce[q] - cw[q] : fma_r(ce[q], re[q], -mul_r(cw[q], rw[q]));
+      const T z = mul_r(mul_r(ui[q], msu[q]), dtr);
+      upx[q] = positive(z);
+      nzx[q] = waf_nz<T>(z, upx[q]);
     }
-  }
-  // the three fluxes' factors in the form vel*(x - zmih*B), once for every
-  // field: the upwind flags (zamu > 0) and zmih
-  bool upy[V], upe[VE], upx[V];
-  T z2y[V], z2e[VE], z2x[V];  // zmi = 2*zmih (FP64 only)
-#pragma unroll
-  for (int q = 0; q < V; ++q) {
-    upy[q] = positive(zmy[q]);
-    upx[q] = positive(zmx[q]);
-    z2y[q] = waf_zmi<T>(zmy[q], upy[q]);
-    z2x[q] = waf_zmi<T>(zmx[q], upx[q]);
-    zmy[q] = z2y[q] * T(0.5);
-    zmx[q] = z2x[q] * T(0.5);
-  }
-#pragma unroll
-  for (int q = 0; q < VE; ++q) {
-    upe[q] = positive(zmye[q]);
-    z2e[q] = waf_zmi<T>(zmye[q], upe[q]);
-    zmye[q] = z2e[q] * T(0.5);
   }
   // rows of the halo tile (global row r at tile row r - I0 + 2) the upwind
   // differences use, with the reference's clamps ih = min(i+1, imax),
@@ -924,13 +775,14 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
   int tA, tB, tC, eA, eB, eC;
   mrows(i, tA, tB, tC);
   mrows(I0 + NW, eA, eB, eC);
-  // columns the lane may write: range columns 2 .. W-3 inside the domain
-  bool wv[V];
+  // columns the lane may write, and among them those it updates (the ring
+  // keeps its values)
+  bool wv[V], rv[V];
   bool wall = true;
 #pragma unroll
   for (int q = 0; q < V; ++q) {
-    const int cc = V * lane + q;
-    wv[q] = inrow && i <= iy - 1 && cc >= 2 && cc <= W - 3 && jq[q] >= 1 && jq[q] <= jx - 1;
+    wv[q] = inrow && i <= iy - 1 && hshape_writes(V, V * lane + q, ob, jx);
+    rv[q] = rowP && jq[q] >= 2 && jq[q] <= jx - 2;
     wall = wall && wv[q];
   }
   const bool rowin = inrow && i <= iy - 1;
@@ -944,38 +796,36 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
     ld_row<T, V>(ppk, pp, e0, i, P, rowin);
     const int b = f % kStages;
     const bool landed = mbar_wait_bounded(&mbar[b], (unsigned)((f / kStages) & 1));
-    T(*wt)[BW] = tile(b);
+    T(*wt)[W] = tile(b);
     T(*zp)[W] = zp_s[f & 1];
-    // meridional fluxes zpby(j,i): j in jce, i in ici1..ice2
+    // meridional fluxes per unit wind: j in jce, i in ici1..ice2 (elsewhere
+    // they are not used)
     T wzi[V];
     {
       T wa[V], wA[V], wB[V], wC[V], x[V];
-      ld_vec<T, V>(wa, &wt[i - I0 + 1][OFF + V * lane]);
-      ld_vec<T, V>(wzi, &wt[i - I0 + 2][OFF + V * lane]);
-      ld_vec<T, V>(wA, &wt[tA][OFF + V * lane]);
-      ld_vec<T, V>(wB, &wt[tB][OFF + V * lane]);
-      ld_vec<T, V>(wC, &wt[tC][OFF + V * lane]);
+      ld_vec<T, V>(wa, &wt[i - I0 + 1][V * lane]);
+      ld_vec<T, V>(wzi, &wt[i - I0 + 2][V * lane]);
+      ld_vec<T, V>(wA, &wt[tA][V * lane]);
+      ld_vec<T, V>(wB, &wt[tB][V * lane]);
+      ld_vec<T, V>(wC, &wt[tC][V * lane]);
 #pragma unroll
       for (int q = 0; q < V; ++q) {
         const bool up = upy[q];
-        const T y = waf_flux_h<T>(vv[q], up, zmy[q], z2y[q], wa[q], wzi[q],
-                                  (up ? wa[q] : wB[q]) - (up ? wA[q] : wC[q]));
-        x[q] = mv[q] ? y : T(0);  // zero outside the flux points
+        x[q] = waf_g<T>(nzy[q], up ? wa[q] : wzi[q], wzi[q] - wa[q], (up ? wa[q] : wB[q]) - (up ? wA[q] : wC[q]));
       }
       st_vec<T, V>(&zp[wp][V * lane], x);
       if (eWarp) {
         T xa[VE], xc[VE], eA_[VE], eB_[VE], eC_[VE], xe[VE];
-        ld_vec<T, VE>(xa, &wt[NW + 1][OFF + ec0]);
-        ld_vec<T, VE>(xc, &wt[NW + 2][OFF + ec0]);
-        ld_vec<T, VE>(eA_, &wt[eA][OFF + ec0]);
-        ld_vec<T, VE>(eB_, &wt[eB][OFF + ec0]);
-        ld_vec<T, VE>(eC_, &wt[eC][OFF + ec0]);
+        ld_vec<T, VE>(xa, &wt[NW + 1][ec0]);
+        ld_vec<T, VE>(xc, &wt[NW + 2][ec0]);
+        ld_vec<T, VE>(eA_, &wt[eA][ec0]);
+        ld_vec<T, VE>(eB_, &wt[eB][ec0]);
+        ld_vec<T, VE>(eC_, &wt[eC][ec0]);
 #pragma unroll
         for (int q = 0; q < VE; ++q) {
           const bool up = upe[q];
-          const T y = waf_flux_h<T>(vve[q], up, zmye[q], z2e[q], xa[q], xc[q],
-                                    (up ? xa[q] : eB_[q]) - (up ? eA_[q] : eC_[q]));
-          xe[q] = me[q] ? y : T(0);
+          xe[q] = waf_g<T>(nze[q], up ? xa[q] : xc[q], xc[q] - xa[q],
+                           (up ? xa[q] : eB_[q]) - (up ? eA_[q] : eC_[q]));
         }
         st_vec<T, VE>(&zp[NW][ec0], xe);
       }
@@ -998,10 +848,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
       ld_vec<T, V>(ys, &zp[wp][V * lane]);
       ld_vec<T, V>(yn, &zp[wp + 1][V * lane]);
 #pragma unroll
-      for (int q = 0; q < V; ++q) {
-        const T x = stencil_update<T>(wzi[q], m2[q], rot, false, ys[q], zs[q], yn[q], zn[q], dvy[q], ppk[q]);
-        p0[q] = pv[q] ? x : T(0);
-      }
+      for (int q = 0; q < V; ++q) p0[q] = waf_update<T>(wzi[q], ys[q], cs[q], yn[q], cn[q], dvy[q], ppk[q]);
     }
     // zonal fluxes zpbw(j,i): j in jci1..jce2, i in ici; p0 at range
     // columns c-2 .. c+1 (the lane's own, two from the lane to the west, one
@@ -1028,8 +875,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
       // jhm1 = max(j-2, jmin) upwind; jh = min(j+1, jmax) downwind:
       // upwind a - p0(jhm1), which is a - a at j = 2; downwind p0(jh) - p0(jh-1)
       const T num = up ? (j == 2 ? self_diff<T>(a) : dat(q - 1)) : (j == jx - 1 ? dq[q] : dat(q + 1));
-      const T x = waf_flux_d<T>(uu[q], up, zmx[q], z2x[q], up ? a : cq, dq[q], num);
-      zx[q] = xv[q] ? x : T(0);
+      zx[q] = waf_g<T>(nzx[q], up ? a : cq, dq[q], num);
     }
     T zxe[V];
     next_col<T, V>(zxe, zx);
@@ -1037,7 +883,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
     T res[V];
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const T x = stencil_update<T>(p0[q], m2[q], rot, true, zx[q], zw[q], zxe[q], ze[q], dvx[q], ppk[q]);
+      const T x = waf_update<T>(p0[q], zx[q], cw[q], zxe[q], ce[q], dvx[q], ppk[q]);
       res[q] = rv[q] ? x : ppk[q];
     }
     if (wall) {
@@ -1187,28 +1033,28 @@ __global__ void k_adv_back(const Dom<R> *__restrict__ doms, int uvoff, int advof
 // Both vertical passes (Main/mod_moloch.F90:858-922) in increment form, one
 // thread per column, streaming the levels upward like k_adv_vertical with
 // pass 2 two levels behind pass 1.  e is the pass input's increment over the
-// field (zero for pass 1), dzs(k) = field(k+1) - field(k).  The flux through
-// interface k+1 is formed relative to cell k and moved to cell k+1 by
-// -s(k+1)*dzs(k).  Writes the increment dz = (field after the passes) -
-// field, as a double-float: the bottom and top cells carry a double-float
-// constant part (no flux through levels 1 and kz+1, where s need not vanish).
-__device__ __forceinline__ float vflux_inc(float dtrdz, float skp, float em1, float ek, float ekp1,
+// field (zero for pass 1), dzs(k) = field(k+1) - field(k).  The flux per unit
+// s through interface k+1 is formed relative to cell k and moved to cell k+1
+// by -dzs(k).  Writes the increment dz = (field after the passes) - field, as
+// a double-float at the bottom and top cells, which carry a double-float
+// constant part (no flux through levels 1 and kz+1, where s need not vanish);
+// elsewhere its low part is zero and is neither written nor read.
+__device__ __forceinline__ float vflux_inc(float nz, bool up, float em1, float ek, float ekp1,
                                            float ekp2, float dzm1, float dzk, float dzp1, int k,
                                            int kz) {
-  const float zamu = skp * dtrdz;
-  const bool up = zamu >= 0.f;
+  const float a = dzk + ekp1;
   float num;
   if (up) num = k + 2 <= kz ? (ekp1 - ekp2) - dzp1 : 0.f;
   else num = k >= 2 ? (em1 - ek) - dzm1 : 0.f;
-  return waf_flux<float>(0.5f * skp, up, zamu, dzk + ekp1, ek, num);
+  return waf_g<float>(nz, up ? a : ek, ek - a, num);
 }
-// the cell update without the bottom/top constant parts; flb is the flux
-// through interface k (relative to cell k-1), fla the flux through k+1
-__device__ __forceinline__ float vupdate_inc(float ek, float flb, float fla, float sk, float skp,
-                                             float zu, float zd, float dzm1, int k, int kz) {
-  const float fb = k >= 2 ? flb - sk * dzm1 : 0.f;
-  const float fa = k <= kz - 1 ? fla : 0.f;
-  return -fb * zu + fa * zd + (sk * zu - skp * zd) * ek;
+// the cell update without the bottom/top constant parts; gb is the flux per
+// unit s through interface k (relative to cell k-1), ga the one through k+1
+__device__ __forceinline__ float vupdate_inc(float ek, float gb, float ga, float cu, float cd,
+                                             float dzm1, int k, int kz) {
+  const float fb = k >= 2 ? gb - dzm1 : 0.f;
+  const float fa = k <= kz - 1 ? ga : 0.f;
+  return fma_r(fa, cd, fma_r(-fb, cu, mul_r(cu - cd, ek)));
 }
 
 template <class R>
@@ -1239,7 +1085,7 @@ __global__ void k_adv_vertical_inc(const Dom<R> *__restrict__ doms, int advoff,
   const R *__restrict__ zup = D.sa.zrfmu + ij;
   const R *__restrict__ zdp = D.sa.zrfmd + ij;
   const unsigned PS = (unsigned)g.PS;
-  const float dtrdz = 0.5f * (c.dtstepaf * c.rdzitaf);
+  const float hdtrdz = -0.25f * (c.dtstepaf * c.rdzitaf);  // -1/2 of the factor of s in zamu
 
   // the bottom cell's and top cell's FP32 parts and double-float constant parts
   float eb32 = 0.f, et32 = 0.f;
@@ -1254,47 +1100,52 @@ __global__ void k_adv_vertical_inc(const Dom<R> *__restrict__ doms, int advoff,
   float sm2 = 0.f, sm1 = 0.f, sk = float(sp[0]);
   float zum2 = 0.f, zdm2 = 0.f, zum1 = 0.f, zdm1 = 0.f;
   float f1k = 0.f, f2m = 0.f;
-  unsigned o = 0;
   F2 n_x = src.ld(2 * PS);
   float n_s = float(sp[PS]), n_zu = float(zup[0]), n_zd = float(zdp[0]);
-  for (int k = 1; k <= kz; ++k, o += PS) {
+  // -zmih of an interface from its s
+  auto nzof = [&](float s) { return fma_r(s, hdtrdz, s >= 0.f ? 0.5f : -0.5f); };
+  // level k; the interior steps (4 <= k <= kz-3) carry no bound checks
+  auto step = [&](int k, auto interior) {
+    constexpr bool I = decltype(interior)::value;
+    const unsigned o = (unsigned)(k - 1) * PS;
     const float skp1 = n_s, zuk = n_zu, zdk = n_zd;
     const F2 xp2 = n_x;  // field at k+2 (k+2 <= kz)
-    if (k < kz) {
+    if (I || k < kz) {
       n_s = float(sp[o + 2 * PS]);
       n_zu = float(zup[o + PS]);
       n_zd = float(zdp[o + PS]);
-      if (k + 3 <= kz) n_x = src.ld(o + 3 * PS);
+      if (I || k + 3 <= kz) n_x = src.ld(o + 3 * PS);
     }
-    const float dp1 = k + 2 <= kz ? df_diff(xp2, xp1) : 0.f;  // dzs(k+1)
+    const float dp1 = I || k + 2 <= kz ? df_diff(xp2, xp1) : 0.f;  // dzs(k+1)
     // pass 1 (input increment zero)
-    const float f1kp = k <= kz - 1 ? vflux_inc(dtrdz, skp1, 0.f, 0.f, 0.f, 0.f, dm1, dk, dp1, k, kz) : 0.f;
-    const float u1 = vupdate_inc(0.f, f1k, f1kp, sk, skp1, zuk, zdk, dm1, k, kz);
-    float e1k;
-    if (k == kz) {
-      et32 += u1;
-      ht = df_add(ht, df_mul(src.ld(o), two_prod(-skp1, zdk)));
-      e1k = et32 + df_f(ht);
-    } else if (k == 1) {
-      eb32 += u1;
-      hb = df_add(hb, df_mul(src1, two_prod(sk, zuk)));
-      e1k = eb32 + df_f(hb);
-    } else {
-      e1k = 0.f + u1;
+    const int kk = I ? 4 : k, kzz = I ? 8 : kz;  // an interior level's checks hold
+    const float f1kp = I || k <= kz - 1
+                           ? vflux_inc(nzof(skp1), skp1 >= 0.f, 0.f, 0.f, 0.f, 0.f, dm1, dk, dp1, kk, kzz)
+                           : 0.f;
+    const float u1 = vupdate_inc(0.f, f1k, f1kp, mul_r(sk, zuk), mul_r(skp1, zdk), dm1, kk, kzz);
+    float e1k = u1;
+    if constexpr (!I) {
+      if (k == kz) {
+        et32 += u1;
+        ht = df_add(ht, df_mul(src.ld(o), two_prod(-skp1, zdk)));
+        e1k = et32 + df_f(ht);
+      } else if (k == 1) {
+        eb32 += u1;
+        hb = df_add(hb, df_mul(src1, two_prod(sk, zuk)));
+        e1k = eb32 + df_f(hb);
+      }
     }
-    if (k >= 3) {  // pass 2 at level m = k-2
-      const int m = k - 2;
-      const float f2n = vflux_inc(dtrdz, sm1, e1m3, e1m2, e1m1, e1k, dm3, dm2, dm1, m, kz);
-      const float u2 = vupdate_inc(e1m2, f2m, f2n, sm2, sm1, zum2, zdm2, dm3, m, kz);
-      F2 d;
-      if (m == 1) {
+    if (I || k >= 3) {  // pass 2 at level m = k-2
+      const int m = I ? 4 : k - 2;
+      const float f2n = vflux_inc(nzof(sm1), sm1 >= 0.f, e1m3, e1m2, e1m1, e1k, dm3, dm2, dm1, m, kzz);
+      const float u2 = vupdate_inc(e1m2, f2m, f2n, mul_r(sm2, zum2), mul_r(sm1, zdm2), dm3, m, kzz);
+      if (!I && m == 1) {
         eb32 += u2;
         hb = df_add(hb, df_mul(src1, two_prod(sm2, zum2)));
-        d = df_add_f(hb, eb32);
+        dst.st(o - 2 * PS, df_add_f(hb, eb32));
       } else {
-        d = F2{e1m2 + u2, 0.f};
+        dst.p[o - 2 * PS] = e1m2 + u2;
       }
-      dst.st(o - 2 * PS, d);
       f2m = f2n;
     }
     dm3 = dm2; dm2 = dm1; dm1 = dk; dk = dp1;
@@ -1303,13 +1154,20 @@ __global__ void k_adv_vertical_inc(const Dom<R> *__restrict__ doms, int advoff,
     sm2 = sm1; sm1 = sk; sk = skp1;
     zum2 = zum1; zdm2 = zdm1; zum1 = zuk; zdm1 = zdk;
     f1k = f1kp;
-  }
+  };
+  using edge = std::integral_constant<bool, false>;
+  using mid = std::integral_constant<bool, true>;
+  const int k1 = min(3, kz), k2 = max(4, kz - 2);
+  for (int k = 1; k <= k1; ++k) step(k, edge{});
+#pragma unroll 4
+  for (int k = 4; k < k2; ++k) step(k, mid{});
+  for (int k = k2; k <= kz; ++k) step(k, edge{});
   // pass 2 at levels kz-1 and kz; dm3 = dzs(kz-2), dm2 = dzs(kz-1) now
   const unsigned ot = (unsigned)(kz - 1) * PS;
-  const float f2n = vflux_inc(dtrdz, sm1, e1m3, e1m2, e1m1, 0.f, dm3, dm2, dm1, kz - 1, kz);
-  const float u2 = vupdate_inc(e1m2, f2m, f2n, sm2, sm1, zum2, zdm2, dm3, kz - 1, kz);
-  dst.st(ot - PS, F2{e1m2 + u2, 0.f});
-  const float ut = vupdate_inc(e1m1, f2n, 0.f, sm1, sk, zum1, zdm1, dm2, kz, kz);
+  const float f2n = vflux_inc(nzof(sm1), sm1 >= 0.f, e1m3, e1m2, e1m1, 0.f, dm3, dm2, dm1, kz - 1, kz);
+  const float u2 = vupdate_inc(e1m2, f2m, f2n, mul_r(sm2, zum2), mul_r(sm1, zdm2), dm3, kz - 1, kz);
+  dst.p[ot - PS] = e1m2 + u2;
+  const float ut = vupdate_inc(e1m1, f2n, 0.f, mul_r(sm1, zum1), mul_r(sk, zdm1), dm2, kz, kz);
   et32 += ut;
   ht = df_add(ht, df_mul(src.ld(ot), two_prod(-sk, zdm1)));
   dst.st(ot, df_add_f(ht, et32));
@@ -1325,18 +1183,15 @@ __global__ void k_adv_vertical_inc(const Dom<R> *__restrict__ doms, int advoff,
 // + zonal increments).  Fluxes are formed relative to the cell south (west)
 // of the interface, from FP32 increments and neighbour differences.
 template <class R, int V, int NW>
-__global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW))
+__global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(V == 4 ? MLC_HINC_WARPS_4 : MLC_HINC_WARPS, NW))
     k_adv_horizontal_inc(const Dom<R> *__restrict__ doms,
                                                                int tiles_j, int uvoff,
                                                                int advoff,
                                                                const WorkItem *__restrict__ wl) {
   constexpr int W = 32 * V, S = W - 4;
-  constexpr int OB0 = hshape_ob0(V);
-  constexpr int OFF = hshape_off(4, V);
-  constexpr int BW = W + 2 * OFF;  // tile row: range column c sits at c + OFF
-  constexpr unsigned kBox = (unsigned)((NW + 4) * BW * 4);
+  constexpr unsigned kBox = (unsigned)((NW + 4) * W * 4);
   constexpr unsigned kBuf = (kBox + 127u) / 128u * 128u;
-  constexpr int shape = V == 1 ? 0 : 1;
+  constexpr int shape = V == 1 ? 0 : V == 2 ? 1 : 4;
   static_assert(hshape_inc(shape).v == V && hshape_inc(shape).nw == NW, "tile shape table");
   // per field: the halo tiles (rows I0-2 .. I0+NW+1) of pp hi, pp lo, dz hi,
   // dz lo, landed by TMA, all issued at the start
@@ -1351,9 +1206,9 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
   const int jx = g.jx, iy = g.iy;
   if (k > g.kz) return;
   const int bj = wi.a, bi = wi.b;
-  const int ob = bj * S + OB0;
+  const int ob = bj * S;
   const int I0 = bi * NW + 1;
-  if (ob + 3 > jx - 1 || I0 > iy - 1) return;
+  if (bj >= hshape_tiles(V, jx) || I0 > iy - 1) return;
   const Scal &c = D.c;
   const Stat<R> &sa = D.sa;
   const int uv = (D.clk->uv_role + uvoff) & 1, adv = (D.clk->adv_role + advoff) & 1;
@@ -1367,9 +1222,10 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
   const float *__restrict__ uk = D.u[uv] + ko;
   const float *__restrict__ vk = D.v[uv] + ko;
   const float dta = c.dtstepaf;
-  const float dtrdx = dta * c.rdxf, dtrdy = dta * c.rdxf;
+  const float dtr = dta * c.rdxf;
   const bool rot = c.lrotllr != 0;
   using T = float;
+  const bool dlo = k == 1 || k == g.kz;  // elsewhere dz has no low part (k_adv_vertical_inc)
   const int tid = (int)threadIdx.x;
   if (tid == 0) {
     mbar_init(&mbar[0], 1);
@@ -1380,11 +1236,12 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
   if (tid == 0) {
     const char *tm = static_cast<const char *>(D.tmap) + ((size_t)shape * kTmapSlots + kMaxFields) * kTmapBytes;
     for (int f = 0; f < 2; ++f) {
-      mbar_expect_tx(&mbar[f], 4u * kBox);
+      const int ntile = dlo ? 4 : 3;
+      mbar_expect_tx(&mbar[f], (unsigned)ntile * kBox);
       const int pslot = 4 * f + 2 * adv, dslot = 8 + 2 * f;
       const int slot[4] = {pslot, pslot + 1, dslot, dslot + 1};
-      for (int q = 0; q < 4; ++q)
-        tma_load_3d(tiles[f][q], tm + (size_t)slot[q] * kTmapBytes, ob - OFF, I0 - 3, k - 1, &mbar[f]);
+      for (int q = 0; q < ntile; ++q)
+        tma_load_3d(tiles[f][q], tm + (size_t)slot[q] * kTmapBytes, ob, I0 - 3, k - 1, &mbar[f]);
     }
   }
 
@@ -1396,34 +1253,34 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
   const bool okM = inrow && rowM, okP = inrow && rowP;
   const int ie = I0 + NW;
   const bool okE = wp == NW - 1 && inrow && ie >= 2 && ie <= iy - 1;
-  // ---- coefficients ----
-  T vv[V], zmy[V], vve[V], zmye[V];
-  bool mv[V], me[V];
+  // ---- coefficients, as in k_adv_horizontal ----
+  T nzy[V], nze[V], nzx[V];
+  bool upy[V], upe[V], upx[V], rv[V];
   {
     T a[V], b[V];
     ld_row<T, V>(a, vk, e0, i, P, okM);
     ld_row<T, V>(b, sa.msfv, e0, i, P, okM && !rot);
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const bool ok = okM && jq[q] >= 1 && jq[q] <= jx - 1;
-      mv[q] = ok;
-      vv[q] = ok ? a[q] : T(0);
-      zmy[q] = ok ? (rot ? a[q] * dtrdy : a[q] * b[q] * dtrdy) : T(0);
+      const T z = mul_r(rot ? a[q] : mul_r(a[q], b[q]), dtr);
+      upy[q] = z > 0.f;
+      nzy[q] = waf_nz<T>(z, upy[q]);
     }
     ld_row<T, V>(a, vk, e0, ie, P, okE);
     ld_row<T, V>(b, sa.msfv, e0, ie, P, okE && !rot);
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const bool ok = okE && jq[q] >= 1 && jq[q] <= jx - 1;
-      me[q] = ok;
-      vve[q] = ok ? a[q] : T(0);
-      zmye[q] = ok ? (rot ? a[q] * dtrdy : a[q] * b[q] * dtrdy) : T(0);
+      const T z = mul_r(rot ? a[q] : mul_r(a[q], b[q]), dtr);
+      upe[q] = z > 0.f;
+      nze[q] = waf_nz<T>(z, upe[q]);
     }
   }
-  T zs[V], zn[V], vsv[V], cy[V], m2[V], uu[V], zmx[V], zw[V], ze[V], uwv[V], cx[V];
-  bool pv[V], xv[V], rv[V], cyf[V], cxf[V];
+  // the faces' winds times the cell's metric factors (cs, cn; cw, ce) and the
+  // map-factor terms that a constant field does not cancel (cy, cx)
+  T cs[V], cn[V], cy[V], cw[V], ce[V], cx[V];
+  bool cyf[V], cxf[V];
   {
-    T fz[V], vi[V], vn[V], ri[V], rn[V], fi[V], fn[V], mf[V], ui[V], rmui[V], msu[V];
+    T fz[V], vi[V], vn[V], ri[V], rn[V], fi[V], fn[V], mf[V], ui[V], rw[V], msu[V];
     ld_row<T, V>(fz, sa.fmz + ko, e0, i, P, okP);
     ld_row<T, V>(vi, vk, e0, i, P, okP);
     ld_row<T, V>(vn, vk, e0, i + 1, P, okP);
@@ -1433,48 +1290,28 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
     ld_row<T, V>(fn, (rot ? sa.rfmzv : sa.rfmzu) + ko, e0, i + 1, P, okP);
     ld_row<T, V>(mf, rot ? sa.msfx : sa.mx2, e0, i, P, okP);
     ld_row<T, V>(ui, uk, e0, i, P, okP);
-    ld_row<T, V>(rmui, sa.rmu, e0, i, P, okP && !rot);
+    ld_row<T, V>(rw, sa.rmu, e0, i, P, okP && !rot);
     ld_row<T, V>(msu, sa.msfu, e0, i, P, okP);
-    T fzu[V], fze[V], ue[V], rme[V];
-    ld_row<T, V>(fzu, sa.rfmzu + ko, e0, i, P, okP);
-    next_col<T, V>(fze, fzu);
+    T fw[V], fe[V], ue[V], re[V];
+    ld_row<T, V>(fw, sa.rfmzu + ko, e0, i, P, okP);
+    next_col<T, V>(fe, fw);
     next_col<T, V>(ue, ui);
-    next_col<T, V>(rme, rmui);
+    next_col<T, V>(re, rw);
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const int j = jq[q];
-      pv[q] = okP && j >= 1 && j <= jx - 1;
-      xv[q] = okP && j >= 2 && j <= jx - 1;
-      rv[q] = okP && j >= 2 && j <= jx - 2;
-      vsv[q] = vi[q];
-      uwv[q] = ui[q];
-      if (rot) {
-        const T zhxvtn = dtrdy * rn[q] * mf[q];
-        const T zhxvts = dtrdy * ri[q] * mf[q];
-        zn[q] = zhxvtn * fz[q] * fn[q];
-        zs[q] = zhxvts * fz[q] * fi[q];
-        m2[q] = T(1);
-        cyf[q] = false;
-        cy[q] = T(0);
-        const T zcostx = dtrdx * mf[q];
-        zw[q] = zcostx * fz[q] * fzu[q];
-        ze[q] = zcostx * fz[q] * fze[q];
-        cxf[q] = false;
-        cx[q] = T(0);
-      } else {
-        zn[q] = dtrdy * fz[q] * fn[q];
-        zs[q] = dtrdy * fz[q] * fi[q];
-        m2[q] = mf[q];
-        // the map-factor terms a constant field does not cancel
-        cyf[q] = ri[q] != 1.f || rn[q] != 1.f;
-        cy[q] = mf[q] * (vi[q] * zs[q] * (1.f - ri[q]) - vn[q] * zn[q] * (1.f - rn[q]));
-        zw[q] = dtrdx * fz[q] * fzu[q];
-        ze[q] = dtrdx * fz[q] * fze[q];
-        cxf[q] = rmui[q] != 1.f || rme[q] != 1.f;
-        cx[q] = mf[q] * (ui[q] * zw[q] * (1.f - rmui[q]) - ue[q] * ze[q] * (1.f - rme[q]));
-      }
-      uu[q] = xv[q] ? ui[q] : T(0);
-      zmx[q] = xv[q] ? ui[q] * msu[q] * dtrdx : T(0);
+      const T a = mul_r(dtr, mul_r(fz[q], mf[q]));
+      cs[q] = mul_r(mul_r(vi[q], rot ? mul_r(fi[q], ri[q]) : fi[q]), a);
+      cn[q] = mul_r(mul_r(vn[q], rot ? mul_r(fn[q], rn[q]) : fn[q]), a);
+      cw[q] = mul_r(mul_r(ui[q], fw[q]), a);
+      ce[q] = mul_r(mul_r(ue[q], fe[q]), a);
+      cyf[q] = !rot && (ri[q] != 1.f || rn[q] != 1.f);
+      cxf[q] = !rot && (rw[q] != 1.f || re[q] != 1.f);
+      cy[q] = fma_r(cs[q], 1.f - ri[q], -mul_r(cn[q], 1.f - rn[q]));
+      cx[q] = fma_r(cw[q], 1.f - rw[q], -mul_r(ce[q], 1.f - re[q]));
+      const T z = mul_r(mul_r(ui[q], msu[q]), dtr);
+      upx[q] = z > 0.f;
+      nzx[q] = waf_nz<T>(z, upx[q]);
+      rv[q] = okP && jq[q] >= 2 && jq[q] <= jx - 2;
     }
   }
   const bool rowin = inrow && i <= iy - 1;
@@ -1483,23 +1320,23 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
 #pragma unroll
   for (int q = 0; q < V; ++q) {
     const int cc = V * lane + q;
-    wv[q] = rowin && cc >= 2 && cc <= W - 3 && jq[q] >= 1 && jq[q] <= jx - 1;
+    wv[q] = rowin && hshape_writes(V, cc, ob, jx);
     wall = wall && wv[q];
   }
-  // the meridional flux through the south face of row r (relative to pp(r-1))
-  // from dz and pp differences of rows r-2 .. r+1; the reference's clamps
-  // ih = min(r+1, imax), ihm1 = max(ih-1, imin)
-  auto mflux = [&](T (&x)[V], const T (&vvr)[V], const T (&zm)[V], const bool (&ok)[V], int r,
+  // the meridional flux per unit wind through the south face of row r
+  // (relative to pp(r-1)) from dz and pp differences of rows r-2 .. r+1; the
+  // reference's clamps ih = min(r+1, imax), ihm1 = max(ih-1, imin)
+  auto mflux = [&](T (&x)[V], const T (&nz)[V], const bool (&upr)[V], int r,
                    const T (&zm2)[V], const T (&zm1)[V], const T (&z0)[V], const T (&zp1)[V],
                    const T (&dym2)[V], const T (&dym1)[V], const T (&dy0)[V]) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const bool up = zm[q] > 0.f;
+      const bool up = upr[q];
+      const float cq = z0[q] + dym1[q];
       float num;
-      if (up) num = r >= 3 ? (zm1[q] - zm2[q]) + dym2[q] : (zm1[q] - zm1[q]) + 0.f;
+      if (up) num = r >= 3 ? (zm1[q] - zm2[q]) + dym2[q] : zm1[q] - zm1[q];
       else num = r <= iy - 2 ? (zp1[q] - z0[q]) + dy0[q] : (z0[q] - zm1[q]) + dym1[q];
-      const float y = waf_flux<float>(0.5f * vvr[q], up, zm[q], zm1[q], z0[q] + dym1[q], num);
-      x[q] = ok[q] ? y : 0.f;
+      x[q] = waf_g<float>(nz[q], up ? zm1[q] : cq, cq - zm1[q], num);
     }
   };
 
@@ -1507,11 +1344,19 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
     float *outh = reinterpret_cast<float *>(f == 0 ? D.tetav[adv ^ 1] : D.pai[adv ^ 1]);
     float (*fy)[W] = fy_s[f];
     const bool landed = mbar_wait_bounded(&mbar[f], 0u);
-    const float(*tph)[BW] = reinterpret_cast<const float(*)[BW]>(tiles[f][0]);
-    const float(*tpl)[BW] = reinterpret_cast<const float(*)[BW]>(tiles[f][1]);
-    const float(*tzh)[BW] = reinterpret_cast<const float(*)[BW]>(tiles[f][2]);
-    const float(*tzl)[BW] = reinterpret_cast<const float(*)[BW]>(tiles[f][3]);
-    const int cl = OFF + V * lane;
+    const float(*tph)[W] = reinterpret_cast<const float(*)[W]>(tiles[f][0]);
+    const float(*tpl)[W] = reinterpret_cast<const float(*)[W]>(tiles[f][1]);
+    const float(*tzh)[W] = reinterpret_cast<const float(*)[W]>(tiles[f][2]);
+    const float(*tzl)[W] = reinterpret_cast<const float(*)[W]>(tiles[f][3]);
+    const int cl = V * lane;
+    auto low_part = [&](T (&x)[V], const float *p) {
+      if (dlo) {
+        ld_vec<T, V>(x, p);
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q) x[q] = 0.f;
+      }
+    };
     // rows i-2 .. i+1 (tile rows wp .. wp+3) of pp (hi, lo) and dz (rounded
     // to FP32); zero outside the cross points
     T ph[4][V], pl[4][V], zz[4][V], dzi_h[V], dzi_l[V];
@@ -1521,7 +1366,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
       ld_vec<T, V>(pl[rr], &tpl[wp + rr][cl]);
       T zh[V], zl[V];
       ld_vec<T, V>(zh, &tzh[wp + rr][cl]);
-      ld_vec<T, V>(zl, &tzl[wp + rr][cl]);
+      low_part(zl, &tzl[wp + rr][cl]);
 #pragma unroll
       for (int q = 0; q < V; ++q) zz[rr][q] = zh[q] + zl[q];
       if (rr == 2) {
@@ -1538,7 +1383,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
         dy[rr][q] = (ph[rr + 1][q] - ph[rr][q]) + (pl[rr + 1][q] - pl[rr][q]);
     {
       T x[V];
-      mflux(x, vv, zmy, mv, i, zz[0], zz[1], zz[2], zz[3], dy[0], dy[1], dy[2]);
+      mflux(x, nzy, upy, i, zz[0], zz[1], zz[2], zz[3], dy[0], dy[1], dy[2]);
       st_vec<T, V>(&fy[wp][V * lane], x);
     }
     if (wp == NW - 1) {  // the flux of row I0+NW: rows ie-2 .. ie+1 = i-1 .. i+2
@@ -1546,14 +1391,14 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
       ld_vec<T, V>(h4, &tph[NW + 3][cl]);
       ld_vec<T, V>(l4, &tpl[NW + 3][cl]);
       ld_vec<T, V>(zh, &tzh[NW + 3][cl]);
-      ld_vec<T, V>(zl, &tzl[NW + 3][cl]);
+      low_part(zl, &tzl[NW + 3][cl]);
 #pragma unroll
       for (int q = 0; q < V; ++q) {
         z4[q] = zh[q] + zl[q];
         dy3[q] = (h4[q] - ph[3][q]) + (l4[q] - pl[3][q]);
       }
       T x[V];
-      mflux(x, vve, zmye, me, ie, zz[1], zz[2], zz[3], z4, dy[1], dy[2], dy3);
+      mflux(x, nze, upe, ie, zz[1], zz[2], zz[3], z4, dy[1], dy[2], dy3);
       st_vec<T, V>(&fy[NW][V * lane], x);
     }
     if (__syncthreads_or(!landed)) {
@@ -1573,12 +1418,10 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
       ld_vec<T, V>(yn, &fy[wp + 1][V * lane]);
 #pragma unroll
       for (int q = 0; q < V; ++q) {
-        const float fs = ys[q] - vsv[q] * dy[1][q];  // moved to pp(i)
-        const float fn = yn[q];
-        float h = m2[q] * (fs * zs[q] - fn * zn[q]);
-        if (rot) h = fs * zs[q] - fn * zn[q];
-        else if (cyf[q]) h += ph[2][q] * cy[q];
-        hy[q] = pv[q] ? h : 0.f;
+        // the south flux moved to pp(i)
+        float h = fma_r(ys[q] - dy[1][q], cs[q], -mul_r(yn[q], cn[q]));
+        if (cyf[q]) h = fma_r(ph[2][q], cy[q], h);
+        hy[q] = h;
         ey[q] = zz[2][q] + hy[q];
       }
     }
@@ -1603,18 +1446,17 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
     auto dxat = [&](int q) -> float {
       return q == -2 ? dxw2 : q == -1 ? dxw1 : dx[q < 0 ? 0 : q >= V ? V - 1 : q];
     };
-    // zonal fluxes at the lane's columns, relative to pp(j-1)
+    // zonal fluxes per unit wind at the lane's columns, relative to pp(j-1)
     T fx[V];
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       const int j = jq[q];
-      const bool up = zmx[q] > 0.f;
-      const float a = eyat(q - 1), cq = eyat(q);
+      const bool up = upx[q];
+      const float a = eyat(q - 1), c0 = eyat(q), cq = c0 + dxat(q - 1);
       float num;
-      if (up) num = j >= 3 ? (a - eyat(q - 2)) + dxat(q - 2) : (a - a) + 0.f;
-      else num = j <= jx - 2 ? (eyat(q + 1) - cq) + dxat(q) : (cq - a) + dxat(q - 1);
-      const float y = waf_flux<float>(0.5f * uu[q], up, zmx[q], a, cq + dxat(q - 1), num);
-      fx[q] = xv[q] ? y : 0.f;
+      if (up) num = j >= 3 ? (a - eyat(q - 2)) + dxat(q - 2) : a - a;
+      else num = j <= jx - 2 ? (eyat(q + 1) - c0) + dxat(q) : (c0 - a) + dxat(q - 1);
+      fx[q] = waf_g<float>(nzx[q], up ? a : cq, cq - a, num);
     }
     T fxe[V];
     next_col<T, V>(fxe, fx);
@@ -1625,15 +1467,9 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(MLC_HINC_WARPS, NW)
       const F2 ppk{ph[2][q], pl[2][q]};
       F2 x = ppk;
       if (rv[q]) {
-        const float fw = fx[q] - uwv[q] * dxat(q - 1);  // moved to pp(j)
-        const float fe = fxe[q];
-        float hx;
-        if (rot) {
-          hx = fw * zw[q] - fe * ze[q];
-        } else {
-          hx = m2[q] * (fw * zw[q] - fe * ze[q]);
-          if (cxf[q]) hx += ppk.hi * cx[q];
-        }
+        // the west flux moved to pp(j)
+        float hx = fma_r(fx[q] - dxat(q - 1), cw[q], -mul_r(fxe[q], ce[q]));
+        if (cxf[q]) hx = fma_r(ppk.hi, cx[q], hx);
         x = df_add_f(df_add(ppk, F2{dzi_h[q], dzi_l[q]}), hy[q] + hx);
       }
       rh[q] = x.hi;
@@ -1688,9 +1524,7 @@ void launch_vertical(const LaunchGeom &L, const Dom<R> *d, int nf, int set, int 
 
 template <class R, int V, int NW>
 void launch_tile(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
-  // tiles along j: tile bj writes j = bj*S + ob0 + 3 .. bj*S + ob0 + S + 2
-  constexpr int S = 32 * V - 4;
-  const int tj = (L.jx - 3 - hshape_ob0(V) + S - 1) / S, ti = (L.iy - 1 + NW - 1) / NW;
+  const int tj = hshape_tiles(V, L.jx), ti = (L.iy - 1 + NW - 1) / NW;
   const dim3 grd = L.wl_h ? dim3((unsigned)L.n_h, 1, 1)
                           : dim3((unsigned)(tj * ti), (unsigned)L.kz, (unsigned)L.nmem);
   k_adv_horizontal<R, V, NW><<<grd, 32 * NW, 0, s>>>(d, tj, uvoff, advoff, L.wl_h);
@@ -1699,7 +1533,10 @@ void launch_tile(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cu
 template <class R>
 void launch_horizontal(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
   constexpr int eb = (int)sizeof(R);
-  switch (L.htile) {
+  switch (waf_tile(L)) {
+    case 4:
+      if constexpr (sizeof(R) == sizeof(float)) launch_tile<R, 4, hshape(4, 4).nw>(L, d, uvoff, advoff, s);
+      break;
     case 1: launch_tile<R, hshape(eb, 1).v, hshape(eb, 1).nw>(L, d, uvoff, advoff, s); break;
     case 2: launch_tile<R, hshape(eb, 2).v, hshape(eb, 2).nw>(L, d, uvoff, advoff, s); break;
     case 3: launch_tile<R, hshape(eb, 3).v, hshape(eb, 3).nw>(L, d, uvoff, advoff, s); break;
@@ -1718,8 +1555,7 @@ void launch_vertical_inc(const LaunchGeom &L, const Dom<R> *d, int advoff, cudaS
 
 template <class R, int V, int NW>
 void launch_tile_inc(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
-  constexpr int S = 32 * V - 4;
-  const int tj = (L.jx - 3 - hshape_ob0(V) + S - 1) / S, ti = (L.iy - 1 + NW - 1) / NW;
+  const int tj = hshape_tiles(V, L.jx), ti = (L.iy - 1 + NW - 1) / NW;
   const dim3 grd = L.wl_hinc ? dim3((unsigned)L.n_hinc, 1, 1)
                              : dim3((unsigned)(tj * ti), (unsigned)L.kz, (unsigned)L.nmem);
   k_adv_horizontal_inc<R, V, NW><<<grd, 32 * NW, 0, s>>>(d, tj, uvoff, advoff, L.wl_hinc);
@@ -1728,8 +1564,11 @@ void launch_tile_inc(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff
 template <class R>
 void launch_horizontal_inc(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff,
                            cudaStream_t s) {
-  if (hshape_inc(L.htile).v == 2) launch_tile_inc<R, 2, hshape_inc(1).nw>(L, d, uvoff, advoff, s);
-  else launch_tile_inc<R, 1, hshape_inc(0).nw>(L, d, uvoff, advoff, s);
+  switch (hshape_inc(waf_tile_inc(L)).v) {
+    case 4: launch_tile_inc<R, 4, hshape_inc(4).nw>(L, d, uvoff, advoff, s); break;
+    case 2: launch_tile_inc<R, 2, hshape_inc(1).nw>(L, d, uvoff, advoff, s); break;
+    default: launch_tile_inc<R, 1, hshape_inc(0).nw>(L, d, uvoff, advoff, s); break;
+  }
 }
 
 template <class R>

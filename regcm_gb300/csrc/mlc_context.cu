@@ -152,9 +152,9 @@ void carve_dom(Carver &cv, Dom<R> &D, const Geom &g, const mlc_dims &d, const ml
   for (int f = 0; f < kMaxFields; ++f) D.wz[f] = f < nr ? cv.take<R>(F) : nullptr;
   for (int f = 0; f < 2; ++f) D.wz_d[f] = f64 ? nullptr : cv.take<double>(F);
   D.vdiv = f64 ? cv.take<double>(F) : nullptr;
-  D.vzamu = f64 ? cv.take<double>(F) : nullptr;
-  D.vzmih = f64 ? cv.take<double>(F) : nullptr;
-  D.vzmi = f64 ? cv.take<double>(F) : nullptr;
+  D.vcu = f64 ? cv.take<double>(F) : nullptr;
+  D.vcd = f64 ? cv.take<double>(F) : nullptr;
+  D.vnz = f64 ? cv.take<double>(F) : nullptr;
   Stat<R> &s = D.sa;
   s.fmz = cv.take<R>(F); s.fmzf = cv.take<R>(F1); s.rfmzu = cv.take<R>(F); s.rfmzv = cv.take<R>(F);
   if (f64) {
@@ -350,7 +350,7 @@ struct mlc_ctx {
   WorkItem *wl_buf = nullptr;
   size_t wl_cap = 0;           // entries
   bool wl_dirty = true;        // members changed since the lists were built
-  int wl_key[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
+  int wl_key[10] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
   const WorkItem *wl_ptr[9] = {};  // the lists in wl_buf (null: none) ...
   int wl_n[9] = {};                // ... and their lengths
 };
@@ -385,10 +385,8 @@ int ensure_staging(mlc_ctx *x, const mlc_dims &d) {
 // and the increment form the planes of theta_v, Exner and their vertical
 // increments the same way.  The map's extents are the cross points (jx-1,
 // iy-1, kz), so everything outside them reads as zero, as the kernels need.
-// A copy must start on a 16-byte boundary: tile offsets step by 32*v - 4
-// columns, a multiple of 16 bytes, and the first tile starts hshape_off
-// columns left of its range so that its x times the element size is a
-// multiple of 16; every box row is a multiple of 16 bytes.
+// A copy must start on a 16-byte boundary: tile offsets are multiples of
+// 32*v - 4 columns, a multiple of 16 bytes, and so is every box row.
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -420,7 +418,7 @@ int encode_tmaps(mlc_ctx *x, const Member &m, const Dom<R> &D) {
   const cuuint32_t estr[3] = {1, 1, 1};
   auto encode = [&](CUtensorMap *mp, const void *base, size_t ebytes, HShape h) {
     const cuuint64_t strides[2] = {(cuuint64_t)g.P * ebytes, (cuuint64_t)g.PS * ebytes};
-    const cuuint32_t box[3] = {(cuuint32_t)(32 * h.v + 2 * hshape_off((int)ebytes, h.v)),
+    const cuuint32_t box[3] = {(cuuint32_t)(32 * h.v),
                                (cuuint32_t)(h.nw + 4), 1};
     return enc(mp, ebytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
                const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -528,6 +526,49 @@ int solve_kind(const std::vector<Dom<R>> &t) {
   return n <= (f64 ? 8 : 16) * 152 ? kSolveCols3 : kSolveStream;
 }
 
+// Tile shapes of the horizontal WAF.  A tile's time goes with its columns,
+// those outside the domain included, so the width is the one whose tiles
+// cover the members' rows with the least weighted columns; the weights are
+// the measured times a column of 32-, 64- and 128-column tiles (64: 100).
+// FP64 spends the same at either width (arithmetic): 256x256x41 0.911 ms in
+// 9 tiles of 32 columns, 1.017 in 5 of 64; 512x512x41 3.80 and 3.60 (19 and
+// 9).  FP32 saves address arithmetic and shuffles with wider lanes: fields
+// (146, 100, 83) 32 members of 128x128x30 0.68, 0.53, 0.29 ms; increments,
+// whose rows in flight fill the registers, (142, 100, 108) 0.50, 0.42, 0.32.
+// Eight rows a tile (FP64 at 64 columns four, 1 % faster); FP64 tiles of 32
+// columns take four where eight would leave SMs with a block or two (47x33x23:
+// 26 us against 32).
+template <class R>
+void size_tiles(const std::vector<Dom<R>> &t, LaunchGeom &L) {
+  const bool f64 = sizeof(R) == sizeof(double);
+  static constexpr int kWidth[3] = {1, 2, 4};
+  static constexpr int kCost[3][3] = {{100, 100, 0}, {146, 100, 83}, {142, 100, 108}};
+  auto pick = [&](int kind) {
+    double best = 0.0;
+    int v = 0;
+    for (int q = 0; q < 3; ++q) {
+      if (kCost[kind][q] == 0) continue;
+      double cost = 0.0;
+      for (const Dom<R> &D : t)
+        cost += (double)hshape_tiles(kWidth[q], D.g.jx) * 32 * kWidth[q] * D.g.iy * D.g.kz * kCost[kind][q];
+      if (v == 0 || cost < best) {
+        best = cost;
+        v = kWidth[q];
+      }
+    }
+    return v;
+  };
+  const int v = pick(f64 ? 0 : 1), vi = f64 ? v : pick(2);
+  if (f64) {
+    long blocks = 0;  // of eight rows
+    for (const Dom<R> &D : t) blocks += (long)hshape_tiles(1, D.g.jx) * ((D.g.iy - 1 + 7) / 8) * D.g.kz;
+    L.size_tile = v == 2 ? 2 : blocks < 2 * 152 ? 3 : 0;
+  } else {
+    L.size_tile = v == 4 ? 4 : v == 2 ? 1 : 0;
+  }
+  L.size_tile_inc = vi == 4 ? 4 : vi == 2 ? 1 : 0;
+}
+
 // Upload the descriptor table of the active members and derive the launch
 // geometry (maxima over the members; the launch shapes are kept).
 template <class R>
@@ -567,6 +608,7 @@ int refresh(mlc_ctx *x) {
   }
   L.nmem = (int)t.size();
   L.solve = solve_kind<R>(t);
+  size_tiles<R>(t, L);
   size_t pts = 0;
   L.frame_points = 0;
   for (const Dom<R> &D : t) {
@@ -602,7 +644,8 @@ int ensure_lists(mlc_ctx *x) {
   bool uneven = false;
   for (const Member *m : act)
     uneven = uneven || m->g.jx != L.jx || m->g.iy != L.iy || m->g.kz != L.kz;
-  const int key[9] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, L.htile, L.solve, L.lv, L.wind_rows};
+  const int key[10] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, waf_tile(L), waf_tile_inc(L),
+                       L.solve, L.lv, L.wind_rows};
   // the launch geometry always takes the lists from the context (a copy of
   // an older geometry may carry stale ones)
   auto apply = [&]() {
@@ -676,19 +719,18 @@ int ensure_lists(mlc_ctx *x) {
     }
   // horizontal WAF tiles of the shape in use, every level
   auto htiles = [&](HShape h) {
-    const int S = 32 * h.v - 4;
     for (int m = 0; m < (int)act.size(); ++m) {
       const Geom &g = act[m]->g;
-      const int tj = cdiv(g.jx - 3 - hshape_ob0(h.v), S), ti = cdiv(g.iy - 1, h.nw);
+      const int tj = hshape_tiles(h.v, g.jx), ti = cdiv(g.iy - 1, h.nw);
       for (int k = 0; k < g.kz; ++k)
         for (int bi = 0; bi < ti; ++bi)
           for (int bj = 0; bj < tj; ++bj) push(m, bj, bi, k);
     }
   };
   off[5] = all.size();
-  htiles(hshape((int)sizeof(R), L.htile));
+  htiles(hshape((int)sizeof(R), waf_tile(L)));
   off[6] = all.size();
-  if (!f64) htiles(hshape_inc(L.htile));
+  if (!f64) htiles(hshape_inc(waf_tile_inc(L)));
   // the step end: 16-byte lanes, and the winds' tiles
   off[7] = all.size();
   for (int m = 0; m < (int)act.size(); ++m) {
@@ -1458,7 +1500,7 @@ int create_common(const mlc_params *params, int capacity, size_t budget, mlc_ctx
   L.col_x = 32; L.col_y = 4;
   L.solve_x = 32; L.solve_y = 2;
   L.vert_x = 32; L.vert_y = 4;
-  L.htile = 1;  // 64x8 tiles; the autotuner's fixed configuration is 32x8
+  L.htile = -1;  // by size; the autotuner's fixed configuration is 32x8
   L.solve_df = 1;  // the mixed solve's recurrence to FP64 accuracy
   cudaError_t e = cudaGetDevice(&x->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking);
@@ -2006,9 +2048,10 @@ int autotune_impl(mlc_ctx *x, int steps, mlc_tune_report *rep) {
   int pick[4] = {0, 0, 0, 0};
   int st = MLC_OK;
   const int ntrial = 6;
-  for (int tr = 0; tr < ntrial && st == MLC_OK; ++tr) {
+  for (int tr = 0; tr <= ntrial && st == MLC_OK; ++tr) {
     LaunchGeom L = base;
-    int idx[4] = {tr % kNCol, tr % kNSolve, tr % kNVert, tr % kNTile};
+    // the last trial: the horizontal WAF tiles by size
+    int idx[4] = {tr % kNCol, tr % kNSolve, tr % kNVert, tr < ntrial ? tr % kNTile : -1};
     set_shapes(L, idx[0], idx[1], idx[2], idx[3]);
     if (!shapes_fit(L)) {  // keep the base solve/vertical shapes for this trial
       L.solve_x = base.solve_x; L.solve_y = base.solve_y;
@@ -2055,7 +2098,8 @@ int autotune_impl(mlc_ctx *x, int steps, mlc_tune_report *rep) {
     rep->col_x = tuned.col_x; rep->col_y = tuned.col_y;
     rep->solve_x = tuned.solve_x; rep->solve_y = tuned.solve_y;
     rep->vert_x = tuned.vert_x; rep->vert_y = tuned.vert_y;
-    rep->htile = tuned.htile;
+    // (128-column tiles, which only the rule on sizes takes, as 64-column ones)
+    rep->htile = waf_tile(tuned) < kNTile ? waf_tile(tuned) : 1;
     rep->ms_fixed = msf[0] + msf[1] + msf[2] + msf[3];
     rep->ms_tuned = mst[0] + mst[1] + mst[2] + mst[3];
   }

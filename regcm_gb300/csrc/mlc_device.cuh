@@ -171,12 +171,10 @@ struct Dom {
   DiagDev *diag;
   double *partials;
   R *spec;               // spectral nudging: per field and level, iy rows of km2 coefficients
-  // an FP64 member's s(k)*zrfmu(k) - s(k+1)*zrfmd(k) of the advection round
-  // (the vertical WAF update's divergence factor, the same for every field)
-  double *vdiv;
-  // an FP64 member's flux factors of interface k+1 at level k's offset:
-  // zamu = s*dtrdz, zmi = zamu - is and zmih = zmi/2 (the vertical WAF's)
-  double *vzamu, *vzmih, *vzmi;
+  // an FP64 member's vertical WAF factors of the advection round, the same for
+  // every field, at level k's offset: s(k)*zrfmu(k), s(k+1)*zrfmd(k), their
+  // difference, and -zmih = (is - zamu)/2 of interface k+1
+  double *vcu, *vcd, *vdiv, *vnz;
   // physics tendencies of the open step (null: zero), fields of the state's
   // layout: tten, uten, vten, then nqx qxten, then ntr chiten
   const R *tend;
@@ -190,7 +188,7 @@ struct Dom {
   // [horizontal tile shape][field], for the horizontal WAF's halo tiles
   const void *tmap;
 };
-constexpr int kTileShapes = 4;
+constexpr int kTileShapes = 5;
 constexpr int kTmapBytes = 128;
 // Tensor maps per tile shape: the kMaxFields wz fields of the R table, then
 // the planes the increment form of a mixed member reads: theta_v and Exner
@@ -204,29 +202,40 @@ constexpr int kTmapSlots = kMaxFields + kIncMaps;
 // Tile shapes of the horizontal WAF (LaunchGeom::htile).  A warp is one row
 // of 32*v columns, lane l holding columns v*l .. v*l+v-1; a block is nw rows.
 // Every warp computes its whole range and writes all but two columns at each
-// end (the zonal fluxes of a column need the intermediate field two columns
-// either side), so consecutive tiles overlap by four columns.
-//   0 = 32x8, 1 = 64x8, 2 = 64x4, 3 = 32x4 (columns x rows)
+// end (hshape_writes), so consecutive tiles overlap by four columns.
+//   0 = 32x8, 1 = 64x8, 2 = 64x4, 3 = 32x4 (columns x rows), and, for FP32
+//   members by the rule on sizes alone, 4 = 128x8
+// All shapes give the same bits.
 struct HShape {
   int v, nw;
 };
 __host__ __device__ constexpr HShape hshape(int elem_bytes, int idx) {
-  return (void)elem_bytes,
-         idx == 1 ? HShape{2, 8} : idx == 2 ? HShape{2, 4} : idx == 3 ? HShape{1, 4} : HShape{1, 8};
+  return idx == 4 && elem_bytes == 4 ? HShape{4, 8}
+         : idx == 1 || idx == 4      ? HShape{2, 8}
+         : idx == 2                  ? HShape{2, 4}
+         : idx == 3                  ? HShape{1, 4}
+                                     : HShape{1, 8};
 }
 // The increment-form WAF (theta_v and Exner of a mixed member, two planes per
 // field) runs the same lanes in blocks of four rows.
 __host__ __device__ constexpr HShape hshape_inc(int idx) {
   return HShape{hshape(4, idx).v, 4};
 }
-// Column offset (j - 1) of the first tile's first column: at most -2, so the
-// first written column is j <= 1, and a multiple of v (aligned lane vectors).
-__host__ __device__ constexpr int hshape_ob0(int v) { return -(v > 2 ? v : 2); }
-// Columns the halo tile's TMA box starts left of the warp range, so that the
-// copy starts on 16 bytes (tile offsets step by 32*v - 4, a multiple of 16
-// bytes); the box is 32*v + 2*off columns by nw + 4 rows.
-__host__ __device__ constexpr int hshape_off(int elem_bytes, int v) {
-  return ((hshape_ob0(v) % (16 / elem_bytes)) + 16 / elem_bytes) % (16 / elem_bytes);
+// Tile bj's range starts at column offset (j - 1) bj*(32*v - 4), which is a
+// multiple of 16 bytes (the halo tile's TMA copy starts there).  The zonal
+// flux at a column needs the intermediate field two columns either side, but
+// for the domain's first and last columns, whose upwind differences are
+// clamped: the first tile writes from its first column on and the last to its
+// last, so a domain of n columns takes the fewest tiles with
+// tiles*(32*v - 4) + 4 >= n.
+__host__ __device__ constexpr int hshape_tiles(int v, int jx) {
+  const int s = 32 * v - 4;
+  return jx - 1 <= s + 4 ? 1 : (jx - 1 - 4 + s - 1) / s;
+}
+// whether the tile starting at column offset ob writes its range column cc
+__host__ __device__ constexpr bool hshape_writes(int v, int cc, int ob, int jx) {
+  const int j = ob + cc + 1, w = 32 * v;
+  return j <= jx - 1 && (cc >= 2 || ob == 0) && (cc <= w - 3 || ob + w >= jx - 1);
 }
 
 // A per-domain constant in the kernel's field type: the FP64 value for an

@@ -39,7 +39,8 @@ struct LaunchGeom {
   int frame_points;      // points a level of the largest member's frame (Scal::frame)
   int lv;                // levels a thread of the point kernels runs (1 or 4)
   int vert_x, vert_y;    // adv_vertical
-  int htile;             // adv_horizontal tile shape (hshape)
+  int htile;             // adv_horizontal tile shape (hshape) asked for, -1: by size
+  int size_tile, size_tile_inc;  // the shapes by size (refresh)
   int nadv_r;            // advected fields of type R per member
   int nadv_d;            // advected FP64 fields per member (mixed: theta_v, Exner)
   int red_blocks;        // reduction blocks of the largest member
@@ -53,10 +54,14 @@ struct LaunchGeom {
   const WorkItem *wl_solve;  // row segments of solve_segment columns
   const WorkItem *wl_vert;   // vert_x x vert_y column tiles, R fields
   const WorkItem *wl_vinc;   // the same, the two double-float fields
-  const WorkItem *wl_h;      // horizontal WAF tiles (shape htile), levels
+  const WorkItem *wl_h;      // horizontal WAF tiles (shape waf_tile), levels
   const WorkItem *wl_hinc;   // increment-form WAF tiles, levels
   int n_pt, n_v4, n_vec, n_wind, n_solve, n_vert, n_vinc, n_h, n_hinc;
 };
+
+// Tile shapes of the horizontal WAF kernels
+inline int waf_tile(const LaunchGeom &L) { return L.htile >= 0 ? L.htile : L.size_tile; }
+inline int waf_tile_inc(const LaunchGeom &L) { return L.htile >= 0 ? L.htile : L.size_tile_inc; }
 
 template <class R> struct Launch {
   // one-off kernel attributes (large dynamic shared memory); call before capture
