@@ -963,31 +963,12 @@ Clock get_clock(mlc_ctx *x, int slot, int *st) {
 // Copy a packed (Fortran extents nj x ni x nk) host array into the padded
 // device layout through the staging buffer at element offset `soff`.  One
 // stream orders every copy and (un)pack, so consecutive fields may reuse the
-// same staging slice.
-// An FP64 array goes straight between the packed host array and the padded
-// device layout in one pitched copy (rows of nj, ni rows of a plane on the
-// host, iy on the device); a conversion to FP32 goes through the staging buffer.
-cudaMemcpy3DParms pitched(const Geom &g, const double *host, double *dev, int nj, int ni, int nk,
-                          bool to_device) {
-  cudaMemcpy3DParms c{};
-  cudaPitchedPtr hp = make_cudaPitchedPtr(const_cast<double *>(host), (size_t)nj * sizeof(double),
-                                          (size_t)nj, (size_t)ni);
-  cudaPitchedPtr dp = make_cudaPitchedPtr(dev, (size_t)g.P * sizeof(double), (size_t)g.P, (size_t)g.iy);
-  c.srcPtr = to_device ? hp : dp;
-  c.dstPtr = to_device ? dp : hp;
-  c.extent = make_cudaExtent((size_t)nj * sizeof(double), (size_t)ni, (size_t)nk);
-  c.kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-  return c;
-}
-
+// same staging slice.  (A pitched copy straight into the layout is slower
+// wherever rows are not whole 32-byte sectors or the host array is pageable:
+// the state of 201x157x35 3.88 ms pitched, 1.02 so; 512x512x41 4.80 and 4.62.)
 template <class R>
 int put3(mlc_ctx *x, const Geom &g, const double *h, R *dst, int nj, int ni, int nk, size_t soff) {
   if (!h) return MLC_OK;
-  if constexpr (sizeof(R) == sizeof(double)) {
-    const cudaMemcpy3DParms c = pitched(g, h, reinterpret_cast<double *>(dst), nj, ni, nk, true);
-    MLC_TRY(cudaMemcpy3DAsync(&c, x->stream));
-    return MLC_OK;
-  }
   const size_t n = (size_t)nj * ni * nk;
   if (soff + n > x->staging_elems) return MLC_ERR_INVALID;
   MLC_TRY(cudaMemcpyAsync(x->staging + soff, h, n * sizeof(double), cudaMemcpyHostToDevice, x->stream));
@@ -1013,12 +994,20 @@ template <class R>
 int get3x(mlc_ctx *x, const Geom &g, const double *src, double *h, int nj, int ni, int nk,
           size_t soff, size_t nplane);
 
+// An FP64 array goes back from the padded device layout to the packed host
+// array in one pitched copy (rows of nj, ni rows of a plane on the host, iy on
+// the device), the faster way in this direction (512x512x41 4.53 ms against
+// 5.03 packed first); a mixed member's FP32 field is packed and converted
+// through the staging buffer.
 template <class R>
 int get3(mlc_ctx *x, const Geom &g, const R *src, double *h, int nj, int ni, int nk, size_t soff) {
   if (!h) return MLC_OK;
   if constexpr (sizeof(R) == sizeof(double)) {
-    const cudaMemcpy3DParms c =
-        pitched(g, h, reinterpret_cast<double *>(const_cast<R *>(src)), nj, ni, nk, false);
+    cudaMemcpy3DParms c{};
+    c.srcPtr = make_cudaPitchedPtr(const_cast<R *>(src), (size_t)g.P * sizeof(double), (size_t)g.P, (size_t)g.iy);
+    c.dstPtr = make_cudaPitchedPtr(h, (size_t)nj * sizeof(double), (size_t)nj, (size_t)ni);
+    c.extent = make_cudaExtent((size_t)nj * sizeof(double), (size_t)ni, (size_t)nk);
+    c.kind = cudaMemcpyDeviceToHost;
     MLC_TRY(cudaMemcpy3DAsync(&c, x->stream));
     return MLC_OK;
   }
@@ -1105,47 +1094,33 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
       if (b[e] > p.nspgx || b[e] == 0 || b[e] < -1) return MLC_ERR_INVALID;
   c.rdzita = 1.0 / s->zita[kz - 1];
   c.rdzitaf = float(c.rdzita);
-  // 3-D metric: one field at a time through the staging buffer
-  MLC_CHK(put3<R>(x, g, s->fmz, W(a.fmz), jx - 1, iy - 1, kz, 0));
-  MLC_CHK(put3<R>(x, g, s->fmzf, W(a.fmzf), jx - 1, iy - 1, kz + 1, 0));
-  if (sizeof(R) != sizeof(double)) {
-    // the hydrostatic factor of the mixed solve, cp*fmzf*dtrdz, in FP64
-    const double dtrdz = c.dtsound * (1.0 / s->zita[kz - 1]);
-    const size_t n = (size_t)(jx - 1) * (iy - 1) * (kz + 1);
-    std::vector<double> cf(n);
-    for (size_t e = 0; e < n; ++e) cf[e] = kCpd * s->fmzf[e] * dtrdz;
-    MLC_CHK(put3x<R>(x, g, cf.data(), W(a.cfz), jx - 1, iy - 1, kz + 1, 0, g.PS * (size_t)(kz + 1)));
-    MLC_TRY(cudaStreamSynchronize(x->stream));
+  // 3-D metric: FP64 members straight into place; mixed members' fmz and fmzf
+  // stay in the staging buffer for bind_derived
+  const size_t nc = (size_t)(jx - 1) * (iy - 1) * kz;
+  const double *fmz_src, *fmzf_src;
+  size_t fp, fps;
+  if constexpr (sizeof(R) == sizeof(double)) {
+    MLC_CHK(put3<R>(x, g, s->fmz, W(a.fmz), jx - 1, iy - 1, kz, 0));
+    MLC_CHK(put3<R>(x, g, s->fmzf, W(a.fmzf), jx - 1, iy - 1, kz + 1, 0));
+    fmz_src = a.fmz;
+    fmzf_src = a.fmzf;
+    fp = g.P;
+    fps = g.PS;
+  } else {
+    const size_t nf = (size_t)(jx - 1) * (iy - 1) * (kz + 1);
+    if (nc + nf > x->staging_elems) return MLC_ERR_INVALID;
+    MLC_TRY(cudaMemcpyAsync(x->staging, s->fmz, nc * sizeof(double), cudaMemcpyHostToDevice, x->stream));
+    MLC_TRY(cudaMemcpyAsync(x->staging + nc, s->fmzf, nf * sizeof(double), cudaMemcpyHostToDevice, x->stream));
+    fmz_src = x->staging;
+    fmzf_src = x->staging + nc;
+    fp = (size_t)(jx - 1);
+    fps = (size_t)(jx - 1) * (iy - 1);
   }
-  MLC_CHK(put3<R>(x, g, s->rfmzu, W(a.rfmzu), jx, iy - 1, kz, 0));
-  MLC_CHK(put3<R>(x, g, s->rfmzv, W(a.rfmzv), jx - 1, iy, kz, 0));
-  MLC_CHK(put3<double>(x, g, s->zeta, W(a.zeta), jx - 1, iy - 1, kz, 0));
-  MLC_CHK(put3<double>(x, g, s->dz, W(a.dz), jx - 1, iy - 1, kz, 0));
-  if (sizeof(R) != sizeof(double)) {
-    MLC_CHK(put3<R>(x, g, s->dz, W(a.dz_r), jx - 1, iy - 1, kz, 0));
-    // the remainder dz - (float)dz, so that {dz_r, dz_lo} carries dz to FP64 accuracy
-    const size_t n = (size_t)(jx - 1) * (iy - 1) * kz;
-    std::vector<double> lo(n);
-    for (size_t e = 0; e < n; ++e) lo[e] = s->dz[e] - (double)(float)s->dz[e];
-    MLC_CHK(put3<R>(x, g, lo.data(), W(a.dz_lo), jx - 1, iy - 1, kz, 0));
-    MLC_TRY(cudaStreamSynchronize(x->stream));
-  }
-  // vertical WAF ratios (dtrdz*fmz)/fmzf, Main/mod_moloch.F90:888-889
-  {
-    const double mo_dzita = s->zita[kz - 1];
-    const double dtrdz = 0.5 * (c.dtstepa * (1.0 / mo_dzita));
-    const size_t c2 = (size_t)(jx - 1) * (iy - 1);
-    std::vector<double> zu(c2 * kz), zd(c2 * kz);
-    for (int k = 0; k < kz; ++k)
-      for (size_t e = 0; e < c2; ++e) {
-        const double fz = s->fmz[e + c2 * k];
-        zu[e + c2 * k] = dtrdz * fz / s->fmzf[e + c2 * k];
-        zd[e + c2 * k] = dtrdz * fz / s->fmzf[e + c2 * (k + 1)];
-      }
-    MLC_CHK(put3<R>(x, g, zu.data(), W(a.zrfmu), jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3<R>(x, g, zd.data(), W(a.zrfmd), jx - 1, iy - 1, kz, 0));
-    MLC_TRY(cudaStreamSynchronize(x->stream));
-  }
+  const size_t soff = sizeof(R) == sizeof(double) ? 0 : nc + (size_t)(jx - 1) * (iy - 1) * (kz + 1);
+  MLC_CHK(put3<R>(x, g, s->rfmzu, W(a.rfmzu), jx, iy - 1, kz, soff));
+  MLC_CHK(put3<R>(x, g, s->rfmzv, W(a.rfmzv), jx - 1, iy, kz, soff));
+  MLC_CHK(put3<double>(x, g, s->zeta, W(a.zeta), jx - 1, iy - 1, kz, soff));
+  MLC_CHK(put3<double>(x, g, s->dz, W(a.dz), jx - 1, iy - 1, kz, soff));
   // 2-D fields and init_moloch derivations (Main/mod_moloch.F90:258-271)
   std::vector<double> t2(nd);
   auto copy2 = [&](const double *h, size_t n) { t2.assign(h, h + n); };
@@ -1239,93 +1214,24 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
     MLC_CHK(put1(x, sl.data(), a.slat, iy));
   }
   if (sizeof(R) == sizeof(double)) {
-    // the acoustic substep's constant factors, in the kernels' operand order
-    // (the same products the kernels formed every substep)
-    const bool rot = p.lrotllr != 0;
-    const double dtrdx = c.dtrdxs, dtrdy = c.dtrdxs, dxrdt = c.dxrdt, dts = c.dtsound;
-    const double zfz = kGrav * dts;
-    std::vector<double> xkd(kz), gkh(kz);
-    for (int k = 1; k <= kz; ++k) {
-      xkd[k - 1] = kNuMax * kDdamp * (1.0 / (k + 1.0) - 1.0 / (kz + 2.0));
-      gkh[k - 1] = gzita(s->zitah[k - 1], p.mo_ztop, p.mo_a0);
-    }
-    const size_t nu = (size_t)jx * (iy - 1), nv = (size_t)(jx - 1) * iy, nc = (size_t)(jx - 1) * (iy - 1);
-    std::vector<double> fu(nu * kz), fv(nv * kz), fc(nc * kz), gu(nu * kz), gv(nv * kz);
-    std::vector<double> cu(nu), cvv(nv);
-    for (int k = 0; k < kz; ++k)
-      for (int i = 0; i < iy - 1; ++i)
-        for (int j = 0; j < jx; ++j) {
-          const size_t e = (size_t)j + (size_t)i * jx, e3 = e + nu * k;
-          const double rmu = 1.0 / s->msfu[e];
-          fu[e3] = rot ? dtrdx * s->rfmzu[e3] : dtrdx * s->rfmzu[e3] * rmu;
-          gu[e3] = zfz * s->hx[e] * gkh[k];
-        }
-    for (int k = 0; k < kz; ++k)
-      for (int i = 0; i < iy; ++i)
-        for (int j = 0; j < jx - 1; ++j) {
-          const size_t e2 = (size_t)j + (size_t)i * jx;          // msfv (jx, iy)
-          const size_t e = (size_t)j + (size_t)i * (jx - 1), e3 = e + nv * k;
-          const double rmv = 1.0 / s->msfv[e2];
-          fv[e3] = dtrdy * s->rfmzv[e3] * rmv;
-          gv[e3] = zfz * s->hy[e] * gkh[k];
-        }
-    for (int k = 0; k < kz; ++k)
-      for (int i = 0; i < iy - 1; ++i)
-        for (int j = 0; j < jx - 1; ++j) {
-          const size_t e2 = (size_t)j + (size_t)i * jx;
-          const size_t e3 = (size_t)j + (size_t)i * (jx - 1) + nc * k;
-          const double mfac = rot ? s->msfx[e2] : s->msfx[e2] * s->msfx[e2];
-          fc[e3] = s->fmz[e3] * mfac;
-        }
-    MLC_CHK(put3<double>(x, g, fu.data(), W(a.dv_cu), jx, iy - 1, kz, 0));
-    MLC_CHK(put3<double>(x, g, fv.data(), W(a.dv_cv), jx - 1, iy, kz, 0));
-    MLC_CHK(put3<double>(x, g, fc.data(), W(a.dv_cf), jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3<double>(x, g, gu.data(), W(a.mo_gu), jx, iy - 1, kz, 0));
-    MLC_CHK(put3<double>(x, g, gv.data(), W(a.mo_gv), jx - 1, iy, kz, 0));
-    MLC_TRY(cudaStreamSynchronize(x->stream));
-    for (int k = 0; k < kz; ++k)
-      for (int i = 0; i < iy - 1; ++i)
-        for (int j = 0; j < jx; ++j) {
-          const size_t e = (size_t)j + (size_t)i * jx;
-          fu[e + nu * k] = dxrdt * xkd[k] * s->msfu[e];
-        }
-    for (int k = 0; k < kz; ++k)
-      for (int i = 0; i < iy; ++i)
-        for (int j = 0; j < jx - 1; ++j) {
-          const size_t e2 = (size_t)j + (size_t)i * jx;
-          const size_t e = (size_t)j + (size_t)i * (jx - 1);
-          fv[e + nv * k] = rot ? dxrdt * xkd[k] : dxrdt * xkd[k] * s->msfv[e2];
-        }
-    for (size_t e = 0; e < nu; ++e) cu[e] = kOmega2 * std::sin(s->ulat[e] * kDegrad) * dts;
-    for (size_t e = 0; e < nv; ++e) cvv[e] = kOmega2 * std::sin(s->vlat[e] * kDegrad) * dts;
-    MLC_CHK(put3<double>(x, g, fu.data(), W(a.mo_du), jx, iy - 1, kz, 0));
-    MLC_CHK(put3<double>(x, g, fv.data(), W(a.mo_dv), jx - 1, iy, kz, 0));
+    std::vector<double> cu((size_t)jx * (iy - 1)), cvv((size_t)(jx - 1) * iy);
+    for (size_t e = 0; e < cu.size(); ++e) cu[e] = kOmega2 * std::sin(s->ulat[e] * kDegrad) * c.dtsound;
+    for (size_t e = 0; e < cvv.size(); ++e) cvv[e] = kOmega2 * std::sin(s->vlat[e] * kDegrad) * c.dtsound;
     MLC_CHK(put3<double>(x, g, cu.data(), W(a.mo_cu), jx, iy - 1, 1, 0));
     MLC_CHK(put3<double>(x, g, cvv.data(), W(a.mo_cv), jx - 1, iy, 1, 0));
     MLC_TRY(cudaStreamSynchronize(x->stream));
-    // the solve's factors: (bw*dtrdz)*fmz, (dtrdz*R/cv)*fmz and dtrdz*fmz
-    // (dtrdz = dtsound*rdzita)
-    const double sdtrdz = c.dtsound * c.rdzita;
-    const double zcs = sdtrdz * kRdrcv;
-    const int nsp = p.nspgx;
-    std::vector<double> fa(nc * kz), fb(nc * kz);
-    for (int k = 0; k < kz; ++k)
-      for (int i = 0; i < iy - 1; ++i)
-        for (int j = 0; j < jx - 1; ++j) {
-          const size_t e2 = (size_t)j + (size_t)i * jx;
-          const size_t e3 = (size_t)j + (size_t)i * (jx - 1) + nc * k;
-          const int ib = s->ibnd_cr[e2];
-          const double bw = ib > 0 ? 1.0 - s->hefc[(size_t)(ib - 1) + (size_t)k * nsp] : 1.0;
-          fa[e3] = (bw * sdtrdz) * s->fmz[e3];
-          fb[e3] = zcs * s->fmz[e3];
-        }
-    MLC_CHK(put3<double>(x, g, fa.data(), W(a.sv_a), jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3<double>(x, g, fb.data(), W(a.sv_b), jx - 1, iy - 1, kz, 0));
-    MLC_TRY(cudaStreamSynchronize(x->stream));
-    for (size_t e = 0; e < nc * kz; ++e) fa[e] = sdtrdz * s->fmz[e];
-    MLC_CHK(put3<double>(x, g, fa.data(), W(a.sv_c), jx - 1, iy - 1, kz, 0));
-    MLC_TRY(cudaStreamSynchronize(x->stream));
   }
+  BindPar bp{};
+  bp.dtrdz_adv = 0.5 * (c.dtstepa * c.rdzita);
+  bp.dtrdz = c.dtsound * c.rdzita;
+  bp.zcs = bp.dtrdz * kRdrcv;
+  bp.dtrdx = c.dtrdxs;
+  bp.dxrdt = c.dxrdt;
+  bp.zfz = kGrav * c.dtsound;
+  bp.rot = p.lrotllr != 0;
+  bp.nspgx = p.nspgx;
+  Launch<R>::bind_derived(a, g, fmz_src, fmzf_src, fp, fps, bp, x->stream);
+  MLC_TRY(cudaGetLastError());
   if (p.mo_spectral_nudge) {
     // lowpass_init (Main/mod_bdycod.F90:3844-3896, one process: njcross =
     // jx-1, nicross = iy-1) in FP64, rows of the modes k = 1..2km over

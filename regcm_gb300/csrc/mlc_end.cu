@@ -1655,6 +1655,74 @@ __global__ void k_unpack3(const double *__restrict__ src, R *__restrict__ dst, G
   }
 }
 
+// What a member keeps derived from the bound 3-D fields, formed where the data
+// is: each source crosses the host link once and the host forms no 3-D array
+// (binding members of 96x96x30 and 157x157x30: mixed 6.0 ms with these products
+// formed on the host, 1.9 so; FP64 16.9 and 2.3).  Every product and quotient
+// is rounded by itself.
+// Points of the cross grid: the vertical WAF's ratios; mixed members' FP32
+// copies, the hydrostatic factor cp*fmzf*dtrdz and dz as a double-float; FP64
+// members' factors of the divergence and of the solve.
+template <class R>
+__global__ void k_bind_cross(Stat<R> sa, Geom g, const double *__restrict__ fmz,
+                             const double *__restrict__ fmzf, size_t fp, size_t fps, BindPar b) {
+  constexpr bool f64 = sizeof(R) == sizeof(double);
+  const size_t nj = (size_t)g.jx - 1, ni = (size_t)g.iy - 1, n = nj * ni * (size_t)(g.kz + 1);
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const size_t j = e % nj, r = e / nj, i = r % ni;
+    const int k = (int)(r / ni);
+    const size_t o2 = j + i * g.P, o = o2 + (size_t)k * g.PS, f = j + i * fp + (size_t)k * fps;
+    const double zf = fmzf[f];
+    if constexpr (!f64) {
+      const_cast<R *>(sa.fmzf)[o] = (R)zf;
+      const double c = __dmul_rn(__dmul_rn(kCpd, zf), b.dtrdz);
+      float *cf = reinterpret_cast<float *>(const_cast<double *>(sa.cfz));
+      cf[o] = (float)c;
+      cf[o + g.PS * (size_t)(g.kz + 1)] = (float)(c - (double)(float)c);
+    }
+    if (k >= g.kz) continue;
+    const double fz = fmz[f];
+    const double a = __dmul_rn(b.dtrdz_adv, fz);
+    const_cast<R *>(sa.zrfmu)[o] = (R)__ddiv_rn(a, zf);
+    const_cast<R *>(sa.zrfmd)[o] = (R)__ddiv_rn(a, fmzf[f + fps]);
+    if constexpr (f64) {
+      const int ib = sa.ibnd_cr[o2];
+      const double bw = ib > 0 ? 1.0 - sa.hefc[(size_t)(ib - 1) + (size_t)k * b.nspgx] : 1.0;
+      const_cast<double *>(sa.dv_cf)[o] = __dmul_rn(fz, b.rot ? sa.msfx[o2] : sa.mx2[o2]);
+      const_cast<double *>(sa.sv_a)[o] = __dmul_rn(__dmul_rn(bw, b.dtrdz), fz);
+      const_cast<double *>(sa.sv_b)[o] = __dmul_rn(b.zcs, fz);
+      const_cast<double *>(sa.sv_c)[o] = __dmul_rn(b.dtrdz, fz);
+    } else {
+      const_cast<R *>(sa.fmz)[o] = (R)fz;
+      const double dz = sa.dz[o];
+      const_cast<R *>(sa.dz_r)[o] = (R)dz;
+      const_cast<R *>(sa.dz_lo)[o] = (R)(dz - (double)(R)dz);
+    }
+  }
+}
+
+// Wind points of an FP64 member: the acoustic substep's constant factors.
+__global__ void k_bind_wind(Stat<double> sa, Geom g, BindPar b) {
+  const size_t nj = (size_t)g.jx, ni = (size_t)g.iy, n = nj * ni * (size_t)g.kz;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const size_t j = e % nj, r = e / nj, i = r % ni;
+    const int k = (int)(r / ni);
+    const size_t o2 = j + i * g.P, o = o2 + (size_t)k * g.PS;
+    const double gk = sa.gzitakh[k], dk = __dmul_rn(b.dxrdt, sa.xkdamp[k]);
+    if (i < ni - 1) {
+      const double c = __dmul_rn(b.dtrdx, sa.rfmzu[o]);
+      const_cast<double *>(sa.dv_cu)[o] = b.rot ? c : __dmul_rn(c, sa.rmu[o2]);
+      const_cast<double *>(sa.mo_gu)[o] = __dmul_rn(__dmul_rn(b.zfz, sa.hx[o2]), gk);
+      const_cast<double *>(sa.mo_du)[o] = __dmul_rn(dk, sa.msfu[o2]);
+    }
+    if (j < nj - 1) {
+      const_cast<double *>(sa.dv_cv)[o] = __dmul_rn(__dmul_rn(b.dtrdx, sa.rfmzv[o]), sa.rmv[o2]);
+      const_cast<double *>(sa.mo_gv)[o] = __dmul_rn(__dmul_rn(b.zfz, sa.hy[o2]), gk);
+      const_cast<double *>(sa.mo_dv)[o] = b.rot ? dk : __dmul_rn(dk, sa.msfv[o2]);
+    }
+  }
+}
+
 template <class R>
 __global__ void k_pack3(const R *__restrict__ src, double *__restrict__ dst, Geom g, int nj, int ni, int nk) {
   const size_t n = (size_t)nj * ni * nk;
@@ -1854,6 +1922,13 @@ void Launch<R>::end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int 
                            cudaStream_t s) {
   k_reduce_partial<R><<<dim3((unsigned)L.red_blocks, (unsigned)L.nmem), kRedThreads, 0, s>>>(
       d, uvoff, advoff, form_ps ? 1 : 0);
+}
+
+template <class R>
+void Launch<R>::bind_derived(const Stat<R> &sa, const Geom &g, const double *fmz, const double *fmzf,
+                             size_t fp, size_t fps, const BindPar &b, cudaStream_t s) {
+  k_bind_cross<R><<<152 * 8, 256, 0, s>>>(sa, g, fmz, fmzf, fp, fps, b);
+  if constexpr (sizeof(R) == sizeof(double)) k_bind_wind<<<152 * 8, 256, 0, s>>>(sa, g, b);
 }
 
 template <class R>

@@ -63,6 +63,15 @@ struct LaunchGeom {
 inline int waf_tile(const LaunchGeom &L) { return L.htile >= 0 ? L.htile : L.size_tile; }
 inline int waf_tile_inc(const LaunchGeom &L) { return L.htile >= 0 ? L.htile : L.size_tile_inc; }
 
+// Constants of the derived time-invariant fields (bind_cross, bind_wind)
+struct BindPar {
+  double dtrdz_adv;  // 0.5*dtstepa/dzita
+  double dtrdz;      // dtsound/dzita
+  double zcs;        // dtrdz*R/cv
+  double dtrdx, dxrdt, zfz;  // dtsound/dx, dx/dtsound, g*dtsound
+  int rot, nspgx;
+};
+
 template <class R> struct Launch {
   // one-off kernel attributes (large dynamic shared memory); call before capture
   static cudaError_t configure_sound();
@@ -109,6 +118,10 @@ template <class R> struct Launch {
   static void end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps,
                          cudaStream_t s);
   // ---- layout conversion (one member, from the host) ----
+  // the 3-D fields derived from the bound ones (fmz, fmzf: of row pitch fp and
+  // plane fps; the 1-D and 2-D fields and, for FP64, rfmzu and rfmzv in place)
+  static void bind_derived(const Stat<R> &sa, const Geom &g, const double *fmz, const double *fmzf,
+                           size_t fp, size_t fps, const BindPar &b, cudaStream_t s);
   static void unpack3(const double *src, R *dst, const Geom &g, int nj, int ni, int nk,
                       cudaStream_t s);
   static void pack3(const R *src, double *dst, const Geom &g, int nj, int ni, int nk,
