@@ -267,6 +267,7 @@ __device__ __forceinline__ void field_t(const Dom<R> &D, int set, int f, int adv
 template <class R, int LV>
 __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -379,6 +380,7 @@ template <class R, class T>
 __global__ void __launch_bounds__(256, vert_min_blocks<T>())
     k_adv_vertical(const Dom<R> *__restrict__ doms, int nf, int set, int advoff,
                                const WorkItem *__restrict__ wl) {
+  grid_begin();
   const WorkItem wi = wl ? wl[blockIdx.x]
                           : WorkItem{(int16_t)blockIdx.z, (int16_t)(blockIdx.x / (unsigned)nf),
                                      (int16_t)blockIdx.y, (int16_t)(blockIdx.x % (unsigned)nf)};
@@ -612,6 +614,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
     k_adv_horizontal(const Dom<R> *__restrict__ doms,
                                                            int tiles_j, int uvoff, int advoff,
     const WorkItem *__restrict__ wl) {
+  grid_begin();
   using T = R;
   constexpr int W = 32 * V;       // columns of a warp's range
   constexpr int S = W - 4;        // columns from a tile to the next (hshape_writes)
@@ -901,6 +904,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(sizeof(R) == sizeof
 template <class R, int LV>
 __global__ void k_species_copy(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -920,6 +924,7 @@ __global__ void k_species_copy(const Dom<R> *__restrict__ doms, int advoff, int 
 template <class R, int LV>
 __global__ void k_adv_curvature(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active || !D.c.curvature) return;
@@ -959,6 +964,7 @@ __global__ void k_adv_curvature(const Dom<R> *__restrict__ doms, int advoff, int
 template <class R, int LV>
 __global__ void k_adv_back(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -1060,6 +1066,7 @@ __device__ __forceinline__ float vupdate_inc(float ek, float gb, float ga, float
 template <class R>
 __global__ void k_adv_vertical_inc(const Dom<R> *__restrict__ doms, int advoff,
                                    const WorkItem *__restrict__ wl) {
+  grid_begin();
   const WorkItem wi = wl ? wl[blockIdx.x]
                           : WorkItem{(int16_t)blockIdx.z, (int16_t)(blockIdx.x >> 1), (int16_t)blockIdx.y,
                                      (int16_t)(blockIdx.x & 1u)};
@@ -1188,6 +1195,7 @@ __global__ void __launch_bounds__(32 * NW, waf_min_blocks<R>(V == 4 ? MLC_HINC_W
                                                                int tiles_j, int uvoff,
                                                                int advoff,
                                                                const WorkItem *__restrict__ wl) {
+  grid_begin();
   constexpr int W = 32 * V, S = W - 4;
   constexpr unsigned kBox = (unsigned)((NW + 4) * W * 4);
   constexpr unsigned kBuf = (kBox + 127u) / 128u * 128u;
@@ -1505,8 +1513,8 @@ void Launch<R>::adv_prep(const LaunchGeom &L, const Dom<R> *d, int uvoff, int ad
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (L.lv == 1) k_adv_prep<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_adv_prep<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_adv_prep<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_adv_prep<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R, class T>
@@ -1519,7 +1527,7 @@ void launch_vertical(const LaunchGeom &L, const Dom<R> *d, int nf, int set, int 
   const dim3 grd = wl ? dim3((unsigned)nw, 1, 1)
                       : dim3((unsigned)(((L.jx - 1 + L.vert_x - 1) / L.vert_x) * nf),
                              (unsigned)((L.iy - 1 + L.vert_y - 1) / L.vert_y), (unsigned)L.nmem);
-  k_adv_vertical<R, T><<<grd, b, 0, s>>>(d, nf, set, advoff, wl);
+  step_launch(L, k_adv_vertical<R, T>, grd, b, 0, s, d, nf, set, advoff, wl);
 }
 
 template <class R, int V, int NW>
@@ -1527,7 +1535,7 @@ void launch_tile(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cu
   const int tj = hshape_tiles(V, L.jx), ti = (L.iy - 1 + NW - 1) / NW;
   const dim3 grd = L.wl_h ? dim3((unsigned)L.n_h, 1, 1)
                           : dim3((unsigned)(tj * ti), (unsigned)L.kz, (unsigned)L.nmem);
-  k_adv_horizontal<R, V, NW><<<grd, 32 * NW, 0, s>>>(d, tj, uvoff, advoff, L.wl_h);
+  step_launch(L, k_adv_horizontal<R, V, NW>, grd, 32 * NW, 0, s, d, tj, uvoff, advoff, L.wl_h);
 }
 
 template <class R>
@@ -1550,7 +1558,7 @@ void launch_vertical_inc(const LaunchGeom &L, const Dom<R> *d, int advoff, cudaS
   const dim3 grd = L.wl_vinc ? dim3((unsigned)L.n_vinc, 1, 1)
                              : dim3((unsigned)(((L.jx - 1 + L.vert_x - 1) / L.vert_x) * 2),
                                     (unsigned)((L.iy - 1 + L.vert_y - 1) / L.vert_y), (unsigned)L.nmem);
-  k_adv_vertical_inc<R><<<grd, b, 0, s>>>(d, advoff, L.wl_vinc);
+  step_launch(L, k_adv_vertical_inc<R>, grd, b, 0, s, d, advoff, L.wl_vinc);
 }
 
 template <class R, int V, int NW>
@@ -1558,7 +1566,7 @@ void launch_tile_inc(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff
   const int tj = hshape_tiles(V, L.jx), ti = (L.iy - 1 + NW - 1) / NW;
   const dim3 grd = L.wl_hinc ? dim3((unsigned)L.n_hinc, 1, 1)
                              : dim3((unsigned)(tj * ti), (unsigned)L.kz, (unsigned)L.nmem);
-  k_adv_horizontal_inc<R, V, NW><<<grd, 32 * NW, 0, s>>>(d, tj, uvoff, advoff, L.wl_hinc);
+  step_launch(L, k_adv_horizontal_inc<R, V, NW>, grd, 32 * NW, 0, s, d, tj, uvoff, advoff, L.wl_hinc);
 }
 
 template <class R>
@@ -1599,8 +1607,8 @@ void Launch<R>::adv_species_copy(const LaunchGeom &L, const Dom<R> *d, int advof
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (L.lv == 1) k_species_copy<R, 1><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
-  else k_species_copy<R, 4><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_species_copy<R, 1>, grd, b, 0, s, d, advoff, tj, L.wl_pt);
+  else step_launch(L, k_species_copy<R, 4>, grd, b, 0, s, d, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1608,8 +1616,8 @@ void Launch<R>::adv_curvature(const LaunchGeom &L, const Dom<R> *d, int advoff, 
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 3, L.iy - 3, tj);
-  if (L.lv == 1) k_adv_curvature<R, 1><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
-  else k_adv_curvature<R, 4><<<grd, b, 0, s>>>(d, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_adv_curvature<R, 1>, grd, b, 0, s, d, advoff, tj, L.wl_pt);
+  else step_launch(L, k_adv_curvature<R, 4>, grd, b, 0, s, d, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1617,8 +1625,8 @@ void Launch<R>::adv_back(const LaunchGeom &L, const Dom<R> *d, int uvoff, int ad
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-  if (L.lv == 1) k_adv_back<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_adv_back<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_adv_back<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_adv_back<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>

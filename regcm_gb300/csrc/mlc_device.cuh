@@ -387,6 +387,17 @@ struct DF {
   __device__ __forceinline__ float hi(size_t o) const { return p[o]; }
 };
 
+// ---- consecutive launches of a step ------------------------------------------
+// Small domains' kernels are launched with programmatic serialization
+// (step_launch): a kernel's launch overlaps the end of the kernel before it,
+// and its blocks wait here, before any access to memory, until that kernel
+// has finished and its writes are visible.  Every block of every step kernel
+// calls this first, also those with no work, so a kernel finishes only after
+// all earlier ones have.  (Without the launch attribute it does nothing; the
+// four-level point kernels, never launched so, leave it out: as a barrier to
+// the compiler it cost the mixed momentum update 20 %.)
+__device__ __forceinline__ void grid_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- work lists of an uneven batch ------------------------------------------
 // A launch over members of different extents covers, by default, the largest
 // member's tiles for every member (blockIdx.z is the member; blocks outside a

@@ -86,6 +86,7 @@ constexpr int kRingThreads = 128;
 template <class R>
 __global__ void __launch_bounds__(kRingThreads) k_bdy_ring(const Dom<R> *__restrict__ doms, int uvoff,
                                                            int advoff) {
+  grid_begin();
   const Dom<R> &D = doms[blockIdx.z];
   if (!D.active) return;
   const Geom g = D.g;
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(kRingThreads) k_bdy_ring(const Dom<R> *__restr
 template <class R, int LV>
 __global__ void k_end_relax(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -423,6 +425,7 @@ __device__ __forceinline__ R spec_departure(const Dom<R> &D, const State<R> &st,
 // kz*3, members), 256 threads.
 template <class R>
 __global__ void __launch_bounds__(256) k_spec_rows(const Dom<R> *__restrict__ doms, int uvoff, int advoff) {
+  grid_begin();
   const Dom<R> &D = doms[blockIdx.z];
   if (!D.active) return;
   const Scal &c = D.c;
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(256) k_spec_rows(const Dom<R> *__restrict__ do
 // threads per field, level and member.
 template <class R>
 __global__ void __launch_bounds__(256) k_spec_modes(const Dom<R> *__restrict__ doms) {
+  grid_begin();
   const Dom<R> &D = doms[blockIdx.z];
   if (!D.active) return;
   const Scal &c = D.c;
@@ -499,6 +503,7 @@ __global__ void __launch_bounds__(256) k_spec_modes(const Dom<R> *__restrict__ d
 template <class R, int LV>
 __global__ void k_spec_apply(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -576,6 +581,7 @@ __device__ __forceinline__ void ps_column(const Dom<R> &D, const State<R> &st, s
 // nudging (the reduction forms it in the others)
 template <class R>
 __global__ void k_end_ps(const Dom<R> *__restrict__ doms, int uvoff, int advoff) {
+  grid_begin();
   const Dom<R> &D = doms[blockIdx.z];
   if (!D.active) return;
   const Geom g = D.g;
@@ -664,6 +670,7 @@ constexpr double kTracFloor = 1.0e-50;  // mkslice's tracer floor (Main/mod_slic
 template <class R, int PH, int LV>
 __global__ void k_end_cross(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -843,6 +850,7 @@ __device__ __forceinline__ void stv(R *p, const R (&x)[V], const bool (&ok)[V], 
 template <class R, int LV, bool FRAME>
 __global__ void __launch_bounds__(128, FRAME ? 10 : 7) k_end_point(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
                                                    int tiles_j, const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   constexpr int V = FRAME ? 1 : 16 / (int)sizeof(R);
   constexpr bool mixed = sizeof(R) == sizeof(float);
   const WorkItem wi = FRAME ? WorkItem{(int16_t)blockIdx.z, 0, 0, (int16_t)blockIdx.y} : work_item(wl, tiles_j);
@@ -1183,6 +1191,7 @@ template <class R>
 __global__ void __launch_bounds__(32 * kWindWarps) k_end_winds(const Dom<R> *__restrict__ doms, int uvoff,
                                                                int advoff, int rows, int tiles_j,
                                                                const WorkItem *__restrict__ wl) {
+  grid_begin();
   constexpr int V = 4;
   static_assert(sizeof(R) == sizeof(float), "FP32 fields");
   static_assert(kWindCols == 32 * V - 8, "a lane either side is halo");
@@ -1330,6 +1339,7 @@ __global__ void __launch_bounds__(32 * kWindWarps) k_end_winds(const Dom<R> *__r
 template <class R, int LV>
 __global__ void k_end_uvx(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active || !D.c.apply_bdy) return;
@@ -1356,6 +1366,7 @@ __global__ void k_end_uvx(const Dom<R> *__restrict__ doms, int uvoff, int advoff
 template <class R, int LV>
 __global__ void k_end_uvstag(const Dom<R> *__restrict__ doms, int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -1464,6 +1475,7 @@ __device__ __forceinline__ RedSum red_block(RedSum a, bool flux, RedSum *sh) {
 template <class R>
 __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__restrict__ doms,
                                                                 int uvoff, int advoff, int form_ps) {
+  grid_begin();
   __shared__ RedSum sh[kRedWarps];
   __shared__ bool last;
   const Dom<R> &D = doms[blockIdx.y];
@@ -1795,6 +1807,7 @@ int reduce_blocks(const Geom &g) {
 template <class R, int LV>
 __global__ void k_end_tke(const Dom<R> *__restrict__ doms, int whole, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active || !D.c.tke) return;
@@ -1818,7 +1831,7 @@ __global__ void k_end_tke(const Dom<R> *__restrict__ doms, int whole, int tiles_
 template <class R>
 void Launch<R>::bdy_ring(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
   const unsigned nb = (unsigned)((2 * (L.iy - 2) + 2 * L.jx + kRingThreads - 1) / kRingThreads);
-  k_bdy_ring<R><<<dim3(nb, (unsigned)L.kz, (unsigned)L.nmem), kRingThreads, 0, s>>>(d, uvoff, advoff);
+  step_launch(L, k_bdy_ring<R>, dim3(nb, (unsigned)L.kz, (unsigned)L.nmem), kRingThreads, 0, s, d, uvoff, advoff);
 }
 
 template <class R>
@@ -1826,21 +1839,21 @@ void Launch<R>::end_relax(const LaunchGeom &L, const Dom<R> *d, int uvoff, int a
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (L.lv == 1) k_end_relax<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_end_relax<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_end_relax<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_end_relax<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
 void Launch<R>::bdy_spectral(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff,
                              cudaStream_t s) {
   const unsigned fk = (unsigned)(L.kz * 3);
-  k_spec_rows<R><<<dim3((unsigned)((L.iy + 7) / 8), fk, (unsigned)L.nmem), 256, 0, s>>>(d, uvoff, advoff);
-  k_spec_modes<R><<<dim3(1, fk, (unsigned)L.nmem), 256, 0, s>>>(d);
+  step_launch(L, k_spec_rows<R>, dim3((unsigned)((L.iy + 7) / 8), fk, (unsigned)L.nmem), 256, 0, s, d, uvoff, advoff);
+  step_launch(L, k_spec_modes<R>, dim3(1, fk, (unsigned)L.nmem), 256, 0, s, d);
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 2, L.iy - 2, tj);
-  if (L.lv == 1) k_spec_apply<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_spec_apply<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_spec_apply<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_spec_apply<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1849,14 +1862,14 @@ void Launch<R>::end_point(const LaunchGeom &L, const Dom<R> *d, int uvoff, int a
   const int tj = (L.jx - 1 + W - 1) / W, ti = (L.iy - 1 + 3) / 4;
   const dim3 grd = L.wl_vec ? dim3((unsigned)L.n_vec, 1, 1)
                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
-  if (L.lv == 1) k_end_point<R, 1, false><<<grd, 128, 0, s>>>(d, uvoff, advoff, tj, L.wl_vec);
-  else k_end_point<R, 4, false><<<grd, 128, 0, s>>>(d, uvoff, advoff, tj, L.wl_vec);
+  if (L.lv == 1) step_launch(L, k_end_point<R, 1, false>, grd, 128, 0, s, d, uvoff, advoff, tj, L.wl_vec);
+  else step_launch(L, k_end_point<R, 4, false>, grd, 128, 0, s, d, uvoff, advoff, tj, L.wl_vec);
 }
 
 template <class R>
 void Launch<R>::end_frame(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
   const dim3 grd((unsigned)((L.frame_points + 127) / 128), (unsigned)L.kz, (unsigned)L.nmem);
-  k_end_point<R, 1, true><<<grd, 128, 0, s>>>(d, uvoff, advoff, 1, nullptr);
+  step_launch(L, k_end_point<R, 1, true>, grd, 128, 0, s, d, uvoff, advoff, 1, nullptr);
 }
 
 template <class R>
@@ -1864,8 +1877,8 @@ void Launch<R>::end_uvx(const LaunchGeom &L, const Dom<R> *d, int uvoff, int adv
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (L.lv == 1) k_end_uvx<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_end_uvx<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_end_uvx<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_end_uvx<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1874,7 +1887,7 @@ void Launch<R>::end_winds(const LaunchGeom &L, const Dom<R> *d, int uvoff, int a
   const dim3 grd = L.wl_wind ? dim3((unsigned)L.n_wind, 1, 1)
                              : dim3((unsigned)(tj * ti), (unsigned)L.kz, (unsigned)L.nmem);
   if constexpr (sizeof(R) == sizeof(float))
-    k_end_winds<R><<<grd, 32 * kWindWarps, 0, s>>>(d, uvoff, advoff, L.wind_rows, tj, L.wl_wind);
+    step_launch(L, k_end_winds<R>, grd, 32 * kWindWarps, 0, s, d, uvoff, advoff, L.wind_rows, tj, L.wl_wind);
 }
 
 template <class R, int PH>
@@ -1882,9 +1895,9 @@ void launch_cross(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, c
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (PH != kEndPost) k_end_ps<R><<<grid2(L.jx - 3, L.iy - 3, b, L.nmem), b, 0, s>>>(d, uvoff, advoff);
-  if (L.lv == 1) k_end_cross<R, PH, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_end_cross<R, PH, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (PH != kEndPost) step_launch(L, k_end_ps<R>, grid2(L.jx - 3, L.iy - 3, b, L.nmem), b, 0, s, d, uvoff, advoff);
+  if (L.lv == 1) step_launch(L, k_end_cross<R, PH, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_end_cross<R, PH, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1904,8 +1917,8 @@ void Launch<R>::end_uvstag(const LaunchGeom &L, const Dom<R> *d, int uvoff, int 
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-  if (L.lv == 1) k_end_uvstag<R, 1><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-  else k_end_uvstag<R, 4><<<grd, b, 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_end_uvstag<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  else step_launch(L, k_end_uvstag<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1913,15 +1926,14 @@ void Launch<R>::end_tke(const LaunchGeom &L, const Dom<R> *d, bool whole_step, c
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-  if (L.lv == 1) k_end_tke<R, 1><<<grd, b, 0, s>>>(d, whole_step ? 1 : 0, tj, L.wl_pt);
-  else k_end_tke<R, 4><<<grd, b, 0, s>>>(d, whole_step ? 1 : 0, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_end_tke<R, 1>, grd, b, 0, s, d, whole_step ? 1 : 0, tj, L.wl_pt);
+  else step_launch(L, k_end_tke<R, 4>, grd, b, 0, s, d, whole_step ? 1 : 0, tj, L.wl_pt);
 }
 
 template <class R>
 void Launch<R>::end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps,
                            cudaStream_t s) {
-  k_reduce_partial<R><<<dim3((unsigned)L.red_blocks, (unsigned)L.nmem), kRedThreads, 0, s>>>(
-      d, uvoff, advoff, form_ps ? 1 : 0);
+  step_launch(L, k_reduce_partial<R>, dim3((unsigned)L.red_blocks, (unsigned)L.nmem), kRedThreads, 0, s, d, uvoff, advoff, form_ps ? 1 : 0);
 }
 
 template <class R>

@@ -72,6 +72,7 @@ __device__ __forceinline__ double relax_weight(const int32_t *ibnd, const double
 template <class R, int LV>
 __global__ void k_sound_prep(const Dom<R> *__restrict__ doms, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
   if (!D.active) return;
@@ -130,6 +131,7 @@ __device__ __forceinline__ R slope_wind(R u0, R hx0, R u1, R hx1, R v0, R hy0, R
 template <class R, int LV>
 __global__ void k_sound_div(const Dom<R> *__restrict__ doms, int uvoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   static_assert(sizeof(R) == sizeof(double), "FP64 member");
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
@@ -327,6 +329,7 @@ __device__ __forceinline__ SolveLane solve_lane(const Geom &g, int x0) {
 template <class R, int AW>
 __global__ void __launch_bounds__(solve_threads(AW), 512 / solve_threads(AW)) k_solve_cols_d(const Dom<R> *__restrict__ doms, int advoff,
                                                                   int last, const WorkItem *__restrict__ wl) {
+  grid_begin();
   static_assert(sizeof(R) == sizeof(double), "FP64 member");
   constexpr int NL = kSolveLevels, NR = AW * NL;  // interfaces a warp, a round
   extern __shared__ __align__(16) double dv_smem[];
@@ -449,6 +452,7 @@ __global__ void __launch_bounds__(solve_threads(AW), 512 / solve_threads(AW)) k_
 template <class R, int AW, bool DFR>
 __global__ void __launch_bounds__(solve_threads(AW), 1024 / solve_threads(AW)) k_solve_cols_f(const Dom<R> *__restrict__ doms, int advoff,
                                                                   int last, const WorkItem *__restrict__ wl) {
+  grid_begin();
   static_assert(sizeof(R) == sizeof(float), "FP32 fields");
   constexpr int NL = kSolveLevels, NR = AW * NL;
   extern __shared__ __align__(16) float sv_smem[];
@@ -633,6 +637,7 @@ __device__ __forceinline__ void block_sync() {
 template <class R, int CW>
 __global__ void __launch_bounds__(CW, CW == 32 ? 24 : 768 / CW) k_solve_stream_d(const Dom<R> *__restrict__ doms,
     int advoff, int last, const WorkItem *__restrict__ wl) {
+  grid_begin();
   static_assert(sizeof(R) == sizeof(double), "FP64 member");
   using Sh = SolveShape<R, CW>;
   constexpr int NS = Sh::kStages, ZW = Sh::kZW;
@@ -826,6 +831,7 @@ __global__ void __launch_bounds__(CW, CW == 32 ? 24 : 768 / CW) k_solve_stream_d
 template <class R, int CW, bool DFR>
 __global__ void __launch_bounds__(CW, 7) k_solve_stream_f(const Dom<R> *__restrict__ doms,
     int advoff, int last, const WorkItem *__restrict__ wl) {
+  grid_begin();
   static_assert(sizeof(R) == sizeof(float), "FP32 fields");
   using Sh = SolveShape<R, CW>;
   constexpr int NS = Sh::kStages, ZW = Sh::kZW;
@@ -1046,6 +1052,7 @@ template <class R, int LV>
 __global__ void k_sound_momentum(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
                                  int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   const WorkItem wi = work_item(wl, tiles_j);
   static_assert(sizeof(R) == sizeof(double), "FP64 member");
   const Dom<R> &D = doms[wi.m];
@@ -1131,6 +1138,7 @@ template <class R, int LV>
 __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<R> *__restrict__ doms, int uvoff,
                                                       int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   static_assert(sizeof(R) == sizeof(float), "FP32 fields");
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
@@ -1256,6 +1264,7 @@ template <class R, int LV>
 __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const Dom<R> *__restrict__ doms,
                                                            int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
   static_assert(sizeof(R) == sizeof(float), "FP32 fields");
   const WorkItem wi = work_item(wl, tiles_j);
   const Dom<R> &D = doms[wi.m];
@@ -1410,8 +1419,8 @@ template <class R>
 void Launch<R>::sound_prep(const LaunchGeom &L, const Dom<R> *d, int advoff, cudaStream_t s) {
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-  if (L.lv == 1) k_sound_prep<R, 1><<<grd, col_block(L), 0, s>>>(d, advoff, tj, L.wl_pt);
-  else k_sound_prep<R, 4><<<grd, col_block(L), 0, s>>>(d, advoff, tj, L.wl_pt);
+  if (L.lv == 1) step_launch(L, k_sound_prep<R, 1>, grd, col_block(L), 0, s, d, advoff, tj, L.wl_pt);
+  else step_launch(L, k_sound_prep<R, 4>, grd, col_block(L), 0, s, d, advoff, tj, L.wl_pt);
 }
 
 template <class R>
@@ -1421,13 +1430,13 @@ void Launch<R>::sound_div(const LaunchGeom &L, const Dom<R> *d, int uvoff, cudaS
     const dim3 grd = L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
                              : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv),
                                     (unsigned)L.nmem);
-    if (L.lv == 1) k_sound_div_v4<R, 1><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, tj, L.wl_v4);
-    else k_sound_div_v4<R, 4><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, tj, L.wl_v4);
+    if (L.lv == 1) step_launch(L, k_sound_div_v4<R, 1>, grd, dim3(32, 4), 0, s, d, uvoff, tj, L.wl_v4);
+    else step_launch(L, k_sound_div_v4<R, 4>, grd, dim3(32, 4), 0, s, d, uvoff, tj, L.wl_v4);
   } else {
     int tj;
     const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
-    if (L.lv == 1) k_sound_div<R, 1><<<grd, col_block(L), 0, s>>>(d, uvoff, tj, L.wl_pt);
-    else k_sound_div<R, 4><<<grd, col_block(L), 0, s>>>(d, uvoff, tj, L.wl_pt);
+    if (L.lv == 1) step_launch(L, k_sound_div<R, 1>, grd, col_block(L), 0, s, d, uvoff, tj, L.wl_pt);
+    else step_launch(L, k_sound_div<R, 4>, grd, col_block(L), 0, s, d, uvoff, tj, L.wl_pt);
   }
 }
 
@@ -1435,10 +1444,10 @@ template <class R, int AW>
 void launch_cols(const LaunchGeom &L, const Dom<R> *d, dim3 grid, int advoff, int last, cudaStream_t s) {
   const size_t smem = solve_smem<R>(L.kz);
   if constexpr (sizeof(R) == sizeof(float)) {
-    if (L.solve_df) k_solve_cols_f<R, AW, true><<<grid, solve_threads(AW), smem, s>>>(d, advoff, last, L.wl_solve);
-    else k_solve_cols_f<R, AW, false><<<grid, solve_threads(AW), smem, s>>>(d, advoff, last, L.wl_solve);
+    if (L.solve_df) step_launch(L, k_solve_cols_f<R, AW, true>, grid, solve_threads(AW), smem, s, d, advoff, last, L.wl_solve);
+    else step_launch(L, k_solve_cols_f<R, AW, false>, grid, solve_threads(AW), smem, s, d, advoff, last, L.wl_solve);
   } else {
-    k_solve_cols_d<R, AW><<<grid, solve_threads(AW), smem, s>>>(d, advoff, last, L.wl_solve);
+    step_launch(L, k_solve_cols_d<R, AW>, grid, solve_threads(AW), smem, s, d, advoff, last, L.wl_solve);
   }
 }
 
@@ -1459,10 +1468,10 @@ void Launch<R>::sound_solve(const LaunchGeom &L, const Dom<R> *d, int uvoff, int
     using Sh = SolveShape<R, CW>;
     constexpr size_t smem = (size_t)Sh::kStages * Sh::kStage * sizeof(R);
     if constexpr (sizeof(R) == sizeof(float)) {
-      if (L.solve_df) k_solve_stream_f<R, CW, true><<<grid, CW, smem, s>>>(d, advoff, lst, L.wl_solve);
-      else k_solve_stream_f<R, CW, false><<<grid, CW, smem, s>>>(d, advoff, lst, L.wl_solve);
+      if (L.solve_df) step_launch(L, k_solve_stream_f<R, CW, true>, grid, CW, smem, s, d, advoff, lst, L.wl_solve);
+      else step_launch(L, k_solve_stream_f<R, CW, false>, grid, CW, smem, s, d, advoff, lst, L.wl_solve);
     } else {
-      k_solve_stream_d<R, CW><<<grid, CW, smem, s>>>(d, advoff, lst, L.wl_solve);
+      step_launch(L, k_solve_stream_d<R, CW>, grid, CW, smem, s, d, advoff, lst, L.wl_solve);
     }
   }
 }
@@ -1476,13 +1485,13 @@ void Launch<R>::sound_momentum(const LaunchGeom &L, const Dom<R> *d, int uvoff, 
     const dim3 grd = L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
                              : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv),
                                     (unsigned)L.nmem);
-    if (L.lv == 1) k_sound_momentum_v4<R, 1><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, advoff, tj, L.wl_v4);
-    else k_sound_momentum_v4<R, 4><<<grd, dim3(32, 4), 0, s>>>(d, uvoff, advoff, tj, L.wl_v4);
+    if (L.lv == 1) step_launch(L, k_sound_momentum_v4<R, 1>, grd, dim3(32, 4), 0, s, d, uvoff, advoff, tj, L.wl_v4);
+    else step_launch(L, k_sound_momentum_v4<R, 4>, grd, dim3(32, 4), 0, s, d, uvoff, advoff, tj, L.wl_v4);
   } else {
     int tj;
     const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
-    if (L.lv == 1) k_sound_momentum<R, 1><<<grd, col_block(L), 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
-    else k_sound_momentum<R, 4><<<grd, col_block(L), 0, s>>>(d, uvoff, advoff, tj, L.wl_pt);
+    if (L.lv == 1) step_launch(L, k_sound_momentum<R, 1>, grd, col_block(L), 0, s, d, uvoff, advoff, tj, L.wl_pt);
+    else step_launch(L, k_sound_momentum<R, 4>, grd, col_block(L), 0, s, d, uvoff, advoff, tj, L.wl_pt);
   }
 }
 
