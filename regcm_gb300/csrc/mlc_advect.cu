@@ -100,15 +100,19 @@ template <class T>
 __device__ __forceinline__ T waf_b(T den, T num) {
   T B;
   if constexpr (sizeof(T) == sizeof(float)) {
-    // FP32: the branch-free clamp, signs moved by bit operations; the guard
-    // of tiny denominators is left out - it changes B only where
-    // |den| < 1e-15, by less than 2|den|, far below FP32 rounding of the
-    // flux
-    const unsigned sg = __float_as_uint(den) & 0x80000000u;
-    const float q = __uint_as_float(__float_as_uint(num) ^ sg);
-    const float d = fabsf(den);
-    const float bd = fmaxf(0.f, fminf(d + d, fmaxf(q, fminf(q + q, d))));
-    B = __uint_as_float(__float_as_uint(bd) ^ sg);
+    // FP32: |B| = max(0, min(|2 num|, |den|), min(|num|, |2 den|)), the two
+    // minima with num*den's sign (superbee in its other form, the same
+    // candidates in every region), B with den's: four instructions of the
+    // half-rate pipe instead of seven (moist 512x512x41, a step: vertical
+    // passes 0.227 -> 0.212 ms, increments 0.109 -> 0.094, horizontal 0.351 ->
+    // 0.338).  The guard of tiny
+    // denominators is left out - it changes B only where |den| < 1e-15, by
+    // less than 2|den|, far below FP32 rounding of the flux
+    float t1, t2, bd;
+    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(t1) : "f"(num + num), "f"(den));
+    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(t2) : "f"(num), "f"(den + den));
+    asm("max.f32 %0, %1, %2, 0f00000000;" : "=f"(bd) : "f"(t1), "f"(t2));
+    B = __uint_as_float(__float_as_uint(bd) ^ (__float_as_uint(den) & 0x80000000u));
   } else {
     // FP64: the region tests on the integer pipe.  Non-negative doubles order
     // like their bit patterns read as integers, and for a normal d (d >= minden
@@ -358,55 +362,56 @@ __device__ __forceinline__ T vupdate(T pk, T gb, T ga, T dv, T cu, T cd) {
 }
 
 // Blocks of 256 threads an SM the vertical WAF is compiled for, FP64 and FP32
-// (0: no bound, the compiler's own register choice).  FP32 3/4/5/6 blocks:
-// 309/283/252/313 us a moist 512x512x41 step; FP64 2 (by its registers) and 3:
-// 1820 and 1988 us.
+// (0: no bound, the compiler's own register choice).  Moist 512x512x41 step:
+// FP32, one field a thread, 3/4/5/6 blocks 309/283/252/313 us; two fields
+// 3/4/5 blocks 220/212/318; FP64 2 (by its registers) and 3 1820 and 1988.
 #ifndef MLC_VERT_MINB_D
 #define MLC_VERT_MINB_D 0
 #endif
 #ifndef MLC_VERT_MINB_F
 #define MLC_VERT_MINB_F 5
 #endif
-template <class T>
+#ifndef MLC_VERT_MINB_2
+#define MLC_VERT_MINB_2 4
+#endif
+template <class T, int NF>
 constexpr int vert_min_blocks() {
-  return sizeof(T) == sizeof(double) ? (MLC_VERT_MINB_D > 0 ? MLC_VERT_MINB_D : 1) : MLC_VERT_MINB_F;
+  if (sizeof(T) == sizeof(double)) return MLC_VERT_MINB_D > 0 ? MLC_VERT_MINB_D : 1;
+  return NF == 2 ? MLC_VERT_MINB_2 : MLC_VERT_MINB_F;
+}
+// a pointer into a field as one to global memory (fields are picked from a
+// table, which hides that from the compiler)
+template <class T>
+__device__ __forceinline__ T *global_ptr(T *p) {
+  return (T *)__cvta_global_to_generic(__cvta_generic_to_global((const void *)p));
 }
 // Levels an FP32 column loads ahead of the one it computes (1 or 2; two
 // measured no faster on the moist 512x512x41 step, 0.256 ms a step both).
-// grid: x = column tiles along j times the fields (field fastest, so the
-// blocks reading one column's s and metric run together), y = row tiles,
-// z = member; block (vert_x, vert_y) columns along (j, i)
-template <class R, class T>
-__global__ void __launch_bounds__(256, vert_min_blocks<T>())
-    k_adv_vertical(const Dom<R> *__restrict__ doms, int nf, int set, int advoff,
-                               const WorkItem *__restrict__ wl) {
-  grid_begin();
-  const WorkItem wi = wl ? wl[blockIdx.x]
-                          : WorkItem{(int16_t)blockIdx.z, (int16_t)(blockIdx.x / (unsigned)nf),
-                                     (int16_t)blockIdx.y, (int16_t)(blockIdx.x % (unsigned)nf)};
-  const Dom<R> &D = doms[wi.m];
-  if (!D.active) return;
-  const int f = wi.c;
-  const int bj = wi.a;
-  if (set == 0 && f >= n_table_r(D)) return;  // a member with fewer species
-  const Geom g = D.g;
-  const int kz = g.kz;
-  const int j = bj * (int)blockDim.x + (int)threadIdx.x + 1;
-  const int i = (int)wi.b * (int)blockDim.y + (int)threadIdx.y + 1;
-  if (j > g.jx - 1 || i > g.iy - 1) return;
+// Fields f0 .. f0+NF-1 of the column (j, i), both passes.  FP32 members of
+// large launches take two fields a thread, which share the level's loads and
+// factors: the kernel is bound by instructions (54 against 119 a level and
+// field; moist 512x512x41 0.256 -> 0.212 ms a step, 32 members of 128x128x30
+// 0.239 -> 0.207).  Small ones need the threads (64x64x30 15.0 us against
+// 14.2).  Copies further ahead (a shared-memory ring of 3 to 8 levels) gained
+// nothing.
+template <class R, class T, int NF>
+__device__ __forceinline__ void vertical_column(const Dom<R> &D, int set, int f0, int adv, size_t ij) {
   const Scal &c = D.c;
-  const int adv = (D.clk->adv_role + advoff) & 1;
-  const T *src;
-  T *outp, *dst;
-  field_t<R, T>(D, set, f, adv, src, outp, dst);
-  (void)outp;
-  const size_t ij = g.at2(j, i);
-  src += ij;
-  dst += ij;
+  const int kz = D.g.kz;
+  const T *src[NF];
+  T *dst[NF];
+#pragma unroll
+  for (int n = 0; n < NF; ++n) {
+    T *outp;
+    field_t<R, T>(D, set, f0 + n, adv, src[n], outp, dst[n]);
+    (void)outp;
+    src[n] = global_ptr(src[n]) + ij;
+    dst[n] = global_ptr(dst[n]) + ij;
+  }
   const R *__restrict__ sp = D.s + ij;
   const R *__restrict__ zup = D.sa.zrfmu + ij;
   const R *__restrict__ zdp = D.sa.zrfmd + ij;
-  const unsigned PS = (unsigned)g.PS;  // a domain's fields stay below 2^31 elements
+  const unsigned PS = (unsigned)D.g.PS;  // a domain's fields stay below 2^31 elements
   // -1/2 of the factor of s in zamu
   const T hdtrdz = T(-0.25) * (pick<T>(c.dtstepa, c.dtstepaf) * pick<T>(c.rdzita, c.rdzitaf));
 
@@ -418,8 +423,7 @@ __global__ void __launch_bounds__(256, vert_min_blocks<T>())
   // A level's factors: FP64 those of k_adv_prep.  FP32 forms them from s(k),
   // s(k+1) and the metric (a plane less to read), for the second pass again:
   // what a level carries between the passes is then four registers instead of
-  // five, which fits five blocks an SM (moist 512x512x41: 252 us a step; 268
-  // with the wind in the fluxes, 280 with the factors kept)
+  // five
   struct Fac {
     T cu, cd, dv, nz;
     bool up;  // of interface k+1: the cell below is upwind
@@ -452,25 +456,34 @@ __global__ void __launch_bounds__(256, vert_min_blocks<T>())
       return Fac{cu, cd, cu - cd, fma_r(r.sp, hdtrdz, up ? T(0.5) : T(-0.5)), up};
     }
   };
-  T c0k = src[0], c0p1 = src[PS];
-  T c1m2 = T(0), c1m1 = T(0);
-  T sk = kPre ? T(0) : T(sp[0]);
-  T f1k = T(0), f2m = T(0);
-  T d1p = T(0), d1c = c0k - c0p1, d2p = T(0), d2c = T(0);
-  Lev l1{}, l2{};  // levels k-1, k-2
+  T c0k[NF], c0p1[NF], c1m2[NF], c1m1[NF], f1k[NF], f2m[NF], d1p[NF], d1c[NF], d2p[NF], d2c[NF], n_c[NF];
   // the next level's loads, issued one level ahead
   Lev n_l = load(0);
-  T n_c = src[2 * PS];
+#pragma unroll
+  for (int n = 0; n < NF; ++n) {
+    c0k[n] = src[n][0];
+    c0p1[n] = src[n][PS];
+    n_c[n] = src[n][2 * PS];
+    c1m2[n] = c1m1[n] = f1k[n] = f2m[n] = d1p[n] = d2p[n] = d2c[n] = T(0);
+    d1c[n] = c0k[n] - c0p1[n];
+  }
+  T sk = kPre ? T(0) : T(sp[0]);
+  Lev l1{}, l2{};  // levels k-1, k-2
   // level k; every bound check is known to hold inside the column
   // (4 <= k <= kz-3), so the interior steps carry none
   auto step = [&](int k, auto interior) {
     constexpr bool I = decltype(interior)::value;
     const unsigned o = (unsigned)(k - 1) * PS;
     Lev l = n_l;
-    const T c0p2 = (I || k + 2 <= kz) ? n_c : T(0);
+    T c0p2[NF];
+#pragma unroll
+    for (int n = 0; n < NF; ++n) c0p2[n] = (I || k + 2 <= kz) ? n_c[n] : T(0);
     if (I || k < kz) {
       n_l = load(o + PS);
-      if (I || k + 3 <= kz) n_c = src[o + 3 * PS];
+      if (I || k + 3 <= kz) {
+#pragma unroll
+        for (int n = 0; n < NF; ++n) n_c[n] = src[n][o + 3 * PS];
+      }
     }
     if constexpr (kPre) {
       l.up = nonneg(l.sp);  // zamu has s's sign
@@ -478,26 +491,28 @@ __global__ void __launch_bounds__(256, vert_min_blocks<T>())
       l.s = sk;
       sk = l.sp;
     }
-    const Fac t = factors(l);
-    const T d1n = c0p1 - c0p2;  // the next interface's difference, this one's upwind one
-    T f1kp;
-    if (I) f1kp = vflux_in<T>(t.nz, t.up, c0k, c0p1, d1p, d1c, d1n);
-    else f1kp = k <= kz - 1 ? vflux<T>(t.nz, t.up, c0k, c0p1, d1p, d1c, d1n, k, kz) : T(0);
-    const T c1k = vupdate<T>(c0k, f1k, f1kp, t.dv, t.cu, t.cd);
-    const T d2n = c1m1 - c1k;
-    if (I || k >= 3) {  // pass 2 at level m = k-2
-      const Fac t2 = factors(l2);
-      T f2n;
-      if (I) f2n = vflux_in<T>(t2.nz, t2.up, c1m2, c1m1, d2p, d2c, d2n);
-      else f2n = vflux<T>(t2.nz, t2.up, c1m2, c1m1, d2p, d2c, d2n, k - 2, kz);
-      dst[o - 2 * PS] = vupdate<T>(c1m2, f2m, f2n, t2.dv, t2.cu, t2.cd);
-      f2m = f2n;
+    const Fac t = factors(l), t2 = factors(l2);
+#pragma unroll
+    for (int n = 0; n < NF; ++n) {
+      const T d1n = c0p1[n] - c0p2[n];  // the next interface's difference, this one's upwind one
+      T f1kp;
+      if (I) f1kp = vflux_in<T>(t.nz, t.up, c0k[n], c0p1[n], d1p[n], d1c[n], d1n);
+      else f1kp = k <= kz - 1 ? vflux<T>(t.nz, t.up, c0k[n], c0p1[n], d1p[n], d1c[n], d1n, k, kz) : T(0);
+      const T c1k = vupdate<T>(c0k[n], f1k[n], f1kp, t.dv, t.cu, t.cd);
+      const T d2n = c1m1[n] - c1k;
+      if (I || k >= 3) {  // pass 2 at level m = k-2
+        T f2n;
+        if (I) f2n = vflux_in<T>(t2.nz, t2.up, c1m2[n], c1m1[n], d2p[n], d2c[n], d2n);
+        else f2n = vflux<T>(t2.nz, t2.up, c1m2[n], c1m1[n], d2p[n], d2c[n], d2n, k - 2, kz);
+        dst[n][o - 2 * PS] = vupdate<T>(c1m2[n], f2m[n], f2n, t2.dv, t2.cu, t2.cd);
+        f2m[n] = f2n;
+      }
+      c0k[n] = c0p1[n]; c0p1[n] = c0p2[n];
+      c1m2[n] = c1m1[n]; c1m1[n] = c1k;
+      d1p[n] = d1c[n]; d1c[n] = d1n; d2p[n] = d2c[n]; d2c[n] = d2n;
+      f1k[n] = f1kp;
     }
-    c0k = c0p1; c0p1 = c0p2;
-    c1m2 = c1m1; c1m1 = c1k;
-    d1p = d1c; d1c = d1n; d2p = d2c; d2c = d2n;
     l2 = l1; l1 = l;
-    f1k = f1kp;
   };
   using edge = std::integral_constant<bool, false>;
   using mid = std::integral_constant<bool, true>;
@@ -509,9 +524,41 @@ __global__ void __launch_bounds__(256, vert_min_blocks<T>())
   // pass 2 at levels kz-1 (flux through interface kz) and kz (none above)
   const unsigned ot = (unsigned)(kz - 1) * PS;
   const Fac t1 = factors(l1), t2 = factors(l2);
-  const T f2n = vflux<T>(t2.nz, t2.up, c1m2, c1m1, d2p, d2c, T(0), kz - 1, kz);
-  dst[ot - PS] = vupdate<T>(c1m2, f2m, f2n, t2.dv, t2.cu, t2.cd);
-  dst[ot] = vupdate<T>(c1m1, f2n, T(0), t1.dv, t1.cu, t1.cd);
+#pragma unroll
+  for (int n = 0; n < NF; ++n) {
+    const T f2n = vflux<T>(t2.nz, t2.up, c1m2[n], c1m1[n], d2p[n], d2c[n], T(0), kz - 1, kz);
+    dst[n][ot - PS] = vupdate<T>(c1m2[n], f2m[n], f2n, t2.dv, t2.cu, t2.cd);
+    dst[n][ot] = vupdate<T>(c1m1[n], f2n, T(0), t1.dv, t1.cu, t1.cd);
+  }
+}
+
+// grid: x = column tiles along j times the groups of NF fields (group fastest,
+// so the blocks reading one column's s and metric run together), y = row
+// tiles, z = member; block (vert_x, vert_y) columns along (j, i)
+template <class R, class T, int NF>
+__global__ void __launch_bounds__(256, vert_min_blocks<T, NF>())
+    k_adv_vertical(const Dom<R> *__restrict__ doms, int ng, int set, int advoff,
+                               const WorkItem *__restrict__ wl) {
+  grid_begin();
+  const WorkItem wi = wl ? wl[blockIdx.x]
+                          : WorkItem{(int16_t)blockIdx.z, (int16_t)(blockIdx.x / (unsigned)ng),
+                                     (int16_t)blockIdx.y, (int16_t)(blockIdx.x % (unsigned)ng)};
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const int f0 = wi.c * NF, nf = set == 0 ? n_table_r(D) : 2;
+  if (f0 >= nf) return;  // a member with fewer species
+  const int j = wi.a * (int)blockDim.x + (int)threadIdx.x + 1;
+  const int i = (int)wi.b * (int)blockDim.y + (int)threadIdx.y + 1;
+  if (j > D.g.jx - 1 || i > D.g.iy - 1) return;
+  const int adv = (D.clk->adv_role + advoff) & 1;
+  const size_t ij = D.g.at2(j, i);
+  if constexpr (NF == 2) {
+    if (f0 + 1 >= nf) {
+      vertical_column<R, T, 1>(D, set, f0, adv, ij);
+      return;
+    }
+  }
+  vertical_column<R, T, NF>(D, set, f0, adv, ij);
 }
 
 // ---- lane vectors ---------------------------------------------------------
@@ -1522,12 +1569,17 @@ void launch_vertical(const LaunchGeom &L, const Dom<R> *d, int nf, int set, int 
                      cudaStream_t s) {
   // one thread per column: blocks of vert_x x vert_y columns along (j, i)
   const dim3 b((unsigned)L.vert_x, (unsigned)L.vert_y);
-  const WorkItem *wl = set == 0 ? L.wl_vert : L.wl_vinc;
-  const int nw = set == 0 ? L.n_vert : L.n_vinc;
-  const dim3 grd = wl ? dim3((unsigned)nw, 1, 1)
-                      : dim3((unsigned)(((L.jx - 1 + L.vert_x - 1) / L.vert_x) * nf),
-                             (unsigned)((L.iy - 1 + L.vert_y - 1) / L.vert_y), (unsigned)L.nmem);
-  step_launch(L, k_adv_vertical<R, T>, grd, b, 0, s, d, nf, set, advoff, wl);
+  const int ng = (nf + L.vert_nf - 1) / L.vert_nf;
+  const dim3 grd = L.wl_vert ? dim3((unsigned)L.n_vert, 1, 1)
+                             : dim3((unsigned)(((L.jx - 1 + L.vert_x - 1) / L.vert_x) * ng),
+                                    (unsigned)((L.iy - 1 + L.vert_y - 1) / L.vert_y), (unsigned)L.nmem);
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (L.vert_nf == 2) {
+      step_launch(L, k_adv_vertical<R, T, 2>, grd, b, 0, s, d, ng, set, advoff, L.wl_vert);
+      return;
+    }
+  }
+  step_launch(L, k_adv_vertical<R, T, 1>, grd, b, 0, s, d, ng, set, advoff, L.wl_vert);
 }
 
 template <class R, int V, int NW>

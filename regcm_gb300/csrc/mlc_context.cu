@@ -350,7 +350,7 @@ struct mlc_ctx {
   WorkItem *wl_buf = nullptr;
   size_t wl_cap = 0;           // entries
   bool wl_dirty = true;        // members changed since the lists were built
-  int wl_key[10] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
+  int wl_key[11] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
   const WorkItem *wl_ptr[9] = {};  // the lists in wl_buf (null: none) ...
   int wl_n[9] = {};                // ... and their lengths
 };
@@ -617,6 +617,7 @@ int refresh(mlc_ctx *x) {
     L.frame_points = std::max(L.frame_points, nx * ny - std::max(0, nx - f) * std::max(0, ny - f));
   }
   L.lv = point_levels(pts);
+  L.vert_nf = x->mixed && L.lv > 1 ? 2 : 1;
   L.wind_rows = !x->mixed ? 0 : pts <= (size_t)256 << 10 ? 2 : 4;  // (eight and more measured slower)
   if (!t.empty()) {
     MLC_TRY(cudaMemcpyAsync(x->table, t.data(), t.size() * sizeof(Dom<R>), cudaMemcpyHostToDevice,
@@ -644,8 +645,8 @@ int ensure_lists(mlc_ctx *x) {
   bool uneven = false;
   for (const Member *m : act)
     uneven = uneven || m->g.jx != L.jx || m->g.iy != L.iy || m->g.kz != L.kz;
-  const int key[10] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, waf_tile(L), waf_tile_inc(L),
-                       L.solve, L.lv, L.wind_rows};
+  const int key[11] = {uneven ? 1 : 0, L.col_x, L.col_y, L.vert_x, L.vert_y, waf_tile(L), waf_tile_inc(L),
+                       L.solve, L.lv, L.wind_rows, L.vert_nf};
   // the launch geometry always takes the lists from the context (a copy of
   // an older geometry may carry stale ones)
   auto apply = [&]() {
@@ -706,7 +707,7 @@ int ensure_lists(mlc_ctx *x) {
     const int nf = n_table_r(act[m]->dims, x->prm, f64);
     for (int bi = 0; bi < cdiv(g.iy - 1, L.vert_y); ++bi)
       for (int bj = 0; bj < cdiv(g.jx - 1, L.vert_x); ++bj)
-        for (int f = 0; f < nf; ++f) push(m, bj, bi, f);
+        for (int f = 0; f < cdiv(nf, L.vert_nf); ++f) push(m, bj, bi, f);
   }
   // the same for theta_v and Exner of mixed members
   off[4] = all.size();

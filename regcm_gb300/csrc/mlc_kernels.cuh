@@ -39,6 +39,7 @@ struct LaunchGeom {
   int frame_points;      // points a level of the largest member's frame (Scal::frame)
   int lv;                // levels a thread of the point kernels runs (1 or 4)
   int vert_x, vert_y;    // adv_vertical
+  int vert_nf;           // fields a thread of it carries (1; mixed members by size 2)
   int htile;             // adv_horizontal tile shape (hshape) asked for, -1: by size
   int size_tile, size_tile_inc;  // the shapes by size (refresh)
   int nadv_r;            // advected fields of type R per member

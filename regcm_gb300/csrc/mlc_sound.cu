@@ -1123,19 +1123,23 @@ struct West4 {
 };
 
 // Blocks of 128 threads an SM the four-column point kernels are compiled for
-// (the register budget follows; a few registers spill to L1).  Measured on the
-// moist 512x512x41 step: 5 blocks (about 100 registers) momentum 0.37 and
-// divergence 0.30 ms a step, against 0.39 and 0.35 at 4 (128 registers).
-#ifndef MLC_PT4_BLOCKS
-#define MLC_PT4_BLOCKS 5
-#endif
+// (the register budget follows).  Four levels a thread: 5 blocks (96
+// registers, a few spilled to L1) momentum 0.377 and divergence 0.300 ms a
+// moist 512x512x41 step, against 0.377 and 0.330 at 4 and 0.409 and 0.299 at
+// 6.  One level a thread, where few blocks run anyway: 4 blocks (no spills)
+// momentum 0.215 and divergence 0.168 ms a rotated 150x187x40 step, against
+// 0.223 and 0.178 at 5.
+template <int LV>
+constexpr int pt4_blocks() {
+  return LV == 1 ? 4 : 5;
+}
 
 // The divergence and s of a mixed member (the same equations as
 // k_sound_div) with lanes of four consecutive columns: 16-byte loads at the
 // lane's points and the row north of them, the east neighbour of the last
 // element read singly, the level below carried from the previous level.
 template <class R, int LV>
-__global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<R> *__restrict__ doms, int uvoff,
+__global__ void __launch_bounds__(128, pt4_blocks<LV>()) k_sound_div_v4(const Dom<R> *__restrict__ doms, int uvoff,
                                                       int tiles_j,
     const WorkItem *__restrict__ wl) {
   if constexpr (LV == 1) grid_begin();
@@ -1261,7 +1265,7 @@ __global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_div_v4(const Dom<
 // block is 32 lanes x 4 rows; grid x = 128-column tiles times row tiles, y =
 // level chunks, z = member.
 template <class R, int LV>
-__global__ void __launch_bounds__(128, MLC_PT4_BLOCKS) k_sound_momentum_v4(const Dom<R> *__restrict__ doms,
+__global__ void __launch_bounds__(128, pt4_blocks<LV>()) k_sound_momentum_v4(const Dom<R> *__restrict__ doms,
                                                            int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   if constexpr (LV == 1) grid_begin();
