@@ -328,6 +328,10 @@ struct mlc_ctx {
   bool mixed = false;
   int device = 0;
   cudaStream_t stream = nullptr;
+  // a step's second stream, for kernels that do not depend on one another,
+  // and the events that fork it from and join it to the first
+  cudaStream_t side = nullptr;
+  cudaEvent_t forked = nullptr, joined = nullptr;
   cudaMemPool_t pool = nullptr;
   std::vector<Member> mem;     // slots
   Clock *clks = nullptr;       // device, one per slot
@@ -830,6 +834,19 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
   cudaStream_t s = x->stream;
   const int nadv = x->prm.mo_nadv, nsound = x->prm.mo_nsound;
   int nl = 0;
+  // the stream of a group of kernels that may run beside the next ones of s
+  // (timed launches run one after the other), and its end
+  auto fork = [&]() {
+    if (rec) return s;
+    cudaEventRecord(x->forked, s);
+    cudaStreamWaitEvent(x->side, x->forked, 0);
+    return x->side;
+  };
+  auto join = [&](cudaStream_t q) {
+    if (q == s) return;
+    cudaEventRecord(x->joined, q);
+    cudaStreamWaitEvent(s, x->joined, 0);
+  };
   for (int r = 0; r < nadv && phase != kStepFinish; ++r) {
     // ---- sound (Main/mod_moloch.F90:531-765) ----
     REC("sound_prep", K::sound_prep(L, d, r, s)); ++nl;
@@ -842,11 +859,19 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
     // ---- advection (Main/mod_moloch.F90:767-1042) ----
     const int uvo = (r + 1) * nsound;
     REC("adv_prep", K::adv_prep(L, d, uvo, r, s)); ++nl;
+    // theta_v and Exner of mixed members and the species that are not
+    // advected beside the other fields: they share only what they read
+    const bool beside = L.nadv_d || x->key.any_copy;
+    const cudaStream_t q = beside ? fork() : s;
+    if (L.nadv_d) {
+      REC("adv_vertical_inc", K::adv_vertical_inc(L, d, r, q));
+      REC("adv_horizontal_inc", K::adv_horizontal_inc(L, d, uvo, r, q));
+      nl += 2;
+    }
+    if (x->key.any_copy) { REC("adv_species_copy", K::adv_species_copy(L, d, r, q)); ++nl; }
     REC("adv_vertical", K::adv_vertical(L, d, r, s)); ++nl;
-    if (L.nadv_d) { REC("adv_vertical_inc", K::adv_vertical_inc(L, d, r, s)); ++nl; }
     REC("adv_horizontal", K::adv_horizontal(L, d, uvo, r, s)); ++nl;
-    if (L.nadv_d) { REC("adv_horizontal_inc", K::adv_horizontal_inc(L, d, uvo, r, s)); ++nl; }
-    if (x->key.any_copy) { REC("adv_species_copy", K::adv_species_copy(L, d, r, s)); ++nl; }
+    if (beside) join(q);
     if (x->key.any_curv) { REC("adv_curvature", K::adv_curvature(L, d, r + 1, s)); ++nl; }
     REC("adv_back", K::adv_back(L, d, uvo, r + 1, s)); ++nl;
   }
@@ -856,8 +881,11 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
     // the ring first: the point pass after it does tvirt, t and the relaxation
     if (x->prm.do_apply_bdy) { REC("bdy_ring", K::bdy_ring(L, d, uvo, ao, s)); ++nl; }
     if (phase == kStepAll && !(x->prm.do_apply_bdy && x->prm.mo_spectral_nudge)) {
-      REC("end_frame", K::end_frame(L, d, uvo, ao, s)); ++nl;
+      // frame and interior share no point
+      const cudaStream_t q = fork();
+      REC("end_frame", K::end_frame(L, d, uvo, ao, q)); ++nl;
       REC("end_point", K::end_point(L, d, uvo, ao, s)); ++nl;
+      join(q);
       int flip = 0;
       if (L.wind_rows) {
         // (the winds end in the other half of their pairs)
@@ -1382,6 +1410,9 @@ void release(mlc_ctx *x) {
   if (x->table) cudaFree(x->table);
   if (x->wl_buf) cudaFree(x->wl_buf);
   if (x->pool) cudaMemPoolDestroy(x->pool);
+  if (x->forked) cudaEventDestroy(x->forked);
+  if (x->joined) cudaEventDestroy(x->joined);
+  if (x->side) cudaStreamDestroy(x->side);
   if (x->stream) cudaStreamDestroy(x->stream);
   delete x;
 }
@@ -1411,6 +1442,9 @@ int create_common(const mlc_params *params, int capacity, size_t budget, mlc_ctx
   L.solve_df = 1;  // the mixed solve's recurrence to FP64 accuracy
   cudaError_t e = cudaGetDevice(&x->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->forked, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->joined, cudaEventDisableTiming);
   if (e == cudaSuccess) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
