@@ -332,6 +332,158 @@ __global__ void k_adv_prep(const Dom<R> *__restrict__ doms, int uvoff, int advof
   }
 }
 
+// ---- lane vectors ---------------------------------------------------------
+template <int B> struct VecOf;
+template <> struct VecOf<4> { using t = unsigned; };
+template <> struct VecOf<8> { using t = uint2; };
+template <> struct VecOf<16> { using t = uint4; };
+
+// v consecutive elements at p, which is aligned to min(v * sizeof(T), 16)
+template <class T, int V>
+__device__ __forceinline__ void ld_vec(T (&x)[V], const T *p) {
+  constexpr int B = V * (int)sizeof(T);
+  if constexpr (B <= 16) {
+    const typename VecOf<B>::t w = *reinterpret_cast<const typename VecOf<B>::t *>(p);
+    memcpy(x, &w, B);
+  } else {
+#pragma unroll
+    for (int h = 0; h < B / 16; ++h) {
+      const uint4 w = reinterpret_cast<const uint4 *>(p)[h];
+      memcpy(reinterpret_cast<char *>(x) + 16 * h, &w, 16);
+    }
+  }
+}
+template <class T, int V>
+__device__ __forceinline__ void st_vec(T *p, const T (&x)[V]) {
+  constexpr int B = V * (int)sizeof(T);
+  if constexpr (B <= 16) {
+    typename VecOf<B>::t w;
+    memcpy(&w, x, B);
+    *reinterpret_cast<typename VecOf<B>::t *>(p) = w;
+  } else {
+#pragma unroll
+    for (int h = 0; h < B / 16; ++h) {
+      uint4 w;
+      memcpy(&w, reinterpret_cast<const char *>(x) + 16 * h, 16);
+      reinterpret_cast<uint4 *>(p)[h] = w;
+    }
+  }
+}
+// the lane's v elements of row r (1-based) of a plane, or zeros
+template <class T, int V>
+__device__ __forceinline__ void ld_row(T (&x)[V], const T *plane, int e0, int r, unsigned P, bool ok) {
+  if (ok) {
+    ld_vec<T, V>(x, plane + (unsigned)e0 + (unsigned)(r - 1) * P);
+  } else {
+#pragma unroll
+    for (int q = 0; q < V; ++q) x[q] = T(0);
+  }
+}
+// element q+1 of the lane's columns: the lane's own, or the next lane's first
+template <class T, int V>
+__device__ __forceinline__ void next_col(T (&e)[V], const T (&x)[V]) {
+#pragma unroll
+  for (int q = 0; q + 1 < V; ++q) e[q] = x[q + 1];
+  e[V - 1] = __shfl_down_sync(0xffffffffu, x[0], 1);
+}
+
+// Four FP32 points of a row interpolated from the eight around them
+__device__ __forceinline__ void interp_vec(float (&x)[4], const float (&a)[4], const float (&b)[4], const float (&c)[4],
+                                           const float (&d)[4], bool edge) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) x[q] = edge ? interp2<float>(a[q], b[q]) : interp4<float>(a[q], b[q], c[q], d[q]);
+}
+// x stored at p where e0 + q < n (0-based columns)
+__device__ __forceinline__ void store_row4(float *p, const float (&x)[4], int e0, int n) {
+  if (e0 + 4 <= n) {
+    st_vec<float, 4>(p, x);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (e0 + q < n) p[q] = x[q];
+  }
+}
+
+// k_adv_prep of a mixed member in lanes of four columns: 16-byte loads of the
+// rows and levels around a point, w's carried from level to level, so a point
+// takes three loads instead of twelve (moist 512x512x41: 57 us a step
+// against 92).  Block 32 lanes x 4 rows, grid as k_sound_div_v4's.
+template <class R, int LV>
+__global__ void __launch_bounds__(128) k_adv_prep_v4(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
+                                                     int tiles_j, const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
+  const WorkItem wi = work_item(wl, tiles_j);
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const Geom g = D.g;
+  const int jx = g.jx, iy = g.iy, kz = g.kz;
+  const int e0 = ((int)wi.a * 32 + (int)threadIdx.x) * 4, i = (int)wi.b * 4 + (int)threadIdx.y + 1;
+  const int k0 = (int)wi.c * LV + 1;
+  if (e0 + 1 > jx - 1 || i > iy - 1 || k0 > kz) return;
+  const int uv = (D.clk->uv_role + uvoff) & 1, adv = (D.clk->adv_role + advoff) & 1;
+  const unsigned P = (unsigned)g.P, PS = (unsigned)g.PS, ij = (unsigned)e0 + (unsigned)(i - 1) * P;
+  const float *__restrict__ u = D.u[uv] + ij;
+  const float *__restrict__ v = D.v[uv] + ij;
+  const float *__restrict__ w = D.w + ij;
+  const float *__restrict__ tk = D.c.tke ? D.tke + ij : nullptr;
+  float *__restrict__ ux = D.ux[adv] + ij;
+  float *__restrict__ vx = D.vx[adv] + ij;
+  float *__restrict__ wx = D.wx[adv] + ij;
+  float *__restrict__ tkx = D.c.tke ? D.tkex[adv] + ij : nullptr;
+  float w0[4] = {}, w1[4], w2[4], w3[4] = {};  // w at levels k-1 .. k+2
+  unsigned o = (unsigned)(k0 - 1) * PS;
+  if (k0 >= 2) ld_vec<float, 4>(w0, w + o - PS);
+  ld_vec<float, 4>(w1, w + o);
+  ld_vec<float, 4>(w2, w + o + PS);
+  for (int k = k0; k < k0 + LV && k <= kz; ++k, o += PS) {
+    float x[4];
+    {
+      // uvstagtouvx :1535-1549: columns e0-1 .. e0+5
+      float a[7] = {};
+      float m[4];
+      ld_vec<float, 4>(m, u + o);
+      if (e0 >= 1) a[0] = (u + o)[-1];  // (o may be 0: no unsigned o - 1)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[1 + q] = m[q];
+      if (e0 + 4 <= jx - 1) a[5] = u[o + 4];
+      if (e0 + 5 <= jx - 1) a[6] = u[o + 5];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = e0 + q + 1;
+        x[q] = j == 1 || j == jx - 1 ? interp2<float>(a[q + 1], a[q + 2])
+                                     : interp4<float>(a[q + 2], a[q + 1], a[q + 3], a[q]);
+      }
+      store_row4(ux + o, x, e0, jx - 1);
+    }
+    {
+      // :1553-1566: rows i-1 .. i+2
+      float a[4] = {}, b[4], c[4], d[4] = {};
+      if (i >= 2) ld_vec<float, 4>(a, v + o - P);
+      ld_vec<float, 4>(b, v + o);
+      ld_vec<float, 4>(c, v + o + P);
+      if (i <= iy - 2) ld_vec<float, 4>(d, v + o + 2 * P);
+      interp_vec(x, c, b, d, a, i == 1 || i == iy - 1);
+      store_row4(vx + o, x, e0, jx - 1);
+    }
+    // zstagtoh :1445-1459
+    if (k < kz) ld_vec<float, 4>(w3, w + o + 2 * PS);
+    interp_vec(x, w2, w1, w3, w0, k == 1 || k == kz);
+    store_row4(wx + o, x, e0, jx - 1);
+    if (tk) {
+      // zstagtoh(tke, tkex) (Main/mod_moloch.F90:782-784)
+      float a[4] = {}, b[4], c[4], d[4] = {};
+      if (k >= 2) ld_vec<float, 4>(a, tk + o - PS);
+      ld_vec<float, 4>(b, tk + o);
+      ld_vec<float, 4>(c, tk + o + PS);
+      if (k < kz) ld_vec<float, 4>(d, tk + o + 2 * PS);
+      interp_vec(x, c, b, d, a, k == 1 || k == kz);
+      store_row4(tkx + o, x, e0, jx - 1);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { w0[q] = w1[q]; w1[q] = w2[q]; w2[q] = w3[q]; }
+  }
+}
+
 // Two vertical WAF passes (do_vadvtwice, :858-922), one thread per column
 // and field, streaming the levels upward through registers.  Pass 1's flux
 // at interface k+1 needs the input at levels k-1..k+2 and its update at k the
@@ -561,60 +713,6 @@ __global__ void __launch_bounds__(256, vert_min_blocks<T, NF>())
   vertical_column<R, T, NF>(D, set, f0, adv, ij);
 }
 
-// ---- lane vectors ---------------------------------------------------------
-template <int B> struct VecOf;
-template <> struct VecOf<4> { using t = unsigned; };
-template <> struct VecOf<8> { using t = uint2; };
-template <> struct VecOf<16> { using t = uint4; };
-
-// v consecutive elements at p, which is aligned to min(v * sizeof(T), 16)
-template <class T, int V>
-__device__ __forceinline__ void ld_vec(T (&x)[V], const T *p) {
-  constexpr int B = V * (int)sizeof(T);
-  if constexpr (B <= 16) {
-    const typename VecOf<B>::t w = *reinterpret_cast<const typename VecOf<B>::t *>(p);
-    memcpy(x, &w, B);
-  } else {
-#pragma unroll
-    for (int h = 0; h < B / 16; ++h) {
-      const uint4 w = reinterpret_cast<const uint4 *>(p)[h];
-      memcpy(reinterpret_cast<char *>(x) + 16 * h, &w, 16);
-    }
-  }
-}
-template <class T, int V>
-__device__ __forceinline__ void st_vec(T *p, const T (&x)[V]) {
-  constexpr int B = V * (int)sizeof(T);
-  if constexpr (B <= 16) {
-    typename VecOf<B>::t w;
-    memcpy(&w, x, B);
-    *reinterpret_cast<typename VecOf<B>::t *>(p) = w;
-  } else {
-#pragma unroll
-    for (int h = 0; h < B / 16; ++h) {
-      uint4 w;
-      memcpy(&w, reinterpret_cast<const char *>(x) + 16 * h, 16);
-      reinterpret_cast<uint4 *>(p)[h] = w;
-    }
-  }
-}
-// the lane's v elements of row r (1-based) of a plane, or zeros
-template <class T, int V>
-__device__ __forceinline__ void ld_row(T (&x)[V], const T *plane, int e0, int r, unsigned P, bool ok) {
-  if (ok) {
-    ld_vec<T, V>(x, plane + (unsigned)e0 + (unsigned)(r - 1) * P);
-  } else {
-#pragma unroll
-    for (int q = 0; q < V; ++q) x[q] = T(0);
-  }
-}
-// element q+1 of the lane's columns: the lane's own, or the next lane's first
-template <class T, int V>
-__device__ __forceinline__ void next_col(T (&e)[V], const T (&x)[V]) {
-#pragma unroll
-  for (int q = 0; q + 1 < V; ++q) e[q] = x[q + 1];
-  e[V - 1] = __shfl_down_sync(0xffffffffu, x[0], 1);
-}
 
 // Meridional then zonal WAF at one level for a tile of nw rows, every field
 // of the R table (:984-1038; ROTLLR :926-983).  Warp w owns row I0+w; lane l
@@ -1064,6 +1162,97 @@ __global__ void k_adv_back(const Dom<R> *__restrict__ doms, int uvoff, int advof
         D.tke[o] = a;
       }
     }
+  }
+}
+
+// k_adv_back of a mixed member in lanes of four columns, as k_adv_prep_v4
+// (moist 512x512x41: 57 us a step against 94)
+template <class R, int LV>
+__global__ void __launch_bounds__(128) k_adv_back_v4(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
+                                                     int tiles_j, const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
+  const WorkItem wi = work_item(wl, tiles_j);
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const Geom g = D.g;
+  const int jx = g.jx, iy = g.iy, kz = g.kz;
+  const int e0 = ((int)wi.a * 32 + (int)threadIdx.x) * 4, i = (int)wi.b * 4 + (int)threadIdx.y + 1;
+  const int k0 = (int)wi.c * LV + 1;
+  // (no wind is written in the last column and row)
+  if (e0 + 1 > jx - 1 || i > iy - 1 || k0 > kz) return;
+  const int uv = (D.clk->uv_role + uvoff) & 1, adv = (D.clk->adv_role + advoff) & 1;
+  const unsigned P = (unsigned)g.P, PS = (unsigned)g.PS, ij = (unsigned)e0 + (unsigned)(i - 1) * P;
+  const float *__restrict__ ux = D.ux[adv] + ij;
+  const float *__restrict__ vx = D.vx[adv] + ij;
+  const float *__restrict__ wx = D.wx[adv] + ij;
+  const float *__restrict__ tx = D.c.tke ? D.tkex[adv] + ij : nullptr;
+  float *__restrict__ u = D.u[uv] + ij;
+  float *__restrict__ v = D.v[uv] + ij;
+  float *__restrict__ w = D.w + ij;
+  float *__restrict__ tk = D.c.tke ? D.tke + ij : nullptr;
+  const bool do_u = i >= 2 && i <= iy - 2, do_v = i >= 2;
+  // store columns first .. n-1 (0-based) of a lane
+  auto store = [&](float *p, const float (&x)[4], int first, int n) {
+    if (e0 >= first && e0 + 4 <= n) {
+      st_vec<float, 4>(p, x);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (e0 + q >= first && e0 + q < n) p[q] = x[q];
+    }
+  };
+  float w0[4] = {}, w1[4] = {}, w2[4], w3[4] = {};  // wx at levels k-2 .. k+1
+  unsigned o = (unsigned)(k0 - 1) * PS;
+  if (k0 >= 3) ld_vec<float, 4>(w0, wx + o - 2 * PS);
+  if (k0 >= 2) ld_vec<float, 4>(w1, wx + o - PS);
+  ld_vec<float, 4>(w2, wx + o);
+  for (int k = k0; k < k0 + LV && k <= kz; ++k, o += PS) {
+    float x[4];
+    if (do_u) {
+      float a[7] = {};  // columns e0-2 .. e0+4
+      float m[4];
+      ld_vec<float, 4>(m, ux + o);
+      if (e0 >= 2) {
+        a[0] = (ux + o)[-2];  // (o may be 0: no unsigned o - 2)
+        a[1] = (ux + o)[-1];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[2 + q] = m[q];
+      if (e0 + 4 <= jx - 2) a[6] = ux[o + 4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = e0 + q + 1;
+        x[q] = j == 2 || j == jx - 1 ? interp2<float>(a[q + 1], a[q + 2])
+                                     : interp4<float>(a[q + 2], a[q + 1], a[q + 3], a[q]);
+      }
+      store(u + o, x, 1, jx - 1);
+    }
+    if (do_v) {
+      float a[4] = {}, b[4], c[4], d[4] = {};  // rows i-2 .. i+1
+      if (i >= 3) ld_vec<float, 4>(a, vx + o - 2 * P);
+      ld_vec<float, 4>(b, vx + o - P);
+      ld_vec<float, 4>(c, vx + o);
+      if (i <= iy - 2) ld_vec<float, 4>(d, vx + o + P);
+      interp_vec(x, c, b, d, a, i == 2 || i == iy - 1);
+      store(v + o, x, 1, jx - 2);
+    }
+    if (k < kz) ld_vec<float, 4>(w3, wx + o + PS);
+    if (k >= 2) {
+      interp_vec(x, w2, w1, w3, w0, k == 2 || k == kz);
+      store(w + o, x, 0, jx - 1);
+      if (tx) {
+        // htozstag(tkex, tke) (Main/mod_moloch.F90:831-834)
+        float a[4] = {}, b[4], c[4], d[4] = {};
+        if (k >= 3) ld_vec<float, 4>(a, tx + o - 2 * PS);
+        ld_vec<float, 4>(b, tx + o - PS);
+        ld_vec<float, 4>(c, tx + o);
+        if (k < kz) ld_vec<float, 4>(d, tx + o + PS);
+        interp_vec(x, c, b, d, a, k == 2 || k == kz);
+        store(tk + o, x, 0, jx - 1);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { w0[q] = w1[q]; w1[q] = w2[q]; w2[q] = w3[q]; }
   }
 }
 
@@ -1555,13 +1744,29 @@ inline dim3 pt_grid(const LaunchGeom &L, int nj, int ni, int &tiles_j) {
 
 }  // namespace
 
+// grid of the four-column kernels over nj x ni points (128 x 4 tiles)
+dim3 v4_grid(const LaunchGeom &L, int nj, int ni, int &tj) {
+  tj = (nj + 127) / 128;
+  const int ti = (ni + 3) / 4;
+  return L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
+                 : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
+}
+
 template <class R>
 void Launch<R>::adv_prep(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  if constexpr (sizeof(R) == sizeof(float)) {
+    int tj;
+    const dim3 grd = v4_grid(L, L.jx - 1, L.iy - 1, tj), b(32, 4);
+    if (L.lv == 1) step_launch(L, k_adv_prep_v4<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_v4);
+    else step_launch(L, k_adv_prep_v4<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_v4);
+    return;
+  } else {
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx - 1, L.iy - 1, tj);
   if (L.lv == 1) step_launch(L, k_adv_prep<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
   else step_launch(L, k_adv_prep<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  }
 }
 
 template <class R, class T>
@@ -1674,11 +1879,19 @@ void Launch<R>::adv_curvature(const LaunchGeom &L, const Dom<R> *d, int advoff, 
 
 template <class R>
 void Launch<R>::adv_back(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  if constexpr (sizeof(R) == sizeof(float)) {
+    int tj;
+    const dim3 grd = v4_grid(L, L.jx - 1, L.iy - 1, tj), b(32, 4);
+    if (L.lv == 1) step_launch(L, k_adv_back_v4<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_v4);
+    else step_launch(L, k_adv_back_v4<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_v4);
+    return;
+  } else {
   const dim3 b((unsigned)L.col_x, (unsigned)L.col_y);
   int tj;
   const dim3 grd = pt_grid(L, L.jx, L.iy, tj);
   if (L.lv == 1) step_launch(L, k_adv_back<R, 1>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
   else step_launch(L, k_adv_back<R, 4>, grd, b, 0, s, d, uvoff, advoff, tj, L.wl_pt);
+  }
 }
 
 template <class R>
