@@ -989,35 +989,51 @@ Clock get_clock(mlc_ctx *x, int slot, int *st) {
   return c;
 }
 
-// Copy a packed (Fortran extents nj x ni x nk) host array into the padded
-// device layout through the staging buffer at element offset `soff`.  One
-// stream orders every copy and (un)pack, so consecutive fields may reuse the
-// same staging slice.  (A pitched copy straight into the layout is slower
-// wherever rows are not whole 32-byte sectors or the host array is pageable:
-// the state of 201x157x35 3.88 ms pitched, 1.02 so; 512x512x41 4.80 and 4.62.)
-template <class R>
-int put3(mlc_ctx *x, const Geom &g, const double *h, R *dst, int nj, int ni, int nk, size_t soff) {
-  if (!h) return MLC_OK;
-  const size_t n = (size_t)nj * ni * nk;
-  if (soff + n > x->staging_elems) return MLC_ERR_INVALID;
-  MLC_TRY(cudaMemcpyAsync(x->staging + soff, h, n * sizeof(double), cudaMemcpyHostToDevice, x->stream));
-  Launch<R>::unpack3(x->staging + soff, dst, g, nj, ni, nk, x->stream);
-  return MLC_OK;
-}
+// Uploads of packed (Fortran extents nj x ni x nk) host arrays into the padded
+// device layout of one member: each array is copied to the next place of the
+// staging buffer, and flush unpacks them all with one kernel.  (A pitched copy
+// straight into the layout is slower wherever rows are not whole 32-byte
+// sectors or the host array is pageable: the state of 201x157x35 3.88 ms
+// pitched, 1.02 so; 512x512x41 4.80 and 4.62.)
+struct Upload {
+  mlc_ctx *x;
+  const Geom &g;
+  size_t at;  // the next place; the stream's order lets a flushed one be reused
+  UnpackList l{};
 
-// The same for a double-float field of a mixed member (planes of nplane
-// elements: hi, then lo); an FP64 member takes the plain copy.
-template <class R>
-int put3x(mlc_ctx *x, const Geom &g, const double *h, double *dst, int nj, int ni, int nk,
-          size_t soff, size_t nplane) {
-  if (sizeof(R) == sizeof(double)) return put3<double>(x, g, h, dst, nj, ni, nk, soff);
-  if (!h) return MLC_OK;
-  const size_t n = (size_t)nj * ni * nk;
-  if (soff + n > x->staging_elems) return MLC_ERR_INVALID;
-  MLC_TRY(cudaMemcpyAsync(x->staging + soff, h, n * sizeof(double), cudaMemcpyHostToDevice, x->stream));
-  Launch<R>::unpack3_df(x->staging + soff, dst, g, nj, ni, nk, nplane, x->stream);
-  return MLC_OK;
-}
+  Upload(mlc_ctx *x_, const Geom &g_, size_t from = 0) : x(x_), g(g_), at(from), first(from) {}
+  int put(const double *h, void *dst, int nj, int ni, int nk, bool f64, size_t nplane) {
+    if (!h) return MLC_OK;
+    const size_t n = (size_t)nj * ni * nk;
+    if (l.n == UnpackList::kMax || at + n > x->staging_elems) {
+      MLC_CHK(flush());
+      at = first;
+      if (at + n > x->staging_elems) return MLC_ERR_INVALID;
+    }
+    MLC_TRY(cudaMemcpyAsync(x->staging + at, h, n * sizeof(double), cudaMemcpyHostToDevice, x->stream));
+    l.it[l.n++] = {x->staging + at, dst, nplane, nj, ni, nk, f64 ? 1 : 0};
+    at += n;
+    return MLC_OK;
+  }
+  template <class R>
+  int put3(const double *h, R *dst, int nj, int ni, int nk) {
+    return put(h, dst, nj, ni, nk, sizeof(R) == sizeof(double), 0);
+  }
+  // a double-float field of a mixed member (planes of nplane elements: hi,
+  // then lo); an FP64 member takes the plain copy
+  template <class R>
+  int put3x(const double *h, double *dst, int nj, int ni, int nk, size_t nplane) {
+    return put(h, dst, nj, ni, nk, sizeof(R) == sizeof(double), nplane);
+  }
+  int flush() {
+    if (l.n > 0) Launch<double>::unpack(l, g, x->stream);
+    l.n = 0;
+    return cuda_status(cudaGetLastError());
+  }
+
+ private:
+  size_t first;
+};
 
 template <class R>
 int get3x(mlc_ctx *x, const Geom &g, const double *src, double *h, int nj, int ni, int nk,
@@ -1128,15 +1144,16 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
   const size_t nc = (size_t)(jx - 1) * (iy - 1) * kz;
   const double *fmz_src, *fmzf_src;
   size_t fp, fps;
+  const size_t nf = (size_t)(jx - 1) * (iy - 1) * (kz + 1);
+  Upload up(x, g, sizeof(R) == sizeof(double) ? 0 : nc + nf);
   if constexpr (sizeof(R) == sizeof(double)) {
-    MLC_CHK(put3<R>(x, g, s->fmz, W(a.fmz), jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3<R>(x, g, s->fmzf, W(a.fmzf), jx - 1, iy - 1, kz + 1, 0));
+    MLC_CHK(up.put3(s->fmz, W(a.fmz), jx - 1, iy - 1, kz));
+    MLC_CHK(up.put3(s->fmzf, W(a.fmzf), jx - 1, iy - 1, kz + 1));
     fmz_src = a.fmz;
     fmzf_src = a.fmzf;
     fp = g.P;
     fps = g.PS;
   } else {
-    const size_t nf = (size_t)(jx - 1) * (iy - 1) * (kz + 1);
     if (nc + nf > x->staging_elems) return MLC_ERR_INVALID;
     MLC_TRY(cudaMemcpyAsync(x->staging, s->fmz, nc * sizeof(double), cudaMemcpyHostToDevice, x->stream));
     MLC_TRY(cudaMemcpyAsync(x->staging + nc, s->fmzf, nf * sizeof(double), cudaMemcpyHostToDevice, x->stream));
@@ -1145,11 +1162,11 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
     fp = (size_t)(jx - 1);
     fps = (size_t)(jx - 1) * (iy - 1);
   }
-  const size_t soff = sizeof(R) == sizeof(double) ? 0 : nc + (size_t)(jx - 1) * (iy - 1) * (kz + 1);
-  MLC_CHK(put3<R>(x, g, s->rfmzu, W(a.rfmzu), jx, iy - 1, kz, soff));
-  MLC_CHK(put3<R>(x, g, s->rfmzv, W(a.rfmzv), jx - 1, iy, kz, soff));
-  MLC_CHK(put3<double>(x, g, s->zeta, W(a.zeta), jx - 1, iy - 1, kz, soff));
-  MLC_CHK(put3<double>(x, g, s->dz, W(a.dz), jx - 1, iy - 1, kz, soff));
+  MLC_CHK(up.put3(s->rfmzu, W(a.rfmzu), jx, iy - 1, kz));
+  MLC_CHK(up.put3(s->rfmzv, W(a.rfmzv), jx - 1, iy, kz));
+  MLC_CHK(up.put3(s->zeta, W(a.zeta), jx - 1, iy - 1, kz));
+  MLC_CHK(up.put3(s->dz, W(a.dz), jx - 1, iy - 1, kz));
+  MLC_CHK(up.flush());
   // 2-D fields and init_moloch derivations (Main/mod_moloch.F90:258-271)
   std::vector<double> t2(nd);
   auto copy2 = [&](const double *h, size_t n) { t2.assign(h, h + n); };
@@ -1246,8 +1263,9 @@ int bind_static_impl(mlc_ctx *x, Member &mb, const mlc_static_ptrs *s) {
     std::vector<double> cu((size_t)jx * (iy - 1)), cvv((size_t)(jx - 1) * iy);
     for (size_t e = 0; e < cu.size(); ++e) cu[e] = kOmega2 * std::sin(s->ulat[e] * kDegrad) * c.dtsound;
     for (size_t e = 0; e < cvv.size(); ++e) cvv[e] = kOmega2 * std::sin(s->vlat[e] * kDegrad) * c.dtsound;
-    MLC_CHK(put3<double>(x, g, cu.data(), W(a.mo_cu), jx, iy - 1, 1, 0));
-    MLC_CHK(put3<double>(x, g, cvv.data(), W(a.mo_cv), jx - 1, iy, 1, 0));
+    MLC_CHK(up.put3(cu.data(), W(a.mo_cu), jx, iy - 1, 1));
+    MLC_CHK(up.put3(cvv.data(), W(a.mo_cv), jx - 1, iy, 1));
+    MLC_CHK(up.flush());
     MLC_TRY(cudaStreamSynchronize(x->stream));
   }
   BindPar bp{};
@@ -1296,29 +1314,25 @@ int upload_state_impl(mlc_ctx *x, int slot, const mlc_state_ptrs *h) {
   const State<R> st = state_of(dom_of<R>(mb), ck.uv_role, ck.adv_role);
   const Geom &g = mb.g;
   const int jx = mb.dims.jx, iy = mb.dims.iy, kz = mb.dims.kz;
-  size_t off = 0;
   const size_t c3 = (size_t)(jx - 1) * (iy - 1) * kz;
-  auto adv = [&](size_t n) { size_t o = off; off += n; return o; };
-  MLC_CHK(put3<R>(x, g, h->u, st.u, jx, iy - 1, kz, adv((size_t)jx * (iy - 1) * kz)));
-  MLC_CHK(put3<R>(x, g, h->v, st.v, jx - 1, iy, kz, adv((size_t)(jx - 1) * iy * kz)));
-  MLC_CHK(put3<R>(x, g, h->w, st.w, jx - 1, iy - 1, kz + 1, adv((size_t)(jx - 1) * (iy - 1) * (kz + 1))));
-  MLC_CHK(put3x<R>(x, g, h->pai, st.pai, jx - 1, iy - 1, kz, adv(c3), g.field3()));
-  MLC_CHK(put3x<R>(x, g, h->tetav, st.tetav, jx - 1, iy - 1, kz, adv(c3), g.field3()));
+  Upload up(x, g);
+  MLC_CHK(up.put3(h->u, st.u, jx, iy - 1, kz));
+  MLC_CHK(up.put3(h->v, st.v, jx - 1, iy, kz));
+  MLC_CHK(up.put3(h->w, st.w, jx - 1, iy - 1, kz + 1));
+  MLC_CHK(up.put3x<R>(h->pai, st.pai, jx - 1, iy - 1, kz, g.field3()));
+  MLC_CHK(up.put3x<R>(h->tetav, st.tetav, jx - 1, iy - 1, kz, g.field3()));
   R *f3[] = {st.t, st.tvirt, st.ux, st.vx, st.p, st.rho, st.qsat};
   const double *h3[] = {h->t, h->tvirt, h->ux, h->vx, h->p, h->rho, h->qsat};
-  for (int q = 0; q < 7; ++q) MLC_CHK(put3<R>(x, g, h3[q], f3[q], jx - 1, iy - 1, kz, adv(c3)));
+  for (int q = 0; q < 7; ++q) MLC_CHK(up.put3(h3[q], f3[q], jx - 1, iy - 1, kz));
   const size_t F = g.field3();
   for (int n = 0; n < mb.dims.nqx && h->qx; ++n)
-    MLC_CHK(put3<R>(x, g, h->qx + n * c3, st.qx + n * F, jx - 1, iy - 1, kz, adv(c3)));
+    MLC_CHK(up.put3(h->qx + n * c3, st.qx + n * F, jx - 1, iy - 1, kz));
   for (int n = 0; n < mb.dims.ntr && h->trac; ++n)
-    MLC_CHK(put3<R>(x, g, h->trac + n * c3, st.trac + n * F, jx - 1, iy - 1, kz, adv(c3)));
-  if (h->ps) {
-    const size_t c2 = (size_t)(jx - 1) * (iy - 1);
-    MLC_CHK(put3<double>(x, g, h->ps, st.ps, jx - 1, iy - 1, 1, adv(c2)));
-  }
+    MLC_CHK(up.put3(h->trac + n * c3, st.trac + n * F, jx - 1, iy - 1, kz));
+  MLC_CHK(up.put3(h->ps, st.ps, jx - 1, iy - 1, 1));
   if (h->tke && st.tke)
-    MLC_CHK(put3<R>(x, g, h->tke, st.tke, jx - 1, iy - 1, kz + 1,
-                    adv((size_t)(jx - 1) * (iy - 1) * (kz + 1))));
+    MLC_CHK(up.put3(h->tke, st.tke, jx - 1, iy - 1, kz + 1));
+  MLC_CHK(up.flush());
   // init_moloch: w(:,:,1) = 0 (Main/mod_moloch.F90:264-266)
   if (h->w) MLC_TRY(cudaMemsetAsync(st.w, 0, g.PS * sizeof(R), x->stream));
   return cuda_status(cudaStreamSynchronize(x->stream));
@@ -1379,18 +1393,21 @@ int set_boundary_impl(mlc_ctx *x, Member &mb, const mlc_bdy_ptrs *b) {
     if (p.present_qi && !b->xib[s]) return MLC_ERR_INVALID;
     if (d.ntr > 0 && !b->chib[s]) return MLC_ERR_INVALID;
   }
+  Upload up(x, g);
   for (int s = 0; s < 2; ++s) {
-    MLC_CHK(put3x<R>(x, g, b->xtb[s], W(a.xtb[s]), jx - 1, iy - 1, kz, 0, F));
-    MLC_CHK(put3<R>(x, g, b->xqb[s], W(a.xqb[s]), jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3x<R>(x, g, b->xpaib[s], W(a.xpaib[s]), jx - 1, iy - 1, kz, 0, F));
-    if (p.present_qc) MLC_CHK(put3<R>(x, g, b->xlb[s], W(a.xlb[s]), jx - 1, iy - 1, kz, 0));
-    if (p.present_qi) MLC_CHK(put3<R>(x, g, b->xib[s], W(a.xib[s]), jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3<R>(x, g, b->dub[s], W(a.dub[s]), jx, iy - 1, kz, 0));
-    MLC_CHK(put3<R>(x, g, b->dvb[s], W(a.dvb[s]), jx - 1, iy, kz, 0));
+    MLC_CHK(up.put3x<R>(b->xtb[s], W(a.xtb[s]), jx - 1, iy - 1, kz, F));
+    MLC_CHK(up.put3(b->xqb[s], W(a.xqb[s]), jx - 1, iy - 1, kz));
+    MLC_CHK(up.put3x<R>(b->xpaib[s], W(a.xpaib[s]), jx - 1, iy - 1, kz, F));
+    if (p.present_qc) MLC_CHK(up.put3(b->xlb[s], W(a.xlb[s]), jx - 1, iy - 1, kz));
+    if (p.present_qi) MLC_CHK(up.put3(b->xib[s], W(a.xib[s]), jx - 1, iy - 1, kz));
+    MLC_CHK(up.put3(b->dub[s], W(a.dub[s]), jx, iy - 1, kz));
+    MLC_CHK(up.put3(b->dvb[s], W(a.dvb[s]), jx - 1, iy, kz));
     for (int n = 0; n < d.ntr; ++n)
-      MLC_CHK(put3<R>(x, g, b->chib[s] + n * c3, W(a.chib[s]) + n * F, jx - 1, iy - 1, kz, 0));
-    MLC_CHK(put3<double>(x, g, b->xpsb[s], W(a.xpsb[s]), jx - 1, iy - 1, 1, 0));
+      MLC_CHK(up.put3(b->chib[s] + n * c3, W(a.chib[s]) + n * F, jx - 1, iy - 1, kz));
+    MLC_CHK(up.put3(b->xpsb[s], W(a.xpsb[s]), jx - 1, iy - 1, 1));
+    MLC_CHK(up.flush());
     MLC_TRY(cudaStreamSynchronize(x->stream));
+    up.at = 0;
   }
   return MLC_OK;
 }
@@ -1556,15 +1573,17 @@ int set_tendencies_impl(mlc_ctx *x, Member &mb, const mlc_tend_ptrs *t) {
   const int nj = mb.dims.jx - 3, ni = mb.dims.iy - 3, kz = mb.dims.kz;
   const size_t n3 = (size_t)nj * ni * kz;
   const size_t at22 = g.at2(2, 2);
+  Upload up(x, g);
   const double *h[3] = {t->tten, t->uten, t->vten};
-  for (int f = 0; f < 3; ++f) MLC_CHK(put3<R>(x, g, h[f], base + (size_t)f * F + at22, nj, ni, kz, 0));
+  for (int f = 0; f < 3; ++f) MLC_CHK(up.put3(h[f], base + (size_t)f * F + at22, nj, ni, kz));
   for (int n = 0; n < mb.dims.nqx && t->qxten; ++n)
-    MLC_CHK(put3<R>(x, g, t->qxten + n * n3, base + (size_t)(3 + n) * F + at22, nj, ni, kz, 0));
+    MLC_CHK(up.put3(t->qxten + n * n3, base + (size_t)(3 + n) * F + at22, nj, ni, kz));
   for (int n = 0; n < mb.dims.ntr && t->chiten; ++n)
-    MLC_CHK(put3<R>(x, g, t->chiten + n * n3, base + (size_t)(3 + mb.dims.nqx + n) * F + at22, nj, ni,
-                    kz, 0));
+    MLC_CHK(up.put3(t->chiten + n * n3, base + (size_t)(3 + mb.dims.nqx + n) * F + at22, nj, ni,
+                    kz));
   if (mb.c.tke && t->tketen)
-    MLC_CHK(put3<R>(x, g, t->tketen, base + (size_t)nf * F + at22, nj, ni, kz + 1, 0));
+    MLC_CHK(up.put3(t->tketen, base + (size_t)nf * F + at22, nj, ni, kz + 1));
+  MLC_CHK(up.flush());
   return cuda_status(cudaStreamSynchronize(x->stream));
 }
 

@@ -1655,15 +1655,26 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__
   clk->red_done = 0u;
 }
 
-template <class R>
-__global__ void k_unpack3(const double *__restrict__ src, R *__restrict__ dst, Geom g, int nj, int ni, int nk) {
-  const size_t n = (size_t)nj * ni * nk;
+// blockIdx.y: the list's item.  All of an upload's arrays in one launch, after
+// their copies: with a kernel after each copy the two engines waited for one
+// another (state of 47x33x23: 131 us, 66 so).
+__global__ void k_unpack(UnpackList l, Geom g) {
+  const UnpackList::Item &t = l.it[blockIdx.y];
+  const size_t n = (size_t)t.nj * t.ni * t.nk;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e % nj);
-    const size_t r = e / nj;
-    const int i = (int)(r % ni);
-    const int k = (int)(r / ni);
-    dst[(size_t)j + (size_t)i * g.P + (size_t)k * g.PS] = (R)src[e];
+    const int j = (int)(e % t.nj);
+    const size_t r = e / t.nj;
+    const int i = (int)(r % t.ni), k = (int)(r / t.ni);
+    const size_t o = (size_t)j + (size_t)i * g.P + (size_t)k * g.PS;
+    const double x = t.src[e];
+    if (t.f64) {
+      static_cast<double *>(t.dst)[o] = x;
+    } else {
+      // hi = fl(x), lo = fl(x - hi): x to ~48 bits as two floats
+      const float hi = (float)x;
+      static_cast<float *>(t.dst)[o] = hi;
+      if (t.nplane) static_cast<float *>(t.dst)[o + t.nplane] = (float)(x - (double)hi);
+    }
   }
 }
 
@@ -1744,23 +1755,6 @@ __global__ void k_pack3(const R *__restrict__ src, double *__restrict__ dst, Geo
     const int i = (int)(r % ni);
     const int k = (int)(r / ni);
     dst[e] = (double)src[(size_t)j + (size_t)i * g.P + (size_t)k * g.PS];
-  }
-}
-
-// hi = fl(x), lo = fl(x - hi): x to ~48 bits as two floats
-__global__ void k_unpack3_df(const double *__restrict__ src, float *__restrict__ dst, Geom g, int nj,
-                             int ni, int nk, size_t nplane) {
-  const size_t n = (size_t)nj * ni * nk;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e % nj);
-    const size_t r = e / nj;
-    const int i = (int)(r % ni);
-    const int k = (int)(r / ni);
-    const size_t o = (size_t)j + (size_t)i * g.P + (size_t)k * g.PS;
-    const double x = src[e];
-    const float hi = (float)x;
-    dst[o] = hi;
-    dst[o + nplane] = (float)(x - (double)hi);
   }
 }
 
@@ -1944,19 +1938,13 @@ void Launch<R>::bind_derived(const Stat<R> &sa, const Geom &g, const double *fmz
 }
 
 template <class R>
-void Launch<R>::unpack3(const double *src, R *dst, const Geom &g, int nj, int ni, int nk, cudaStream_t s) {
-  k_unpack3<R><<<152 * 8, 256, 0, s>>>(src, dst, g, nj, ni, nk);
+void Launch<R>::unpack(const UnpackList &l, const Geom &g, cudaStream_t s) {
+  k_unpack<<<dim3((unsigned)(152 * 8 / l.n + 1), (unsigned)l.n), 256, 0, s>>>(l, g);
 }
 
 template <class R>
 void Launch<R>::pack3(const R *src, double *dst, const Geom &g, int nj, int ni, int nk, cudaStream_t s) {
   k_pack3<R><<<152 * 8, 256, 0, s>>>(src, dst, g, nj, ni, nk);
-}
-
-template <class R>
-void Launch<R>::unpack3_df(const double *src, double *dst, const Geom &g, int nj, int ni, int nk,
-                           size_t nplane, cudaStream_t s) {
-  k_unpack3_df<<<152 * 8, 256, 0, s>>>(src, reinterpret_cast<float *>(dst), g, nj, ni, nk, nplane);
 }
 
 template <class R>

@@ -88,6 +88,20 @@ void step_launch(const LaunchGeom &L, void (*kernel)(P...), dim3 grid, dim3 bloc
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Packed FP64 arrays (Fortran extents nj x ni x nk) in the staging buffer and
+// the fields in the padded layout that they go to: FP64, FP32, or, with a
+// plane size, double-float (high parts, then low parts nplane floats on).
+struct UnpackList {
+  static constexpr int kMax = 24;
+  struct Item {
+    const double *src;
+    void *dst;
+    size_t nplane;
+    int nj, ni, nk, f64;
+  } it[kMax];
+  int n;
+};
+
 // Constants of the derived time-invariant fields (bind_cross, bind_wind)
 struct BindPar {
   double dtrdz_adv;  // 0.5*dtstepa/dzita
@@ -147,13 +161,10 @@ template <class R> struct Launch {
   // plane fps; the 1-D and 2-D fields and, for FP64, rfmzu and rfmzv in place)
   static void bind_derived(const Stat<R> &sa, const Geom &g, const double *fmz, const double *fmzf,
                            size_t fp, size_t fps, const BindPar &b, cudaStream_t s);
-  static void unpack3(const double *src, R *dst, const Geom &g, int nj, int ni, int nk,
-                      cudaStream_t s);
+  static void unpack(const UnpackList &l, const Geom &g, cudaStream_t s);
   static void pack3(const R *src, double *dst, const Geom &g, int nj, int ni, int nk,
                     cudaStream_t s);
   // double-float planes (hi, lo) of nplane elements each
-  static void unpack3_df(const double *src, double *dst, const Geom &g, int nj, int ni, int nk,
-                         size_t nplane, cudaStream_t s);
   static void pack3_df(const double *src, double *dst, const Geom &g, int nj, int ni, int nk,
                        size_t nplane, cudaStream_t s);
 };

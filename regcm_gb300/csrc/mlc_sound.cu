@@ -1123,14 +1123,14 @@ struct West4 {
 };
 
 // Blocks of 128 threads an SM the four-column point kernels are compiled for
-// (the register budget follows).  Four levels a thread: 5 blocks (96
-// registers, a few spilled to L1) momentum 0.377 and divergence 0.300 ms a
-// moist 512x512x41 step, against 0.377 and 0.330 at 4 and 0.409 and 0.299 at
-// 6.  One level a thread, where few blocks run anyway: 4 blocks (no spills)
-// momentum 0.215 and divergence 0.168 ms a rotated 150x187x40 step, against
-// 0.223 and 0.178 at 5.
+// (the register budget follows).  Momentum, four levels a thread: 5 blocks (96
+// registers, a few spilled to L1) 0.377 ms a moist 512x512x41 step, against
+// 0.385 at 4 and 0.409 at 6; one level a thread, where few blocks run anyway:
+// 4 blocks (no spills) 0.215 ms a rotated 150x187x40 step, 0.223 at 5.  The
+// divergence: 4 blocks with two levels' loads in flight 0.274 ms (one level's
+// 0.330), 5 blocks 0.300, 3 blocks 0.323.
 template <int LV>
-constexpr int pt4_blocks() {
+constexpr int momentum_blocks() {
   return LV == 1 ? 4 : 5;
 }
 
@@ -1139,7 +1139,7 @@ constexpr int pt4_blocks() {
 // lane's points and the row north of them, the east neighbour of the last
 // element read singly, the level below carried from the previous level.
 template <class R, int LV>
-__global__ void __launch_bounds__(128, pt4_blocks<LV>()) k_sound_div_v4(const Dom<R> *__restrict__ doms, int uvoff,
+__global__ void __launch_bounds__(128, 4) k_sound_div_v4(const Dom<R> *__restrict__ doms, int uvoff,
                                                       int tiles_j,
     const WorkItem *__restrict__ wl) {
   if constexpr (LV == 1) grid_begin();
@@ -1207,6 +1207,7 @@ __global__ void __launch_bounds__(128, pt4_blocks<LV>()) k_sound_div_v4(const Do
     ld4(vm, v + om);
     ld4(vpm, v + om + P);
   }
+#pragma unroll 2
   for (int k = k0; k < k0 + LV && k <= kz; ++k) {
     const unsigned o = ij + (unsigned)(k - 1) * PS;
     float u0[4], u1[4], v0[4], v1[4], fu0[4], fu1[4], fv0[4], fv1[4], fz[4], zd[4];
@@ -1265,7 +1266,7 @@ __global__ void __launch_bounds__(128, pt4_blocks<LV>()) k_sound_div_v4(const Do
 // block is 32 lanes x 4 rows; grid x = 128-column tiles times row tiles, y =
 // level chunks, z = member.
 template <class R, int LV>
-__global__ void __launch_bounds__(128, pt4_blocks<LV>()) k_sound_momentum_v4(const Dom<R> *__restrict__ doms,
+__global__ void __launch_bounds__(128, momentum_blocks<LV>()) k_sound_momentum_v4(const Dom<R> *__restrict__ doms,
                                                            int uvoff, int advoff, int tiles_j,
     const WorkItem *__restrict__ wl) {
   if constexpr (LV == 1) grid_begin();
