@@ -1414,6 +1414,7 @@ int set_boundary_impl(mlc_ctx *x, Member &mb, const mlc_bdy_ptrs *b) {
 
 void release(mlc_ctx *x) {
   if (!x) return;
+  if (x->side) cudaStreamSynchronize(x->side);
   if (x->stream) cudaStreamSynchronize(x->stream);
   if (x->graph) cudaGraphExecDestroy(x->graph);
   for (Member &m : x->mem) {
