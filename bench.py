@@ -155,21 +155,22 @@ def kernel_bytes(name: str, case, nadv_fields: int, wbytes: int) -> float | None
 
 
 # DRAM bytes per point of a launch (dram__bytes_read.sum + dram__bytes_write.sum)
-# from one ncu capture of the same kernel and precision on the quarter-size
-# case (moist 256x256x41, 10 advected fields), scaled to the bench case by its
-# points.  These are constants from that capture, not measured by this run:
-# the line prints them with that label and the kernel build they were taken
-# on.  Keyed by (kernel group, precision, advected fields).
+# from one ncu capture of the same kernel and precision on a smaller moist case
+# (10 advected fields; the mixed solve on a size that takes the bench case's
+# form), scaled to the bench case by its points.  These are constants from that
+# capture, not measured by this run: the line prints them with that label and
+# the kernel build they were taken on.  Keyed by (kernel group, precision,
+# advected fields): bytes per point; build and captured case.
 CAPTURED_TRAFFIC_PER_POINT = {
-    ("adv_horizontal", "fp64", 10): (733.3e6 / (256 * 256 * 41), "b130abd"),
-    ("sound_solve", "mixed", 10): (243.0e6 / (256 * 256 * 41), "b130abd"),
+    ("adv_horizontal", "fp64", 10): (713.3e6 / (256 * 256 * 41), "874984a, moist 256x256x41"),
+    ("sound_solve", "mixed", 10): (402.0e6 / (320 * 320 * 41), "874984a, moist 320x320x41"),
 }
 # What limits the dominant kernel besides its roofline, from the same captures.
 CAPTURED_LIMITER = {
     ("adv_horizontal", "fp64"): {
-        "pipe": "fp64", "active": 0.84, "counter": "sm__inst_executed_pipe_fp64"},
+        "pipe": "fp64", "active": 0.86, "counter": "sm__inst_executed_pipe_fp64"},
     ("sound_solve", "mixed"): {
-        "stall": "block barrier (one a level, freeing a copy stage)", "warps_active": 0.21},
+        "stall": "block barrier (one a level, freeing a copy stage)", "warps_active": 0.35},
 }
 
 
@@ -816,8 +817,8 @@ def kernel_roofline(lib, ctx, case, precision):
                              "algorithmic_bytes": bytes_per})
     roofline["share_of_step"] = kms / total_k
     if cap:
-        roofline["traffic_source"] = (f"constant: ncu DRAM bytes of this kernel on moist "
-                                      f"256x256x41 at build {cap[1]}, scaled by points; "
+        roofline["traffic_source"] = (f"constant: ncu DRAM bytes of this kernel at build "
+                                      f"{cap[1]}, scaled by points; "
                                       "not measured by this run")
     lim = CAPTURED_LIMITER.get((dom_name, precision))
     if lim:
