@@ -886,6 +886,11 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
       REC("end_frame", K::end_frame(L, d, uvo, ao, q)); ++nl;
       REC("end_point", K::end_point(L, d, uvo, ao, s)); ++nl;
       join(q);
+      // the budget beside the winds: its face fluxes take the ring's winds,
+      // which the pass from cross points leaves (a mixed member's are in both
+      // halves); the roles that both read advance after them
+      const cudaStream_t q2 = fork();
+      REC("end_reduce", K::end_reduce(L, d, uvo, ao, true, false, q2)); ++nl;
       int flip = 0;
       if (L.wind_rows) {
         // (the winds end in the other half of their pairs)
@@ -896,7 +901,8 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
         REC("end_uvstag", K::end_uvstag(L, d, uvo, ao, s)); ++nl;
       }
       if (x->key.any_tke) { REC("end_tke", K::end_tke(L, d, true, s)); ++nl; }
-      REC("end_reduce", K::end_reduce(L, d, uvo + flip, ao, true, s)); ++nl;
+      join(q2);
+      REC("end_advance", K::end_advance(L, d, uvo + flip, ao, s)); ++nl;
       return nl;
     }
     REC("end_relax", K::end_relax(L, d, uvo, ao, s)); ++nl;
@@ -915,7 +921,7 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
   }
   if (x->key.any_tke) { REC("end_tke", K::end_tke(L, d, phase == kStepAll, s)); ++nl; }
   REC("end_uvstag", K::end_uvstag(L, d, uvo, ao, s)); ++nl;
-  REC("end_reduce", K::end_reduce(L, d, uvo, ao, false, s)); ++nl;
+  REC("end_reduce", K::end_reduce(L, d, uvo, ao, false, true, s)); ++nl;
   return nl;
 }
 
@@ -1944,7 +1950,8 @@ int group_of(const char *name) {
   if (!std::strcmp(name, "sound_solve")) return 1;
   if (!std::strcmp(name, "adv_vertical") || !std::strcmp(name, "adv_vertical_inc")) return 2;
   if (!std::strcmp(name, "adv_horizontal") || !std::strcmp(name, "adv_horizontal_inc")) return 3;
-  if (!std::strcmp(name, "bdy_ring") || !std::strcmp(name, "end_reduce")) return -1;
+  if (!std::strcmp(name, "bdy_ring") || !std::strcmp(name, "end_reduce") || !std::strcmp(name, "end_advance"))
+    return -1;
   return 0;  // column kernels
 }
 

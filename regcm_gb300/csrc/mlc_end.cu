@@ -1459,6 +1459,24 @@ __device__ __forceinline__ RedSum red_block(RedSum a, bool flux, RedSum *sh) {
   return a;
 }
 
+// The boundary clock, the step count and the buffer roles of the next step.
+__device__ __forceinline__ void advance_clock(const Scal &c, Clock *clk, int uvoff, int advoff) {
+  if (c.apply_bdy) clk->xbctime = clk->xbctime + c.dtsec;
+  if (c.apply_bdy && c.spectral) clk->tspectral = clk->tspectral + c.dtsec;
+  clk->step = clk->step + 1;
+  clk->uv_role = (clk->uv_role + uvoff) & 1;
+  clk->adv_role = (clk->adv_role + advoff) & 1;
+}
+// The same after a budget that ran beside the winds (which read the roles): a
+// member a thread.
+template <class R>
+__global__ void k_end_advance(const Dom<R> *__restrict__ doms, int nmem, int uvoff, int advoff) {
+  grid_begin();
+  const int m = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (m >= nmem || !doms[m].active) return;
+  advance_clock(doms[m].c, doms[m].clk, uvoff, advoff);
+}
+
 // Partial sums of the mass budget and the ps extrema of one member, per block.
 // Interior rows go to warps, lanes along the row in 16-byte vectors (every row
 // starts on 128 bytes); the species of a point are summed before they are
@@ -1474,7 +1492,7 @@ __device__ __forceinline__ RedSum red_block(RedSum a, bool flux, RedSum *sh) {
 // 230 without ps; 20 against 25 and 28 at 64x64x30.)
 template <class R>
 __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__restrict__ doms,
-                                                                int uvoff, int advoff, int form_ps) {
+                                                                int uvoff, int advoff, int form_ps, int advance) {
   grid_begin();
   __shared__ RedSum sh[kRedWarps];
   __shared__ bool last;
@@ -1647,11 +1665,7 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__
   diag->ps_min = t.bad ? NAN : __longlong_as_double(order_key(t.pmin));
   diag->nonfinite = t.bad;
   if (t.bad && !clk->nonfinite) { clk->nonfinite = 1; clk->bad_step = clk->step; }
-  if (c.apply_bdy) clk->xbctime = clk->xbctime + c.dtsec;
-  if (c.apply_bdy && c.spectral) clk->tspectral = clk->tspectral + c.dtsec;
-  clk->step = clk->step + 1;
-  clk->uv_role = (clk->uv_role + uvoff) & 1;
-  clk->adv_role = (clk->adv_role + advoff) & 1;
+  if (advance) advance_clock(c, clk, uvoff, advoff);
   clk->red_done = 0u;
 }
 
@@ -1925,9 +1939,15 @@ void Launch<R>::end_tke(const LaunchGeom &L, const Dom<R> *d, bool whole_step, c
 }
 
 template <class R>
-void Launch<R>::end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps,
+void Launch<R>::end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps, bool advance,
                            cudaStream_t s) {
-  step_launch(L, k_reduce_partial<R>, dim3((unsigned)L.red_blocks, (unsigned)L.nmem), kRedThreads, 0, s, d, uvoff, advoff, form_ps ? 1 : 0);
+  step_launch(L, k_reduce_partial<R>, dim3((unsigned)L.red_blocks, (unsigned)L.nmem), kRedThreads, 0, s, d, uvoff,
+              advoff, form_ps ? 1 : 0, advance ? 1 : 0);
+}
+
+template <class R>
+void Launch<R>::end_advance(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
+  step_launch(L, k_end_advance<R>, (unsigned)((L.nmem + 63) / 64), 64, 0, s, d, L.nmem, uvoff, advoff);
 }
 
 template <class R>

@@ -154,8 +154,9 @@ template <class R> struct Launch {
   // status_update of the TKE (ibltyp = 2): tendency (split step) and floor
   static void end_tke(const LaunchGeom &L, const Dom<R> *d, bool whole_step, cudaStream_t s);
   // form_ps: ps from the virtual temperatures end_point left
-  static void end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps,
+  static void end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps, bool advance,
                          cudaStream_t s);
+  static void end_advance(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   // ---- layout conversion (one member, from the host) ----
   // the 3-D fields derived from the bound ones (fmz, fmzf: of row pitch fp and
   // plane fps; the 1-D and 2-D fields and, for FP64, rfmzu and rfmzv in place)
