@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
+#include <climits>
 #include <cstring>
 #include <memory>
 #include <new>
@@ -615,9 +616,11 @@ int refresh(mlc_ctx *x) {
   size_tiles<R>(t, L);
   size_t pts = 0;
   L.frame_points = 0;
+  L.min_frame = INT_MAX;
   for (const Dom<R> &D : t) {
     const int nx = D.g.jx - 1, ny = D.g.iy - 1, f = 2 * D.c.frame;
     pts += (size_t)D.g.jx * D.g.iy * D.g.kz;
+    L.min_frame = std::min(L.min_frame, D.c.frame);
     L.frame_points = std::max(L.frame_points, nx * ny - std::max(0, nx - f) * std::max(0, ny - f));
   }
   L.lv = point_levels(pts);
@@ -878,11 +881,16 @@ int enqueue_step(mlc_ctx *x, Recorder *rec = nullptr, int phase = kStepAll) {
   // ---- step end (Main/mod_moloch.F90:340-446) ----
   const int uvo = nadv * nsound, ao = nadv;
   if (phase != kStepFinish) {
-    // the ring first: the point pass after it does tvirt, t and the relaxation
-    if (x->prm.do_apply_bdy) { REC("bdy_ring", K::bdy_ring(L, d, uvo, ao, s)); ++nl; }
-    if (phase == kStepAll && !(x->prm.do_apply_bdy && x->prm.mo_spectral_nudge)) {
-      // frame and interior share no point
-      const cudaStream_t q = fork();
+    // The ring first: the point pass after it does tvirt, t and the
+    // relaxation.  Interior points need neither the ring nor the frame, which
+    // hold no point of theirs; a ring point reads the point inside it, so the
+    // interior waits for the ring where that point is not the frame's.
+    const bool whole = phase == kStepAll && !(x->prm.do_apply_bdy && x->prm.mo_spectral_nudge);
+    const bool early = whole && L.min_frame >= 2;
+    cudaStream_t q = early ? fork() : s;
+    if (x->prm.do_apply_bdy) { REC("bdy_ring", K::bdy_ring(L, d, uvo, ao, q)); ++nl; }
+    if (whole) {
+      if (!early) q = fork();
       REC("end_frame", K::end_frame(L, d, uvo, ao, q)); ++nl;
       REC("end_point", K::end_point(L, d, uvo, ao, s)); ++nl;
       join(q);

@@ -37,6 +37,7 @@ struct LaunchGeom {
   int solve;             // form of the column solves (kSolveStream ...)
   int wind_rows;         // rows of a warp of end_winds (0: FP64 members, end_uvx and end_uvstag)
   int frame_points;      // points a level of the largest member's frame (Scal::frame)
+  int min_frame;         // the thinnest member's frame
   int lv;                // levels a thread of the point kernels runs (1 or 4)
   int vert_x, vert_y;    // adv_vertical
   int vert_nf;           // fields a thread of it carries (1; mixed members by size 2)
