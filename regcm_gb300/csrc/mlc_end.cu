@@ -1646,8 +1646,9 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const Dom<R> *__
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // store the diagnostics, then advance the boundary clock and the buffer
-  // roles to the next step's and re-arm the block count
+  // store the diagnostics, then, where nothing runs beside this, advance the
+  // boundary clock and the buffer roles to the next step's, and re-arm the
+  // block count
   RedSum t = red_zero();
   for (int b = (int)threadIdx.x; b < nb; b += kRedThreads) {
     const double *p = D.partials + (size_t)b * kNPart;

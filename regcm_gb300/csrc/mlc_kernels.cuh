@@ -154,7 +154,8 @@ template <class R> struct Launch {
   static void end_uvstag(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
   // status_update of the TKE (ibltyp = 2): tendency (split step) and floor
   static void end_tke(const LaunchGeom &L, const Dom<R> *d, bool whole_step, cudaStream_t s);
-  // form_ps: ps from the virtual temperatures end_point left
+  // form_ps: ps from the virtual temperatures end_point left; advance: the
+  // last block also advances the clock and the roles (else end_advance does)
   static void end_reduce(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, bool form_ps, bool advance,
                          cudaStream_t s);
   static void end_advance(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s);
