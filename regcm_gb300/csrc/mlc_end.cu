@@ -841,8 +841,8 @@ __device__ __forceinline__ void stv(R *p, const R (&x)[V], const bool (&ok)[V], 
 // Bound by the FP64 pipe or, mixed, by memory: 56 bytes a point at five
 // species, where the passes it replaces moved 140 (t and its low part,
 // theta_v, Exner and the species went through memory between them).
-// Mixed: where nothing changed t or the species of its factor, theta_v is what
-// it was and is left alone.  FP64 forms t*qf/pai everywhere, as the split step
+// Mixed: where nothing changed t or the species of its factor and t is finite,
+// theta_v is what it was and is left alone.  FP64 forms t*qf/pai everywhere, as the split step
 // does (the two are bit for bit equal).
 // us a step, this pass and k_end_winds against k_end_relax, k_end_cross and
 // k_end_uvstag: mixed 512x512x41 258 against 546, 12 uneven domains 325 against
@@ -960,6 +960,8 @@ __global__ void __launch_bounds__(128, FRAME ? 10 : 7) k_end_point(const Dom<R> 
         t[e] = t2.hi;
         tl[e] = t2.lo;
         tv[e] = df_f(v2);
+        // a species that is not finite reaches theta_v and tvirt through t
+        chg[e] = chg[e] || !isfinite(t2.hi);
       } else {
         tv[e] = mul_r(th[e], pa[e]);
         qf[e] = qfactor_of<R>(x, ipp);
