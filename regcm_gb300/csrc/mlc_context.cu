@@ -510,25 +510,18 @@ int remove_member(mlc_ctx *x, int slot) {
 // 4.36 both, 512x512x41 15.6 and 15.5; mixed 6.8 M points 3.09 and 3.01.
 int point_levels(size_t points) { return points <= (size_t)152 * 16384 ? 1 : 4; }
 
-// The form of the column solves for these members, by their 32-column row
-// segments n an SM (152).  Several warps a column while the segments are few;
-// a thread a column, streamed, once they fill the GPU.  Measured, us a launch
-// (six coefficient warps | three | streamed), moist, 41 levels:
-//   n     FP64               mixed
-//   0.8   30.0  38.5  92.8   17.5  25.2  62.8
-//   3.3   69.5  61.4  93.4   23.0  30.1  64.1
-//   5.2    101   110   104   37.2  34.1  72.6
-//   7.1*   118   101   107   36.4  32.9  62.0   (* 35 levels)
-//   9.1    165   166   134   58.4  64.9  72.9
-//   13.4   229   224   179   79.5  72.8  78.6
-//   20.9   356   332   312    120   107   104
+// The form of the column solves for these members (solve_form): by their
+// 32-column row segments and, as a column's levels decide how many blocks an SM
+// holds, the levels of the deepest.
 template <class R>
 int solve_kind(const std::vector<Dom<R>> &t) {
   long n = 0;
-  for (const Dom<R> &D : t) n += (long)((D.g.jx - 1 + 31) / 32) * (D.g.iy - 3);
-  const bool f64 = sizeof(R) == sizeof(double);
-  if (n <= (f64 ? 2 : 4) * 152) return kSolveCols6;
-  return n <= (f64 ? 8 : 16) * 152 ? kSolveCols3 : kSolveStream;
+  int kz = 1;
+  for (const Dom<R> &D : t) {
+    n += (long)((D.g.jx - 1 + 31) / 32) * (D.g.iy - 3);
+    kz = std::max(kz, D.g.kz);
+  }
+  return solve_form(n, kz, (int)sizeof(R));
 }
 
 // Tile shapes of the horizontal WAF.  A tile's time goes with its columns,

@@ -20,6 +20,51 @@ constexpr int kSolveStream = 0, kSolveCols3 = 3, kSolveCols6 = 6;
 constexpr int solve_segment(int kind, int elem_bytes) {
   return kind == kSolveStream && elem_bytes == 4 ? 128 : 32;
 }
+// The forms with several warps a column keep kSolveArrays values a column and
+// level in shared memory.
+constexpr int kSolveArrays = 5;
+constexpr size_t solve_smem(int kz, int elem_bytes) { return (size_t)kSolveArrays * (kz + 2) * 32 * elem_bytes; }
+// Blocks of such a form resident on an SM: as many as its registers allow
+// (`most`), or as the columns' levels leave room for (228 KB an SM, 1 KB and
+// the barriers' 176 bytes a block beside the columns).
+constexpr int solve_resident(int most, int kz, int elem_bytes) {
+  const int fit = (int)(((size_t)228 << 10) / (solve_smem(kz, elem_bytes) + 1024 + 176));
+  return fit < most ? fit : most;
+}
+// The form for `segments` 32-column row segments of columns of up to kz levels
+// on 152 SMs.  A form with several warps a column takes a time for each wave of
+// resident blocks, three coefficient warps 1.7 times that of six (but twice as
+// many blocks fit); the streamed form takes about the same until its segments
+// fill the GPU.  So the one of the two whose waves take less, and streamed once
+// six warps need more than two waves (FP64; three where a block fills the SM)
+// or four (mixed).  Of 220 measured cases (two precisions, 24 to 128 levels,
+// 0.8 to 21 segments an SM) the form taken is within 5 % of the fastest.  us a
+// launch (six | three | streamed; n segments an SM):
+//          n     FP64                  mixed
+//   41     1.9   37.8  45.1  85.7      19.6  27.7  65.1
+//   levels 3.3   72.3  64.6  90.0      22.9  29.7  65.9
+//          5.2    105   120   102      37.4  33.7  74.1
+//          9.5    172   179   135      59.7  63.8  77.5
+//          13.4   241   238   183      80.8  71.1  81.0
+//          20.9   375   354   300       123   106   107
+//   70     1.9   59.4  79.4   141      27.7  41.4   106
+//          3.3    114   156   148      34.6  47.9   107
+//          5.2    167   233   169      60.5  94.1   120
+//          13.4   384   538   306       127   199   133
+//          20.9   600   845   505       192   301   176
+//   128    1.9    158   269   251      49.1  79.5   187
+//          3.3    312   533   262      98.6   164   188
+//          7.5    622  1073   350       202   340   223
+//          13.4  1085  1872   550       357   602   237
+constexpr int solve_form(long segments, int kz, int elem_bytes) {
+  const bool f64 = elem_bytes == 8;
+  const int r6 = solve_resident(f64 ? 2 : 4, kz, elem_bytes), r3 = solve_resident(f64 ? 5 : 8, kz, elem_bytes);
+  const long w6 = (segments + 152L * r6 - 1) / (152L * r6), w3 = (segments + 152L * r3 - 1) / (152L * r3);
+  const bool three = 17 * w3 < 10 * w6;
+  if (f64 && three) return w3 == 1 ? kSolveCols3 : kSolveStream;
+  if (w6 > (f64 ? (r6 == 1 ? 3 : 2) : 4)) return kSolveStream;
+  return three ? kSolveCols3 : kSolveCols6;
+}
 // Tiles of end_winds: a block is kWindWarps warps, a warp a row segment of 128
 // columns of which it writes kWindCols, marching over some rows.
 constexpr int kWindWarps = 4, kWindCols = 120;

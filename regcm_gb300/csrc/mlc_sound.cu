@@ -176,7 +176,7 @@ __global__ void k_sound_div(const Dom<R> *__restrict__ doms, int uvoff, int tile
 }
 
 // Two forms of each solve, picked by the number of column segments
-// (solve_kind).  Their level arithmetic is the functions below, every rounding
+// (solve_form).  Their level arithmetic is the functions below, every rounding
 // explicit, so the forms agree bit for bit: a member's result does not depend
 // on what else a launch holds.
 //
@@ -299,7 +299,6 @@ constexpr int kSolveCols = 32;
 // interfaces a coefficient warp forms a round (a round's first level costs the
 // filtered divergence once more; 1 and 4 measured slower)
 constexpr int kSolveLevels = 2;
-constexpr int kSolveArrays = 5;  // shared values a column and level
 // threads of a block: with six coefficient warps two share each scheduler but
 // the elimination's, whose second warp only joins the Exner update
 constexpr int solve_threads(int aw) { return 32 * (aw > 3 ? 8 : 4); }
@@ -582,7 +581,7 @@ __global__ void __launch_bounds__(solve_threads(AW), 1024 / solve_threads(AW)) k
 }
 
 // ---- the solves, streamed: one thread a column --------------------------------
-// Where the grid fills the GPU (solve_kind).
+// Where the grid fills the GPU (solve_form).
 // A block is a row segment of CW columns (one thread a column).  The downward
 // pass forms each level's coefficients and eliminates at once, the upward pass
 // substitutes back and updates Exner (and s after the last substep) a level
@@ -1416,10 +1415,6 @@ inline dim3 pt_grid(const LaunchGeom &L, int nj, int ni, int &tiles_j) {
 }
 }  // namespace
 
-// shared memory of a solve block of columns of kz levels
-template <class R>
-constexpr size_t solve_smem(int kz) { return (size_t)kSolveArrays * (kz + 2) * 32 * sizeof(R); }
-
 template <class R>
 void Launch<R>::sound_prep(const LaunchGeom &L, const Dom<R> *d, int advoff, cudaStream_t s) {
   int tj;
@@ -1447,7 +1442,7 @@ void Launch<R>::sound_div(const LaunchGeom &L, const Dom<R> *d, int uvoff, cudaS
 
 template <class R, int AW>
 void launch_cols(const LaunchGeom &L, const Dom<R> *d, dim3 grid, int advoff, int last, cudaStream_t s) {
-  const size_t smem = solve_smem<R>(L.kz);
+  const size_t smem = solve_smem(L.kz, (int)sizeof(R));
   if constexpr (sizeof(R) == sizeof(float)) {
     if (L.solve_df) step_launch(L, k_solve_cols_f<R, AW, true>, grid, solve_threads(AW), smem, s, d, advoff, last, L.wl_solve);
     else step_launch(L, k_solve_cols_f<R, AW, false>, grid, solve_threads(AW), smem, s, d, advoff, last, L.wl_solve);
@@ -1503,7 +1498,7 @@ void Launch<R>::sound_momentum(const LaunchGeom &L, const Dom<R> *d, int uvoff, 
 template <class R>
 cudaError_t Launch<R>::configure_sound() {
   // k_solve_cols holds a column of up to kMaxLevels levels in shared memory
-  const int most = (int)solve_smem<R>(kMaxLevels);
+  const int most = (int)solve_smem(kMaxLevels, (int)sizeof(R));
   cudaError_t e = cudaSuccess;
   auto allow = [&](auto k) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
