@@ -299,8 +299,12 @@ typedef struct mlc_tune_report {
                                 members' sizes whatever these say      */
   int32_t vert_x, vert_y;    /* vertical WAF passes                   */
   int32_t htile;             /* horizontal WAF tile, columns x rows:
-                                0 32x8, 1 64x8, 2 64x4, 3 32x4 (until
-                                shapes are set, by the members' sizes) */
+                                0 32x8, 1 64x8, 2 64x4, 3 32x4        */
+  int32_t by_size;           /* 1: the tiles follow the members' sizes, as
+                                until shapes are set (htile is then the
+                                nearest of the above); else htile. In what
+                                was padding: zero in structures that a
+                                caller zeroes                          */
   double  ms_fixed;          /* tuned kernel groups, fixed shapes [ms/step] */
   double  ms_tuned;          /* the same groups, picked shapes [ms/step]    */
 } mlc_tune_report;

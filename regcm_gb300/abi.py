@@ -109,7 +109,7 @@ class mlc_sav_fields(C.Structure):
 class mlc_tune_report(C.Structure):
     _fields_ = [("col_x", C.c_int32), ("col_y", C.c_int32), ("solve_x", C.c_int32),
                 ("solve_y", C.c_int32), ("vert_x", C.c_int32), ("vert_y", C.c_int32),
-                ("htile", C.c_int32), ("ms_fixed", C.c_double), ("ms_tuned", C.c_double)]
+                ("htile", C.c_int32), ("by_size", C.c_int32), ("ms_fixed", C.c_double), ("ms_tuned", C.c_double)]
 
     def as_dict(self):
         return {n: getattr(self, n) for n, _ in self._fields_}

@@ -2067,7 +2067,8 @@ int autotune_impl(mlc_ctx *x, int steps, mlc_tune_report *rep) {
     rep->col_x = tuned.col_x; rep->col_y = tuned.col_y;
     rep->solve_x = tuned.solve_x; rep->solve_y = tuned.solve_y;
     rep->vert_x = tuned.vert_x; rep->vert_y = tuned.vert_y;
-    // (128-column tiles, which only the rule on sizes takes, as 64-column ones)
+    // (tiles by size: their nearest listed shape, 64 columns for 128)
+    rep->by_size = tuned.htile < 0 ? 1 : 0;
     rep->htile = waf_tile(tuned) < kNTile ? waf_tile(tuned) : 1;
     rep->ms_fixed = msf[0] + msf[1] + msf[2] + msf[3];
     rep->ms_tuned = mst[0] + mst[1] + mst[2] + mst[3];
@@ -2099,7 +2100,7 @@ int mlc_set_launch_shapes(mlc_ctx *x, const mlc_tune_report *r) {
   const int vert = find(kVertCand, kNVert, r->vert_x, r->vert_y);
   if (col < 0 || solve < 0 || vert < 0 || r->htile < 0 || r->htile >= kNTile) return MLC_ERR_INVALID;
   LaunchGeom L = x->key.L;
-  set_shapes(L, col, solve, vert, r->htile);
+  set_shapes(L, col, solve, vert, r->by_size == 1 ? -1 : r->htile);
   if (!shapes_fit(L)) return MLC_ERR_INVALID;
   x->key.L = L;  // the graph is recorded again at the next step
   return MLC_OK;

@@ -139,7 +139,7 @@ def _autotune(lib, ctx, steps_per_trial):
 
 # the fixed configuration the autotuner compares against
 DEFAULT_SHAPES = {"col_x": 32, "col_y": 4, "solve_x": 32, "solve_y": 2, "vert_x": 32, "vert_y": 4,
-                  "htile": 0}
+                  "htile": 0, "by_size": 0}
 
 
 def _set_launch_shapes(lib, ctx, shapes):
