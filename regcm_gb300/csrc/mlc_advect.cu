@@ -22,29 +22,12 @@
 #include <type_traits>
 
 #include "mlc_kernels.cuh"
+#include "mlc_scalar.cuh"
 #include "mlc_tma.cuh"
 
 namespace mlc {
 
 namespace {
-
-
-// Main/mod_moloch.F90:1571-1590; minnum is the 4-byte real holding minden.
-template <class R> struct FlowEps;
-template <> struct FlowEps<double> {
-  static __device__ __forceinline__ double den() { return 1.0e-30; }
-  static __device__ __forceinline__ double num() { return (double)1.0e-30f; }
-};
-
-// The bit pattern of x through an opaque move, for the sign, region and
-// upwind tests that run on the integer pipe: a plain reinterpretation lets the
-// compiler turn an integer test of the pattern back into an FP64 comparison
-// (an instruction of the 1/64-rate FP64 pipe on GB300)
-__device__ __forceinline__ long long bits_of(double x) {
-  long long b;
-  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
-  return b;
-}
 
 // x + (gs*cs - gn*cn + dv*p): a WAF update from the fluxes per unit wind of a
 // cell's two faces, the faces' winds times the cell's metric factors, the
@@ -79,93 +62,6 @@ __device__ __forceinline__ bool positive(T x) {
   }
 }
 
-// WAF flux  hvel*((1+phi)*a + (1-phi)*c)  with  phi = is + zamu*b - is*b  and
-// the limiter  b = max(0, min(2, max(r, min(2r, 1))))  of  r = num/den
-// (local_flow_param, Main/mod_moloch.F90:1571-1590; the flux lines
-// :877-883, :986-993, :1017-1024).  In every use den = c - a, so
-//   (1+phi)*a + (1-phi)*c = (a + c) - phi*den,
-//   phi*den = is*den + (zamu - is)*B,   B = b*den.
-// With d = |den| > 0 and q = num*sign(den) (so r = q/d), multiplying the
-// limiter by d > 0 gives
-//   B = sign(den) * max(0, min(2d, max(q, min(2q, d)))),
-// whose candidates 0, q, 2q, d, 2d are exact: B is one of 0, 2*num, den, num,
-// 2*den exactly, the value of b*den in each region of r, ties included.  No
-// division.  FP32 takes the branch-free clamp; FP64 tests the regions of r in
-// turn (0, 1/2, 1, 2), which usually stops early - on GB300 each FP64 min, max
-// or compare is an instruction of the 1/64-rate FP64 pipe - and keeps the
-// reference's guard of denominators below minden exactly.  is = +1 (up) or
-// -1 enters as a choice of constants and of den's sign (is*den exactly), not
-// as a multiplication.
-template <class T>
-__device__ __forceinline__ T waf_b(T den, T num) {
-  T B;
-  if constexpr (sizeof(T) == sizeof(float)) {
-    // FP32: |B| = max(0, min(|2 num|, |den|), min(|num|, |2 den|)), the two
-    // minima with num*den's sign (superbee in its other form, the same
-    // candidates in every region), B with den's: four instructions of the
-    // half-rate pipe instead of seven (moist 512x512x41, a step: vertical
-    // passes 0.227 -> 0.212 ms, increments 0.109 -> 0.094, horizontal 0.351 ->
-    // 0.338).  The guard of tiny
-    // denominators is left out - it changes B only where |den| < 1e-15, by
-    // less than 2|den|, far below FP32 rounding of the flux
-    float t1, t2, bd;
-    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(t1) : "f"(num + num), "f"(den));
-    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(t2) : "f"(num), "f"(den + den));
-    asm("max.f32 %0, %1, %2, 0f00000000;" : "=f"(bd) : "f"(t1), "f"(t2));
-    B = __uint_as_float(__float_as_uint(bd) ^ (__float_as_uint(den) & 0x80000000u));
-  } else {
-    // FP64: the region tests on the integer pipe.  Non-negative doubles order
-    // like their bit patterns read as integers, and for a normal d (d >= minden
-    // here) d/2 and 2d are d's pattern -/+ 2^52; q = sign(den)*num by a sign-bit
-    // XOR.  The tests are the comparisons above exactly (a NaN num fails every
-    // comparison and takes the last region in both forms); only the flux itself
-    // uses the FP64 pipe.
-    const long long bden = bits_of(den), bnum = bits_of(num);
-    const long long mag = 0x7fffffffffffffffLL, one_exp = 1LL << 52;
-    const long long ad = bden & mag;                    // |den|
-    const long long bq = bnum ^ (bden & ~mag);          // q, as a signed pattern
-    const long long eden = __double_as_longlong(FlowEps<T>::den());
-    const long long enum_ = __double_as_longlong(FlowEps<T>::num());
-    if (ad < eden) B = (bnum & mag) < enum_ ? den : T(0);  // r = 1 or r = 0
-    else if ((bnum & mag) > 0x7ff0000000000000LL) B = den + den;  // num is NaN
-    else if (bq <= 0) B = T(0);                          // q <= 0 (and -0)
-    else if (bq < ad - one_exp) B = num + num;           // q < d/2
-    else if (bq <= ad) B = den;                          // q <= d
-    else if (bq < ad + one_exp) B = num;                 // q < 2d
-    else B = den + den;
-  }
-  return B;
-}
-// The kernels form it per unit wind: vel*g with vel = 2*hvel (the wind itself),
-// g = x - zmih*B, x = a upwind of a positive zamu (is = +1) else c, and
-// zmih = (zamu - is)/2: (a + c) - is*den = 2x exactly, so in exact arithmetic
-//   hvel*((a + c) - (is*den + (zamu - is)*B)) = vel*(x - zmih*B).
-// One fused multiply-add; the wind joins the cells' metric factors, formed
-// once for every field (FP64, moist 512x512x41, a step: horizontal WAF 4.90 ms
-// with the wind in every flux, 3.65 so; vertical 2.35 and 1.82).
-//
-// FP64 keeps the doubling out of the FP64 pipe: in the regions where B is
-// 2*num or 2*den the flux takes 2*zmih (an exponent's increment) as the factor
-// of num or den instead, zmih*(2*sel) = (2*zmih)*sel exactly, so only the
-// differences and one fused multiply-add are FP64 instructions.
-__device__ __forceinline__ double waf_sel(double den, double num, bool &dbl) {
-  // the regions of waf_b, tested on the bit patterns
-  const long long bden = bits_of(den), bnum = bits_of(num);
-  const long long mag = 0x7fffffffffffffffLL, one_exp = 1LL << 52;
-  const long long ad = bden & mag;
-  const long long bq = bnum ^ (bden & ~mag);
-  const long long eden = __double_as_longlong(FlowEps<double>::den());
-  const long long enum_ = __double_as_longlong(FlowEps<double>::num());
-  dbl = false;
-  if (ad < eden) return (bnum & mag) < enum_ ? den : 0.0;
-  if ((bnum & mag) > 0x7ff0000000000000LL) { dbl = true; return den; }
-  if (bq <= 0) return 0.0;
-  if (bq < ad - one_exp) { dbl = true; return num; }
-  if (bq <= ad) return den;
-  if (bq < ad + one_exp) return num;
-  dbl = true;
-  return den;
-}
 // a - a for the limiter's region tests: +0 for a finite a, else a NaN (every
 // NaN takes the same region), formed on the integer pipe in FP64
 template <class T>
@@ -178,12 +74,13 @@ __device__ __forceinline__ T self_diff(T a) {
     return a - a;
   }
 }
-// 2x (if dbl) by the exponent, on the integer pipe; zeros, subnormals,
-// infinities and NaN as they are
-__device__ __forceinline__ double twice(double x, bool dbl) {
-  const int h = __double2hiint(x), e = h & 0x7ff00000;
-  return __hiloint2double(dbl && e && e != 0x7ff00000 ? h + 0x00100000 : h, __double2loint(x));
-}
+// The WAF flux (mlc_scalar.cuh) per unit wind: vel*g with vel = 2*hvel (the wind itself),
+// g = x - zmih*B, x = a upwind of a positive zamu (is = +1) else c, and
+// zmih = (zamu - is)/2: (a + c) - is*den = 2x exactly, so in exact arithmetic
+//   hvel*((a + c) - (is*den + (zamu - is)*B)) = vel*(x - zmih*B).
+// One fused multiply-add; the wind joins the cells' metric factors, formed
+// once for every field (FP64, moist 512x512x41, a step: horizontal WAF 4.90 ms
+// with the wind in every flux, 3.65 so; vertical 2.35 and 1.82).
 // g with den = c - a and the upwind value x given (an interface's den is the
 // num of the interfaces on either side: a caller that has the neighbouring
 // differences forms each once); nz = -zmih
@@ -194,7 +91,7 @@ __device__ __forceinline__ T waf_g(T nz, T x, T den, T num) {
     const double sel = waf_sel(den, num, dbl);
     return __fma_rn(twice(nz, dbl), sel, x);
   } else {
-    return fmaf(nz, waf_b<T>(den, num), x);
+    return fmaf(nz, waf_b(den, num), x);
   }
 }
 // -zmih = (is - zamu)/2 of an interface

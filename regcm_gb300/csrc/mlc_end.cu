@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "mlc_kernels.cuh"
+#include "mlc_scalar.cuh"
 
 namespace mlc {
 
@@ -591,67 +592,6 @@ __global__ void k_end_ps(const Dom<R> *__restrict__ doms, int uvoff, int advoff)
   if (j > g.jx - 2 || i > g.iy - 2) return;
   ps_column<R>(D, st, g.at2(j, i));
 }
-
-// q < c for a positive finite threshold c, exactly as the comparison (false
-// for a NaN q).  FP64: on the bit patterns in the integer pipe, read through
-// an opaque move (a plain reinterpretation would be turned back into an FP64
-// comparison); a negative q, -0 included, has the sign bit set and compares
-// below every positive pattern as a signed integer.  FP32 compares directly.
-__device__ __forceinline__ long long bits_of_d(double x) {
-  long long b;
-  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
-  return b;
-}
-template <class R>
-__device__ __forceinline__ bool below_pos(R q, double c) {
-  if constexpr (sizeof(R) == sizeof(double)) {
-    const long long b = bits_of_d(q);
-    const bool nan = (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
-    return !nan && b < __double_as_longlong(c);
-  } else {
-    return q < R(c);
-  }
-}
-
-// pfwsat (Share/pfwsat.inc) of FP64 fields with few FP64 instructions: the
-// range tests on the bit patterns, explicit fused multiply-adds, div_d.
-__device__ __forceinline__ double pfwsat_d(double t, double p) {
-  double td = t - kTzero;
-  const long long b = bits_of_d(td), mag = b & 0x7fffffffffffffffLL;
-  const bool num = mag <= 0x7ff0000000000000LL;
-  if (num && b < 0 && mag > __double_as_longlong(75.0)) td = -75.0;
-  if (num && b > __double_as_longlong(100.0)) td = 100.0;
-  double es;
-  if (num && b >= 0) {
-    es = __fma_rn(td, 0.209339997e-13, -0.373208410e-10);
-    es = __fma_rn(td, es, 0.892344772e-08);
-    es = __fma_rn(td, es, 0.196237241e-05);
-    es = __fma_rn(td, es, 0.305903558e-03);
-    es = __fma_rn(td, es, 0.264461437e-01);
-    es = __fma_rn(td, es, 0.143064234e+01);
-    es = __fma_rn(td, es, 0.444007856e+02);
-    es = __fma_rn(td, es, 0.611213476e+03);
-  } else {
-    es = __fma_rn(td, 0.262655803e-12, 0.149436277e-09);
-    es = __fma_rn(td, es, 0.387940929e-07);
-    es = __fma_rn(td, es, 0.602780717e-05);
-    es = __fma_rn(td, es, 0.614396778e-03);
-    es = __fma_rn(td, es, 0.420547422e-01);
-    es = __fma_rn(td, es, 0.188369801e+01);
-    es = __fma_rn(td, es, 0.503109514e+02);
-    es = __fma_rn(td, es, 0.611123516e+03);
-  }
-  // (pressures and saturation pressures are positive, so they order like
-  // their patterns; a NaN stays)
-  const double cap = __dmul_rn(0.15, p);
-  const long long be = bits_of_d(es);
-  if (be <= 0x7ff0000000000000LL && bits_of_d(cap) < be) es = cap;
-  return __dmul_rn(kEp2, div_d(es, p - es));
-}
-
-// x differs from c in its bits (-0 from 0 too), on the integer pipe
-__device__ __forceinline__ bool bits_differ(double x, double c) { return bits_of_d(x) != __double_as_longlong(c); }
-__device__ __forceinline__ bool bits_differ(float x, float c) { return __float_as_uint(x) != __float_as_uint(c); }
 
 // Cross-point work after the boundary, per point: uvstagtouvx and
 // temp_to_tvirt of boundary (:520-523), p (:348-352), the edits mkslice
