@@ -378,11 +378,11 @@ int mlc_fp64_peak(int repeats, double *flops);
  * layout above (rho, dz: cross 3-D; qx: cross 3-D x nqx; u, v: staggered
  * 3-D; ps: cross 2-D).  out (device) receives 7 doubles: drymass, dryadv,
  * qmass, qadv, ps max, ps min, non-finite flag.  dt is the model step.
- * Partial sums live in a fixed 256 KiB file-scope device array, so domains
- * with more than 32768 rows ((iy-1)*kz) get MLC_ERR_TOO_LARGE.  The first
- * call on each device looks up that array's address: make it before any
- * stream capture.  The address is kept with the id of the CUDA context it
- * was taken in and looked up again when the current context differs (after
+ * Partial sums live in a fixed 29 KB file-scope device array; domains with
+ * more than 32768 rows ((iy-1)*kz) get MLC_ERR_TOO_LARGE.  The first call
+ * on each device looks up that array's address: make it before any stream
+ * capture.  The address is kept with the id of the CUDA context it was taken
+ * in and looked up again when the current context differs (after
  * cudaDeviceReset the module loads at a new address); a call that does the
  * lookup again must also come outside a capture.  Kernels are enqueued on
  * `stream` (a cudaStream_t, NULL = default stream) and the call returns

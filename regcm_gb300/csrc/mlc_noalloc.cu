@@ -12,8 +12,10 @@
 //
 // Limits and sharing rules:
 // * a domain may have at most kBudgetRows = 32768 rows ((iy-1) * kz); larger
-//   domains are rejected with MLC_ERR_TOO_LARGE;
-// * every GPU that loads the library holds the 256 KiB array until exit;
+//   domains are rejected with MLC_ERR_TOO_LARGE (what callers rely on to fall
+//   back; the array no longer depends on it: one record a block, whatever the
+//   rows);
+// * every GPU that loads the library holds the 29 KB array until exit;
 // * all calls share the one array: calls whose kernels overlap on the GPU
 //   (different streams, or different host threads) race on it; serialise
 //   them (one stream, or events);
@@ -29,7 +31,6 @@
 
 namespace {
 
-constexpr int kBudgetBlocks = 4096;
 constexpr long long kBudgetRows = 32768;
 constexpr int kBudgetRecord = 8;  // dry, dryadv, qmass, qadv, ps max, ps min, bad, pad
 constexpr int kBudgetThreads = 256;
@@ -38,6 +39,7 @@ constexpr int kMaxDevices = 64;
 // domain takes 6 rows and the blocks are resident at once (178 us; 1: 371,
 // 2: 212, 4: 208, 8: 196, the reduction's tail growing with the blocks).
 constexpr int kBudgetBlocksSM = 3;
+constexpr int kBudgetBlocks = 152 * kBudgetBlocksSM;  // at most
 
 static __device__ __align__(256) double g_budget_scratch[kBudgetBlocks * kBudgetRecord];
 
@@ -238,10 +240,9 @@ extern "C" int mlc_mass_budget_noalloc(const mlc_dims *d, double dx, double dt,
   const int st = scratch_for_current_device(&scratch);
   if (st != MLC_OK) return st;
   // whole rows a warp, as few as fill kBudgetBlocksSM blocks on each of 152 SMs
-  constexpr int kWarps = kBudgetThreads / 32, kFull = 152 * kBudgetBlocksSM * kWarps;
+  constexpr int kWarps = kBudgetThreads / 32, kFull = kBudgetBlocks * kWarps;
   const int rows = (d->iy - 3) * d->kz, per = (rows + kFull - 1) / kFull;
   const int nblocks = (rows + per * kWarps - 1) / (per * kWarps);
-  static_assert(kFull / kWarps <= kBudgetBlocks, "the scratch holds every block's record");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto part = d->nqx == 5 ? k_budget_partial<5> : d->nqx == 2 ? k_budget_partial<2> : k_budget_partial<0>;
   part<<<nblocks, kBudgetThreads, 0, s>>>(d->jx, d->iy, d->kz, d->nqx, dx, dt, per, rho, dz, qx, u, v, ps, scratch);
