@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "../../include/moloch_gb300.h"
@@ -132,9 +133,11 @@ __device__ Budget block_budget(Budget a) {
 // Arrays are in the packed reference layout: cross (jx-1, iy-1, kz),
 // u (jx, iy-1, kz), v (jx-1, iy, kz), qx (jx-1, iy-1, kz, nqx), ps (jx-1, iy-1).
 //
-// Interior rows (i, k) go to warps, rows_per_warp in turn each, lanes along j
-// (rows start on 8 bytes only, so wider loads are not possible).  dx^2 is applied to the sums and the
-// species of a point are added before they are weighted by dz*rho: 2 + nqx
+// Pieces of interior rows (i, k) go to warps, `per` in turn each, lanes along j
+// (rows start on 8 bytes only, so wider loads are not possible).  A piece is a
+// whole row unless there are fewer rows than warps (two rows of 30000 columns
+// took 1.6 ms by whole rows).  dx^2 is applied to the sums and the species of a
+// point are added before they are weighted by dz*rho: 2 + nqx
 // FP64 instructions a point.  On GB300, whose FP64 pipe runs two a clock and
 // SM, that pipe bounds the kernel (142 us at 512x512x41 with 5 species; the
 // 0.6 GB of loads need 89 us); the form with each species weighted by itself
@@ -144,7 +147,7 @@ __device__ Budget block_budget(Budget a) {
 // NQ: species (0: nqx at run time).
 template <int NQ>
 __global__ void __launch_bounds__(kBudgetThreads) k_budget_partial(
-    int jx, int iy, int kz, int nqx, double dx, double dt, int rows_per_warp, const double *__restrict__ rho,
+    int jx, int iy, int kz, int nqx, double dx, double dt, int pieces, int per, const double *__restrict__ rho,
     const double *__restrict__ dz, const double *__restrict__ qx, const double *__restrict__ u,
     const double *__restrict__ v, const double *__restrict__ ps, double *scratch) {
   const int nc = jx - 1, nq = NQ > 0 ? NQ : nqx;
@@ -153,13 +156,15 @@ __global__ void __launch_bounds__(kBudgetThreads) k_budget_partial(
   Budget a = budget_zero();
   const int lane = (int)(threadIdx.x & 31u);
   const int warp = (int)(blockIdx.x * (kBudgetThreads / 32) + (threadIdx.x >> 5));
-  const int ni = iy - 3, rows = ni * kz;
-  const int r1 = min(rows, (warp + 1) * rows_per_warp);
-  for (int r = warp * rows_per_warp; r < r1; ++r) {
+  const int ni = iy - 3, items = ni * kz * pieces;
+  const int len = ((nc - 2 + 31) / 32 + pieces - 1) / pieces * 32;  // columns of a piece
+  const int t1 = min(items, (warp + 1) * per);
+  for (int t = warp * per; t < t1; ++t) {
+    const int r = t / pieces, j0 = 1 + (t - r * pieces) * len, j1 = min(nc - 2, j0 + len - 1);
     const int k = r / ni, i = r - k * ni + 1;  // 0-based level and row
     const size_t o0 = c2 * k + (size_t)nc * i;
 #pragma unroll 1  // unrolled by 4 (the compiler's choice) 211 us instead of 178
-    for (int j = 1 + lane; j <= nc - 2; j += 32) {
+    for (int j = j0 + lane; j <= j1; j += 32) {
       const size_t o = o0 + j;
       const double m = dz[o] * rho[o];
       double q = qx[o];
@@ -239,13 +244,16 @@ extern "C" int mlc_mass_budget_noalloc(const mlc_dims *d, double dx, double dt,
   double *scratch = nullptr;
   const int st = scratch_for_current_device(&scratch);
   if (st != MLC_OK) return st;
-  // whole rows a warp, as few as fill kBudgetBlocksSM blocks on each of 152 SMs
+  // pieces a warp: as few as fill kBudgetBlocksSM blocks on each of 152 SMs
   constexpr int kWarps = kBudgetThreads / 32, kFull = kBudgetBlocks * kWarps;
-  const int rows = (d->iy - 3) * d->kz, per = (rows + kFull - 1) / kFull;
-  const int nblocks = (rows + per * kWarps - 1) / (per * kWarps);
+  const int rows = (d->iy - 3) * d->kz, chunks = (d->jx - 3 + 31) / 32;
+  const int pieces = rows >= kFull ? 1 : std::min(chunks, kFull / rows);
+  const int items = rows * pieces, per = (items + kFull - 1) / kFull;
+  const int nblocks = (items + per * kWarps - 1) / (per * kWarps);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto part = d->nqx == 5 ? k_budget_partial<5> : d->nqx == 2 ? k_budget_partial<2> : k_budget_partial<0>;
-  part<<<nblocks, kBudgetThreads, 0, s>>>(d->jx, d->iy, d->kz, d->nqx, dx, dt, per, rho, dz, qx, u, v, ps, scratch);
+  part<<<nblocks, kBudgetThreads, 0, s>>>(d->jx, d->iy, d->kz, d->nqx, dx, dt, pieces, per, rho, dz, qx, u, v, ps,
+                                       scratch);
   k_budget_final<<<1, kBudgetThreads, 0, s>>>(scratch, nblocks, out);
   return cudaGetLastError() == cudaSuccess ? MLC_OK : MLC_ERR_CUDA;
 }
