@@ -762,6 +762,142 @@ __device__ __forceinline__ void stv(R *p, const R (&x)[V], const bool (&ok)[V], 
   }
 }
 
+// k_end_cross<kEndAll> of a mixed member in lanes of four columns (16-byte loads
+// and stores, the same expressions): the end of steps that nudge spectrally.
+// Bound by memory; with ps before it 211 us a step at 512x512x41 and 71 at
+// 256x256x41, a point a thread 453 and 136.
+template <class R, int LV>
+__global__ void __launch_bounds__(128) k_end_cross_v4(const Dom<R> *__restrict__ doms, int uvoff, int advoff,
+                                                      int tiles_j, const WorkItem *__restrict__ wl) {
+  if constexpr (LV == 1) grid_begin();
+  constexpr int V = 4;
+  static_assert(sizeof(R) == sizeof(float), "FP32 fields");
+  const WorkItem wi = work_item(wl, tiles_j);
+  const Dom<R> &D = doms[wi.m];
+  if (!D.active) return;
+  const Geom g = D.g;
+  const Scal &c = D.c;
+  const int jx = g.jx, iy = g.iy, kz = g.kz;
+  const int e0 = ((int)wi.a * 32 + (int)threadIdx.x) * V, i = (int)wi.b * 4 + (int)threadIdx.y + 1;
+  const int k0 = (int)wi.c * LV + 1;
+  if (e0 + 1 > jx - 1 || i > iy - 1 || k0 > kz) return;
+  const State<R> st = state_of(D, (D.clk->uv_role + uvoff) & 1, (D.clk->adv_role + advoff) & 1);
+  const size_t F = g.field3();
+  const unsigned P = (unsigned)g.P, PS = (unsigned)g.PS, ij = (unsigned)e0 + (unsigned)(i - 1) * P;
+  const float *__restrict__ u = st.u + ij;
+  const float *__restrict__ v = st.v + ij;
+  const float *__restrict__ t_h = st.t + ij;
+  const float *__restrict__ t_l = D.wz[1] + ij;
+  const float *__restrict__ pai = reinterpret_cast<const float *>(st.pai) + ij;
+  float *__restrict__ tet = reinterpret_cast<float *>(st.tetav) + ij;
+  float *__restrict__ qx = st.qx + ij;
+  float *__restrict__ trac = st.trac + ij;
+  const int ipp = c.ipptls, nq = qfactor_species(ipp);
+  bool has[V], inner[V], all = true, any_inner = false;
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    const int j = e0 + q + 1;
+    has[q] = j <= jx - 1;
+    inner[q] = j >= 2 && j <= jx - 2 && i >= 2 && i <= iy - 2;
+    all = all && has[q];
+    any_inner = any_inner || inner[q];
+  }
+  unsigned o = (unsigned)(k0 - 1) * PS;
+  for (int k = k0; k < k0 + LV && k <= kz; ++k, o += PS) {
+    if (c.apply_bdy) {
+      // u at columns e0-1 .. e0+5 and v at rows i-1 .. i+2 (:1535-1566)
+      float n[V + 3] = {}, m[V], a[V];
+      ldv<R, V>(m, u + o);
+      if (e0 >= 1) n[0] = (u + o)[-1];  // (o may be 0: no unsigned o - 1)
+#pragma unroll
+      for (int q = 0; q < V; ++q) n[1 + q] = m[q];
+      if (e0 + 4 <= jx - 1) n[5] = u[o + 4];
+      if (e0 + 5 <= jx - 1) n[6] = u[o + 5];
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        const int j = e0 + q + 1;
+        a[q] = j == 1 || j == jx - 1 ? interp2<R>(n[q + 1], n[q + 2]) : interp4<R>(n[q + 2], n[q + 1], n[q + 3], n[q]);
+      }
+      stv<R, V>(st.ux + ij + o, a, has, all);
+      float vs[V] = {}, vc[V], vn[V], vf[V] = {};
+      ldv<R, V>(vc, v + o);
+      ldv<R, V>(vn, v + o + P);
+      const bool edge = i == 1 || i == iy - 1;
+      if (!edge) {
+        ldv<R, V>(vs, v + o - P);
+        ldv<R, V>(vf, v + o + 2 * P);
+      }
+#pragma unroll
+      for (int q = 0; q < V; ++q) a[q] = edge ? interp2<R>(vc[q], vn[q]) : interp4<R>(vn[q], vc[q], vf[q], vs[q]);
+      stv<R, V>(st.vx + ij + o, a, has, all);
+    }
+    float ph[V], pl[V], pk[V], tk[V], tl[V], q[5][V];
+    ldv<R, V>(ph, pai + o);
+    ldv<R, V>(pl, pai + F + o);
+    ldv<R, V>(tk, t_h + o);
+    ldv<R, V>(tl, t_l + o);
+#pragma unroll
+    for (int n = 0; n < 5; ++n)
+      if (n < nq) ldv<R, V>(q[n], qx + o + (size_t)n * F);
+      else
+#pragma unroll
+        for (int e = 0; e < V; ++e) q[n][e] = 0.f;
+    // the floors at inner points (see k_end_cross; in FP32 every tracer below
+    // mkslice's is at most zero)
+    if (any_inner) {
+      auto floors = [&](float (&x)[V], float *p, double check, float zero) {
+        bool ch = false;
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (inner[e] && below_pos<R>(x[e], check)) {
+            x[e] = zero;
+            ch = true;
+          }
+        if (ch) stv<R, V>(p, x, has, all);
+      };
+#pragma unroll
+      for (int n = 0; n < 5; ++n)
+        if (n < nq) floors(q[n], qx + o + (size_t)n * F, qx_check(n), float(qx_zero(n)));
+      for (int n = nq; n < g.nqx; ++n) {
+        float x[V];
+        ldv<R, V>(x, qx + o + (size_t)n * F);
+        floors(x, qx + o + (size_t)n * F, qx_check(n), float(qx_zero(n)));
+      }
+      for (int n = 0; n < g.ntr; ++n) {
+        float x[V];
+        bool ch = false;
+        ldv<R, V>(x, trac + o + (size_t)n * F);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (inner[e] && x[e] <= 0.f) {
+            x[e] = 0.f;
+            ch = true;
+          }
+        if (ch) stv<R, V>(trac + o + (size_t)n * F, x, has, all);
+      }
+    }
+    float tv[V], rh[V], th[V], thl[V], qs[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const float x[5] = {q[0][e], q[1][e], q[2][e], q[3][e], q[4][e]};
+      pk[e] = exner_to_pressure_f(ph[e] + pl[e]);
+      tv[e] = mul_r(tk[e], qfactor_of<R>(x, ipp));
+      rh[e] = divide<R>(pk[e], mul_r(R(kRgas), tk[e]));
+      // theta_v = tvirt/pai from the double-float t (Main/mod_moloch.F90:1403-1443)
+      const F2 t2 = df_div(df_mul(F2{tk[e], tl[e]}, qfactor_df_of(x, ipp)), F2{ph[e], pl[e]});
+      th[e] = t2.hi;
+      thl[e] = t2.lo;
+      qs[e] = pfwsat_f(tk[e], pk[e]);
+    }
+    stv<R, V>(st.p + ij + o, pk, has, all);
+    stv<R, V>(st.tvirt + ij + o, tv, has, all);
+    stv<R, V>(st.rho + ij + o, rh, has, all);
+    stv<R, V>(tet + o, th, has, all);
+    stv<R, V>(tet + F + o, thl, has, all);
+    stv<R, V>(st.qsat + ij + o, qs, has, all);
+  }
+}
+
 // A whole step's pointwise end in one pass (steps that nudge spectrally take
 // k_end_relax and k_end_cross): virtual temperature and temperature of
 // dynamical_core :1121-1123, motopnudge (Main/mod_bdycod.F90:4049-4083) and
@@ -1853,7 +1989,17 @@ void launch_cross(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, c
 
 template <class R>
 void Launch<R>::end_cross(const LaunchGeom &L, const Dom<R> *d, int uvoff, int advoff, cudaStream_t s) {
-  launch_cross<R, kEndAll>(L, d, uvoff, advoff, s);
+  if constexpr (sizeof(R) == sizeof(float)) {
+    const dim3 b((unsigned)L.col_x, (unsigned)L.col_y), b4(32, 4);
+    const int tj = (L.jx - 1 + 127) / 128, ti = (L.iy - 1 + 3) / 4;
+    const dim3 grd = L.wl_v4 ? dim3((unsigned)L.n_v4, 1, 1)
+                             : dim3((unsigned)(tj * ti), (unsigned)((L.kz + L.lv - 1) / L.lv), (unsigned)L.nmem);
+    step_launch(L, k_end_ps<R>, grid2(L.jx - 3, L.iy - 3, b, L.nmem), b, 0, s, d, uvoff, advoff);
+    if (L.lv == 1) step_launch(L, k_end_cross_v4<R, 1>, grd, b4, 0, s, d, uvoff, advoff, tj, L.wl_v4);
+    else step_launch(L, k_end_cross_v4<R, 4>, grd, b4, 0, s, d, uvoff, advoff, tj, L.wl_v4);
+  } else {
+    launch_cross<R, kEndAll>(L, d, uvoff, advoff, s);
+  }
 }
 
 template <class R>
