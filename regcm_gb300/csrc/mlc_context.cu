@@ -504,11 +504,14 @@ int remove_member(mlc_ctx *x, int slot) {
 }
 
 // Levels a thread of the point kernels runs: one while the points are few,
-// because a thread's levels wait on memory one after the other.  Step times
-// with one and four levels: mixed 64x64x30 0.166 and 0.213 ms, FP64 64x64x30
-// 0.331 and 0.369, 201x157x35 (1.1 M points) 2.72 and 2.77, 256x256x41 (2.7 M)
-// 4.36 both, 512x512x41 15.6 and 15.5; mixed 6.8 M points 3.09 and 3.01.
-int point_levels(size_t points) { return points <= (size_t)152 * 16384 ? 1 : 4; }
+// because a thread's levels wait on memory one after the other.  Step times in
+// ms with one and four levels, FP64 and mixed: 64x64x30 (0.13 M points) 0.242
+// and 0.273, 0.125 and 0.153; 110x110x41 (0.51 M) 0.876 and 0.921, 0.262 and
+// 0.288; 170x170x41 (1.2 M) 1.874 and 1.879, 0.493 and 0.502; 16 members of
+// 60x60x25 (1.5 M) 1.79 and 1.77, 0.637 and 0.591; 200x200x41 (1.7 M) 2.40 and
+// 2.39, 0.678 and 0.676; 64 members of 40x40x20 (2.2 M) 3.49 and 3.40, 1.41 and
+// 1.22; 512x512x41 13.4 and 13.1, 2.92 and 2.78.
+int point_levels(size_t points) { return points <= (size_t)152 * 8192 ? 1 : 4; }
 
 // The form of the column solves for these members (solve_form): by their
 // 32-column row segments and, as a column's levels decide how many blocks an SM

@@ -41,7 +41,7 @@ def same(a, b, where):
                                       (False, {"spectral": True, "dtrad": 60.0}), (True, {"apply_bdy": False})])
 @pytest.mark.parametrize("prec", PRECISIONS)
 def test_alone_and_in_a_large_batch(prec, moist, kw, split):
-    case = build(69, 67, 10, moist, prec, **kw)  # 47 600 points: 54 copies pass the threshold (2.49 M)
+    case = build(69, 67, 10, moist, prec, **kw)  # 47 600 points: 54 copies are past the threshold (1.25 M)
 
     def run(copies):
         b = MolochBatch([case] * copies)
