@@ -3,22 +3,27 @@
 // interpolations of :1445-1569 and local_flow_param :1571-1590).
 //
 //   adv_prep        u,v -> ux,vx (4th order, 2nd at the edges) and w -> wx.
-//   adv_vertical    per column and field: both vertical WAF passes
-//                   (do_vadvtwice) with the column in shared memory.
-//   adv_horizontal  per (32 x 8) tile, level and field: meridional then zonal
-//                   WAF.  The tile stages wz with a 2-point halo in shared
-//                   memory, builds the meridional fluxes and the intermediate
-//                   p0 on a 2-column halo, then the zonal fluxes and the
-//                   result, so each field is read and written once.  The
-//                   result goes to a second buffer because the halo columns
-//                   of a tile still need the field's old values.
+//   adv_vertical    a thread a column and field (FP32 in large launches two
+//                   fields): both vertical WAF passes (do_vadvtwice), streamed
+//                   upward through registers.
+//   adv_horizontal  per tile (a warp a row, 32 to 128 columns) and level, field
+//                   by field: meridional then zonal WAF.  The tile's wz lands in
+//                   shared memory with a 2-point halo; from it come the
+//                   meridional fluxes and the intermediate p0 on a 2-column
+//                   halo, then the zonal fluxes and the result, so each field
+//                   is read and written once.  The result goes to a second
+//                   buffer because the halo columns of a tile still need the
+//                   field's old values.
 //   adv_curvature   curvature terms on ux, vx (skipped when they are zero at
 //                   every point: with uniform map factors the reference adds
 //                   an exact zero).
 //   adv_back        ux,vx -> u,v and wx -> w (4th order, 2nd at the edges).
-// Operand order follows the reference expression by expression.  The ratios
-// dtrdz*fmz/fmzf of the vertical passes are per-domain constants read from
-// arrays computed once with the same expression.
+// The fluxes are formed per unit wind and the wind joins the cells' metric
+// factors, and an update's terms are summed before the field (waf_g, waf_update,
+// vupdate): the reference's sums with other operand orders, equal to rounding.
+// The interpolations and curvature terms follow the reference's expressions.
+// The ratios dtrdz*fmz/fmzf of the vertical passes are per-domain constants read
+// from arrays computed once with the same expression.
 #include <type_traits>
 
 #include "mlc_kernels.cuh"
@@ -387,8 +392,7 @@ __global__ void __launch_bounds__(128) k_adv_prep_v4(const Dom<R> *__restrict__ 
 // fluxes at k and k+1; pass 2 needs pass 1's output at m-1..m+2, so it runs
 // two levels behind pass 1 in the same loop.  Every value is loaded once and
 // the column never touches shared memory.  R is the type of the winds and
-// metric, T that of the advected field and of the arithmetic.  Fluxes and
-// updates are the reference's expressions, operand for operand.
+// metric, T that of the advected field and of the arithmetic.
 // the flux per unit s through interface k+1 between levels k and k+1, its
 // upwind difference col(k1) - col(k1p1) with the reference's clamps
 // k1p1 = min(k+2, kz), k1 = max(k-1, 1); d: the differences c(k) - c(k+1) of
@@ -434,8 +438,6 @@ template <class T>
 __device__ __forceinline__ T *global_ptr(T *p) {
   return (T *)__cvta_global_to_generic(__cvta_generic_to_global((const void *)p));
 }
-// Levels an FP32 column loads ahead of the one it computes (1 or 2; two
-// measured no faster on the moist 512x512x41 step, 0.256 ms a step both).
 // Fields f0 .. f0+NF-1 of the column (j, i), both passes.  FP32 members of
 // large launches take two fields a thread, which share the level's loads and
 // factors: the kernel is bound by instructions (54 against 119 a level and

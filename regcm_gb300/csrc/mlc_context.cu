@@ -621,7 +621,11 @@ int refresh(mlc_ctx *x) {
   }
   L.lv = point_levels(pts);
   L.vert_nf = x->mixed && L.lv > 1 ? 2 : 1;
-  L.wind_rows = !x->mixed ? 0 : pts <= (size_t)256 << 10 ? 2 : 4;  // (eight and more measured slower)
+  // Rows a warp of the winds marches: few where warps are few.  us of the pass
+  // with one, two, four and eight rows: 64x64x30 8.1, 9.0, 10.7, 14.0 (beside the
+  // budget, the step the same with one and two); 96x96x35 (0.33 M points) 10.3,
+  // 10.1, 10.5, 14.6; 256x256x41 35, 29, 24, 29; 512x512x41 100, 76, 65, 68.
+  L.wind_rows = !x->mixed ? 0 : pts <= (size_t)256 << 10 ? 2 : 4;
   if (!t.empty()) {
     MLC_TRY(cudaMemcpyAsync(x->table, t.data(), t.size() * sizeof(Dom<R>), cudaMemcpyHostToDevice,
                             x->stream));
@@ -1051,9 +1055,10 @@ int get3x(mlc_ctx *x, const Geom &g, const double *src, double *h, int nj, int n
 
 // An FP64 array goes back from the padded device layout to the packed host
 // array in one pitched copy (rows of nj, ni rows of a plane on the host, iy on
-// the device), the faster way in this direction (512x512x41 4.53 ms against
-// 5.03 packed first); a mixed member's FP32 field is packed and converted
-// through the staging buffer.
+// the device), the faster way in this direction also where rows are odd: the
+// whole state, pinned, 512x512x41 7.7 ms against 8.5 packed first, 333x311x40
+// 3.1 against 3.4, 201x157x35 0.92 against 1.08, 47x33x23 0.12 against 0.22.  A
+// mixed member's FP32 field is packed and converted through the staging buffer.
 template <class R>
 int get3(mlc_ctx *x, const Geom &g, const R *src, double *h, int nj, int ni, int nk, size_t soff) {
   if (!h) return MLC_OK;

@@ -8,8 +8,9 @@
 //
 // The boundary clock lives on the device: bdyval blends with xbctime, then
 // the reference advances it by dtsec (Main/mod_bdycod.F90:2653) before
-// motopnudge and morelax blend again, so those read xbctime + dtsec; the
-// final reduction kernel stores the advanced clock.
+// motopnudge and morelax blend again, so those read xbctime + dtsec; the last
+// kernel of a step stores the advanced clock (end_advance, or the reduction in
+// split steps and those that nudge spectrally).
 #include <algorithm>
 
 #include "mlc_kernels.cuh"

@@ -112,12 +112,11 @@ inline int waf_tile_inc(const LaunchGeom &L) { return L.htile >= 0 ? L.htile : L
 
 // Launch a kernel of the step (its first statement is grid_begin).  Where a
 // step is a few microseconds a kernel (one level a thread, point_levels) the
-// launch overlaps the end of the kernel before it: a step of 64x64x30 mixed
-// 153 -> 149 us, of 47x33x23 FP64 201 -> 195, and 590 -> 536 us launched one
-// by one around the physics.  Larger steps gain nothing, and all lose by
-// letting the next kernel's blocks in as soon as all blocks of this one have
-// started (64x64x30 FP64 262 -> 337 us: they settle where there is room, not
-// evenly).
+// launch overlaps the end of the kernel before it: a step of 64x64x30 mixed 127
+// us without and 123 with, FP64 247 and 242, of 47x33x23 125 and 119, 193 and
+// 189.  From 150x150x40 on nothing changes, and all lose by letting the next
+// kernel's blocks in as soon as all blocks of this one have started (64x64x30
+// FP64 262 -> 337 us: they settle where there is room, not evenly).
 template <class... P, class... A>
 void step_launch(const LaunchGeom &L, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                  A... args) {

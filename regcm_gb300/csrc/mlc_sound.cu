@@ -6,11 +6,12 @@
 //   sound_div       per column of cross points: raw horizontal divergence
 //                   zdiv2 (Eq. 16) and the generalized vertical velocity s
 //                   (Eq. 10), s(kz+1) and the surface w.
-//   sound_solve     per interior column, one thread per column: the 5-point
-//                   divergence filter, the vertical divergence term, the
-//                   implicit w-Exner tridiagonal system (Eq. 19, Thomas
-//                   algorithm, the column streamed through shared memory), the
-//                   Exner update and, after the last substep, the completed s.
+//   sound_solve     per interior column: the 5-point divergence filter, the
+//                   vertical divergence term, the implicit w-Exner tridiagonal
+//                   system (Eq. 19, Thomas algorithm), the Exner update and,
+//                   after the last substep, the completed s.  A column is one
+//                   thread's, streamed through shared memory, or several warps'
+//                   and kept on chip (solve_form).
 //   sound_momentum  u and v (Eq. 17/18): divergence damping, Coriolis with
 //                   the substep's initial winds, pressure gradient with the new
 //                   Exner function, terrain term, relaxation-zone weight.  It
@@ -303,7 +304,8 @@ constexpr int kSolveLevels = 2;
 // the elimination's, whose second warp only joins the Exner update
 constexpr int solve_threads(int aw) { return 32 * (aw > 3 ? 8 : 4); }
 
-// This thread's part of a block: its role (0 eliminates, 1..3 coefficients)
+// This thread's part of a block: its role (0 eliminates, 1..AW coefficients,
+// AW+1 of the six-warp form only the Exner update)
 // and its column; lanes outside the interior work on the nearest interior
 // column and store nothing.
 struct SolveLane {
@@ -602,7 +604,7 @@ struct SolveShape {
   static constexpr int kZW = CW + 2 * kHalo;
   static constexpr int kPlanes = kF64 ? 7 : 8;
   static constexpr int kStage = 3 * kZW + kPlanes * CW;
-  static constexpr int kStages = kF64 ? (CW == 32 ? 4 : 3) : (CW == 32 ? 6 : 4);
+  static constexpr int kStages = 4;
 };
 
 // One plane's copies: where the segment lies in the plane at level 1, where
